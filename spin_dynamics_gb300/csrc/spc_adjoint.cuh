@@ -519,7 +519,7 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
     k_rowpass<PASS_NORM_GATHER><<<nip, blk, 0, st>>>(pa);
     h->prof.end(st, pe, PK_DOT, 4.0 * elems, 16.0 * elems);
     pe = h->prof.begin(st);
-    k_scale<<<nip, blk, 0, st>>>(tiles, d_items, d_map, d_scol, x, d_P, 1, 0, pa.rbeta, d_Q, d_xs);
+    k_scale<<<nip, blk, 0, st>>>(tiles, d_items, d_map, d_scol, x, d_P, 1, 0, pa.rbeta, d_Q, d_xs, nullptr);
     h->prof.end(st, pe, PK_SCALE, 2.0 * elems, 40.0 * elems);
     h->count_launch(2);
     for (int i = 0; i < m; ++i) {
@@ -565,7 +565,8 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
           k_rowpass<PASS_AXPY_NORM><<<nip, blk, 0, st>>>(pa);
         h->prof.end(st, pe, PK_AXPY_NORM, (lanczos ? 8.0 : 12.0) * elems, 48.0 * elems);
         pe = h->prof.begin(st);
-        k_scale<<<nip, blk, 0, st>>>(tiles, d_items, d_map, d_scol, x, d_P, 0, i + 1, pa.rbeta, d_Q, d_xs);
+        k_scale<<<nip, blk, 0, st>>>(tiles, d_items, d_map, d_scol, x, d_P, 0, i + 1, pa.rbeta, d_Q, d_xs,
+                                     nullptr);
         h->prof.end(st, pe, PK_SCALE, 2.0 * elems, 40.0 * elems);
         h->count_launch(2);
       }

@@ -124,6 +124,8 @@ struct Handle {
   // execution copy: Re + Im of every entry (xvs, nnz doubles); Re + Im of
   // the current Krylov vector of every tile (xsum, beside P)
   Buf xvs, xsum;
+  // largest basis component of every slot in flight (high word of the double)
+  Buf qmax;
   // Hamiltonian build scratch: row counts, nucleus tables, nonzero totals
   Buf bcnt, bnuc, btot, btab;
   // autotuner outputs and sample subsets

@@ -38,6 +38,7 @@
 #include <vector>
 
 #include <cooperative_groups.h>
+#include <cuda_fp16.h>
 
 #include "spc_common.cuh"
 #include "spc_internal.h"
@@ -222,22 +223,32 @@ __global__ void __launch_bounds__(256) k_rowpass(PassArgs a) {
   }
 }
 
+// High word of the larger of |re|, |im|: its integer order is the order of
+// the magnitudes, NaN above infinity.
+__device__ __forceinline__ unsigned abs_high(double2 q) {
+  return max((unsigned)__double2hiint(q.x) & 0x7fffffffu, (unsigned)__double2hiint(q.y) & 0x7fffffffu);
+}
+
 // Q_{jd} = P / ||P||  (or Q_0 = psi[:, scol] / ||psi|| when gather != 0),
 // and beside it XS = Re + Im of the stored Q_{jd} (the operand k_spmm's
 // three-product form reads); grid = pass items. XS has P's layout (p_off).
+// qmax (may be null): per slot, the high word of the basis' largest component.
 __global__ void __launch_bounds__(256)
     k_scale(const TileInfo* __restrict__ tiles, const int2* __restrict__ items,
             const int* __restrict__ map, const int* __restrict__ scol,
             const double2* __restrict__ psi, const double2* __restrict__ P, int gather, int jd,
-            const double* __restrict__ rbeta, double2* __restrict__ Q, double* __restrict__ XS) {
+            const double* __restrict__ rbeta, double2* __restrict__ Q, double* __restrict__ XS,
+            unsigned* __restrict__ qmax) {
+  __shared__ unsigned mx[SPC_WARPS][SPC_LANES];
   const int2 it = items[blockIdx.x];
   const TileInfo& T = tiles[it.x];
   if (!gather && jd >= T.m) return;
   const int tx = threadIdx.x;
   const int w = it.x * SPC_LANES + tx;
-  if (map[w] < 0) return;
-  const double rb = rbeta[w];
-  const int n = T.n;
+  const bool act = map[w] >= 0;
+  const double rb = act ? rbeta[w] : 0.0;
+  const int n = act ? T.n : 0;
+  unsigned top = 0;
   const int stride = T.nip * SPC_WARPS;
   double2* dst = Q + T.q_off + (size_t)jd * n * SPC_LANES + tx;
   double* xs = XS + T.p_off + tx;
@@ -248,6 +259,7 @@ __global__ void __launch_bounds__(256)
       const double2 q = make_double2(x.x * rb, x.y * rb);
       dst[(size_t)r * SPC_LANES] = q;
       xs[(size_t)r * SPC_LANES] = q.x + q.y;
+      top = max(top, abs_high(q));
     }
   } else {
     const double2* src = P + T.p_off + tx;
@@ -256,7 +268,16 @@ __global__ void __launch_bounds__(256)
       const double2 q = make_double2(x.x * rb, x.y * rb);
       dst[(size_t)r * SPC_LANES] = q;
       xs[(size_t)r * SPC_LANES] = q.x + q.y;
+      top = max(top, abs_high(q));
     }
+  }
+  if (qmax == nullptr) return;
+  mx[threadIdx.y][tx] = top;
+  __syncthreads();
+  if (threadIdx.y == 0) {
+#pragma unroll
+    for (int y = 1; y < SPC_WARPS; ++y) top = max(top, mx[y][tx]);
+    if (act) atomicMax(qmax + w, top);
   }
 }
 
@@ -916,6 +937,8 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+#include "spc_digits.cuh"
+
 __global__ void k_proj_reduce(const TileInfo* __restrict__ tiles, int nslots, const int* __restrict__ map,
                               int m, int ncombo, int nsplit, int64_t rps, const unsigned* __restrict__ combos,
                               const double2* __restrict__ part, double2* __restrict__ proj) {
@@ -1384,7 +1407,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
   // otherwise every round runs over consecutive chunks of whole 32-sample
   // tiles, the capacities scaled down by one factor. States, populations and
   // clocks stay resident for every sample either way.
-  const double slot_fixed = 16.0 * (6.0 * mm + m + 1 + (double)nsplit_max * ncombo) + 8.0 + 4.0 + 8.0;
+  const double slot_fixed = 16.0 * (6.0 * mm + m + 1 + (double)nsplit_max * ncombo) + 8.0 + 4.0 + 4.0 + 8.0;
   // basis + work vector (complex) + the current vector's Re + Im plane (XS)
   const double need_fl = 16.0 * (double)qcap + 24.0 * (double)pcap + slot_fixed * slots_cap +
                          (double)(sizeof(TileInfo) + sizeof(unsigned)) * tiles_cap;
@@ -1411,6 +1434,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
     reuse(h->projpart, 16.0 * (double)nsplit_max * ncombo * sl);
     reuse(h->cvec, 16.0 * m * sl);
     reuse(h->flag, 4.0 * sl);
+    reuse(h->qmax, 4.0 * sl);
     reuse(h->tt, 8.0 * G);
     reuse(h->kk, 4.0 * G);
     reuse(h->done, 4.0 * G);
@@ -1449,7 +1473,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
       h->ensure(h->cvec, sizeof(double2) * m * slots_fl) || h->ensure(h->tt, sizeof(double) * G) ||
       h->ensure(h->kk, sizeof(int) * G) || h->ensure(h->done, sizeof(int) * G) ||
       h->ensure(h->obs, sizeof(double) * 4 * (size_t)T * G) || h->ensure(h->err, 16) ||
-      h->ensure(h->flag, sizeof(int) * slots_fl) ||
+      h->ensure(h->flag, sizeof(int) * slots_fl) || h->ensure(h->qmax, sizeof(unsigned) * slots_fl) ||
       h->ensure(h->plan, sizeof(TileInfo) * tiles_fl + sizeof(int2) * 2 * items_cap +
                              sizeof(int) * 2 * slots_fl + 256) ||
       h->ensure(h->jobtab, (sizeof(JobInit) + sizeof(JobOut)) * nj + 64))
@@ -1476,6 +1500,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
   int* d_err = (int*)h->err.p;
   long long* d_nsteps = (long long*)((char*)h->err.p + 8);
   int* d_flag = (int*)h->flag.p;
+  unsigned* d_qmax = (unsigned*)h->qmax.p;
   // per-round plan: tiles | pass items | SpMM items | map | scol
   char* plan = (char*)h->plan.p;
   TileInfo* d_tiles = (TileInfo*)plan;
@@ -1568,7 +1593,17 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
   const int res_spmm = resident((const void*)k_spmm, 256, 0);
   const int res_pass = std::min(resident((const void*)k_rowpass<PASS_AXPY_DOT>, 256, 0),
                                 resident((const void*)k_rowpass<PASS_AXPY_NORM>, 256, 0));
-  const int res_proj = resident(proj_fn, proj_threads, proj_smem);
+  // Grams on the tensor cores for m <= 32 (a CTA per projector type; its two
+  // 16-vector blocks hold 32 vectors), in FP64 above. Faster at every measured
+  // size below the line: 0.59 -> 0.26 ms (dim 2304, m = 16, 384 samples),
+  // 71 -> 19 ms (dim 55296, m = 30, 512 samples).
+  const bool gram = m <= 32;
+  const int gram_mt = m <= 16 ? 1 : 2;
+  const void* gram_fn = gram_mt == 1 ? (const void*)k_gram<1> : (const void*)k_gram<2>;
+  const size_t gram_smem = gram_smem_bytes(gram_mt);
+  CK(cudaFuncSetAttribute(gram_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gram_smem));
+  const int res_proj = gram ? std::max(1, resident(gram_fn, 256, gram_smem) / 4)
+                            : resident(proj_fn, proj_threads, proj_smem);
 
   std::vector<int> active;
   if (0.0 < t_end)
@@ -1689,7 +1724,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
           ctas += k;
           rows += (double)z;
         }
-        const double est = (rows + 32.0 * ctas) / res_proj + (double)r;
+        const double est = (rows + (gram ? 96.0 : 32.0) * ctas) / res_proj + (double)r;
         if (est < best) {
           best = est;
           rps = r;
@@ -1703,6 +1738,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
     auto enqueue = [&]() -> int {
       CK(cudaMemsetAsync(d_A, 0, sizeof(double2) * mm * nslots, st));
       CK(cudaMemsetAsync(d_flag, 0, sizeof(int) * nslots, st));
+      CK(cudaMemsetAsync(d_qmax, 0, sizeof(unsigned) * nslots, st));
       PassArgs pa{};
       pa.tiles = d_tiles;
       pa.items = d_items_p;
@@ -1735,7 +1771,8 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
       k_rowpass<PASS_NORM_GATHER><<<nip, blk, 0, st>>>(pa);
       h->prof.end(st, pe, PK_DOT, 4.0 * elems, 16.0 * elems);
       pe = h->prof.begin(st);
-      k_scale<<<nip, blk, 0, st>>>(d_tiles, d_items_p, d_map, d_scol, d_psi, d_P, 1, 0, d_rb, d_Q, d_xs);
+      k_scale<<<nip, blk, 0, st>>>(d_tiles, d_items_p, d_map, d_scol, d_psi, d_P, 1, 0, d_rb, d_Q, d_xs,
+                                  d_qmax);
       h->prof.end(st, pe, PK_SCALE, 2.0 * elems, 40.0 * elems);
       h->count_launch(2);
       for (int i = 0; i < m; ++i) {
@@ -1786,7 +1823,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
           h->prof.end(st, pe, PK_AXPY_NORM, (lanczos ? 8.0 : 12.0) * elems, 48.0 * elems);
           pe = h->prof.begin(st);
           k_scale<<<nip, blk, 0, st>>>(d_tiles, d_items_p, d_map, d_scol, d_psi, d_P, 0, i + 1, d_rb,
-                                       d_Q, d_xs);
+                                       d_Q, d_xs, d_qmax);
           h->prof.end(st, pe, PK_SCALE, 2.0 * elems, 40.0 * elems);
           h->count_launch(2);
         }
@@ -1798,9 +1835,13 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
       launch_expm(m, nslots, d_tiles, d_map, d_A, d_E, dt, d_err, st);
       h->prof.end(st, pe, PK_EXPM, 8.0 * (double)mm * m * 9.0 * list.size(),
                   32.0 * (double)mm * list.size());
-      const dim3 pgrid(nslots, ns);
+      const dim3 pgrid(gram ? 4 * nslots : nslots, ns);
       pe = h->prof.begin(st);
-      {
+      if (gram) {
+        void* args[] = {(void*)&d_tiles, (void*)&d_map, (void*)&m, (void*)&ncombo, (void*)&d_Q, (void*)&d_qmax,
+                        (void*)&ns, (void*)&rps, (void*)&d_ppart, (void*)&nslots};
+        CK(cudaLaunchKernel(gram_fn, pgrid, dim3(256), args, gram_smem, st));
+      } else {
         void* args[] = {(void*)&d_tiles, (void*)&d_map, (void*)&m, (void*)&ncombo, (void*)&d_combos,
                         (void*)&d_Q, (void*)&ns, (void*)&rps, (void*)&d_ppart};
         CK(cudaLaunchKernel(proj_fn, pgrid, dim3(proj_threads), args, proj_smem, st));

@@ -1,0 +1,60 @@
+"""The tensor-core kernels on exact digits against the CPU oracle, on the
+tiled path. Every step carries rounding of order 1e-15 of populations of at
+most 1 and the windows have at most 60 steps, so 1e-12 leaves a factor of
+over ten; a wrong fragment, edge or digit shows at 1e-3 and above (the digit
+weights are 1/256 apart)."""
+import numpy as np
+import pytest
+
+from conftest import general_csr, iso_csr
+from spin_dynamics_gb300 import workloads as W
+from spin_dynamics_gb300.spinsys import GAMMA_E, Electron, SysParam
+
+pytestmark = pytest.mark.gpu
+DT = 1.0 * GAMMA_E / 1000
+KEYS = ("P_S", "P_T0", "P_Tp", "P_Tm")
+
+
+def pair(g1, g2, seed=4, iso=False, kT=1.0):
+    rng = np.random.default_rng(seed)
+    A1, A2 = (W._tensors(rng, len(g), -2.0, 2.0, not iso) for g in (g1, g2))
+    return SysParam.from_input_units(Electron(g_I=list(g1), A=A1), Electron(g_I=list(g2), A=A2), J=0.01,
+                                     D=W.axial_dipolar(-0.4), kS_per_us=1.0, kT_per_us=kT)
+
+
+# dims 8 (m above n), 48, 144 and 1296: Z = 2, 12, 36 and 324 rows against 32-row chunks
+@pytest.mark.parametrize("g1, g2", [((2,), ()), ((2,), (2, 3)), ((3, 3), (2, 2)), ((3, 2, 2), (3, 3, 3))])
+@pytest.mark.parametrize("m", [1, 7, 16, 17, 24, 25, 32, 33])
+@pytest.mark.parametrize("method, M", [("mgs", 3), ("auto", 37)])
+def test_populations(sampler, oracle, g1, g2, m, method, M):
+    s = pair(g1, g2)
+    B = np.array([0.01, 0.03, 0.04])
+    rp, col, val = general_csr(oracle, s, B)
+    zk = W.random_phase_samples(s.Z, M, seed=m)
+    t_end = (60 if m > 1 else 3) * DT
+    ref = oracle.trace_sampling(rp, col, val, zk, DT, t_end, m, 1e-6)
+    sampler.set_krylov(method)
+    sampler.set_sample_path("off")
+    try:
+        sampler.build_h(s, B, "general")
+        got = sampler.trace_sampling(zk, DT, t_end, m, 1e-6)
+    finally:
+        sampler.set_sample_path("auto")
+        sampler.set_krylov("mgs")
+    assert max(np.max(np.abs(getattr(got, k) - ref[k])) for k in KEYS) <= 1e-12
+
+
+def test_undefined_samples_stay_undefined(sampler):
+    """A NaN in one sample vector reaches every population of the mean, as in
+    FP64 arithmetic: the digits of a NaN are no number."""
+    s = pair((3, 3), (2, 2))
+    zk = W.random_phase_samples(s.Z, 5)
+    zk[3, 7] = np.nan
+    sampler.set_sample_path("off")
+    try:
+        sampler.build_h(s, np.array([0.0, 0.0, 0.05]), "general")
+        got = sampler.trace_sampling(zk, DT, 4 * DT, 16, 1e-6)
+    finally:
+        sampler.set_sample_path("auto")
+    for k in KEYS:
+        assert np.all(np.isnan(getattr(got, k)[1:5]))
