@@ -237,6 +237,17 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   }();
   const int items_cap = h->sm_count * 32 + ntiles;
 
+  Handle::BlockStore* blocks = nullptr;
+  {
+    std::vector<int> used;
+    for (const GradJob& J : jobs) {
+      used.push_back(J.sys);
+      used.push_back(J.sys + 1);
+    }
+    const int rc = use_blocks(h, false, used, &blocks);
+    if (rc) return rc;
+  }
+  const double xs_bytes = blocks ? 16.0 : 8.0;
   // tiles, slot maps, costate coefficients
   std::vector<TileInfo> tf(ntiles), tb(ntiles);
   std::vector<int> map(nslots), scol(nslots), tile_n(ntiles), tile_job(ntiles);
@@ -266,6 +277,7 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
           x.val = (const double2*)HB.val.p + HB.nz_off[sy];
           x.vsum = (const double*)HB.vsum.p + HB.nz_off[sy];
           x.kappa = HB.herm[sy] ? &((const HMeta*)HB.meta.p)[sy].kappa : nullptr;
+          if (blocks) tile_blocks(x, *blocks, sy);
         }
         for (int l = 0; l < SPC_LANES; ++l) {
           const int s = c * SPC_LANES + l;
@@ -344,7 +356,7 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
     // to the size asked of it (buffers only grow), so its excess over that
     // size is no help
     auto need = [&](int k, bool keep) {
-      return sb * ((double)m + 4.5 + (nsteps / k + 1) + k + 1.0 + (keep ? (double)k * nq : (double)nq));
+      return sb * ((double)m + 4.0 + xs_bytes / 16.0 + (nsteps / k + 1) + k + 1.0 + (keep ? (double)k * nq : (double)nq));
     };
     auto extra = [&](int k, bool keep) {
       double x = 0.0;
@@ -353,7 +365,7 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
       add(h->gmu, sb);
       add(h->glam, 2.0 * sb);
       add(h->P, sb);
-      add(h->xsum, 0.5 * sb);  // the Re + Im plane of the current Krylov vector beside P
+      add(h->xsum, xs_bytes / 16.0 * sb);  // the current Krylov vector's digits or Re + Im plane beside P
       add(h->gck, sb * (nsteps / k + 1));
       add(h->gseg, sb * (k + 1));
       add(h->gnu, sb * (keep ? (double)k * nq : (double)nq));
@@ -389,12 +401,13 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   const int a_last = ((nsteps - 1) / K) * K;  // first step of the last segment
   const size_t n_ck = want_grad ? nck : 0, n_seg = want_grad ? K + 1 : 0;
   const size_t n_nu = want_grad ? (cache ? (size_t)K * nq : (size_t)nq) : 0;
-  const size_t plan_bytes = 2 * sizeof(TileInfo) * ntiles + sizeof(int2) * 2 * items_cap +
+  const size_t plan_bytes = 2 * sizeof(TileInfo) * ntiles + sizeof(int2) * 3 * items_cap +
                             sizeof(int) * 2 * nslots + sizeof(double2) * ntiles + 64;
   if (h->ensure(h->gck, sizeof(double2) * S * n_ck) || h->ensure(h->gseg, sizeof(double2) * S * n_seg) ||
       h->ensure(h->gnu, sizeof(double2) * S * n_nu) || h->ensure(h->gmu, sizeof(double2) * S) ||
       h->ensure(h->glam, sizeof(double2) * S * 2) || h->ensure(h->Q, sizeof(double2) * m * S) ||
-      h->ensure(h->P, sizeof(double2) * S) || h->ensure(h->xsum, sizeof(double) * S) ||
+      h->ensure(h->P, sizeof(double2) * S) || h->ensure(h->xsum, (size_t)xs_bytes * S) ||
+      h->ensure(h->qmax, 2 * sizeof(unsigned) * nslots) || h->ensure(h->xexp, sizeof(int) * nslots) ||
       h->ensure(h->partial, sizeof(double2) * std::max<size_t>((size_t)items_cap * SPC_LANES, part_cap)) ||
       h->ensure(h->counters, sizeof(unsigned) * std::max<size_t>(ntiles, npairs)) ||
       h->ensure(h->coef, sizeof(double2) * nslots) || h->ensure(h->rbeta, sizeof(double) * nslots) ||
@@ -409,7 +422,7 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   double2 *ck = (double2*)h->gck.p, *seg = (double2*)h->gseg.p, *gnu = (double2*)h->gnu.p;
   double2 *gmu = (double2*)h->gmu.p, *lam = (double2*)h->glam.p, *ulam = lam + S;
   double2 *d_Q = (double2*)h->Q.p, *d_P = (double2*)h->P.p, *d_part = (double2*)h->partial.p;
-  double* d_xs = (double*)h->xsum.p;
+  unsigned* d_qmax = (unsigned*)h->qmax.p;
   unsigned* d_cnt = (unsigned*)h->counters.p;
   double2 *d_A = (double2*)h->Ahess.p, *d_E = (double2*)h->Aexp.p, *d_c = (double2*)h->cvec.p;
   double2* d_c2 = (double2*)h->cvec2.p;
@@ -423,14 +436,15 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   TileInfo* d_tb = d_tf + ntiles;
   int2* d_items = (int2*)(plan + 2 * sizeof(TileInfo) * ntiles);
   int2* d_items_s = d_items + items_cap;
-  int* d_map = (int*)(d_items_s + items_cap);
+  int2* d_items_b = d_items_s + items_cap;
+  int* d_map = (int*)(d_items_b + items_cap);
   int* d_scol = d_map + nslots;
   double2* d_coefs = (double2*)(((uintptr_t)(d_scol + nslots) + 15) & ~(uintptr_t)15);
   int64_t launches0 = h->launches;
 
-  auto resident = [&](const void* fn) {
+  auto resident = [&](const void* fn, int threads = 256) {
     int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, 256, 0) != cudaSuccess) b = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, threads, 0) != cudaSuccess) b = 1;
     return std::max(1, b) * h->sm_count;
   };
   std::vector<int> fp, cp, fs, csn;
@@ -438,8 +452,11 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   plan_items(tile_n, std::min(resident((const void*)k_rowpass<PASS_AXPY_DOT>),
                               resident((const void*)k_rowpass<PASS_AXPY_NORM>)), fp, cp, items_p);
   plan_items(tile_n, resident((const void*)k_spmm), fs, csn, items_s);
-  const int nip = (int)items_p.size(), nis = (int)items_s.size();
-  if (nip > items_cap || nis > items_cap) return set_error(SPC_ERR_ARG, "internal: work plan exceeds its buffer");
+  std::vector<int> fb, cb;
+  std::vector<int2> items_b;
+  if (blocks) plan_items(tile_n, resident((const void*)k_spmm_blk<true>, BLK_THREADS), fb, cb, items_b, 4 * BLK_IDX);
+  const int nip = (int)items_p.size(), nis = (int)items_s.size(), nib = (int)items_b.size();
+  if (nip > items_cap || nis > items_cap || nib > items_cap) return set_error(SPC_ERR_ARG, "internal: work plan exceeds its buffer");
   // SpMM work per sample column: all entries (bytes); FP64 operations issued
   // 6 per complex entry, 4 per real one, 3 per row closing the three-product
   // sums (forward and adjoint Hamiltonians of a job share the pattern), plus
@@ -451,6 +468,7 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
     tf[t].nip = tb[t].nip = cp[t];
     tf[t].is0 = tb[t].is0 = fs[t];
     tf[t].nis = tb[t].nis = csn[t];
+    if (blocks) tf[t].nib = tb[t].nib = cb[t];
     const int sy = jobs[tile_job[t]].sys;
     nnz_tiles += HB.nnz[sy];
     spmm_flops += 6.0 * (double)HB.nnz_cplx[sy] + 4.0 * (double)(HB.nnz[sy] - HB.nnz_cplx[sy]) + 3.0 * tile_n[t];
@@ -460,6 +478,7 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   CK(cudaMemcpyAsync(d_tb, tb.data(), sizeof(TileInfo) * ntiles, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(d_items, items_p.data(), sizeof(int2) * nip, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(d_items_s, items_s.data(), sizeof(int2) * nis, cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(d_items_b, items_b.data(), sizeof(int2) * nib, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(d_map, map.data(), sizeof(int) * nslots, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(d_scol, scol.data(), sizeof(int) * nslots, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(d_coefs, coefs.data(), sizeof(double2) * ntiles, cudaMemcpyHostToDevice, st));
@@ -499,78 +518,36 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   // Krylov basis of the states `x` (psi layout) under the tiles' Hamiltonians
   auto build = [&](const double2* x, const TileInfo* tiles) {
     CK(cudaMemsetAsync(d_A, 0, sizeof(double2) * mm * nslots, st));
-    PassArgs pa{};
-    pa.tiles = tiles;
-    pa.items = d_items;
-    pa.m = m;
-    pa.Q = d_Q;
-    pa.P = d_P;
-    pa.psi = x;
-    pa.map = d_map;
-    pa.scol = d_scol;
-    pa.coef = (double2*)h->coef.p;
-    pa.rbeta = (double*)h->rbeta.p;
-    pa.Ahess = d_A;
-    pa.cvec = d_c;
-    pa.partial = d_part;
-    pa.counters = d_cnt;
-    pa.lanczos = lanczos ? 1 : 0;
-    int pe = h->prof.begin(st);
-    k_rowpass<PASS_NORM_GATHER><<<nip, blk, 0, st>>>(pa);
-    h->prof.end(st, pe, PK_DOT, 4.0 * elems, 16.0 * elems);
-    pe = h->prof.begin(st);
-    k_scale<<<nip, blk, 0, st>>>(tiles, d_items, d_map, d_scol, x, d_P, 1, 0, pa.rbeta, d_Q, d_xs, nullptr);
-    h->prof.end(st, pe, PK_SCALE, 2.0 * elems, 40.0 * elems);
-    h->count_launch(2);
-    for (int i = 0; i < m; ++i) {
-      pe = h->prof.begin(st);
-      k_spmm<<<nis, blk, 0, st>>>(tiles, d_items_s, d_map, i, d_Q, d_xs, d_P, lanczos ? 0 : 1);
-      h->prof.end(st, pe, PK_SPMM, (spmm_flops + (lanczos ? 0.0 : 4.0 * herm_rows)) * SPC_LANES,
-                  28.0 * (double)nnz_tiles + 40.0 * elems);
-      h->count_launch();
-      pa.col_i = i;
-      int j0 = 0;
-      if (lanczos && i > 0) {
-        j0 = i - 1;
-      } else {
-        pa.row_j = 0;
-        pa.jx = 0;
-        pe = h->prof.begin(st);
-        if (lanczos)
-          k_rowpass<PASS_DOT, true><<<nip, blk, 0, st>>>(pa);
-        else
-          k_rowpass<PASS_DOT><<<nip, blk, 0, st>>>(pa);
-        h->prof.end(st, pe, PK_DOT, (lanczos ? 4.0 : 8.0) * elems, 32.0 * elems);
-        h->count_launch();
-      }
-      for (int j = j0; j < i; ++j) {
-        pa.jx = j;
-        pa.jn = j + 1;
-        pa.row_j = j + 1;
-        pe = h->prof.begin(st);
-        if (lanczos)
-          k_rowpass<PASS_AXPY_DOT, true><<<nip, blk, 0, st>>>(pa);
-        else
-          k_rowpass<PASS_AXPY_DOT><<<nip, blk, 0, st>>>(pa);
-        h->prof.end(st, pe, PK_AXPY_DOT, (lanczos ? 8.0 : 16.0) * elems, 64.0 * elems);
-        h->count_launch();
-      }
-      if (i < m - 1) {
-        pa.jx = i;
-        pa.row_j = i + 1;
-        pe = h->prof.begin(st);
-        if (lanczos)
-          k_rowpass<PASS_AXPY_NORM, true><<<nip, blk, 0, st>>>(pa);
-        else
-          k_rowpass<PASS_AXPY_NORM><<<nip, blk, 0, st>>>(pa);
-        h->prof.end(st, pe, PK_AXPY_NORM, (lanczos ? 8.0 : 12.0) * elems, 48.0 * elems);
-        pe = h->prof.begin(st);
-        k_scale<<<nip, blk, 0, st>>>(tiles, d_items, d_map, d_scol, x, d_P, 0, i + 1, pa.rbeta, d_Q, d_xs,
-                                     nullptr);
-        h->prof.end(st, pe, PK_SCALE, 2.0 * elems, 40.0 * elems);
-        h->count_launch(2);
-      }
-    }
+    CK(cudaMemsetAsync(d_qmax, 0, 2 * sizeof(unsigned) * nslots, st));
+    BasisRun br{};
+    br.tiles = tiles;
+    br.items_p = d_items;
+    br.items_s = d_items_s;
+    br.items_b = d_items_b;
+    br.nip = nip;
+    br.nis = nis;
+    br.nib = nib;
+    br.xs = h->xsum.p;
+    br.lanczos = lanczos;
+    br.pa.m = m;
+    br.pa.Q = d_Q;
+    br.pa.P = d_P;
+    br.pa.psi = x;
+    br.pa.map = d_map;
+    br.pa.scol = d_scol;
+    br.pa.coef = (double2*)h->coef.p;
+    br.pa.rbeta = (double*)h->rbeta.p;
+    br.pa.Ahess = d_A;
+    br.pa.cvec = d_c;
+    br.pa.partial = d_part;
+    br.pa.counters = d_cnt;
+    br.pa.qmax = d_qmax;
+    br.pa.pmax = d_qmax + nslots;
+    br.pa.xexp = (int*)h->xexp.p;
+    br.elems = elems;
+    br.nnz_work = (double)nnz_tiles;
+    br.spmm_flops = spmm_flops + (lanczos ? 0.0 : 4.0 * herm_rows);
+    enqueue_basis(h, br);
     builds += Mtot;
     return SPC_OK;
   };

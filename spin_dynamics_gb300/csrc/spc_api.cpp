@@ -170,6 +170,7 @@ int spc_set_h(spc_handle* h, const spc_csr* H) {
   h->h.n = n;
   h->h.nnz = nnz;
   h->h.herm_shift = is_hermitian_plus_shift(n, rp, cl, H->val);
+  h->h.blk_one.describe({spc::BlockSys{}});
   return spc::prepare_spmm_rows(&h->h);
 }
 
@@ -287,6 +288,7 @@ static int batch_jobs(spc_handle* h, int n_jobs, const int* job_sys, const int* 
     j.herm_shift = B.herm[s] != 0;
     j.kappa = j.herm_shift ? &((const spc::HMeta*)B.meta.p)[s].kappa : nullptr;
     j.nnz_cplx = B.nnz_cplx[s];
+    j.sys = s;
     zoff += (int64_t)M[k] * (j.n / 4);
   }
   return SPC_OK;

@@ -6,29 +6,33 @@
 // for mma.sync m16n8k16). A double is therefore cut into radix-256 digits (the
 // splitting of Ozaki, Ogita, Oishi and Rump, "Error-free transformations of
 // matrix multiplication by using fast routines of matrix multiplication",
-// Numer. Algorithms 59 (2012)): x = sum_i d_i 256^(6-i) in units of a common
-// power of two, d_i in [-128, 127] (exact in FP16). Products of digits are at
-// most 2^14, so sums of up to 2^10 of them are integers below 2^24 and exact
-// in the FP32 accumulators. The product sums S_l of equal weight (i + j = l)
-// are kept for l <= 6 and closed in integers: the only errors are the
-// rounding of x to the common unit and the dropped l >= 7.
+// Numer. Algorithms 59 (2012)): x = sum_i d_i 256^(7-i), i = 0..7, in units
+// of a common power of two, d_i in [-128, 127] (exact in FP16). Products of
+// digits are at most 2^14, so sums of up to 2^10 of them are integers of at
+// most 2^24 and exact in the FP32 accumulators. The product sums S_l of equal
+// weight (i + j = l) are kept down to a level and closed in integers: the
+// only errors are the rounding of x to the common unit (61 or 62 bits below
+// the largest component), the dropped levels and the last rounding. Measured
+// against extended precision they are no larger than the FP64 kernels'.
 //
 // The digits of a two's-complement integer v are the bytes of
-// v + 0x80808080808080, each 128 too large; a byte b becomes the FP16 number
+// v + 0x8080808080808080, each 128 too large; a byte b becomes the FP16 number
 // b - 128 as (0x6400 | b) - 1152 (0x6400 is 1024, whose unit is 1).
 
-#define DIGITS 7
-#define DIGIT_BIAS 0x0080808080808080ll
+#define DIGITS 8
+#define DIGIT_BIAS 0x8080808080808080ull
 
-// x (sign-magnitude double) as an integer in units of 2^(E - 52), E the
-// biased exponent `emax` of the largest |x| of its set: |result| < 2^53,
-// rounded to nearest (half up in magnitude). Subnormals count as zero.
+// x (sign-magnitude double) as an integer in units of 2^(E - 52 - BITS), E the
+// exponent of the largest |x| of its set (biased: emax): |result| <=
+// 2^(53 + BITS), rounded to nearest (half up in magnitude). Subnormals count
+// as zero.
+template <int BITS>
 __device__ __forceinline__ long long to_fixed(double x, int emax) {
   const long long b = __double_as_longlong(x);
   const int ex = (int)(b >> 52) & 0x7ff;
   const unsigned long long man = (b & 0xfffffffffffffll) | (1ull << 52);
-  const int sh = min(emax - ex, 62);
-  unsigned long long v = (((man << 1) >> sh) + 1) >> 1;
+  const int sh = min(emax - ex, 63);
+  unsigned long long v = (((man << (BITS + 1)) >> sh) + 1) >> 1;
   v = ex == 0 ? 0 : v;
   return b < 0 ? -(long long)v : (long long)v;
 }
@@ -46,198 +50,4 @@ __device__ __forceinline__ void mma_digits(float (&d)[4], const unsigned (&a)[4]
   asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%0,%1,%2,%3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-__device__ __forceinline__ unsigned twice(unsigned x) {
-  const __half2 h = *reinterpret_cast<const __half2*>(&x);
-  const __half2 v = __hadd2(h, h);
-  return *reinterpret_cast<const unsigned*>(&v);
-}
-
-// ---------------------------------------------------------------------------
-// The Krylov-space projectors (k_proj's Grams, same `part` layout) for m <= 32.
-// CTA = (sample, type, split of the nuclear rows). Staged per chunk of GRAM_R
-// rows: the type's vectors V (q1, q2 - q3, q2 + q3 or q4, formed exactly in
-// integers) as digit pairs (re, im), 32 bits each, [digit][vector][row]. With
-// k = (row, part) both operands of V^H V are the same words: the A fragment
-// of 16 vectors is the B fragments of its two 8-column halves; the imaginary
-// part takes B = (im, -re).
-// A warp holds one 16 x 16 block of the real or imaginary part (MT = 2: 8
-// blocks; MT = 1: 2 blocks, four warps each over every fourth k-step). Digit
-// pairs (i, j) and (j, i) give transposed blocks, so only i <= j is formed,
-// with A_i doubled for i < j: T = sum_(i<j) 2 A_i B_j + sum_i A_i B_i, 16
-// products instead of 28, and G = (T + T^T) / 2 (Re), (T - T^T) / 2 (Im).
-// A k-step adds at most 7 * 16 * 2^14 < 2^20.9 to a level: after 8 steps the
-// FP32 sums are closed into 64-bit integers in shared memory.
-// Row stride GRAM_LD = 36 words: the 8 vectors x 4 rows of a fragment load
-// fall into 32 different banks.
-// Measured, all four Grams of 512 samples at dim 55296, m = 30: 19.3 ms
-// against 71.4 ms for k_proj (which holds the FP64 pipe at 92 %); 64 samples
-// at dim 9216, m = 24: 0.40 against 1.17 ms; 384 samples at dim 2304, m = 16:
-// 0.26 against 0.59 ms. The 256 clocks of products per nuclear row and sample
-// (m = 30) are a third of the time: staging (one 16-byte load per line, the
-// conversion to digits) and the products do not overlap within a CTA.
-#define GRAM_R 32
-#define GRAM_LD 36
-__host__ __device__ __forceinline__ size_t gram_smem_bytes(int mt) {
-  return sizeof(unsigned) * DIGITS * 16 * mt * GRAM_LD + sizeof(longlong2) * 8 * 256;
-}
-template <int MT>
-__global__ void __launch_bounds__(256, 2)
-    k_gram(const TileInfo* __restrict__ tiles, const int* __restrict__ map, int m, int ncombo,
-           const double2* __restrict__ Q, const unsigned* __restrict__ qmax, int nsplit, int64_t rps,
-           double2* __restrict__ part, int nslots) {
-  constexpr int MP = 16 * MT;
-  extern __shared__ __align__(16) unsigned char gsm[];
-  longlong2* acc64 = reinterpret_cast<longlong2*>(gsm);               // [8][256]
-  unsigned* V = reinterpret_cast<unsigned*>(acc64 + 8 * 256);         // [DIGITS][MP][GRAM_LD]
-  const int type = blockIdx.x & 3;
-  const int w = blockIdx.x >> 2;
-  if (map[w] < 0) return;
-  const TileInfo& Ti = tiles[w / SPC_LANES];
-  const int64_t Z = Ti.n / 4;
-  const int nsp = proj_splits(nsplit, rps, Z);
-  const int split = blockIdx.y;
-  if (split >= nsp) return;
-  const int me = Ti.m;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
-  const int64_t per = (Z + nsp - 1) / nsp;
-  const int64_t n0 = (int64_t)split * per, n1 = min(Z, n0 + per);
-  const unsigned top = qmax[w];
-  const int emax = (int)(top >> 20);
-  // this warp's block: part (0 Re, 1 Im), rows 16 mi, columns 16 ni, k-steps
-  const int im = warp & 1;
-  const int mi = MT == 2 ? (warp >> 1) & 1 : 0, ni = MT == 2 ? warp >> 2 : 0;
-  const int k0 = MT == 2 ? 0 : warp >> 1, kstep = MT == 2 ? 1 : 4;
-  const bool two = 16 * ni + 8 < m;  // the second 8 columns hold basis vectors
-  float acc[2][DIGITS][4];
-#pragma unroll
-  for (int t = 0; t < 2; ++t)
-#pragma unroll
-    for (int l = 0; l < DIGITS; ++l)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) acc[t][l][r] = 0.f;
-#pragma unroll
-  for (int r = 0; r < 8; ++r) acc64[r * 256 + tid] = make_longlong2(0, 0);
-  auto close = [&]() {
-#pragma unroll
-    for (int t = 0; t < 2; ++t)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        long long s[DIGITS];
-#pragma unroll
-        for (int l = 0; l < DIGITS; ++l) {
-          s[l] = __float2int_rn(acc[t][l][r]);
-          acc[t][l][r] = 0.f;
-        }
-        longlong2 a = acc64[(4 * t + r) * 256 + tid];
-        a.x += (s[0] << 16) + (s[1] << 8) + s[2];
-        a.y += (s[3] << 24) + (s[4] << 16) + (s[5] << 8) + s[6];
-        acc64[(4 * t + r) * 256 + tid] = a;
-      }
-  };
-  const size_t vs = (size_t)Ti.n * SPC_LANES;
-  const int64_t e0 = type == 0 ? 0 : (type == 3 ? 3 * Z : Z);
-  const double2* Qt = Q + Ti.q_off + (w % SPC_LANES) + (size_t)e0 * SPC_LANES;
-  int steps = 0;
-  for (int64_t c0 = n0; c0 < n1; c0 += GRAM_R) {
-    const int len = (int)min((int64_t)GRAM_R, n1 - c0);
-#pragma unroll 4
-    for (int idx = tid; idx < MP * GRAM_R; idx += 256) {
-      const int j = idx / GRAM_R, nn = idx % GRAM_R;
-      long long vr = 0, vi = 0;
-      if (j < me && nn < len) {
-        const double2* p = Qt + (size_t)j * vs + (size_t)(c0 + nn) * SPC_LANES;
-        const double2 a = *p;
-        vr = to_fixed(a.x, emax);
-        vi = to_fixed(a.y, emax);
-        if (type == 1 || type == 2) {
-          const double2 b = p[(size_t)Z * SPC_LANES];
-          const long long br = to_fixed(b.x, emax), bi = to_fixed(b.y, emax);
-          vr = type == 1 ? vr - br : vr + br;
-          vi = type == 1 ? vi - bi : vi + bi;
-        }
-      }
-      vr += DIGIT_BIAS;
-      vi += DIGIT_BIAS;
-      const unsigned rl = (unsigned)vr, rh = (unsigned)(vr >> 32), il = (unsigned)vi, ih = (unsigned)(vi >> 32);
-      unsigned* dst = V + j * GRAM_LD + nn;
-#pragma unroll
-      for (int d = 0; d < DIGITS; ++d)
-        dst[d * MP * GRAM_LD] = d < 3 ? digit_pair(rh, ih, 2 - d) : digit_pair(rl, il, 6 - d);
-    }
-    __syncthreads();
-    for (int ks = k0; ks * 8 < len; ks += kstep) {
-      const unsigned* Vk = V + ks * 8 + q;
-      unsigned B[2][DIGITS][2];
-#pragma unroll
-      for (int t = 0; t < 2; ++t)
-        if (t == 0 || two)
-#pragma unroll
-          for (int d = 0; d < DIGITS; ++d)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const unsigned x = Vk[(d * MP + 16 * ni + 8 * t + g) * GRAM_LD + 4 * h];
-              B[t][d][h] = im ? __byte_perm(x, x, 0x1032) ^ 0x80000000u : x;
-            }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        unsigned A[4];
-        const unsigned* Va = Vk + (i * MP + 16 * mi + g) * GRAM_LD;
-        A[0] = Va[0];
-        A[1] = Va[8 * GRAM_LD];
-        A[2] = Va[4];
-        A[3] = Va[8 * GRAM_LD + 4];
-        mma_digits(acc[0][2 * i], A, B[0][i][0], B[0][i][1]);
-        if (two) mma_digits(acc[1][2 * i], A, B[1][i][0], B[1][i][1]);
-#pragma unroll
-        for (int r = 0; r < 4; ++r) A[r] = twice(A[r]);
-#pragma unroll
-        for (int j = i + 1; j <= 6 - i; ++j) {
-          mma_digits(acc[0][i + j], A, B[0][j][0], B[0][j][1]);
-          if (two) mma_digits(acc[1][i + j], A, B[1][j][0], B[1][j][1]);
-        }
-      }
-      if (++steps == 8) {
-        close();
-        steps = 0;
-      }
-    }
-    __syncthreads();
-  }
-  close();
-  __syncthreads();
-  // T of every block in units of the digit products, then G = (T +- T^T) / 2
-  double* Tm = reinterpret_cast<double*>(V);  // [2][MP][MP + 1]
-  constexpr int TL = MP + 1;
-  if (MT == 2 || k0 == 0) {
-#pragma unroll
-    for (int t = 0; t < 2; ++t)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        longlong2 a = acc64[(4 * t + r) * 256 + tid];
-        if (MT == 1)
-          for (int o = 1; o < 4; ++o) {
-            const longlong2 b = acc64[(4 * t + r) * 256 + tid + 64 * o];
-            a.x += b.x;
-            a.y += b.y;
-          }
-        const int row = 16 * mi + g + (r >> 1) * 8, colm = 16 * ni + 8 * t + 2 * q + (r & 1);
-        Tm[(im * MP + row) * TL + colm] = fma((double)a.x, 4294967296.0, (double)a.y);
-      }
-  }
-  __syncthreads();
-  // units: v in 2^(emax - 1023 - 52), products closed at 256^6
-  const double unit = ldexp(1.0, 2 * (emax - 1023) - 104 + 48 - 1);
-  const int nc = ncombo / 4;
-  double2* out = part + ((size_t)split * nslots + w) * ncombo + type * nc;
-  const bool bad = top >= 0x7ff00000u;  // an infinite or undefined basis gives undefined Grams
-  for (int idx = tid; idx < MP * MP; idx += 256) {
-    const int i = idx / MP, j = idx % MP;
-    if (i > j || j >= m) continue;
-    double2 gv = make_double2((Tm[i * TL + j] + Tm[j * TL + i]) * unit,
-                              (Tm[(MP + i) * TL + j] - Tm[(MP + j) * TL + i]) * unit);
-    if (bad) gv = make_double2(__longlong_as_double(0x7ff8000000000000ll), __longlong_as_double(0x7ff8000000000000ll));
-    out[i * m - i * (i - 1) / 2 + (j - i)] = gv;
-  }
 }

@@ -67,7 +67,8 @@ int Handle::ensure_h_entries(size_t count) {
 Handle::~Handle() {
   Buf* all[] = {&psi, &Q,  &P,    &partial, &counters, &coef, &rbeta, &Ahess, &Aexp, &proj, &projpart,
                 &cvec, &tt, &kk, &done, &map, &obs, &out, &zk, &err, &nbuild, &flag, &xcol, &xval, &xsplit, &plan, &jobtab,
-                &hmeta, &xvs, &xsum, &qmax, &hb.rowptr, &hb.split, &hb.col, &hb.val, &hb.vsum, &hb.meta, &gck, &gseg, &gnu, &gmu, &glam, &cvec2,
+                &hmeta, &xvs, &xsum, &qmax, &xexp, &blk_one.self, &blk_one.tab, &blk_one.nbr, &blk_one.desc,
+                &blk_batch.self, &blk_batch.tab, &blk_batch.nbr, &blk_batch.desc, &hb.rowptr, &hb.split, &hb.col, &hb.val, &hb.vsum, &hb.meta, &gck, &gseg, &gnu, &gmu, &glam, &cvec2,
                 &gslots, &gracc, &gfacc, &bcnt, &bnuc, &btot, &btab, &tune_out, &tune_zk};
   for (Buf* b : all)
     if (b->p) cudaFree(b->p);
@@ -263,6 +264,68 @@ int make_host_system(const spc_system* sys, int mode, HostSystem& hs) {
     general_tables(hs);
   }
   return SPC_OK;
+}
+
+BlockSys make_block_sys(const HostSystem& hs, int mode) {
+  BlockSys b;
+  if (mode != SPC_H_GENERAL) return b;
+  auto comp = [](double2 v) { return std::max(std::fabs(v.x), std::fabs(v.y)); };
+  auto l1 = [](double2 v) { return std::fabs(v.x) + std::fabs(v.y); };
+  // largest off-diagonal component, bound of the diagonal blocks' components
+  // and of the rows' absolute sums
+  double off = 0.0, self = 0.0, rows = 0.0;
+  for (int e = 0; e < 4; ++e) {
+    double r = 0.0;
+    for (int f = 0; f < 4; ++f) {
+      self = std::max(self, comp(hs.gen.H[e][f]));
+      r += l1(hs.gen.H[e][f]);
+    }
+    for (const NucInfo& q : hs.nuc) {
+      double best = 0.0;
+      for (int m = 0; m < q.g; ++m) {
+        double t = 0.0;
+        for (int f = 0; f < 4; ++f)
+          for (int d = 0; d < 3; ++d) t += l1(hs.gen_tab[q.tab_off + ((size_t)(e * 4 + f) * q.g + m) * 3 + d]);
+        best = std::max(best, t);
+      }
+      r += best;
+    }
+    rows = std::max(rows, r);
+  }
+  int nbr = 0;
+  for (const NucInfo& q : hs.nuc) {
+    double diag = 0.0;
+    for (size_t i = 0; i < (size_t)48 * q.g; ++i) {
+      const double c = comp(hs.gen_tab[q.tab_off + i]);
+      if (i % 3 == 1)
+        diag = std::max(diag, c);
+      else
+        off = std::max(off, c);
+      // std::max passes over a NaN
+      if (!std::isfinite(c)) rows = c;
+    }
+    self += diag;
+    nbr += std::min(2, q.g - 1);
+    b.g.push_back(q.g);
+    b.stride.push_back(q.stride);
+  }
+  for (int e = 0; e < 4; ++e)
+    for (int f = 0; f < 4; ++f)
+      if (!std::isfinite(l1(hs.gen.H[e][f]))) return b;
+  if (!std::isfinite(rows) || nbr > 19 || hs.N > INT32_MAX) return b;
+  b.Z = hs.Z;
+  b.bk = std::max(4, (nbr + 2) / 2 * 2);
+  const int eo = off > 0.0 ? std::ilogb(off) : -1000, es = self > 0.0 ? std::ilogb(self) : -1000;
+  b.eoff = std::max(eo, es - 7);  // a diagonal component has at most 8 more bits
+  if (b.eoff < -900 || b.eoff > 900) {
+    if (off > 0.0 || self > 0.0) return b;
+    b.eoff = 0;
+  }
+  // units of H, of X and of the closed levels (k + d = 8 is 256^6 units):
+  // 2^(eoff - 53 + E - 61 + 48)
+  b.bexp = b.eoff - 66;
+  b.ok = true;
+  return b;
 }
 
 int64_t predict_nnz(const HostSystem& hs, int mode) {

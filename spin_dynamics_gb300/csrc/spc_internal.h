@@ -100,6 +100,19 @@ struct HMeta {
   unsigned long long ncplx;  // entries with a nonzero imaginary part
 };
 
+// Block structure of a general-builder Hamiltonian: multiplicities and strides
+// of the nuclei, length of a nuclear index's block list (itself first, even),
+// unit exponent of the entries and exponent of the closed sums.
+struct BlockSys {
+  bool ok = false;  // false: the CSR kernel is the only path
+  int64_t Z = 0;
+  std::vector<int> g;
+  std::vector<int64_t> stride;
+  int bk = 0, eoff = 0, bexp = 0;
+  int64_t self_off = 0, tab_off = 0, nbr_off = 0;  // place in the store, once built
+};
+BlockSys make_block_sys(const HostSystem& hs, int mode);
+
 struct Handle {
   Prof prof;
   int device = 0;
@@ -126,6 +139,9 @@ struct Handle {
   Buf xvs, xsum;
   // largest basis component of every slot in flight (high word of the double)
   Buf qmax;
+  // exponent of the current Krylov vector of every slot, and its maximum while
+  // a pass forms it
+  Buf xexp;
   // Hamiltonian build scratch: row counts, nucleus tables, nonzero totals
   Buf bcnt, bnuc, btot, btab;
   // autotuner outputs and sample subsets
@@ -141,6 +157,18 @@ struct Handle {
     std::vector<int64_t> nnz_cplx;
     Buf rowptr, split, col, val, vsum, meta;  // meta: one HMeta per system; vsum: Re + Im per entry
   } hb;
+  // Digit fragments of a general-builder Hamiltonian's 4 x 4 blocks for the
+  // tensor-core SpMM (spc_blocks.cuh): host description at build time, device
+  // fragments on the first propagation that uses them
+  struct BlockStore {
+    Buf self, tab, nbr, desc;
+    std::vector<BlockSys> sys;
+    bool ready = false;
+    void describe(std::vector<BlockSys> s) {
+      sys = std::move(s);
+      ready = false;
+    }
+  } blk_one, blk_batch;
   // Krylov method: 0 full MGS (the reference's get_krylov), 1 Lanczos, 2 auto
   int krylov_method = 0;
   // replay each build round's launches as a captured CUDA graph
@@ -187,6 +215,7 @@ struct JobSpec {
   // and kappa (device) the shift, H_eff = A - i*kappa*1
   const double* kappa = nullptr;
   int64_t nnz_cplx = 0;  // entries of the execution copy with a nonzero imaginary part
+  int sys = 0;           // the job's entry of the block store
 };
 
 // One reduced-matrix slot of the yield gradient: the electron pair (G = 4,
@@ -225,9 +254,10 @@ void enqueue_split_rows(int64_t N, const int* rowptr, const int* col, const doub
                         double2* xval, double* xvs, int* split, bool herm, HMeta* meta, cudaStream_t st);
 int propagate(Handle* h, const double* theta, const double* init_pop, const double* zk_dev,
               int M, double dt, double t_end, int m, double tol, double* out_dev, int T);
+// `single`: the jobs are on the handle's own Hamiltonian, not the batch store.
 int propagate_batch(Handle* h, const double* theta, const double* init_pop,
                     const std::vector<JobSpec>& jobs, double dt, double t_end, int m, double tol,
-                    int T);
+                    int T, bool single = false);
 // Adjoint sweeps of spc_yield_gradient(_batch) over the batch store's
 // Hamiltonians: per job, the sample sums of the reduced matrices of the
 // gradient integrals (rsum[job]: nslot x 36 complex) and of

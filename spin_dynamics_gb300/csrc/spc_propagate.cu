@@ -35,6 +35,7 @@
 #include <cstring>
 #include <map>
 #include <set>
+#include <type_traits>
 #include <vector>
 
 #include <cooperative_groups.h>
@@ -64,6 +65,11 @@ struct TileInfo {
   // non-null: the execution copy holds the Hermitian part A of
   // H_eff = A - i*kappa*1 (real diagonal) and *kappa the shift
   const double* kappa;
+  // digit fragments of the Hamiltonian's blocks (k_spmm_blk) and the tile's items there
+  const uint4* bself;
+  const uint4* btab;
+  const int2* bnbr;
+  int bk, bexp, nib;
 };
 
 enum PassKind { PASS_NORM_GATHER = 0, PASS_DOT = 1, PASS_AXPY_DOT = 2, PASS_AXPY_NORM = 3 };
@@ -72,6 +78,7 @@ struct PassArgs {
   const TileInfo* tiles;
   const int2* items;  // pass items (tile, phase)
   int m, col_i, row_j;
+  int shift;          // k_spmm_blk: add -i kappa x where the copy holds the Hermitian part
   int lanczos;        // AXPY_NORM also seeds the next Lanczos coefficient
   int jx, jn;         // basis indices: DOT reads Q_jx; AXPY removes Q_jx, dots with Q_jn
   const double2* Q;
@@ -85,7 +92,28 @@ struct PassArgs {
   double2* cvec;      // Krylov coordinates per slot
   double2* partial;   // [items][32]
   unsigned* counters; // per tile
+  unsigned* pmax;     // per slot: high word of P's (psi's) largest component (norm passes; zero between them)
+  int* xexp;          // per slot: biased exponent bound of the vector that the norm is for
+  unsigned* qmax;     // per slot: largest such high word of the basis
 };
+
+// High word of the larger of |re|, |im|: its integer order is the order of
+// the magnitudes, NaN above infinity.
+__device__ __forceinline__ unsigned abs_high(double2 q) {
+  return max((unsigned)__double2hiint(q.x) & 0x7fffffffu, (unsigned)__double2hiint(q.y) & 0x7fffffffu);
+}
+
+// After a norm pass: a bound of the scaled vector's largest component (the
+// maximum's high word rounded up, times 1/norm as k_scale forms it), its
+// exponent for the digits of k_spmm_blk and the basis' maximum for k_gram.
+__device__ __forceinline__ void pass_exponent(const PassArgs& a, int w) {
+  const unsigned top = __ldcg(a.pmax + w);
+  a.pmax[w] = 0u;
+  const double q = top == 0u ? 0.0 : __hiloint2double((int)(top + 1u), 0) * a.rbeta[w];
+  const unsigned hq = (unsigned)__double2hiint(q) & 0x7fffffffu;
+  a.xexp[w] = (int)(hq >> 20);
+  a.qmax[w] = max(a.qmax[w], hq);
+}
 
 // REAL: the Hermitian Lanczos recurrence on A of H_eff = A - i*kappa*1
 // (tile's kappa non-null): every coefficient is real, the dots keep their real
@@ -99,6 +127,7 @@ __device__ __forceinline__ void pass_finalize(const PassArgs& a, int w, double2 
     c[0] = make_double2(b, 0.0);
     for (int j = 1; j < a.m; ++j) c[j] = cz();
     a.rbeta[w] = b > 0.0 ? 1.0 / b : 0.0;
+    pass_exponent(a, w);
   } else if (KIND == PASS_DOT || KIND == PASS_AXPY_DOT) {
     if (REAL) {
       a.coef[w] = make_double2(tot.x, 0.0);
@@ -112,6 +141,7 @@ __device__ __forceinline__ void pass_finalize(const PassArgs& a, int w, double2 
     a.Ahess[(size_t)w * mm + a.row_j + (size_t)a.col_i * a.m] = make_double2(b, 0.0);
     // exact breakdown (p == 0): the next basis vector is 0 instead of 0/0
     a.rbeta[w] = b > 0.0 ? 1.0 / b : 0.0;
+    pass_exponent(a, w);
     if (a.lanczos) {
       // Hermitian tridiagonal: A(i, i+1) = beta_i, the coefficient of Q_i
       // in the next step's three-term recurrence
@@ -127,7 +157,10 @@ __device__ __forceinline__ void pass_finalize(const PassArgs& a, int w, double2 
 template <int KIND, bool REAL = false>
 __global__ void __launch_bounds__(256) k_rowpass(PassArgs a) {
   __shared__ double2 red[SPC_WARPS][SPC_LANES];
+  __shared__ unsigned mx[SPC_WARPS][SPC_LANES];
   __shared__ bool am_last;
+  constexpr bool NORM = KIND == PASS_NORM_GATHER || KIND == PASS_AXPY_NORM;
+  unsigned top = 0;
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int2 it = a.items[blockIdx.x];
   const TileInfo& T = a.tiles[it.x];
@@ -147,6 +180,7 @@ __global__ void __launch_bounds__(256) k_rowpass(PassArgs a) {
         double2 x = src[(size_t)r * T.ldp];
         acc.x = fma(x.x, x.x, acc.x);
         acc.x = fma(x.y, x.y, acc.x);
+        top = max(top, abs_high(x));
       }
     } else if (KIND == PASS_DOT) {
       const double2* X = a.Q + T.q_off + a.jx * vs + tx;
@@ -188,17 +222,24 @@ __global__ void __launch_bounds__(256) k_rowpass(PassArgs a) {
         } else {
           acc.x = fma(p.x, p.x, acc.x);
           acc.x = fma(p.y, p.y, acc.x);
+          top = max(top, abs_high(p));
         }
       }
     }
   }
   red[ty][tx] = acc;
+  if (NORM) mx[ty][tx] = top;
   __syncthreads();
   if (ty == 0) {
     double2 s = red[0][tx];
 #pragma unroll
     for (int y = 1; y < SPC_WARPS; ++y) s = cadd(s, red[y][tx]);
     a.partial[(size_t)blockIdx.x * SPC_LANES + tx] = s;
+    if (NORM && act) {
+#pragma unroll
+      for (int y = 1; y < SPC_WARPS; ++y) top = max(top, mx[y][tx]);
+      atomicMax(a.pmax + w, top);
+    }
   }
   __threadfence();
   __syncthreads();
@@ -223,61 +264,55 @@ __global__ void __launch_bounds__(256) k_rowpass(PassArgs a) {
   }
 }
 
-// High word of the larger of |re|, |im|: its integer order is the order of
-// the magnitudes, NaN above infinity.
-__device__ __forceinline__ unsigned abs_high(double2 q) {
-  return max((unsigned)__double2hiint(q.x) & 0x7fffffffu, (unsigned)__double2hiint(q.y) & 0x7fffffffu);
-}
+#include "spc_digits.cuh"
+#include "spc_blocks.cuh"
 
 // Q_{jd} = P / ||P||  (or Q_0 = psi[:, scol] / ||psi|| when gather != 0),
-// and beside it XS = Re + Im of the stored Q_{jd} (the operand k_spmm's
-// three-product form reads); grid = pass items. XS has P's layout (p_off).
-// qmax (may be null): per slot, the high word of the basis' largest component.
+// and beside it the operand of the next SpMM: with DIG the packed digits of
+// Q_{jd} that k_spmm_blk reads, [n][32][4] (a thread takes the four electron
+// rows of a nuclear index and writes 64 bytes), else the plane Re + Im of
+// k_spmm's three-product form in P's layout (p_off); grid = pass items.
+template <bool DIG>
 __global__ void __launch_bounds__(256)
     k_scale(const TileInfo* __restrict__ tiles, const int2* __restrict__ items,
             const int* __restrict__ map, const int* __restrict__ scol,
             const double2* __restrict__ psi, const double2* __restrict__ P, int gather, int jd,
-            const double* __restrict__ rbeta, double2* __restrict__ Q, double* __restrict__ XS,
-            unsigned* __restrict__ qmax) {
-  __shared__ unsigned mx[SPC_WARPS][SPC_LANES];
+            const double* __restrict__ rbeta, const int* __restrict__ xexp, double2* __restrict__ Q,
+            void* __restrict__ XS) {
   const int2 it = items[blockIdx.x];
   const TileInfo& T = tiles[it.x];
   if (!gather && jd >= T.m) return;
   const int tx = threadIdx.x;
   const int w = it.x * SPC_LANES + tx;
-  const bool act = map[w] >= 0;
-  const double rb = act ? rbeta[w] : 0.0;
-  const int n = act ? T.n : 0;
-  unsigned top = 0;
+  if (map[w] < 0) return;
+  const double rb = rbeta[w];
+  const int n = T.n;
   const int stride = T.nip * SPC_WARPS;
   double2* dst = Q + T.q_off + (size_t)jd * n * SPC_LANES + tx;
-  double* xs = XS + T.p_off + tx;
-  if (gather) {
-    const double2* src = psi + T.psi_off + scol[w];
-    for (int r = it.y * SPC_WARPS + threadIdx.y; r < n; r += stride) {
-      const double2 x = src[(size_t)r * T.ldp];
-      const double2 q = make_double2(x.x * rb, x.y * rb);
-      dst[(size_t)r * SPC_LANES] = q;
-      xs[(size_t)r * SPC_LANES] = q.x + q.y;
-      top = max(top, abs_high(q));
+  const double2* src = gather ? psi + T.psi_off + scol[w] : P + T.p_off + tx;
+  const size_t ld = gather ? T.ldp : SPC_LANES;
+  if (DIG) {
+    const int ex = xexp[w], Z = n / 4;
+    uint4* dx = (uint4*)XS + T.p_off + tx * 4;
+    for (int k = it.y * SPC_WARPS + threadIdx.y; k < Z; k += stride) {
+      double2 x[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[e] = src[((size_t)e * Z + k) * ld];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const double2 q = make_double2(x[e].x * rb, x[e].y * rb);
+        dst[((size_t)e * Z + k) * SPC_LANES] = q;
+        dx[(size_t)k * 128 + e] = pack_digits(q, ex);
+      }
     }
   } else {
-    const double2* src = P + T.p_off + tx;
+    double* xs = (double*)XS + T.p_off + tx;
     for (int r = it.y * SPC_WARPS + threadIdx.y; r < n; r += stride) {
-      const double2 x = src[(size_t)r * SPC_LANES];
+      const double2 x = src[(size_t)r * ld];
       const double2 q = make_double2(x.x * rb, x.y * rb);
       dst[(size_t)r * SPC_LANES] = q;
       xs[(size_t)r * SPC_LANES] = q.x + q.y;
-      top = max(top, abs_high(q));
     }
-  }
-  if (qmax == nullptr) return;
-  mx[threadIdx.y][tx] = top;
-  __syncthreads();
-  if (threadIdx.y == 0) {
-#pragma unroll
-    for (int y = 1; y < SPC_WARPS; ++y) top = max(top, mx[y][tx]);
-    if (act) atomicMax(qmax + w, top);
   }
 }
 
@@ -937,7 +972,7 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-#include "spc_digits.cuh"
+#include "spc_gram.cuh"
 
 __global__ void k_proj_reduce(const TileInfo* __restrict__ tiles, int nslots, const int* __restrict__ map,
                               int m, int ncombo, int nsplit, int64_t rps, const unsigned* __restrict__ combos,
@@ -1347,9 +1382,9 @@ int num_time_points(double dt, double t_end) {
   } while (0)
 
 // Work items per tile, proportional to the tile's rows and summing to about
-// one wave of `resident` CTAs; at least 32 rows per item.
+// one wave of `resident` CTAs; at least min_rows rows per item.
 static void plan_items(const std::vector<int>& tile_n, int resident, std::vector<int>& first,
-                       std::vector<int>& count, std::vector<int2>& items) {
+                       std::vector<int>& count, std::vector<int2>& items, int min_rows = 32) {
   int64_t W = 0;
   for (int n : tile_n) W += n;
   first.resize(tile_n.size());
@@ -1358,18 +1393,146 @@ static void plan_items(const std::vector<int>& tile_n, int resident, std::vector
   for (size_t t = 0; t < tile_n.size(); ++t) {
     const int n = tile_n[t];
     int64_t c = W > 0 ? (int64_t)n * resident / W : 1;
-    c = std::max<int64_t>(1, std::min<int64_t>(c, (n + 31) / 32));
+    c = std::max<int64_t>(1, std::min<int64_t>(c, (n + min_rows - 1) / min_rows));
     first[t] = (int)items.size();
     count[t] = (int)c;
     for (int q = 0; q < c; ++q) items.push_back(make_int2((int)t, q));
   }
 }
 
+// One Krylov basis per slot (get_krylov): what a round's launches need.
+struct BasisRun {
+  const TileInfo* tiles;  // device
+  const int2 *items_p, *items_s, *items_b;
+  int nip, nis, nib;       // nib: 0 for k_spmm on the CSR, else k_spmm_blk's items
+  PassArgs pa;
+  void* xs;                // Re + Im plane or packed digits of the current vector
+  bool lanczos;
+  // profile: vector elements, all stored entries, FP64 operations of k_spmm
+  double elems, nnz_work, spmm_flops;
+};
+static void enqueue_basis(Handle* h, BasisRun& B) {
+  cudaStream_t st = h->stream;
+  PassArgs& pa = B.pa;
+  const int m = pa.m;
+  const dim3 blk(SPC_LANES, SPC_WARPS);
+  const double elems = B.elems;
+  pa.tiles = B.tiles;
+  pa.items = B.items_p;
+  pa.lanczos = B.lanczos ? 1 : 0;
+  pa.shift = B.lanczos ? 0 : 1;
+  const auto scale = [&](int gather, int jd) {
+    const int pe = h->prof.begin(st);
+    if (B.nib)
+      k_scale<true><<<B.nip, blk, 0, st>>>(B.tiles, B.items_p, pa.map, pa.scol, pa.psi, pa.P, gather, jd, pa.rbeta,
+                                           pa.xexp, (double2*)pa.Q, B.xs);
+    else
+      k_scale<false><<<B.nip, blk, 0, st>>>(B.tiles, B.items_p, pa.map, pa.scol, pa.psi, pa.P, gather, jd, pa.rbeta,
+                                            pa.xexp, (double2*)pa.Q, B.xs);
+    h->prof.end(st, pe, PK_SCALE, 2.0 * elems, (B.nib ? 48.0 : 40.0) * elems);
+  };
+  int pe = h->prof.begin(st);
+  k_rowpass<PASS_NORM_GATHER><<<B.nip, blk, 0, st>>>(pa);
+  h->prof.end(st, pe, PK_DOT, 4.0 * elems, 16.0 * elems);
+  scale(1, 0);
+  h->count_launch(2);
+  for (int i = 0; i < m; ++i) {
+    pe = h->prof.begin(st);
+    pa.col_i = pa.row_j = i;
+    if (B.nib && B.lanczos)
+      k_spmm_blk<true><<<B.nib, BLK_THREADS, 0, st>>>(pa, B.items_b, (const uint4*)B.xs);
+    else if (B.nib)
+      k_spmm_blk<false><<<B.nib, BLK_THREADS, 0, st>>>(pa, B.items_b, (const uint4*)B.xs);
+    else
+      k_spmm<<<B.nis, blk, 0, st>>>(B.tiles, B.items_s, pa.map, i, pa.Q, (const double*)B.xs, pa.P, B.lanczos ? 0 : 1);
+    // algorithmic traffic: H (with its Re + Im) once per tile, X and its
+    // Re + Im plane once, Y once
+    h->prof.end(st, pe, PK_SPMM, B.spmm_flops * SPC_LANES + (B.nib && B.lanczos ? 8.0 * elems : 0.0),
+                28.0 * B.nnz_work + (B.nib ? (B.lanczos ? 64.0 : 32.0) : 40.0) * elems);
+    h->count_launch();
+    // MGS (get_krylov :453-456) projects p on Q_0..Q_i in order. Lanczos
+    // (H_eff Hermitian up to -i*kappa) needs only Q_{i-1} (coefficient
+    // beta_{i-1}, already in coef) and Q_i.
+    int j0 = 0;
+    if (B.lanczos && B.nib) {
+      j0 = i;  // projected on both by the SpMM's kernel
+    } else if (B.lanczos && i > 0) {
+      j0 = i - 1;
+    } else {
+      pa.row_j = 0;
+      pa.jx = 0;
+      pe = h->prof.begin(st);
+      if (B.lanczos)
+        k_rowpass<PASS_DOT, true><<<B.nip, blk, 0, st>>>(pa);
+      else
+        k_rowpass<PASS_DOT><<<B.nip, blk, 0, st>>>(pa);
+      h->prof.end(st, pe, PK_DOT, (B.lanczos ? 4.0 : 8.0) * elems, 32.0 * elems);
+      h->count_launch();
+    }
+    for (int j = j0; j < i; ++j) {
+      pa.jx = j;
+      pa.jn = j + 1;
+      pa.row_j = j + 1;
+      pe = h->prof.begin(st);
+      if (B.lanczos)
+        k_rowpass<PASS_AXPY_DOT, true><<<B.nip, blk, 0, st>>>(pa);
+      else
+        k_rowpass<PASS_AXPY_DOT><<<B.nip, blk, 0, st>>>(pa);
+      h->prof.end(st, pe, PK_AXPY_DOT, (B.lanczos ? 8.0 : 16.0) * elems, 64.0 * elems);
+      h->count_launch();
+    }
+    if (i < m - 1) {
+      pa.jx = i;
+      pa.row_j = i + 1;
+      pe = h->prof.begin(st);
+      if (B.lanczos)
+        k_rowpass<PASS_AXPY_NORM, true><<<B.nip, blk, 0, st>>>(pa);
+      else
+        k_rowpass<PASS_AXPY_NORM><<<B.nip, blk, 0, st>>>(pa);
+      h->prof.end(st, pe, PK_AXPY_NORM, (B.lanczos ? 8.0 : 12.0) * elems, 48.0 * elems);
+      scale(0, i + 1);
+      h->count_launch(2);
+    }
+  }
+}
+
+// The block store of the handle's own Hamiltonian (single) or of the batch,
+// built if every system that the call uses has one; null otherwise: CSRs the
+// caller gave, the reference builder's (about 9 mostly real entries a row, 20
+// FP64 operations: k_spmm takes 77 us for 32 samples at dim 55296, where
+// k_spmm_blk takes 102 us for the general builder's 15 blocks a row) and systems
+// of more than
+// BLK_MAXNBR neighbours.
+static int use_blocks(Handle* h, bool single, const std::vector<int>& systems, Handle::BlockStore** out) {
+  *out = nullptr;
+  Handle::BlockStore& S = single ? h->blk_one : h->blk_batch;
+  for (int k : systems)
+    if (k >= (int)S.sys.size() || !S.sys[k].ok) return SPC_OK;
+  std::vector<const int*> rp(S.sys.size()), cl(S.sys.size());
+  std::vector<const double2*> vl(S.sys.size());
+  for (size_t k = 0; k < S.sys.size(); ++k) {
+    rp[k] = single ? h->d_rowptr : (const int*)h->hb.rowptr.p + h->hb.rp_off[k];
+    cl[k] = single ? (const int*)h->xcol.p : (const int*)h->hb.col.p + h->hb.nz_off[k];
+    vl[k] = single ? (const double2*)h->xval.p : (const double2*)h->hb.val.p + h->hb.nz_off[k];
+  }
+  const int rc = prepare_blocks(h, S, rp, cl, vl);
+  if (rc == SPC_OK) *out = &S;
+  return rc;
+}
+static void tile_blocks(TileInfo& t, const Handle::BlockStore& S, int sys) {
+  const BlockSys& b = S.sys[sys];
+  t.bself = (const uint4*)S.self.p + 64 * b.self_off;
+  t.btab = (const uint4*)S.tab.p + 64 * b.tab_off;
+  t.bnbr = (const int2*)S.nbr.p + b.nbr_off;
+  t.bk = b.bk;
+  t.bexp = b.bexp;
+}
+
 #include "spc_small.cuh"
 
 int propagate_batch(Handle* h, const double* theta, const double* init_pop,
                     const std::vector<JobSpec>& jobs, double dt, double t_end, int m, double tol,
-                    int T) {
+                    int T, bool single) {
   if (h->sample_path != SPC_SAMPLE_OFF) {
     size_t smem = 0;
     if (small_path_fits(h, jobs, m, T, smem))
@@ -1407,9 +1570,18 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
   // otherwise every round runs over consecutive chunks of whole 32-sample
   // tiles, the capacities scaled down by one factor. States, populations and
   // clocks stay resident for every sample either way.
-  const double slot_fixed = 16.0 * (6.0 * mm + m + 1 + (double)nsplit_max * ncombo) + 8.0 + 4.0 + 4.0 + 8.0;
-  // basis + work vector (complex) + the current vector's Re + Im plane (XS)
-  const double need_fl = 16.0 * (double)qcap + 24.0 * (double)pcap + slot_fixed * slots_cap +
+  const double slot_fixed = 16.0 * (6.0 * mm + m + 1 + (double)nsplit_max * ncombo) + 8.0 + 4.0 + 12.0 + 8.0;
+  Handle::BlockStore* blocks = nullptr;
+  {
+    std::vector<int> used(nj);
+    for (int k = 0; k < nj; ++k) used[k] = jobs[k].sys;
+    const int rc = use_blocks(h, single, used, &blocks);
+    if (rc) return rc;
+  }
+  // basis + work vector (complex) + the current vector's digits or Re + Im
+  // plane (XS)
+  const double xs_bytes = blocks ? 16.0 : 8.0;
+  const double need_fl = 16.0 * (double)qcap + (16.0 + xs_bytes) * (double)pcap + slot_fixed * slots_cap +
                          (double)(sizeof(TileInfo) + sizeof(unsigned)) * tiles_cap;
   const double need_global = 16.0 * (double)psi_total + 8.0 * 4.0 * (double)T * G + 16.0 * G;
   double budget;
@@ -1422,7 +1594,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
     auto reuse = [&](const Handle::Buf& b, double bytes) { held += std::min((double)b.bytes, bytes); };
     reuse(h->Q, 16.0 * (double)qcap);
     reuse(h->P, 16.0 * (double)pcap);
-    reuse(h->xsum, 8.0 * (double)pcap);
+    reuse(h->xsum, xs_bytes * (double)pcap);
     reuse(h->psi, 16.0 * (double)psi_total);
     reuse(h->obs, 8.0 * 4.0 * (double)T * G);
     const double sl = (double)slots_cap;
@@ -1434,7 +1606,8 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
     reuse(h->projpart, 16.0 * (double)nsplit_max * ncombo * sl);
     reuse(h->cvec, 16.0 * m * sl);
     reuse(h->flag, 4.0 * sl);
-    reuse(h->qmax, 4.0 * sl);
+    reuse(h->qmax, 8.0 * sl);
+    reuse(h->xexp, 4.0 * sl);
     reuse(h->tt, 8.0 * G);
     reuse(h->kk, 4.0 * G);
     reuse(h->done, 4.0 * G);
@@ -1450,7 +1623,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
     pfl = std::max<int64_t>((int64_t)(f * (double)pcap), (int64_t)nmax * SPC_LANES);
     tiles_fl = std::max(1, (int)(f * tiles_cap));
     slots_fl = tiles_fl * SPC_LANES;
-    const double fl = 16.0 * (double)qfl + 24.0 * (double)pfl + slot_fixed * slots_fl +
+    const double fl = 16.0 * (double)qfl + (16.0 + xs_bytes) * (double)pfl + slot_fixed * slots_fl +
                       (double)(sizeof(TileInfo) + sizeof(unsigned)) * tiles_fl;
     if (fl > budget)
       return set_error(SPC_ERR_ALLOC,
@@ -1461,7 +1634,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
   // upper bound on work items per round: one wave of the most resident kernel plus one per tile
   const int items_cap = h->sm_count * 32 + tiles_fl;
   if (h->ensure(h->psi, sizeof(double2) * psi_total) || h->ensure(h->Q, sizeof(double2) * qfl) ||
-      h->ensure(h->P, sizeof(double2) * pfl) || h->ensure(h->xsum, sizeof(double) * pfl) ||
+      h->ensure(h->P, sizeof(double2) * pfl) || h->ensure(h->xsum, (size_t)xs_bytes * pfl) ||
       h->ensure(h->partial, sizeof(double2) * (size_t)items_cap * SPC_LANES) ||
       h->ensure(h->counters, sizeof(unsigned) * tiles_fl) ||
       h->ensure(h->coef, sizeof(double2) * slots_fl) || h->ensure(h->rbeta, sizeof(double) * slots_fl) ||
@@ -1473,15 +1646,15 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
       h->ensure(h->cvec, sizeof(double2) * m * slots_fl) || h->ensure(h->tt, sizeof(double) * G) ||
       h->ensure(h->kk, sizeof(int) * G) || h->ensure(h->done, sizeof(int) * G) ||
       h->ensure(h->obs, sizeof(double) * 4 * (size_t)T * G) || h->ensure(h->err, 16) ||
-      h->ensure(h->flag, sizeof(int) * slots_fl) || h->ensure(h->qmax, sizeof(unsigned) * slots_fl) ||
-      h->ensure(h->plan, sizeof(TileInfo) * tiles_fl + sizeof(int2) * 2 * items_cap +
+      h->ensure(h->flag, sizeof(int) * slots_fl) || h->ensure(h->qmax, 2 * sizeof(unsigned) * slots_fl) ||
+      h->ensure(h->xexp, sizeof(int) * slots_fl) ||
+      h->ensure(h->plan, sizeof(TileInfo) * tiles_fl + sizeof(int2) * 3 * items_cap +
                              sizeof(int) * 2 * slots_fl + 256) ||
       h->ensure(h->jobtab, (sizeof(JobInit) + sizeof(JobOut)) * nj + 64))
     return SPC_ERR_ALLOC;
   double2* d_psi = (double2*)h->psi.p;
   double2* d_Q = (double2*)h->Q.p;
   double2* d_P = (double2*)h->P.p;
-  double* d_xs = (double*)h->xsum.p;
   double2* d_part = (double2*)h->partial.p;
   unsigned* d_cnt = (unsigned*)h->counters.p;
   double2* d_coef = (double2*)h->coef.p;
@@ -1501,12 +1674,13 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
   long long* d_nsteps = (long long*)((char*)h->err.p + 8);
   int* d_flag = (int*)h->flag.p;
   unsigned* d_qmax = (unsigned*)h->qmax.p;
-  // per-round plan: tiles | pass items | SpMM items | map | scol
+  // per-round plan: tiles | pass items | SpMM items | block SpMM items | map | scol
   char* plan = (char*)h->plan.p;
   TileInfo* d_tiles = (TileInfo*)plan;
   int2* d_items_p = (int2*)(plan + sizeof(TileInfo) * tiles_fl);
   int2* d_items_s = d_items_p + items_cap;
-  int* d_map = (int*)(d_items_s + items_cap);
+  int2* d_items_b = d_items_s + items_cap;
+  int* d_map = (int*)(d_items_b + items_cap);
   int* d_scol = d_map + slots_fl;
   JobInit* d_jinit = (JobInit*)h->jobtab.p;
   JobOut* d_jout = (JobOut*)((char*)h->jobtab.p + sizeof(JobInit) * nj);
@@ -1591,6 +1765,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
     return std::max(1, b) * h->sm_count;
   };
   const int res_spmm = resident((const void*)k_spmm, 256, 0);
+  const int res_blk = resident((const void*)k_spmm_blk<true>, BLK_THREADS, 0);
   const int res_pass = std::min(resident((const void*)k_rowpass<PASS_AXPY_DOT>, 256, 0),
                                 resident((const void*)k_rowpass<PASS_AXPY_NORM>, 256, 0));
   // Grams on the tensor cores for m <= 32 (a CTA per projector type; its two
@@ -1657,6 +1832,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
         ti.vsum = jobs[k].vsum;
         ti.kappa = jobs[k].herm_shift ? jobs[k].kappa : nullptr;
         ti.m = std::min(m, ti.n);
+        if (blocks) tile_blocks(ti, *blocks, jobs[k].sys);
         qo += (int64_t)m * ti.n * SPC_LANES;
         po += (int64_t)ti.n * SPC_LANES;
         for (int l = 0; l < SPC_LANES; ++l) {
@@ -1676,29 +1852,33 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
     }
     const int ntiles = (int)tiles.size();
     const int nslots = ntiles * SPC_LANES;
-    std::vector<int> fp, cp, fs, cs;
-    std::vector<int2> items_p, items_s;
+    std::vector<int> fp, cp, fs, cs, fb, cb;
+    std::vector<int2> items_p, items_s, items_b;
     plan_items(tile_n, res_pass, fp, cp, items_p);
     plan_items(tile_n, res_spmm, fs, cs, items_s);
+    if (blocks) plan_items(tile_n, res_blk, fb, cb, items_b, 4 * BLK_IDX);
     for (int t = 0; t < ntiles; ++t) {
       tiles[t].ip0 = fp[t];
       tiles[t].nip = cp[t];
       tiles[t].is0 = fs[t];
       tiles[t].nis = cs[t];
+      if (blocks) tiles[t].nib = cb[t];
     }
-    const int nip = (int)items_p.size(), nis = (int)items_s.size();
-    if (nip > items_cap || nis > items_cap || ntiles > tiles_fl || qo > qfl || po > pfl)
+    const int nip = (int)items_p.size(), nis = (int)items_s.size(), nib = (int)items_b.size();
+    if (nip > items_cap || nis > items_cap || nib > items_cap || ntiles > tiles_fl || qo > qfl || po > pfl)
       return set_error(SPC_ERR_ARG, "internal: work plan exceeds its buffer");
     // one host->device copy of the plan
     const size_t off_items_p = sizeof(TileInfo) * tiles_fl;
     const size_t off_items_s = off_items_p + sizeof(int2) * items_cap;
-    const size_t off_map = off_items_s + sizeof(int2) * items_cap;
+    const size_t off_items_b = off_items_s + sizeof(int2) * items_cap;
+    const size_t off_map = off_items_b + sizeof(int2) * items_cap;
     const size_t off_scol = off_map + sizeof(int) * slots_fl;
     const size_t plan_bytes = off_scol + sizeof(int) * nslots;
     hplan.resize(plan_bytes);
     std::memcpy(hplan.data(), tiles.data(), sizeof(TileInfo) * ntiles);
     std::memcpy(hplan.data() + off_items_p, items_p.data(), sizeof(int2) * nip);
     std::memcpy(hplan.data() + off_items_s, items_s.data(), sizeof(int2) * nis);
+    std::memcpy(hplan.data() + off_items_b, items_b.data(), sizeof(int2) * nib);
     std::memcpy(hplan.data() + off_map, map.data(), sizeof(int) * nslots);
     std::memcpy(hplan.data() + off_scol, scol.data(), sizeof(int) * nslots);
     CK(cudaMemcpyAsync(plan, hplan.data(), plan_bytes, cudaMemcpyHostToDevice, st));
@@ -1738,23 +1918,32 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
     auto enqueue = [&]() -> int {
       CK(cudaMemsetAsync(d_A, 0, sizeof(double2) * mm * nslots, st));
       CK(cudaMemsetAsync(d_flag, 0, sizeof(int) * nslots, st));
-      CK(cudaMemsetAsync(d_qmax, 0, sizeof(unsigned) * nslots, st));
-      PassArgs pa{};
-      pa.tiles = d_tiles;
-      pa.items = d_items_p;
-      pa.m = m;
-      pa.Q = d_Q;
-      pa.P = d_P;
-      pa.psi = d_psi;
-      pa.map = d_map;
-      pa.scol = d_scol;
-      pa.coef = d_coef;
-      pa.rbeta = d_rb;
-      pa.Ahess = d_A;
-      pa.cvec = d_c;
-      pa.partial = d_part;
-      pa.counters = d_cnt;
-      pa.lanczos = lanczos ? 1 : 0;
+      CK(cudaMemsetAsync(d_qmax, 0, 2 * sizeof(unsigned) * slots_fl, st));
+      BasisRun br{};
+      br.tiles = d_tiles;
+      br.items_p = d_items_p;
+      br.items_s = d_items_s;
+      br.items_b = d_items_b;
+      br.nip = nip;
+      br.nis = nis;
+      br.nib = nib;
+      br.xs = h->xsum.p;
+      br.lanczos = lanczos;
+      br.pa.m = m;
+      br.pa.Q = d_Q;
+      br.pa.P = d_P;
+      br.pa.psi = d_psi;
+      br.pa.map = d_map;
+      br.pa.scol = d_scol;
+      br.pa.coef = d_coef;
+      br.pa.rbeta = d_rb;
+      br.pa.Ahess = d_A;
+      br.pa.cvec = d_c;
+      br.pa.partial = d_part;
+      br.pa.counters = d_cnt;
+      br.pa.qmax = d_qmax;
+      br.pa.pmax = d_qmax + slots_fl;
+      br.pa.xexp = (int*)h->xexp.p;
       // SpMM work of the round: all entries (bytes) and the FP64 operations
       // issued (3 DFMA per complex entry, 2 per real one, 3 DADD per row to
       // close the three-product sums, 2 DFMA per row for the -i*kappa shift
@@ -1767,67 +1956,11 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
         spmm_flops += 6.0 * (double)J.nnz_cplx + 4.0 * (double)(J.nnz - J.nnz_cplx) + 3.0 * ti.n +
                       (!lanczos && ti.kappa ? 4.0 * ti.n : 0.0);
       }
-      int pe = h->prof.begin(st);
-      k_rowpass<PASS_NORM_GATHER><<<nip, blk, 0, st>>>(pa);
-      h->prof.end(st, pe, PK_DOT, 4.0 * elems, 16.0 * elems);
-      pe = h->prof.begin(st);
-      k_scale<<<nip, blk, 0, st>>>(d_tiles, d_items_p, d_map, d_scol, d_psi, d_P, 1, 0, d_rb, d_Q, d_xs,
-                                  d_qmax);
-      h->prof.end(st, pe, PK_SCALE, 2.0 * elems, 40.0 * elems);
-      h->count_launch(2);
-      for (int i = 0; i < m; ++i) {
-        pe = h->prof.begin(st);
-        k_spmm<<<nis, blk, 0, st>>>(d_tiles, d_items_s, d_map, i, d_Q, d_xs, d_P, lanczos ? 0 : 1);
-        // algorithmic traffic: H (with its Re + Im) once per tile, X and its
-        // Re + Im plane once, Y once
-        h->prof.end(st, pe, PK_SPMM, spmm_flops * SPC_LANES, 28.0 * (double)nnz_work + 40.0 * elems);
-        h->count_launch();
-        pa.col_i = i;
-        // MGS (get_krylov :453-456) projects p on Q_0..Q_i in order. Lanczos
-        // (H_eff Hermitian up to -i*kappa) needs only Q_{i-1} (coefficient
-        // beta_{i-1}, already in coef) and Q_i.
-        int j0 = 0;
-        if (lanczos && i > 0) {
-          j0 = i - 1;
-        } else {
-          pa.row_j = 0;
-          pa.jx = 0;
-          pe = h->prof.begin(st);
-          if (lanczos)
-            k_rowpass<PASS_DOT, true><<<nip, blk, 0, st>>>(pa);
-          else
-            k_rowpass<PASS_DOT><<<nip, blk, 0, st>>>(pa);
-          h->prof.end(st, pe, PK_DOT, (lanczos ? 4.0 : 8.0) * elems, 32.0 * elems);
-          h->count_launch();
-        }
-        for (int j = j0; j < i; ++j) {
-          pa.jx = j;
-          pa.jn = j + 1;
-          pa.row_j = j + 1;
-          pe = h->prof.begin(st);
-          if (lanczos)
-            k_rowpass<PASS_AXPY_DOT, true><<<nip, blk, 0, st>>>(pa);
-          else
-            k_rowpass<PASS_AXPY_DOT><<<nip, blk, 0, st>>>(pa);
-          h->prof.end(st, pe, PK_AXPY_DOT, (lanczos ? 8.0 : 16.0) * elems, 64.0 * elems);
-          h->count_launch();
-        }
-        if (i < m - 1) {
-          pa.jx = i;
-          pa.row_j = i + 1;
-          pe = h->prof.begin(st);
-          if (lanczos)
-            k_rowpass<PASS_AXPY_NORM, true><<<nip, blk, 0, st>>>(pa);
-          else
-            k_rowpass<PASS_AXPY_NORM><<<nip, blk, 0, st>>>(pa);
-          h->prof.end(st, pe, PK_AXPY_NORM, (lanczos ? 8.0 : 12.0) * elems, 48.0 * elems);
-          pe = h->prof.begin(st);
-          k_scale<<<nip, blk, 0, st>>>(d_tiles, d_items_p, d_map, d_scol, d_psi, d_P, 0, i + 1, d_rb,
-                                       d_Q, d_xs, d_qmax);
-          h->prof.end(st, pe, PK_SCALE, 2.0 * elems, 40.0 * elems);
-          h->count_launch(2);
-        }
-      }
+      br.elems = elems;
+      br.nnz_work = (double)nnz_work;
+      br.spmm_flops = spmm_flops;
+      enqueue_basis(h, br);
+      int pe;
       double zsum = 0.0;  // sum over active slots of Z
       for (size_t c = 0; c < map.size(); ++c)
         if (map[c] >= 0) zsum += tiles[c / SPC_LANES].n / 4;
@@ -1889,7 +2022,8 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
     };
     // a shape is captured the second time it occurs (calls whose rounds never
     // repeat a shape pay no capture)
-    const std::vector<int64_t> key = {nip, nis, nslots, ns, rps, lanczos ? 1 : 0, (int64_t)list.size()};
+    const std::vector<int64_t> key = {nip, nis, nib, nslots, ns, rps, lanczos ? 1 : 0,
+                                       (int64_t)list.size()};
     const bool graphs = h->use_graphs && !h->prof.on && !shapes_seen.insert(key).second;
     if (graphs) {
       auto itg = graph_cache.find(key);
@@ -2017,7 +2151,7 @@ int propagate(Handle* h, const double* theta, const double* init_pop, const doub
   j.zk = (const double2*)zk_dev;
   j.out = out_dev;
   j.herm_shift = h->herm_shift;
-  return propagate_batch(h, theta, init_pop, std::vector<JobSpec>{j}, dt, t_end, m, tol, T);
+  return propagate_batch(h, theta, init_pop, std::vector<JobSpec>{j}, dt, t_end, m, tol, T, true);
 }
 
 #include "spc_adjoint.cuh"

@@ -25,9 +25,9 @@ def pair(g1, g2, seed=4, iso=False, kT=1.0):
 # dims 8 (m above n), 48, 144 and 1296: Z = 2, 12, 36 and 324 rows against 32-row chunks
 @pytest.mark.parametrize("g1, g2", [((2,), ()), ((2,), (2, 3)), ((3, 3), (2, 2)), ((3, 2, 2), (3, 3, 3))])
 @pytest.mark.parametrize("m", [1, 7, 16, 17, 24, 25, 32, 33])
-@pytest.mark.parametrize("method, M", [("mgs", 3), ("auto", 37)])
-def test_populations(sampler, oracle, g1, g2, m, method, M):
-    s = pair(g1, g2)
+@pytest.mark.parametrize("method, M, kT", [("mgs", 3, 1.0), ("mgs", 33, 0.3), ("auto", 37, 1.0)])
+def test_populations(sampler, oracle, g1, g2, m, method, M, kT):
+    s = pair(g1, g2, kT=kT)
     B = np.array([0.01, 0.03, 0.04])
     rp, col, val = general_csr(oracle, s, B)
     zk = W.random_phase_samples(s.Z, M, seed=m)
