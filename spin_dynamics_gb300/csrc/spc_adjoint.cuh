@@ -277,6 +277,7 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
           x.val = (const double2*)HB.val.p + HB.nz_off[sy];
           x.vsum = (const double*)HB.vsum.p + HB.nz_off[sy];
           x.kappa = HB.herm[sy] ? &((const HMeta*)HB.meta.p)[sy].kappa : nullptr;
+          x.rexp = HB.rexp[sy];
           if (blocks) tile_blocks(x, *blocks, sy);
         }
         for (int l = 0; l < SPC_LANES; ++l) {
@@ -366,6 +367,8 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
       add(h->glam, 2.0 * sb);
       add(h->P, sb);
       add(h->xsum, xs_bytes / 16.0 * sb);  // the current Krylov vector's digits or Re + Im plane beside P
+      add(h->acc, (double)acc_bytes(ntiles));
+      add(h->gram, (double)gram_bytes(ntiles, m));
       add(h->gck, sb * (nsteps / k + 1));
       add(h->gseg, sb * (k + 1));
       add(h->gnu, sb * (keep ? (double)k * nq : (double)nq));
@@ -401,13 +404,14 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   const int a_last = ((nsteps - 1) / K) * K;  // first step of the last segment
   const size_t n_ck = want_grad ? nck : 0, n_seg = want_grad ? K + 1 : 0;
   const size_t n_nu = want_grad ? (cache ? (size_t)K * nq : (size_t)nq) : 0;
-  const size_t plan_bytes = 2 * sizeof(TileInfo) * ntiles + sizeof(int2) * 3 * items_cap +
+  const size_t plan_bytes = 2 * sizeof(TileInfo) * ntiles + sizeof(int2) * 4 * items_cap +
                             sizeof(int) * 2 * nslots + sizeof(double2) * ntiles + 64;
   if (h->ensure(h->gck, sizeof(double2) * S * n_ck) || h->ensure(h->gseg, sizeof(double2) * S * n_seg) ||
       h->ensure(h->gnu, sizeof(double2) * S * n_nu) || h->ensure(h->gmu, sizeof(double2) * S) ||
       h->ensure(h->glam, sizeof(double2) * S * 2) || h->ensure(h->Q, sizeof(double2) * m * S) ||
       h->ensure(h->P, sizeof(double2) * S) || h->ensure(h->xsum, (size_t)xs_bytes * S) ||
       h->ensure(h->qmax, 2 * sizeof(unsigned) * nslots) || h->ensure(h->xexp, sizeof(int) * nslots) ||
+      h->ensure(h->acc, acc_bytes(ntiles)) || h->ensure(h->gram, gram_bytes(ntiles, m)) ||
       h->ensure(h->partial, sizeof(double2) * std::max<size_t>((size_t)items_cap * SPC_LANES, part_cap)) ||
       h->ensure(h->counters, sizeof(unsigned) * std::max<size_t>(ntiles, npairs)) ||
       h->ensure(h->coef, sizeof(double2) * nslots) || h->ensure(h->rbeta, sizeof(double) * nslots) ||
@@ -437,7 +441,8 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   int2* d_items = (int2*)(plan + 2 * sizeof(TileInfo) * ntiles);
   int2* d_items_s = d_items + items_cap;
   int2* d_items_b = d_items_s + items_cap;
-  int* d_map = (int*)(d_items_b + items_cap);
+  int2* d_items_o = d_items_b + items_cap;
+  int* d_map = (int*)(d_items_o + items_cap);
   int* d_scol = d_map + nslots;
   double2* d_coefs = (double2*)(((uintptr_t)(d_scol + nslots) + 15) & ~(uintptr_t)15);
   int64_t launches0 = h->launches;
@@ -447,16 +452,22 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, threads, 0) != cudaSuccess) b = 1;
     return std::max(1, b) * h->sm_count;
   };
+  // the three-term recurrence only on explicit request: no projector Gram
+  // verifies these bases (the trace-sampling path checks its own)
+  bool lanczos = h->krylov_method == 1;
+  for (const GradJob& J : jobs) lanczos = lanczos && HB.herm[J.sys] && HB.herm[J.sys + 1];
   std::vector<int> fp, cp, fs, csn;
   std::vector<int2> items_p, items_s;
-  plan_items(tile_n, std::min(resident((const void*)k_rowpass<PASS_AXPY_DOT>),
-                              resident((const void*)k_rowpass<PASS_AXPY_NORM>)), fp, cp, items_p);
+  plan_items(tile_n, resident((const void*)k_scale<true>), fp, cp, items_p);
   plan_items(tile_n, resident((const void*)k_spmm), fs, csn, items_s);
-  std::vector<int> fb, cb;
-  std::vector<int2> items_b;
+  std::vector<int> fb, cb, fo, co;
+  std::vector<int2> items_b, items_o;
+  plan_items(tile_n, resident(lanczos ? (const void*)k_ortho<1, 1, false, true>
+                                      : (const void*)k_ortho<8, 8, true, false>), fo, co, items_o);
   if (blocks) plan_items(tile_n, resident((const void*)k_spmm_blk<true>, BLK_THREADS), fb, cb, items_b, 4 * BLK_IDX);
   const int nip = (int)items_p.size(), nis = (int)items_s.size(), nib = (int)items_b.size();
-  if (nip > items_cap || nis > items_cap || nib > items_cap) return set_error(SPC_ERR_ARG, "internal: work plan exceeds its buffer");
+  const int nio = (int)items_o.size();
+  if (nip > items_cap || nis > items_cap || nib > items_cap || nio > items_cap) return set_error(SPC_ERR_ARG, "internal: work plan exceeds its buffer");
   // SpMM work per sample column: all entries (bytes); FP64 operations issued
   // 6 per complex entry, 4 per real one, 3 per row closing the three-product
   // sums (forward and adjoint Hamiltonians of a job share the pattern), plus
@@ -468,6 +479,7 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
     tf[t].nip = tb[t].nip = cp[t];
     tf[t].is0 = tb[t].is0 = fs[t];
     tf[t].nis = tb[t].nis = csn[t];
+    tf[t].nio = tb[t].nio = co[t];
     if (blocks) tf[t].nib = tb[t].nib = cb[t];
     const int sy = jobs[tile_job[t]].sys;
     nnz_tiles += HB.nnz[sy];
@@ -479,6 +491,7 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   CK(cudaMemcpyAsync(d_items, items_p.data(), sizeof(int2) * nip, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(d_items_s, items_s.data(), sizeof(int2) * nis, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(d_items_b, items_b.data(), sizeof(int2) * nib, cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(d_items_o, items_o.data(), sizeof(int2) * nio, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(d_map, map.data(), sizeof(int) * nslots, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(d_scol, scol.data(), sizeof(int) * nslots, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(d_coefs, coefs.data(), sizeof(double2) * ntiles, cudaMemcpyHostToDevice, st));
@@ -507,10 +520,6 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   }
   CK(set_expm_smem(m));
   const dim3 blk(SPC_LANES, SPC_WARPS);
-  // the three-term recurrence only on explicit request: no projector Gram
-  // verifies these bases (the trace-sampling path checks its own)
-  bool lanczos = h->krylov_method == 1;
-  for (const GradJob& J : jobs) lanczos = lanczos && HB.herm[J.sys] && HB.herm[J.sys + 1];
   std::vector<double> xq, wq;
   gauss_legendre01(nq, xq, wq);
   int64_t builds = 0;
@@ -527,6 +536,11 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
     br.nip = nip;
     br.nis = nis;
     br.nib = nib;
+    br.items_o = d_items_o;
+    br.nio = nio;
+    br.acc = (acc_t*)h->acc.p;
+    br.gram = (double2*)h->gram.p;
+    br.ntiles = ntiles;
     br.xs = h->xsum.p;
     br.lanczos = lanczos;
     br.pa.m = m;
@@ -547,7 +561,7 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
     br.elems = elems;
     br.nnz_work = (double)nnz_tiles;
     br.spmm_flops = spmm_flops + (lanczos ? 0.0 : 4.0 * herm_rows);
-    enqueue_basis(h, br);
+    CK(enqueue_basis(h, br));
     builds += Mtot;
     return SPC_OK;
   };

@@ -171,6 +171,14 @@ int spc_set_h(spc_handle* h, const spc_csr* H) {
   h->h.nnz = nnz;
   h->h.herm_shift = is_hermitian_plus_shift(n, rp, cl, H->val);
   h->h.blk_one.describe({spc::BlockSys{}});
+  // ||H|| <= sqrt(n) max row sum
+  double rows = 0.0;
+  for (int r = 0; r < n; ++r) {
+    double t = 0.0;
+    for (int k = rp[r]; k < rp[r + 1]; ++k) t += std::fabs(H->val[2 * (size_t)k]) + std::fabs(H->val[2 * (size_t)k + 1]);
+    if (!(t <= rows)) rows = t;
+  }
+  h->h.rexp = spc::norm_exponent(rows * std::sqrt((double)n));
   return spc::prepare_spmm_rows(&h->h);
 }
 
@@ -289,6 +297,7 @@ static int batch_jobs(spc_handle* h, int n_jobs, const int* job_sys, const int* 
     j.kappa = j.herm_shift ? &((const spc::HMeta*)B.meta.p)[s].kappa : nullptr;
     j.nnz_cplx = B.nnz_cplx[s];
     j.sys = s;
+    j.rexp = B.rexp[s];
     zoff += (int64_t)M[k] * (j.n / 4);
   }
   return SPC_OK;

@@ -168,9 +168,9 @@ __device__ __forceinline__ void copy16(void* dst, const void* src) {
 // step's list entry and rows cost two L2 latencies that five warps per
 // scheduler do not cover.
 // LZ false (MGS rounds): a Hermitian-part copy gets -i kappa x added, as
-// k_spmm. LZ true: the kernel also does k_rowpass<AXPY_DOT, true> of the same
-// Lanczos step on the rows it holds, P = H Q_i - beta_{i-1} Q_{i-1} and the
-// sample's alpha_i = Re <Q_i, P>, with the same two-level sums.
+// k_spmm. LZ true: the kernel also does the first projection of the same Lanczos
+// step (k_ortho<1, 1, false, true>) on the rows it holds, P = H Q_i - beta_{i-1}
+// Q_{i-1} and the sum alpha_i = Re <Q_i, P>.
 //
 // Measured: dim 55296, 512 samples, 1.62 ms with the Lanczos projection against
 // 4.60 ms for k_spmm and 0.27 ms for the pass; dim 9216, 64 samples, MGS: 36
@@ -182,12 +182,11 @@ __device__ __forceinline__ void copy16(void* dst, const void* src) {
 // same within 3 %.
 template <bool LZ>
 __global__ void __launch_bounds__(BLK_THREADS, 4)
-    k_spmm_blk(PassArgs a, const int2* __restrict__ items, const uint4* __restrict__ DX) {
+    k_spmm_blk(PassArgs a, AccArgs A, const int2* __restrict__ items, const uint4* __restrict__ DX) {
   __shared__ uint4 s_x[BLK_AHEAD + 1][4][BLK_THREADS];
   __shared__ double2 s_q[LZ ? 4 : 2][BLK_THREADS];
   __shared__ int s_exp[SPC_LANES];
   __shared__ double s_beta[SPC_LANES], s_dot[2][BLK_THREADS];
-  __shared__ bool am_last;
   const int i = a.col_i;
   const int2 it = items[blockIdx.x];
   const TileInfo& T = a.tiles[it.x];
@@ -205,6 +204,7 @@ __global__ void __launch_bounds__(BLK_THREADS, 4)
     s_beta[lane] = LZ && i > 0 ? a.coef[w].x : 0.0;
   }
   s_dot[0][tid] = s_dot[1][tid] = 0.0;
+  if (LZ && it.y == 0) acc_clear(A, it.x, tid, BLK_THREADS);
   __syncthreads();
   const uint4* X = DX + T.p_off + (s0 + g) * 4 + q;
   const uint4* bself = T.bself + lane;
@@ -335,41 +335,17 @@ __global__ void __launch_bounds__(BLK_THREADS, 4)
     }
   }
   if (!LZ) return;
-  // the CTA's sums: sample c = 16 half + 8 h + gs from the four rows and the
-  // warps of its half, in that order
+  // the CTA's sum of sample c = 16 half + 8 h + gs: the four rows and the warps
+  // of its half
   __syncthreads();
-  auto cta_sum = [&](int c) {
+  if (warp == 0 && map[lane] >= 0) {
     double s = 0.0;
 #pragma unroll
     for (int v = 0; v < BLK_IDX; ++v)
 #pragma unroll
-      for (int r = 0; r < 4; ++r) s += s_dot[(c >> 3) & 1][(2 * v + (c >> 4)) * 32 + 8 * r + (c & 7)];
-    return s;
-  };
-  if (warp == 0) a.partial[(size_t)blockIdx.x * SPC_LANES + lane] = make_double2(cta_sum(lane), 0.0);
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) am_last = atomicAdd(&a.counters[it.x], 1u) == (unsigned)T.nib - 1;
-  __syncthreads();
-  if (!am_last) return;
-  __threadfence();
-  const double2* part = a.partial + (size_t)(blockIdx.x - it.y) * SPC_LANES + lane;
-  double s[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int b = warp; b < T.nib; b += 4 * (BLK_THREADS / 32))
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int c = b + u * (BLK_THREADS / 32);
-      if (c < T.nib) s[u] += __ldcg(&part[(size_t)c * SPC_LANES].x);
-    }
-  s_dot[0][tid] = (s[0] + s[1]) + (s[2] + s[3]);
-  __syncthreads();
-  if (warp == 0) {
-    double t = s_dot[0][lane];
-#pragma unroll
-    for (int v = 1; v < BLK_THREADS / 32; ++v) t += s_dot[0][32 * v + lane];
-    if (map[lane] >= 0)
-      pass_finalize<PASS_AXPY_DOT, true>(a, it.x * SPC_LANES + lane, make_double2(t, 0.0), T.kappa);
-    if (lane == 0) a.counters[it.x] = 0u;
+      for (int r = 0; r < 4; ++r) s += s_dot[(lane >> 3) & 1][(2 * v + (lane >> 4)) * 32 + 8 * r + (lane & 7)];
+    acc_t* out = acc_tile(A, A.out, it.x) + lane;
+    acc_add(out, out + ACC_BAD * SPC_LANES, s, acc_dot_exp(T));
   }
 }
 

@@ -371,6 +371,7 @@ int build_h_device(Handle* h, const HostSystem& hs, int mode) {
   h->nnz = nnz;
   h->nnz_cplx = (int64_t)meta.ncplx;
   h->herm_shift = hs.herm_shift;
+  h->rexp = norm_exponent(hs, mode);
   h->blk_one.describe({make_block_sys(hs, mode)});
   return SPC_OK;
 }
@@ -428,7 +429,11 @@ int build_h_batch_device(Handle* h, const std::vector<HostSystem>& hs, int mode)
   rc = build_slices(h, sl, B.nnz, mode);
   B.nnz_cplx.assign(ns, 0);
   std::vector<BlockSys> bs(ns);
-  for (size_t k = 0; k < ns; ++k) bs[k] = make_block_sys(hs[k], mode);
+  B.rexp.assign(ns, 0);
+  for (size_t k = 0; k < ns; ++k) {
+    bs[k] = make_block_sys(hs[k], mode);
+    B.rexp[k] = norm_exponent(hs[k], mode);
+  }
   h->blk_batch.describe(std::move(bs));
   if (!rc && ns) {
     std::vector<HMeta> meta(ns);

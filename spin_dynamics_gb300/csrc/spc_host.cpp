@@ -67,7 +67,7 @@ int Handle::ensure_h_entries(size_t count) {
 Handle::~Handle() {
   Buf* all[] = {&psi, &Q,  &P,    &partial, &counters, &coef, &rbeta, &Ahess, &Aexp, &proj, &projpart,
                 &cvec, &tt, &kk, &done, &map, &obs, &out, &zk, &err, &nbuild, &flag, &xcol, &xval, &xsplit, &plan, &jobtab,
-                &hmeta, &xvs, &xsum, &qmax, &xexp, &blk_one.self, &blk_one.tab, &blk_one.nbr, &blk_one.desc,
+                &hmeta, &xvs, &xsum, &qmax, &xexp, &acc, &gram, &blk_one.self, &blk_one.tab, &blk_one.nbr, &blk_one.desc,
                 &blk_batch.self, &blk_batch.tab, &blk_batch.nbr, &blk_batch.desc, &hb.rowptr, &hb.split, &hb.col, &hb.val, &hb.vsum, &hb.meta, &gck, &gseg, &gnu, &gmu, &glam, &cvec2,
                 &gslots, &gracc, &gfacc, &bcnt, &bnuc, &btot, &btab, &tune_out, &tune_zk};
   for (Buf* b : all)
@@ -264,6 +264,37 @@ int make_host_system(const spc_system* sys, int mode, HostSystem& hs) {
     general_tables(hs);
   }
   return SPC_OK;
+}
+
+int norm_exponent(double bound) {
+  return std::isfinite(bound) && bound > 0.0 ? std::min(400, std::max(-400, std::ilogb(bound) + 2)) : 0;
+}
+
+int norm_exponent(const HostSystem& hs, int mode) {
+  auto l1 = [](double2 v) { return std::fabs(v.x) + std::fabs(v.y); };
+  double rows = 0.0;
+  for (int e = 0; e < 4; ++e) {
+    double r = 0.0;
+    if (mode == SPC_H_REFERENCE) {
+      r = l1(hs.ref.diag[e]) + l1(hs.ref.flip_ab) + l1(hs.ref.flip_ba);
+      for (const NucInfo& q : hs.nuc) r += std::fabs(q.a_iso) * q.g * q.g + std::fabs(q.zf) * q.g;
+    } else {
+      for (int f = 0; f < 4; ++f) r += l1(hs.gen.H[e][f]);
+      for (const NucInfo& q : hs.nuc) {
+        double best = 0.0;
+        for (int m = 0; m < q.g; ++m) {
+          double t = 0.0;
+          for (int f = 0; f < 4; ++f)
+            for (int d = 0; d < 3; ++d) t += l1(hs.gen_tab[q.tab_off + ((size_t)(e * 4 + f) * q.g + m) * 3 + d]);
+          best = std::max(best, t);
+        }
+        r += best;
+      }
+    }
+    rows = std::max(rows, r);
+    if (!(r <= rows)) rows = r;  // NaN
+  }
+  return norm_exponent(rows);
 }
 
 BlockSys make_block_sys(const HostSystem& hs, int mode) {

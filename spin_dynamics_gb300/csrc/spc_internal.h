@@ -112,6 +112,9 @@ struct BlockSys {
   int64_t self_off = 0, tab_off = 0, nbr_off = 0;  // place in the store, once built
 };
 BlockSys make_block_sys(const HostSystem& hs, int mode);
+// An exponent with ||H|| <= 2^e, from the rows' absolute sums (|H| is symmetric).
+int norm_exponent(const HostSystem& hs, int mode);
+int norm_exponent(double bound);
 
 struct Handle {
   Prof prof;
@@ -142,6 +145,8 @@ struct Handle {
   // exponent of the current Krylov vector of every slot, and its maximum while
   // a pass forms it
   Buf xexp;
+  // integer accumulators of the orthogonalisation sums, and products of basis vectors (spc_ortho.cuh)
+  Buf acc, gram;
   // Hamiltonian build scratch: row counts, nucleus tables, nonzero totals
   Buf bcnt, bnuc, btot, btab;
   // autotuner outputs and sample subsets
@@ -155,6 +160,7 @@ struct Handle {
     std::vector<int64_t> nnz, rp_off, nz_off;
     std::vector<char> herm;
     std::vector<int64_t> nnz_cplx;
+    std::vector<int> rexp;
     Buf rowptr, split, col, val, vsum, meta;  // meta: one HMeta per system; vsum: Re + Im per entry
   } hb;
   // Digit fragments of a general-builder Hamiltonian's 4 x 4 blocks for the
@@ -179,6 +185,8 @@ struct Handle {
   // one-CTA-per-sample kernel for small systems: 0 when it pays, 1 never,
   // 2 whenever the call fits it
   int sample_path = 0;
+  // ||H|| <= 2^rexp for the current Hamiltonian (its basis vectors' rounding included)
+  int rexp = 0;
   // H_eff = (Hermitian) - i*kappa*1 for the current Hamiltonian: Lanczos applies
   bool herm_shift = false;
   bool lanczos_active() const {
@@ -216,6 +224,7 @@ struct JobSpec {
   const double* kappa = nullptr;
   int64_t nnz_cplx = 0;  // entries of the execution copy with a nonzero imaginary part
   int sys = 0;           // the job's entry of the block store
+  int rexp = 0;          // ||H|| <= 2^rexp
 };
 
 // One reduced-matrix slot of the yield gradient: the electron pair (G = 4,

@@ -1,0 +1,325 @@
+// Orthogonalisation passes of the Krylov basis (get_krylov,
+// src/qm_dynamics.f90:445-465). Included by spc_propagate.cu inside namespace
+// spc.
+//
+// Sums over a tile's rows. GB300 adds two doubles per clock and SM, so a last
+// CTA that adds the partial sums of several hundred others (32 samples each)
+// takes 10 us and more. Here every CTA adds its sums to per-sample integers
+// with 64-bit atomics: a double is an integer multiple of 2^(e - 110), e the
+// exponent of a bound on the sum, held as two words (the bits from 2^50 up,
+// the 50 below) that no carry couples. Integer sums do not depend on their
+// order, so results repeat bit for bit, and their only rounding is the last
+// one. The kernel that needs a sum reads it in its prologue. Three sets of
+// accumulators rotate: a kernel adds to one, reads the one before and clears
+// the one after.
+#define ACC_VECS 15             // complex sums per sample (8 dots + 7 basis products)
+#define ACC_MAX (4 * ACC_VECS)  // largest component's high word
+#define ACC_BAD (4 * ACC_VECS + 1)
+#define ACC_ROWS 64
+typedef unsigned long long acc_t;
+
+struct AccArgs {
+  acc_t* acc;  // [3][tiles][ACC_ROWS][32]
+  int ntiles, in, out, clear;
+};
+__device__ __forceinline__ acc_t* acc_tile(const AccArgs& A, int set, int tile) {
+  return A.acc + ((size_t)set * A.ntiles + tile) * ACC_ROWS * SPC_LANES;
+}
+// x to the accumulator pair at p (stride 32), |sum| <= 2^e; NaN, infinities and
+// values past the bound mark the sample
+__device__ __forceinline__ void acc_add(acc_t* p, acc_t* bad, double x, int e) {
+  const long long b = __double_as_longlong(x);
+  const int ex = (int)(b >> 52) & 0x7ff;
+  if (ex == 0) return;
+  if (ex - 1023 > e + 1) {
+    *bad = 1;
+    return;
+  }
+  const acc_t man = (b & 0xfffffffffffffll) | (1ull << 52);
+  const int sh = ex - 965 - e;  // <= 59
+  acc_t lo, hi;                 // man * 2^sh as hi 2^50 + lo
+  if (sh >= 0) {
+    lo = (man << sh) & ((1ull << 50) - 1);
+    hi = sh >= 50 ? man << (sh - 50) : man >> (50 - sh);
+  } else {
+    const acc_t v = sh < -62 ? 0 : ((man >> (-sh - 1)) + 1) >> 1;
+    lo = v & ((1ull << 50) - 1);
+    hi = v >> 50;
+  }
+  if (b < 0) {
+    lo = 0 - lo;
+    hi = 0 - hi;
+  }
+  atomicAdd(p, hi);
+  atomicAdd(p + SPC_LANES, lo);
+}
+__device__ __forceinline__ double acc_get(const acc_t* p, int e) {
+  return ldexp(fma((double)(long long)p[0], 1125899906842624.0, (double)(long long)p[SPC_LANES]), e - 110);
+}
+__device__ __forceinline__ void acc_clear(const AccArgs& A, int tile, int tid, int nth) {
+  acc_t* p = acc_tile(A, A.clear, tile);
+  for (int k = tid; k < ACC_ROWS * SPC_LANES; k += nth) p[k] = 0;
+}
+// exponents of the bounds: dots of a basis vector with p, p's square norm,
+// products of two basis vectors
+__device__ __forceinline__ int acc_dot_exp(const TileInfo& T) { return T.rexp; }
+__device__ __forceinline__ int acc_norm_exp(const TileInfo& T) { return 2 * T.rexp; }
+#define ACC_GRAM_EXP 4
+
+struct OrthoArgs {
+  PassArgs p;
+  AccArgs a;
+  int ja, jd;      // first vector to subtract, first to project on
+  double2* gram;   // [tile][basis vector][8][32]: <Q_j, Q_k> of the vectors k < j of j's block
+};
+#define ORTHO_NB 8
+
+// One pass over the rows of a work item: p -= sum_{v < NA} h_v Q_{ja+v}, then
+// ND > 0: the sums <Q_{jd+v}, p>, v < ND;  ND = 0: ||p||^2 and p's largest
+// component. Modified Gram-Schmidt projects on the basis in blocks of
+// ORTHO_NB: with d_v = <Q_v, p> on the p that enters the block,
+//   h_v = <Q_v, p - sum_{k < v} h_k Q_k> = d_v - sum_{k < v} <Q_v, Q_k> h_k,
+// the coefficient of the one-vector pass in exact arithmetic (as the blocked
+// forms of Swirydowicz, Langou, Ananthan, Yang and Thomas, "Low synchronization
+// Gram-Schmidt and generalized minimal residual algorithms", Numer. Linear
+// Algebra Appl. 28 (2021), e2343). The products of basis vectors are formed once,
+// by the pass that first projects on the newer one (GRAM: Q_{jd+ND-1} is new).
+// What bounds it: FP64 issue, 8 FMAs per vector and row as the one-vector pass;
+// that pass took a launch, a read and a write of p and a serial last sum for each
+// vector. Per Krylov step at m = 24, dim 9216, 64 samples (MGS): 12.5 passes of
+// 29 us before, 3 of 31-82 us now; dim 55296, 32 samples, m = 30: 56.5 -> 27 ms a
+// build. Blocks of eight: the newest block's pass holds 15 complex sums and 8
+// vectors in 126 registers. Lanczos at dim 2304, 77 samples: the norm pass 15.3
+// -> 10.1 us, k_spmm_blk with its projection 27.9 -> 19.5 us without the last sum.
+// REAL: Lanczos on the Hermitian part; NA = 1 with ND = 1 takes beta_{i-1}
+// (coef), with ND = 0 alpha_i.
+template <int NA, int ND, bool GRAM, bool REAL>
+__global__ void __launch_bounds__(256, 2) k_ortho(OrthoArgs o) {
+  constexpr int NG = GRAM && ND > 1 ? ND - 1 : 0, NS = ND + NG;
+  constexpr int NR = ND == 0 ? 1 : (NS < 4 ? NS : 4);  // sums reduced at a time
+  __shared__ double2 h[NA > 0 ? NA : 1][SPC_LANES];
+  __shared__ double2 red[NR][SPC_WARPS][SPC_LANES];
+  __shared__ unsigned mx[SPC_WARPS][SPC_LANES];
+  const PassArgs& a = o.p;
+  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
+  const int2 it = a.items[blockIdx.x];
+  const TileInfo& T = a.tiles[it.x];
+  const int i = a.col_i;
+  if (i >= T.m) return;  // past this job's Krylov dimension
+  const int w = it.x * SPC_LANES + tx;
+  const bool act = a.map[w] >= 0;
+  const bool first = it.y == 0;  // the CTA that records the tile's coefficients
+  // the last column ends with its coefficients: no next vector
+  const bool tail = ND == 0 && i == T.m - 1;
+  if (tail && !first) return;
+  if (first) acc_clear(o.a, it.x, tid, 256);
+  if (NA > 0) {
+    const size_t mm = (size_t)a.m * a.m;
+    const acc_t* in = acc_tile(o.a, o.a.in, it.x) + tx;
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
+    if (REAL) {
+      if (ty == 0) {
+        double c;
+        if (ND == 1) {
+          c = act ? a.coef[w].x : 0.0;
+        } else {
+          c = in[ACC_BAD * SPC_LANES] ? nan : acc_get(in, acc_dot_exp(T));
+          if (first && act)
+            a.Ahess[(size_t)w * mm + i + (size_t)i * a.m] = make_double2(c, -*T.kappa);
+        }
+        h[0][tx] = make_double2(c, 0.0);
+      }
+      __syncthreads();
+    } else {
+      // d_v by warp v, then the corrections; the last block's newest vector has
+      // its basis products in the accumulators
+      const bool last = o.ja + NA == i + 1;
+      const int jv = o.ja + ty;
+      double2 d = cz();
+      float2 gk[ORTHO_NB - 1];
+      bool big = false;
+      double2* G = o.gram + ((size_t)it.x * a.m + jv) * ORTHO_NB * SPC_LANES + tx;
+      if (ty < NA) {
+        d = make_double2(acc_get(in + 4 * ty * SPC_LANES, acc_dot_exp(T)),
+                         acc_get(in + (4 * ty + 2) * SPC_LANES, acc_dot_exp(T)));
+        if (in[ACC_BAD * SPC_LANES]) d = make_double2(nan, nan);
+        h[ty][tx] = d;
+#pragma unroll
+        for (int k = 0; k < NA - 1; ++k) {
+          gk[k] = make_float2(0.f, 0.f);
+          if (k < ty) {
+            double2 gv;
+            if (last && ty == NA - 1) {
+              // <Q_k, Q_new>, stored as <Q_new, Q_k>
+              gv = make_double2(acc_get(in + 4 * (NA + k) * SPC_LANES, ACC_GRAM_EXP),
+                                -acc_get(in + (4 * (NA + k) + 2) * SPC_LANES, ACC_GRAM_EXP));
+              if (first) G[k * SPC_LANES] = gv;
+            } else {
+              gv = G[k * SPC_LANES];
+            }
+            gk[k] = make_float2((float)gv.x, (float)gv.y);
+            big |= act && !(fabsf(gk[k].x) + fabsf(gk[k].y) < 1e-8f);
+          }
+        }
+      }
+      // an orthonormal basis (products of rounding size): the corrections are
+      // below 1e-8 of the coefficients, first order and single precision leave
+      // an error below 1e-15 of them. A basis past a breakdown takes the
+      // recurrence in full.
+      if (!__syncthreads_or(big ? 1 : 0)) {
+        float2 c = make_float2(0.f, 0.f);
+        if (ty < NA) {
+#pragma unroll
+          for (int k = 0; k < NA - 1; ++k) {
+            const float hx = (float)h[k][tx].x, hy = (float)h[k][tx].y;
+            c.x += gk[k].x * hx - gk[k].y * hy;
+            c.y += gk[k].x * hy + gk[k].y * hx;
+          }
+          d = make_double2(d.x - (double)c.x, d.y - (double)c.y);
+        }
+        __syncthreads();
+        if (ty < NA) h[ty][tx] = d;
+      } else {
+        for (int k = 0; k + 1 < NA; ++k) {
+          __syncthreads();  // h_k is final
+          if (ty > k && ty < NA) {
+            double2 gv;
+            if (last && ty == NA - 1)
+              gv = make_double2(acc_get(in + 4 * (NA + k) * SPC_LANES, ACC_GRAM_EXP),
+                                -acc_get(in + (4 * (NA + k) + 2) * SPC_LANES, ACC_GRAM_EXP));
+            else
+              gv = G[k * SPC_LANES];
+            d = cfms(gv, h[k][tx], d);
+            h[ty][tx] = d;
+          }
+        }
+      }
+      if (first && act && ty < NA) a.Ahess[(size_t)w * mm + jv + (size_t)i * a.m] = d;
+      __syncthreads();
+    }
+  }
+  if (tail) return;
+  const int n = act ? T.n : 0;
+  const int stride = T.nio * SPC_WARPS;
+  const size_t vs = (size_t)T.n * SPC_LANES;
+  const double2* Qa = a.Q + T.q_off + (size_t)o.ja * vs + tx;
+  const double2* Qd = a.Q + T.q_off + (size_t)o.jd * vs + tx;
+  double2* P = a.P + T.p_off + tx;
+  double2 acc[NS > 0 ? NS : 1];
+#pragma unroll
+  for (int v = 0; v < (NS > 0 ? NS : 1); ++v) acc[v] = cz();
+  unsigned top = 0;
+  for (int r = it.y * SPC_WARPS + ty; r < n; r += stride) {
+    const size_t off = (size_t)r * SPC_LANES;
+    double2 p = P[off];
+    double2 qd[ND > 0 ? ND : 1];
+#pragma unroll
+    for (int v = 0; v < ND; ++v) qd[v] = Qd[v * vs + off];
+    if (NA > 0) {
+#pragma unroll
+      for (int v = 0; v < NA; ++v) {
+        const double2 q = Qa[v * vs + off];
+        if (REAL) {
+          const double c = h[v][tx].x;
+          p.x = fma(-c, q.x, p.x);
+          p.y = fma(-c, q.y, p.y);
+        } else {
+          p = cfms(h[v][tx], q, p);
+        }
+      }
+      P[off] = p;
+    }
+    if (ND == 0) {
+      acc[0].x = fma(p.x, p.x, acc[0].x);
+      acc[0].x = fma(p.y, p.y, acc[0].x);
+      top = max(top, abs_high(p));
+    }
+#pragma unroll
+    for (int v = 0; v < ND; ++v) {
+      if (REAL) {
+        acc[v].x = fma(qd[v].x, p.x, acc[v].x);
+        acc[v].x = fma(qd[v].y, p.y, acc[v].x);
+      } else {
+        acc[v] = cjfma(qd[v], p, acc[v]);
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < NG; ++v) acc[ND + v] = cjfma(qd[v], qd[ND > 0 ? ND - 1 : 0], acc[ND + v]);
+  }
+  // the CTA's sums over its warps, then to the accumulators: warp y takes sum
+  // y / 2's real or imaginary part
+  acc_t* out = acc_tile(o.a, o.a.out, it.x) + tx;
+#pragma unroll
+  for (int v0 = 0; v0 < (ND == 0 ? 1 : NS); v0 += NR) {
+    if (v0 > 0) __syncthreads();
+#pragma unroll
+    for (int u = 0; u < NR; ++u)
+      if (v0 + u < (ND == 0 ? 1 : NS)) red[u][ty][tx] = acc[v0 + u];
+    if (ND == 0) mx[ty][tx] = top;
+    __syncthreads();
+    const int u = ty >> 1, im = ty & 1, v = v0 + u;
+    if (act && u < NR && v < (ND == 0 ? 1 : NS) && !(im && (REAL || ND == 0))) {
+      double s = im ? red[u][0][tx].y : red[u][0][tx].x;
+#pragma unroll
+      for (int y = 1; y < SPC_WARPS; ++y) s += im ? red[u][y][tx].y : red[u][y][tx].x;
+      const int e = ND == 0 ? acc_norm_exp(T) : (v < ND ? acc_dot_exp(T) : ACC_GRAM_EXP);
+      acc_add(out + (4 * v + 2 * im) * SPC_LANES, out + ACC_BAD * SPC_LANES, s, e);
+      if (ND == 0) {
+#pragma unroll
+        for (int y = 1; y < SPC_WARPS; ++y) top = max(top, mx[y][tx]);
+        atomicMax(out + ACC_MAX * SPC_LANES, (acc_t)top);
+      }
+    }
+  }
+}
+
+// After the norm pass: 1/||p||, the exponent bound of p/||p|| and, recorded by
+// the tile's first CTA, the Hessenberg's subdiagonal, the next Lanczos
+// coefficient, the exponent and the basis' maximum. Called by 32 lanes.
+__device__ __forceinline__ double ortho_norm(const PassArgs& a, const AccArgs& A, const TileInfo& T, int tile, int lane,
+                                             bool record, int* ex) {
+  const int w = tile * SPC_LANES + lane;
+  const acc_t* in = acc_tile(A, A.in, tile) + lane;
+  double b = sqrt(acc_get(in, acc_norm_exp(T)));
+  if (in[ACC_BAD * SPC_LANES]) b = __longlong_as_double(0x7ff8000000000000ll);
+  // exact breakdown (p == 0): the next basis vector is 0 instead of 0/0
+  const double rb = b > 0.0 ? 1.0 / b : (b == 0.0 ? 0.0 : b);
+  const unsigned top = (unsigned)in[ACC_MAX * SPC_LANES];
+  const double q = top == 0u ? 0.0 : __hiloint2double((int)(top + 1u), 0) * rb;
+  const unsigned hq = (unsigned)__double2hiint(q) & 0x7fffffffu;
+  *ex = (int)(hq >> 20);
+  if (record && a.map[w] >= 0) {
+    const size_t mm = (size_t)a.m * a.m;
+    const int i = a.col_i;
+    a.Ahess[(size_t)w * mm + (i + 1) + (size_t)i * a.m] = make_double2(b, 0.0);
+    if (a.lanczos) {
+      // Hermitian tridiagonal: A(i, i+1) = beta_i, the coefficient of Q_i in
+      // the next step's three-term recurrence
+      a.Ahess[(size_t)w * mm + i + (size_t)(i + 1) * a.m] = make_double2(b, 0.0);
+      a.coef[w] = make_double2(b, 0.0);
+    }
+    a.xexp[w] = *ex;
+    a.qmax[w] = max(a.qmax[w], hq);
+  }
+  return rb;
+}
+
+typedef void (*OrthoFn)(OrthoArgs);
+// The pass of a block: `nd` dots after subtracting nothing or a full block (nd
+// = 8 on an older block; the newest block also forms its basis products), or
+// the norm after the last block's `na` vectors.
+static OrthoFn ortho_fn(int na, int nd, bool newest) {
+  static const OrthoFn old[2] = {k_ortho<0, 8, false, false>, k_ortho<8, 8, false, false>};
+  static const OrthoFn lone[8] = {k_ortho<0, 1, true, false>, k_ortho<0, 2, true, false>, k_ortho<0, 3, true, false>,
+                                  k_ortho<0, 4, true, false>, k_ortho<0, 5, true, false>, k_ortho<0, 6, true, false>,
+                                  k_ortho<0, 7, true, false>, k_ortho<0, 8, true, false>};
+  static const OrthoFn next[8] = {k_ortho<8, 1, true, false>, k_ortho<8, 2, true, false>, k_ortho<8, 3, true, false>,
+                                  k_ortho<8, 4, true, false>, k_ortho<8, 5, true, false>, k_ortho<8, 6, true, false>,
+                                  k_ortho<8, 7, true, false>, k_ortho<8, 8, true, false>};
+  static const OrthoFn norm[8] = {k_ortho<1, 0, false, false>, k_ortho<2, 0, false, false>, k_ortho<3, 0, false, false>,
+                                  k_ortho<4, 0, false, false>, k_ortho<5, 0, false, false>, k_ortho<6, 0, false, false>,
+                                  k_ortho<7, 0, false, false>, k_ortho<8, 0, false, false>};
+  if (nd == 0) return norm[na - 1];
+  if (!newest) return old[na > 0];
+  return na > 0 ? next[nd - 1] : lone[nd - 1];
+}

@@ -70,31 +70,29 @@ struct TileInfo {
   const uint4* btab;
   const int2* bnbr;
   int bk, bexp, nib;
+  int nio, rexp;  // items of the orthogonalisation passes; exponent bound of ||H||
 };
-
-enum PassKind { PASS_NORM_GATHER = 0, PASS_DOT = 1, PASS_AXPY_DOT = 2, PASS_AXPY_NORM = 3 };
 
 struct PassArgs {
   const TileInfo* tiles;
   const int2* items;  // pass items (tile, phase)
-  int m, col_i, row_j;
+  int m, col_i;
   int shift;          // k_spmm_blk: add -i kappa x where the copy holds the Hermitian part
-  int lanczos;        // AXPY_NORM also seeds the next Lanczos coefficient
-  int jx, jn;         // basis indices: DOT reads Q_jx; AXPY removes Q_jx, dots with Q_jn
+  int lanczos;        // the norm pass also records the next Lanczos coefficient
   const double2* Q;
   double2* P;
   const double2* psi;
   const int* map;     // slot -> global sample (or -1)
   const int* scol;    // slot -> column in its job's psi
-  double2* coef;      // current MGS coefficient per slot
-  double* rbeta;      // 1/norm per slot
+  double2* coef;      // current Lanczos coefficient beta per slot
+  double* rbeta;      // 1/||psi|| per slot
   double2* Ahess;     // Hessenberg matrices, m x m column-major per slot
   double2* cvec;      // Krylov coordinates per slot
   double2* partial;   // [items][32]
   unsigned* counters; // per tile
-  unsigned* pmax;     // per slot: high word of P's (psi's) largest component (norm passes; zero between them)
-  int* xexp;          // per slot: biased exponent bound of the vector that the norm is for
-  unsigned* qmax;     // per slot: largest such high word of the basis
+  unsigned* pmax;     // per slot: high word of psi's largest component (k_norm; zero between its launches)
+  int* xexp;          // per slot: biased exponent bound of the current basis vector
+  unsigned* qmax;     // per slot: high word bounding the basis' largest component
 };
 
 // High word of the larger of |re|, |im|: its integer order is the order of
@@ -103,196 +101,112 @@ __device__ __forceinline__ unsigned abs_high(double2 q) {
   return max((unsigned)__double2hiint(q.x) & 0x7fffffffu, (unsigned)__double2hiint(q.y) & 0x7fffffffu);
 }
 
-// After a norm pass: a bound of the scaled vector's largest component (the
-// maximum's high word rounded up, times 1/norm as k_scale forms it), its
-// exponent for the digits of k_spmm_blk and the basis' maximum for k_gram.
-__device__ __forceinline__ void pass_exponent(const PassArgs& a, int w) {
-  const unsigned top = __ldcg(a.pmax + w);
-  a.pmax[w] = 0u;
-  const double q = top == 0u ? 0.0 : __hiloint2double((int)(top + 1u), 0) * a.rbeta[w];
-  const unsigned hq = (unsigned)__double2hiint(q) & 0x7fffffffu;
-  a.xexp[w] = (int)(hq >> 20);
-  a.qmax[w] = max(a.qmax[w], hq);
-}
-
-// REAL: the Hermitian Lanczos recurrence on A of H_eff = A - i*kappa*1
-// (tile's kappa non-null): every coefficient is real, the dots keep their real
-// part, and the tridiagonal's diagonal gets the shift: alpha - i*kappa.
-template <int KIND, bool REAL>
-__device__ __forceinline__ void pass_finalize(const PassArgs& a, int w, double2 tot, const double* kappa) {
-  const size_t mm = (size_t)a.m * a.m;
-  if (KIND == PASS_NORM_GATHER) {
-    double b = sqrt(tot.x);
-    double2* c = a.cvec + (size_t)w * a.m;
-    c[0] = make_double2(b, 0.0);
-    for (int j = 1; j < a.m; ++j) c[j] = cz();
-    a.rbeta[w] = b > 0.0 ? 1.0 / b : 0.0;
-    pass_exponent(a, w);
-  } else if (KIND == PASS_DOT || KIND == PASS_AXPY_DOT) {
-    if (REAL) {
-      a.coef[w] = make_double2(tot.x, 0.0);
-      a.Ahess[(size_t)w * mm + a.row_j + (size_t)a.col_i * a.m] = make_double2(tot.x, -*kappa);
-    } else {
-      a.coef[w] = tot;
-      a.Ahess[(size_t)w * mm + a.row_j + (size_t)a.col_i * a.m] = tot;
-    }
-  } else {  // PASS_AXPY_NORM: A(i+1, i) = ||p||, and 1/||p|| for the scale
-    double b = sqrt(tot.x);
-    a.Ahess[(size_t)w * mm + a.row_j + (size_t)a.col_i * a.m] = make_double2(b, 0.0);
-    // exact breakdown (p == 0): the next basis vector is 0 instead of 0/0
-    a.rbeta[w] = b > 0.0 ? 1.0 / b : 0.0;
-    pass_exponent(a, w);
-    if (a.lanczos) {
-      // Hermitian tridiagonal: A(i, i+1) = beta_i, the coefficient of Q_i
-      // in the next step's three-term recurrence
-      a.Ahess[(size_t)w * mm + a.col_i + (size_t)a.row_j * a.m] = make_double2(b, 0.0);
-      a.coef[w] = make_double2(b, 0.0);
-    }
-  }
-}
-
-// One pass over the rows of a work item: element update + per-slot
-// reduction. Grid = pass items, block (32, SPC_WARPS). REAL (Lanczos on the
-// Hermitian part): real coefficients (2 DFMA per axpy) and real dots.
-template <int KIND, bool REAL = false>
-__global__ void __launch_bounds__(256) k_rowpass(PassArgs a) {
-  __shared__ double2 red[SPC_WARPS][SPC_LANES];
+// c = ||psi|| e_1 (get_krylov :440-447), 1/||psi|| and an exponent bound of
+// psi / ||psi||: the largest component's high word rounded up, times 1/||psi||
+// as k_scale forms it. Grid = pass items, block (32, SPC_WARPS). psi has any
+// norm, so its sum is a double's, by the last CTA of the tile.
+__global__ void __launch_bounds__(256) k_norm(PassArgs a) {
+  __shared__ double red[SPC_WARPS][SPC_LANES];
   __shared__ unsigned mx[SPC_WARPS][SPC_LANES];
   __shared__ bool am_last;
-  constexpr bool NORM = KIND == PASS_NORM_GATHER || KIND == PASS_AXPY_NORM;
-  unsigned top = 0;
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int2 it = a.items[blockIdx.x];
   const TileInfo& T = a.tiles[it.x];
-  // steps past this job's Krylov dimension (whole tile, so whole CTA)
-  if (KIND != PASS_NORM_GATHER && (a.col_i >= T.m || (KIND == PASS_AXPY_NORM && a.col_i >= T.m - 1)))
-    return;
   const int w = it.x * SPC_LANES + tx;
   const bool act = a.map[w] >= 0;
-  const int n = T.n;
+  const int n = act ? T.n : 0;
   const int stride = T.nip * SPC_WARPS;
-  const size_t vs = (size_t)n * SPC_LANES;
-  double2 acc = cz();
-  if (act) {
-    if (KIND == PASS_NORM_GATHER) {
-      const double2* src = a.psi + T.psi_off + a.scol[w];
-      for (int r = it.y * SPC_WARPS + ty; r < n; r += stride) {
-        double2 x = src[(size_t)r * T.ldp];
-        acc.x = fma(x.x, x.x, acc.x);
-        acc.x = fma(x.y, x.y, acc.x);
-        top = max(top, abs_high(x));
-      }
-    } else if (KIND == PASS_DOT) {
-      const double2* X = a.Q + T.q_off + a.jx * vs + tx;
-      const double2* P = a.P + T.p_off + tx;
-      for (int r = it.y * SPC_WARPS + ty; r < n; r += stride) {
-        const size_t o = (size_t)r * SPC_LANES;
-        if (REAL) {
-          const double2 x = X[o], p = P[o];
-          acc.x = fma(x.x, p.x, acc.x);
-          acc.x = fma(x.y, p.y, acc.x);
-        } else {
-          acc = cjfma(X[o], P[o], acc);
-        }
-      }
-    } else {
-      const double2 cf = a.coef[w];
-      const double2* Qj = a.Q + T.q_off + a.jx * vs + tx;
-      const double2* Qn = a.Q + T.q_off + a.jn * vs + tx;
-      double2* P = a.P + T.p_off + tx;
-      for (int r = it.y * SPC_WARPS + ty; r < n; r += stride) {
-        const size_t o = (size_t)r * SPC_LANES;
-        double2 p;
-        if (REAL) {
-          const double2 q = Qj[o], p0 = P[o];
-          p.x = fma(-cf.x, q.x, p0.x);
-          p.y = fma(-cf.x, q.y, p0.y);
-        } else {
-          p = cfms(cf, Qj[o], P[o]);
-        }
-        P[o] = p;
-        if (KIND == PASS_AXPY_DOT) {
-          if (REAL) {
-            const double2 q = Qn[o];
-            acc.x = fma(q.x, p.x, acc.x);
-            acc.x = fma(q.y, p.y, acc.x);
-          } else {
-            acc = cjfma(Qn[o], p, acc);
-          }
-        } else {
-          acc.x = fma(p.x, p.x, acc.x);
-          acc.x = fma(p.y, p.y, acc.x);
-          top = max(top, abs_high(p));
-        }
-      }
-    }
+  double acc = 0.0;
+  unsigned top = 0;
+  const double2* src = a.psi + T.psi_off + (act ? a.scol[w] : 0);
+  for (int r = it.y * SPC_WARPS + ty; r < n; r += stride) {
+    const double2 x = src[(size_t)r * T.ldp];
+    acc = fma(x.x, x.x, acc);
+    acc = fma(x.y, x.y, acc);
+    top = max(top, abs_high(x));
   }
   red[ty][tx] = acc;
-  if (NORM) mx[ty][tx] = top;
+  mx[ty][tx] = top;
   __syncthreads();
   if (ty == 0) {
-    double2 s = red[0][tx];
+    double s = red[0][tx];
 #pragma unroll
-    for (int y = 1; y < SPC_WARPS; ++y) s = cadd(s, red[y][tx]);
-    a.partial[(size_t)blockIdx.x * SPC_LANES + tx] = s;
-    if (NORM && act) {
-#pragma unroll
-      for (int y = 1; y < SPC_WARPS; ++y) top = max(top, mx[y][tx]);
-      atomicMax(a.pmax + w, top);
+    for (int y = 1; y < SPC_WARPS; ++y) {
+      s += red[y][tx];
+      top = max(top, mx[y][tx]);
     }
+    a.partial[(size_t)blockIdx.x * SPC_LANES + tx] = make_double2(s, 0.0);
+    if (act) atomicMax(a.pmax + w, top);
   }
   __threadfence();
   __syncthreads();
-  if (tx == 0 && ty == 0) {
-    unsigned t = atomicAdd(&a.counters[it.x], 1u);
-    am_last = (t == (unsigned)T.nip - 1);
-  }
+  if (tx == 0 && ty == 0) am_last = atomicAdd(&a.counters[it.x], 1u) == (unsigned)T.nip - 1;
   __syncthreads();
   if (!am_last) return;
   __threadfence();
-  double2 s = cz();
-  for (int b = ty; b < T.nip; b += SPC_WARPS)
-    s = cadd(s, __ldcg(&a.partial[(size_t)(T.ip0 + b) * SPC_LANES + tx]));
+  double s = 0.0;
+  for (int b = ty; b < T.nip; b += SPC_WARPS) s += __ldcg(&a.partial[(size_t)(T.ip0 + b) * SPC_LANES + tx].x);
   red[ty][tx] = s;
   __syncthreads();
   if (ty == 0) {
-    double2 tot = red[0][tx];
+    double tot = red[0][tx];
 #pragma unroll
-    for (int y = 1; y < SPC_WARPS; ++y) tot = cadd(tot, red[y][tx]);
-    if (act) pass_finalize<KIND, REAL>(a, w, tot, T.kappa);
+    for (int y = 1; y < SPC_WARPS; ++y) tot += red[y][tx];
+    if (act) {
+      const double b = sqrt(tot);
+      double2* c = a.cvec + (size_t)w * a.m;
+      c[0] = make_double2(b, 0.0);
+      for (int j = 1; j < a.m; ++j) c[j] = cz();
+      const double rb = b > 0.0 ? 1.0 / b : 0.0;
+      a.rbeta[w] = rb;
+      const unsigned hi = __ldcg(a.pmax + w);
+      a.pmax[w] = 0u;
+      const double q = hi == 0u ? 0.0 : __hiloint2double((int)(hi + 1u), 0) * rb;
+      const unsigned hq = (unsigned)__double2hiint(q) & 0x7fffffffu;
+      a.xexp[w] = (int)(hq >> 20);
+      a.qmax[w] = max(a.qmax[w], hq);
+    }
     if (tx == 0) a.counters[it.x] = 0u;
   }
 }
 
+#include "spc_ortho.cuh"
 #include "spc_digits.cuh"
 #include "spc_blocks.cuh"
 
-// Q_{jd} = P / ||P||  (or Q_0 = psi[:, scol] / ||psi|| when gather != 0),
+// Q_{jd} = P / ||P||  (Q_0 = psi[:, scol] / ||psi||),
 // and beside it the operand of the next SpMM: with DIG the packed digits of
 // Q_{jd} that k_spmm_blk reads, [n][32][4] (a thread takes the four electron
 // rows of a nuclear index and writes 64 bytes), else the plane Re + Im of
 // k_spmm's three-product form in P's layout (p_off); grid = pass items.
+// Q_0 takes the norm that k_norm left, Q_{jd > 0} the accumulated one.
 template <bool DIG>
-__global__ void __launch_bounds__(256)
-    k_scale(const TileInfo* __restrict__ tiles, const int2* __restrict__ items,
-            const int* __restrict__ map, const int* __restrict__ scol,
-            const double2* __restrict__ psi, const double2* __restrict__ P, int gather, int jd,
-            const double* __restrict__ rbeta, const int* __restrict__ xexp, double2* __restrict__ Q,
-            void* __restrict__ XS) {
-  const int2 it = items[blockIdx.x];
-  const TileInfo& T = tiles[it.x];
-  if (!gather && jd >= T.m) return;
+__global__ void __launch_bounds__(256) k_scale(PassArgs a, AccArgs A, int jd, void* __restrict__ XS) {
+  __shared__ double s_rb[SPC_LANES];
+  __shared__ int s_ex[SPC_LANES];
+  const int2 it = a.items[blockIdx.x];
+  const TileInfo& T = a.tiles[it.x];
+  if (jd >= T.m) return;
   const int tx = threadIdx.x;
   const int w = it.x * SPC_LANES + tx;
-  if (map[w] < 0) return;
-  const double rb = rbeta[w];
+  if (threadIdx.y == 0) {
+    if (jd == 0) {
+      s_rb[tx] = a.rbeta[w];
+      s_ex[tx] = a.xexp[w];
+    } else {
+      s_rb[tx] = ortho_norm(a, A, T, it.x, tx, it.y == 0, &s_ex[tx]);
+    }
+  }
+  __syncthreads();
+  if (a.map[w] < 0) return;
+  const double rb = s_rb[tx];
   const int n = T.n;
   const int stride = T.nip * SPC_WARPS;
-  double2* dst = Q + T.q_off + (size_t)jd * n * SPC_LANES + tx;
-  const double2* src = gather ? psi + T.psi_off + scol[w] : P + T.p_off + tx;
-  const size_t ld = gather ? T.ldp : SPC_LANES;
+  double2* dst = const_cast<double2*>(a.Q) + T.q_off + (size_t)jd * n * SPC_LANES + tx;
+  const double2* src = jd == 0 ? a.psi + T.psi_off + a.scol[w] : a.P + T.p_off + tx;
+  const size_t ld = jd == 0 ? T.ldp : SPC_LANES;
   if (DIG) {
-    const int ex = xexp[w], Z = n / 4;
+    const int ex = s_ex[tx], Z = n / 4;
     uint4* dx = (uint4*)XS + T.p_off + tx * 4;
     for (int k = it.y * SPC_WARPS + threadIdx.y; k < Z; k += stride) {
       double2 x[4];
@@ -1403,15 +1317,20 @@ static void plan_items(const std::vector<int>& tile_n, int resident, std::vector
 // One Krylov basis per slot (get_krylov): what a round's launches need.
 struct BasisRun {
   const TileInfo* tiles;  // device
-  const int2 *items_p, *items_s, *items_b;
-  int nip, nis, nib;       // nib: 0 for k_spmm on the CSR, else k_spmm_blk's items
+  const int2 *items_p, *items_s, *items_b, *items_o;
+  int nip, nis, nib, nio;  // nib: 0 for k_spmm on the CSR, else k_spmm_blk's items
   PassArgs pa;
+  acc_t* acc;              // accumulators, acc_bytes(ntiles)
+  double2* gram;           // products of basis vectors, gram_bytes(ntiles, m)
+  int ntiles;
   void* xs;                // Re + Im plane or packed digits of the current vector
   bool lanczos;
   // profile: vector elements, all stored entries, FP64 operations of k_spmm
   double elems, nnz_work, spmm_flops;
 };
-static void enqueue_basis(Handle* h, BasisRun& B) {
+static size_t acc_bytes(int64_t ntiles) { return sizeof(acc_t) * 3 * ACC_ROWS * SPC_LANES * ntiles; }
+static size_t gram_bytes(int64_t ntiles, int m) { return sizeof(double2) * ORTHO_NB * SPC_LANES * m * ntiles; }
+static cudaError_t enqueue_basis(Handle* h, BasisRun& B) {
   cudaStream_t st = h->stream;
   PassArgs& pa = B.pa;
   const int m = pa.m;
@@ -1421,79 +1340,78 @@ static void enqueue_basis(Handle* h, BasisRun& B) {
   pa.items = B.items_p;
   pa.lanczos = B.lanczos ? 1 : 0;
   pa.shift = B.lanczos ? 0 : 1;
-  const auto scale = [&](int gather, int jd) {
+  const cudaError_t e = cudaMemsetAsync(B.acc, 0, acc_bytes(B.ntiles), st);
+  if (e != cudaSuccess) return e;
+  // every kernel that adds moves the three sets on by one
+  AccArgs A{B.acc, B.ntiles, 2, 0, 1};
+  const auto rotate = [&]() {
+    A.in = A.out;
+    A.out = A.clear;
+    A.clear = (A.clear + 1) % 3;
+  };
+  const auto scale = [&](int jd) {
     const int pe = h->prof.begin(st);
     if (B.nib)
-      k_scale<true><<<B.nip, blk, 0, st>>>(B.tiles, B.items_p, pa.map, pa.scol, pa.psi, pa.P, gather, jd, pa.rbeta,
-                                           pa.xexp, (double2*)pa.Q, B.xs);
+      k_scale<true><<<B.nip, blk, 0, st>>>(pa, A, jd, B.xs);
     else
-      k_scale<false><<<B.nip, blk, 0, st>>>(B.tiles, B.items_p, pa.map, pa.scol, pa.psi, pa.P, gather, jd, pa.rbeta,
-                                            pa.xexp, (double2*)pa.Q, B.xs);
+      k_scale<false><<<B.nip, blk, 0, st>>>(pa, A, jd, B.xs);
     h->prof.end(st, pe, PK_SCALE, 2.0 * elems, (B.nib ? 48.0 : 40.0) * elems);
+    h->count_launch();
+  };
+  // na vectors from ja subtracted, nd from jd projected on (0: the norm)
+  const auto ortho = [&](OrthoFn fn, int ja, int na, int jd, int nd, int extra, double per) {
+    OrthoArgs o{pa, A, ja, jd, B.gram};
+    o.p.items = B.items_o;
+    const int pe = h->prof.begin(st);
+    fn<<<B.nio, blk, 0, st>>>(o);
+    h->prof.end(st, pe, nd == 0 ? PK_AXPY_NORM : (na ? PK_AXPY_DOT : PK_DOT),
+                (per * (na + nd + extra) + (nd == 0 ? 4.0 : 0.0)) * elems,
+                16.0 * (na + nd + (na ? 2.0 : 1.0)) * elems);
+    h->count_launch();
+    rotate();
   };
   int pe = h->prof.begin(st);
-  k_rowpass<PASS_NORM_GATHER><<<B.nip, blk, 0, st>>>(pa);
+  k_norm<<<B.nip, blk, 0, st>>>(pa);
   h->prof.end(st, pe, PK_DOT, 4.0 * elems, 16.0 * elems);
-  scale(1, 0);
-  h->count_launch(2);
+  h->count_launch();
+  scale(0);
   for (int i = 0; i < m; ++i) {
+    pa.col_i = i;
     pe = h->prof.begin(st);
-    pa.col_i = pa.row_j = i;
-    if (B.nib && B.lanczos)
-      k_spmm_blk<true><<<B.nib, BLK_THREADS, 0, st>>>(pa, B.items_b, (const uint4*)B.xs);
-    else if (B.nib)
-      k_spmm_blk<false><<<B.nib, BLK_THREADS, 0, st>>>(pa, B.items_b, (const uint4*)B.xs);
-    else
+    if (B.nib && B.lanczos) {
+      k_spmm_blk<true><<<B.nib, BLK_THREADS, 0, st>>>(pa, A, B.items_b, (const uint4*)B.xs);
+      rotate();
+    } else if (B.nib) {
+      k_spmm_blk<false><<<B.nib, BLK_THREADS, 0, st>>>(pa, A, B.items_b, (const uint4*)B.xs);
+    } else {
       k_spmm<<<B.nis, blk, 0, st>>>(B.tiles, B.items_s, pa.map, i, pa.Q, (const double*)B.xs, pa.P, B.lanczos ? 0 : 1);
+    }
     // algorithmic traffic: H (with its Re + Im) once per tile, X and its
-    // Re + Im plane once, Y once
+    // digits or Re + Im plane once, Y once
     h->prof.end(st, pe, PK_SPMM, B.spmm_flops * SPC_LANES + (B.nib && B.lanczos ? 8.0 * elems : 0.0),
                 28.0 * B.nnz_work + (B.nib ? (B.lanczos ? 64.0 : 32.0) : 40.0) * elems);
     h->count_launch();
-    // MGS (get_krylov :453-456) projects p on Q_0..Q_i in order. Lanczos
-    // (H_eff Hermitian up to -i*kappa) needs only Q_{i-1} (coefficient
-    // beta_{i-1}, already in coef) and Q_i.
-    int j0 = 0;
-    if (B.lanczos && B.nib) {
-      j0 = i;  // projected on both by the SpMM's kernel
-    } else if (B.lanczos && i > 0) {
-      j0 = i - 1;
+    if (B.lanczos) {
+      // H_eff Hermitian up to -i*kappa: only Q_{i-1} (coefficient beta_{i-1})
+      // and Q_i; k_spmm_blk has done the first half
+      if (!B.nib && i == 0) ortho(k_ortho<0, 1, false, true>, 0, 0, 0, 1, 0, 4.0);
+      if (!B.nib && i > 0) ortho(k_ortho<1, 1, false, true>, i - 1, 1, i, 1, 0, 4.0);
+      ortho(k_ortho<1, 0, false, true>, i, 1, 0, 0, 0, 4.0);
     } else {
-      pa.row_j = 0;
-      pa.jx = 0;
-      pe = h->prof.begin(st);
-      if (B.lanczos)
-        k_rowpass<PASS_DOT, true><<<B.nip, blk, 0, st>>>(pa);
-      else
-        k_rowpass<PASS_DOT><<<B.nip, blk, 0, st>>>(pa);
-      h->prof.end(st, pe, PK_DOT, (B.lanczos ? 4.0 : 8.0) * elems, 32.0 * elems);
-      h->count_launch();
+      // MGS (get_krylov :453-456): p projected on Q_0..Q_i in order, by blocks
+      int ja = 0, na = 0;
+      for (int jd = 0; jd <= i; jd += ORTHO_NB) {
+        const int nd = std::min(ORTHO_NB, i + 1 - jd);
+        const bool newest = jd + nd == i + 1;
+        ortho(ortho_fn(na, nd, newest), ja, na, jd, nd, newest ? nd - 1 : 0, 8.0);
+        ja = jd;
+        na = nd;
+      }
+      ortho(ortho_fn(na, 0, false), ja, na, 0, 0, 0, 8.0);
     }
-    for (int j = j0; j < i; ++j) {
-      pa.jx = j;
-      pa.jn = j + 1;
-      pa.row_j = j + 1;
-      pe = h->prof.begin(st);
-      if (B.lanczos)
-        k_rowpass<PASS_AXPY_DOT, true><<<B.nip, blk, 0, st>>>(pa);
-      else
-        k_rowpass<PASS_AXPY_DOT><<<B.nip, blk, 0, st>>>(pa);
-      h->prof.end(st, pe, PK_AXPY_DOT, (B.lanczos ? 8.0 : 16.0) * elems, 64.0 * elems);
-      h->count_launch();
-    }
-    if (i < m - 1) {
-      pa.jx = i;
-      pa.row_j = i + 1;
-      pe = h->prof.begin(st);
-      if (B.lanczos)
-        k_rowpass<PASS_AXPY_NORM, true><<<B.nip, blk, 0, st>>>(pa);
-      else
-        k_rowpass<PASS_AXPY_NORM><<<B.nip, blk, 0, st>>>(pa);
-      h->prof.end(st, pe, PK_AXPY_NORM, (B.lanczos ? 8.0 : 12.0) * elems, 48.0 * elems);
-      scale(0, i + 1);
-      h->count_launch(2);
-    }
+    if (i < m - 1) scale(i + 1);
   }
+  return cudaSuccess;
 }
 
 // The block store of the handle's own Hamiltonian (single) or of the batch,
@@ -1571,6 +1489,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
   // tiles, the capacities scaled down by one factor. States, populations and
   // clocks stay resident for every sample either way.
   const double slot_fixed = 16.0 * (6.0 * mm + m + 1 + (double)nsplit_max * ncombo) + 8.0 + 4.0 + 12.0 + 8.0;
+  const double tile_fixed = (double)(sizeof(TileInfo) + sizeof(unsigned)) + (double)acc_bytes(1) + (double)gram_bytes(1, m);
   Handle::BlockStore* blocks = nullptr;
   {
     std::vector<int> used(nj);
@@ -1582,7 +1501,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
   // plane (XS)
   const double xs_bytes = blocks ? 16.0 : 8.0;
   const double need_fl = 16.0 * (double)qcap + (16.0 + xs_bytes) * (double)pcap + slot_fixed * slots_cap +
-                         (double)(sizeof(TileInfo) + sizeof(unsigned)) * tiles_cap;
+                         tile_fixed * tiles_cap;
   const double need_global = 16.0 * (double)psi_total + 8.0 * 4.0 * (double)T * G + 16.0 * G;
   double budget;
   {
@@ -1608,6 +1527,8 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
     reuse(h->flag, 4.0 * sl);
     reuse(h->qmax, 8.0 * sl);
     reuse(h->xexp, 4.0 * sl);
+    reuse(h->acc, (double)acc_bytes(tiles_cap));
+    reuse(h->gram, (double)gram_bytes(tiles_cap, m));
     reuse(h->tt, 8.0 * G);
     reuse(h->kk, 4.0 * G);
     reuse(h->done, 4.0 * G);
@@ -1624,7 +1545,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
     tiles_fl = std::max(1, (int)(f * tiles_cap));
     slots_fl = tiles_fl * SPC_LANES;
     const double fl = 16.0 * (double)qfl + (16.0 + xs_bytes) * (double)pfl + slot_fixed * slots_fl +
-                      (double)(sizeof(TileInfo) + sizeof(unsigned)) * tiles_fl;
+                      tile_fixed * tiles_fl;
     if (fl > budget)
       return set_error(SPC_ERR_ALLOC,
                        "one 32-sample tile of dimension %d at Krylov dimension %d needs %.3g bytes; "
@@ -1647,8 +1568,9 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
       h->ensure(h->kk, sizeof(int) * G) || h->ensure(h->done, sizeof(int) * G) ||
       h->ensure(h->obs, sizeof(double) * 4 * (size_t)T * G) || h->ensure(h->err, 16) ||
       h->ensure(h->flag, sizeof(int) * slots_fl) || h->ensure(h->qmax, 2 * sizeof(unsigned) * slots_fl) ||
-      h->ensure(h->xexp, sizeof(int) * slots_fl) ||
-      h->ensure(h->plan, sizeof(TileInfo) * tiles_fl + sizeof(int2) * 3 * items_cap +
+      h->ensure(h->xexp, sizeof(int) * slots_fl) || h->ensure(h->acc, acc_bytes(tiles_fl)) ||
+      h->ensure(h->gram, gram_bytes(tiles_fl, m)) ||
+      h->ensure(h->plan, sizeof(TileInfo) * tiles_fl + sizeof(int2) * 4 * items_cap +
                              sizeof(int) * 2 * slots_fl + 256) ||
       h->ensure(h->jobtab, (sizeof(JobInit) + sizeof(JobOut)) * nj + 64))
     return SPC_ERR_ALLOC;
@@ -1674,13 +1596,15 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
   long long* d_nsteps = (long long*)((char*)h->err.p + 8);
   int* d_flag = (int*)h->flag.p;
   unsigned* d_qmax = (unsigned*)h->qmax.p;
-  // per-round plan: tiles | pass items | SpMM items | block SpMM items | map | scol
+  // per-round plan: tiles | pass items | SpMM items | block SpMM items |
+  // orthogonalisation items | map | scol
   char* plan = (char*)h->plan.p;
   TileInfo* d_tiles = (TileInfo*)plan;
   int2* d_items_p = (int2*)(plan + sizeof(TileInfo) * tiles_fl);
   int2* d_items_s = d_items_p + items_cap;
   int2* d_items_b = d_items_s + items_cap;
-  int* d_map = (int*)(d_items_b + items_cap);
+  int2* d_items_o = d_items_b + items_cap;
+  int* d_map = (int*)(d_items_o + items_cap);
   int* d_scol = d_map + slots_fl;
   JobInit* d_jinit = (JobInit*)h->jobtab.p;
   JobOut* d_jout = (JobOut*)((char*)h->jobtab.p + sizeof(JobInit) * nj);
@@ -1766,8 +1690,10 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
   };
   const int res_spmm = resident((const void*)k_spmm, 256, 0);
   const int res_blk = resident((const void*)k_spmm_blk<true>, BLK_THREADS, 0);
-  const int res_pass = std::min(resident((const void*)k_rowpass<PASS_AXPY_DOT>, 256, 0),
-                                resident((const void*)k_rowpass<PASS_AXPY_NORM>, 256, 0));
+  const int res_pass = resident((const void*)k_scale<true>, 256, 0);
+  // Lanczos passes hold one vector and need the loads of many CTAs in flight
+  const int res_ortho[2] = {resident((const void*)k_ortho<8, 8, true, false>, 256, 0),
+                            resident((const void*)k_ortho<1, 1, false, true>, 256, 0)};
   // Grams on the tensor cores for m <= 32 (a CTA per projector type; its two
   // 16-vector blocks hold 32 vectors), in FP64 above. Faster at every measured
   // size below the line: 0.59 -> 0.26 ms (dim 2304, m = 16, 384 samples),
@@ -1832,6 +1758,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
         ti.vsum = jobs[k].vsum;
         ti.kappa = jobs[k].herm_shift ? jobs[k].kappa : nullptr;
         ti.m = std::min(m, ti.n);
+        ti.rexp = jobs[k].rexp;
         if (blocks) tile_blocks(ti, *blocks, jobs[k].sys);
         qo += (int64_t)m * ti.n * SPC_LANES;
         po += (int64_t)ti.n * SPC_LANES;
@@ -1852,8 +1779,9 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
     }
     const int ntiles = (int)tiles.size();
     const int nslots = ntiles * SPC_LANES;
-    std::vector<int> fp, cp, fs, cs, fb, cb;
-    std::vector<int2> items_p, items_s, items_b;
+    std::vector<int> fp, cp, fs, cs, fb, cb, fo, co;
+    std::vector<int2> items_p, items_s, items_b, items_o;
+    plan_items(tile_n, res_ortho[lanczos ? 1 : 0], fo, co, items_o);
     plan_items(tile_n, res_pass, fp, cp, items_p);
     plan_items(tile_n, res_spmm, fs, cs, items_s);
     if (blocks) plan_items(tile_n, res_blk, fb, cb, items_b, 4 * BLK_IDX);
@@ -1862,16 +1790,19 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
       tiles[t].nip = cp[t];
       tiles[t].is0 = fs[t];
       tiles[t].nis = cs[t];
+      tiles[t].nio = co[t];
       if (blocks) tiles[t].nib = cb[t];
     }
     const int nip = (int)items_p.size(), nis = (int)items_s.size(), nib = (int)items_b.size();
-    if (nip > items_cap || nis > items_cap || nib > items_cap || ntiles > tiles_fl || qo > qfl || po > pfl)
+    const int nio = (int)items_o.size();
+    if (nip > items_cap || nis > items_cap || nib > items_cap || nio > items_cap || ntiles > tiles_fl || qo > qfl || po > pfl)
       return set_error(SPC_ERR_ARG, "internal: work plan exceeds its buffer");
     // one host->device copy of the plan
     const size_t off_items_p = sizeof(TileInfo) * tiles_fl;
     const size_t off_items_s = off_items_p + sizeof(int2) * items_cap;
     const size_t off_items_b = off_items_s + sizeof(int2) * items_cap;
-    const size_t off_map = off_items_b + sizeof(int2) * items_cap;
+    const size_t off_items_o = off_items_b + sizeof(int2) * items_cap;
+    const size_t off_map = off_items_o + sizeof(int2) * items_cap;
     const size_t off_scol = off_map + sizeof(int) * slots_fl;
     const size_t plan_bytes = off_scol + sizeof(int) * nslots;
     hplan.resize(plan_bytes);
@@ -1879,6 +1810,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
     std::memcpy(hplan.data() + off_items_p, items_p.data(), sizeof(int2) * nip);
     std::memcpy(hplan.data() + off_items_s, items_s.data(), sizeof(int2) * nis);
     std::memcpy(hplan.data() + off_items_b, items_b.data(), sizeof(int2) * nib);
+    std::memcpy(hplan.data() + off_items_o, items_o.data(), sizeof(int2) * nio);
     std::memcpy(hplan.data() + off_map, map.data(), sizeof(int) * nslots);
     std::memcpy(hplan.data() + off_scol, scol.data(), sizeof(int) * nslots);
     CK(cudaMemcpyAsync(plan, hplan.data(), plan_bytes, cudaMemcpyHostToDevice, st));
@@ -1927,6 +1859,11 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
       br.nip = nip;
       br.nis = nis;
       br.nib = nib;
+      br.items_o = d_items_o;
+      br.nio = nio;
+      br.acc = (acc_t*)h->acc.p;
+      br.gram = (double2*)h->gram.p;
+      br.ntiles = ntiles;
       br.xs = h->xsum.p;
       br.lanczos = lanczos;
       br.pa.m = m;
@@ -1959,7 +1896,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
       br.elems = elems;
       br.nnz_work = (double)nnz_work;
       br.spmm_flops = spmm_flops;
-      enqueue_basis(h, br);
+      CK(enqueue_basis(h, br));
       int pe;
       double zsum = 0.0;  // sum over active slots of Z
       for (size_t c = 0; c < map.size(); ++c)
@@ -2022,7 +1959,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
     };
     // a shape is captured the second time it occurs (calls whose rounds never
     // repeat a shape pay no capture)
-    const std::vector<int64_t> key = {nip, nis, nib, nslots, ns, rps, lanczos ? 1 : 0,
+    const std::vector<int64_t> key = {nip, nis, nib, nio, nslots, ns, rps, lanczos ? 1 : 0,
                                        (int64_t)list.size()};
     const bool graphs = h->use_graphs && !h->prof.on && !shapes_seen.insert(key).second;
     if (graphs) {
@@ -2151,6 +2088,7 @@ int propagate(Handle* h, const double* theta, const double* init_pop, const doub
   j.zk = (const double2*)zk_dev;
   j.out = out_dev;
   j.herm_shift = h->herm_shift;
+  j.rexp = h->rexp;
   return propagate_batch(h, theta, init_pop, std::vector<JobSpec>{j}, dt, t_end, m, tol, T, true);
 }
 

@@ -1,5 +1,5 @@
-"""The tensor-core kernels on exact digits against the CPU oracle, on the
-tiled path. Every step carries rounding of order 1e-15 of populations of at
+"""The tensor-core kernels on exact digits and the orthogonalisation in blocks
+of eight with integer sums, against the CPU oracle on the tiled path. Every step carries rounding of order 1e-15 of populations of at
 most 1 and the windows have at most 60 steps, so 1e-12 leaves a factor of
 over ten; a wrong fragment, edge or digit shows at 1e-3 and above (the digit
 weights are 1/256 apart)."""
@@ -24,7 +24,7 @@ def pair(g1, g2, seed=4, iso=False, kT=1.0):
 
 # dims 8 (m above n), 48, 144 and 1296: Z = 2, 12, 36 and 324 rows against 32-row chunks
 @pytest.mark.parametrize("g1, g2", [((2,), ()), ((2,), (2, 3)), ((3, 3), (2, 2)), ((3, 2, 2), (3, 3, 3))])
-@pytest.mark.parametrize("m", [1, 7, 16, 17, 24, 25, 32, 33])
+@pytest.mark.parametrize("m", [1, 7, 8, 9, 16, 17, 24, 25, 32, 33])
 @pytest.mark.parametrize("method, M, kT", [("mgs", 3, 1.0), ("mgs", 33, 0.3), ("auto", 37, 1.0)])
 def test_populations(sampler, oracle, g1, g2, m, method, M, kT):
     s = pair(g1, g2, kT=kT)
@@ -41,6 +41,26 @@ def test_populations(sampler, oracle, g1, g2, m, method, M, kT):
     finally:
         sampler.set_sample_path("auto")
         sampler.set_krylov("mgs")
+    assert max(np.max(np.abs(getattr(got, k) - ref[k])) for k in KEYS) <= 1e-12
+
+
+@pytest.mark.parametrize("m", [8, 9, 17])
+@pytest.mark.parametrize("scale", [1e-3, 1.0, 1e3])
+def test_given_csr(sampler, oracle, m, scale):
+    """A CSR from the caller (only the FP64 product, its own bound for the
+    sums): the oracle's reference Hamiltonian times a scale, over a step that
+    keeps scale * dt."""
+    s = W.small_pair()
+    rp, col, val = iso_csr(oracle, s, 0.05)
+    zk = W.random_phase_samples(s.Z, 5, seed=m)
+    dt = DT / scale
+    ref = oracle.trace_sampling(rp, col, val * scale, zk, dt, 40 * dt, m, 1e-6)
+    sampler.set_sample_path("off")
+    try:
+        sampler.set_h(rp, col, val * scale)
+        got = sampler.trace_sampling(zk, dt, 40 * dt, m, 1e-6)
+    finally:
+        sampler.set_sample_path("auto")
     assert max(np.max(np.abs(getattr(got, k) - ref[k])) for k in KEYS) <= 1e-12
 
 
