@@ -40,18 +40,26 @@ struct ConPair {
   int64_t roff;
 };
 
+// Node states of a step: node q at q * stride from each base.
+struct ConNodes {
+  double w[16];  // weights
+  int n;
+  size_t stride;
+};
+
 // Partial reduced matrices P[a][b] = sum_{o in chunk} conj(mu_row(a,o))
 // nu_row(b,o) for the (tile, slot) pairs [p0, p0 + cnt), all of slot size G:
 // CTA b = ((pair * nch) + chunk) * (G / RB) + row block; one warp per CTA,
 // lanes = samples; rows a of the block [rb*RB, rb*RB + RB) against all G
 // columns (RB x G accumulators keep the register footprint small enough for
-// many resident warps). k_contract_close adds the chunks in order.
+// many resident warps); grid y = quadrature node. k_contract_close adds the
+// chunks and nodes in order.
 template <int G, int RB>
 __global__ void __launch_bounds__(32, (RB * G > 20 ? 8 : 16))
     k_contract(const TileInfo* __restrict__ tiles, const int* __restrict__ map,
                const int* __restrict__ scol, const GradSlot* __restrict__ slots,
                const ConPair* __restrict__ pairs, int p0, int nch, const double2* __restrict__ mu,
-               const double2* __restrict__ nu, double2* __restrict__ partial) {
+               const double2* __restrict__ nu, size_t node, double2* __restrict__ partial) {
   constexpr int NRB = G / RB;
   const int b = blockIdx.x;
   const int rb = b % NRB;
@@ -72,8 +80,8 @@ __global__ void __launch_bounds__(32, (RB * G > 20 ? 8 : 16))
   for (int i = 0; i < RB * G; ++i) acc[i] = cz();
   if (act) {
     const int64_t ld = T.ldp;
-    const double2* Mu = mu + T.psi_off + scol[wslot];
-    const double2* Nu = nu + T.psi_off + scol[wslot];
+    const double2* Mu = mu + blockIdx.y * node + T.psi_off + scol[wslot];
+    const double2* Nu = nu + blockIdx.y * node + T.psi_off + scol[wslot];
     const int64_t zg = S.owner == -1 ? Z : Z / S.g;
     for (int64_t o = o0; o < o1; ++o) {
       // o = nuclear index (electron pair), else (electron state or spin of
@@ -110,18 +118,18 @@ __global__ void __launch_bounds__(32, (RB * G > 20 ? 8 : 16))
         for (int j = 0; j < G; ++j) acc[i * G + j] = cjfma(a[i], v[j], acc[i * G + j]);
     }
   }
-  // partial[(pair * nch + chunk)][entry][lane]
-  double2* P = partial + ((size_t)pc * G * G + (size_t)rb * RB * G) * SPC_LANES + lane;
+  // partial[node][(pair * nch + chunk)][entry][lane]
+  double2* P = partial + ((size_t)(blockIdx.y * (gridDim.x / NRB) + pc) * G * G + (size_t)rb * RB * G) * SPC_LANES + lane;
 #pragma unroll
   for (int i = 0; i < RB * G; ++i) P[(size_t)i * SPC_LANES] = acc[i];
 }
 
-// R += w * sum over chunks (in chunk order) of the partials, one thread per
-// (pair, entry, lane).
+// R += sum over nodes of w * (sum over chunks, in chunk order) of the partials,
+// one thread per (pair, entry, lane).
 template <int G>
 __global__ void __launch_bounds__(256)
     k_contract_close(const int* __restrict__ map, const ConPair* __restrict__ pairs, int p0, int cnt,
-                     int nch, const double2* __restrict__ partial, double w, double2* __restrict__ racc) {
+                     int nch, const double2* __restrict__ partial, ConNodes N, double2* __restrict__ racc) {
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (int64_t)cnt * G * G * SPC_LANES) return;
   const int lane = (int)(idx % SPC_LANES);
@@ -129,17 +137,121 @@ __global__ void __launch_bounds__(256)
   const int pl = (int)(idx / ((int64_t)SPC_LANES * G * G));
   const ConPair PR = pairs[p0 + pl];
   if (map[PR.t * SPC_LANES + lane] < 0) return;
-  double2 s = cz();
-  const double2* src = partial + ((size_t)pl * nch * G * G + e) * SPC_LANES + lane;
-  for (int c = 0; c < nch; ++c) s = cadd(s, src[(size_t)c * G * G * SPC_LANES]);
   double2* R = racc + ((size_t)PR.roff + (size_t)lane * PR.nsl + PR.jl) * CON_MAXG * CON_MAXG + e;
-  *R = make_double2(fma(w, s.x, R->x), fma(w, s.y, R->y));
+  double2 r = *R;
+  for (int q = 0; q < N.n; ++q) {
+    double2 s = cz();
+    const double2* src = partial + (((size_t)q * cnt + pl) * nch * G * G + e) * SPC_LANES + lane;
+    for (int c = 0; c < nch; ++c) s = cadd(s, src[(size_t)c * G * G * SPC_LANES]);
+    r = make_double2(fma(N.w[q], s.x, r.x), fma(N.w[q], s.y, r.y));
+  }
+  *R = r;
 }
 
-// Krylov coordinates of y = exp(-i tau A) (beta e1): beta * E[:, 0] per slot,
-// beta = ||x|| as the norm pass left it in cvec[w][0].
-__global__ void k_first_col(int nslots, const TileInfo* __restrict__ tiles, const int* __restrict__ map,
-                            int m, const double2* __restrict__ Aexp, const double2* __restrict__ cvec,
+// Krylov coordinates of y_t = exp(-i tau_t H) x for several times from one
+// basis: beta exp(-i tau_t A) e_1, beta = ||x|| as the norm pass left it in
+// cvec[w][0]. Only this column of the exponential is needed, so it is summed
+// as a Taylor series of the vector (terms until they fall below 2^-58 of beta,
+// in ceil(||tau A|| / 2) substeps, where the largest term is at most 2 beta):
+// about 22 matrix-vector products in place of the m^3 products of the Pade form.
+// CTA = (slot, time), 128 threads. TRI: A is the Lanczos tridiagonal.
+// FP64 latency bounds it: 32 samples, m = 16, seven times in one launch take
+// 55 us, where an expm and a launch for each time took 7 x 210 us.
+struct Times {
+  double tau[17];
+  double2* y[17];
+  int n;
+};
+template <bool TRI>
+__global__ void __launch_bounds__(128)
+    k_expm_col(const TileInfo* __restrict__ tiles, const int* __restrict__ map, int m,
+               const double2* __restrict__ Ahess, const double2* __restrict__ cvec, Times tm, int t0,
+               double2* __restrict__ cout) {
+  extern __shared__ double2 esm[];  // [m * m]
+  __shared__ double2 v[SPC_MAX_M], part[4][SPC_MAX_M];
+  __shared__ double s_norm[4];
+  const int w = blockIdx.x, t = t0 + blockIdx.y;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (map[w] < 0) return;
+  const int me = tiles[w / SPC_LANES].m;
+  const double tau = tm.tau[t], beta = cvec[(size_t)w * m].x;
+  const double2* A = Ahess + (size_t)w * m * m;
+  for (int k = tid; k < me * me; k += 128) {
+    const double2 x = A[(k % me) + (size_t)(k / me) * m];
+    esm[k] = make_double2(tau * x.y, -tau * x.x);  // -i tau A
+  }
+  __syncthreads();
+  // largest row sum of |re| + |im|
+  double rs = 0.0;
+  for (int r = tid; r < me; r += 128) {
+    double x = 0.0;
+    for (int c = 0; c < me; ++c) x += fabs(esm[r + c * me].x) + fabs(esm[r + c * me].y);
+    rs = x > rs ? x : rs;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) rs = fmax(rs, __shfl_xor_sync(0xffffffffu, rs, o));
+  if (lane == 0) s_norm[warp] = rs;
+  __syncthreads();
+  const double norm = fmax(fmax(s_norm[0], s_norm[1]), fmax(s_norm[2], s_norm[3]));
+  const int steps = norm < 8192.0 ? max(1, (int)ceil(0.5 * norm)) : 1;  // the caller bounds ||tau H||; NaN passes
+  const double h = 1.0 / steps, small = beta * 3.5e-18;
+  double2 acc = cz();
+  if (tid < me) {
+    acc = tid == 0 ? make_double2(beta, 0.0) : cz();
+    v[tid] = acc;
+  }
+  __syncthreads();
+  for (int s = 0; s < steps; ++s) {
+    for (int k = 1; k < 80; ++k) {
+      const double f = h / k;
+      bool on = false;
+      if (TRI) {
+        double2 x = cz();
+        if (tid < me) {
+          x = cmul(esm[tid + tid * me], v[tid]);
+          if (tid > 0) x = cfma(esm[tid + (tid - 1) * me], v[tid - 1], x);
+          if (tid + 1 < me) x = cfma(esm[tid + (tid + 1) * me], v[tid + 1], x);
+          x = make_double2(x.x * f, x.y * f);
+        }
+        __syncthreads();
+        if (tid < me) {
+          v[tid] = x;
+          acc = cadd(acc, x);
+          on = fabs(x.x) > small || fabs(x.y) > small;
+        }
+      } else {
+        // columns j = warp mod 4, rows in the lanes
+        double2 x0 = cz(), x1 = cz();
+        for (int j = warp; j < me; j += 4) {
+          const double2 vj = v[j];
+          if (lane < me) x0 = cfma(esm[lane + j * me], vj, x0);
+          if (lane + 32 < me) x1 = cfma(esm[lane + 32 + j * me], vj, x1);
+        }
+        part[warp][lane] = x0;
+        part[warp][lane + 32] = x1;
+        __syncthreads();
+        if (tid < me) {
+          double2 x = cadd(cadd(part[0][tid], part[1][tid]), cadd(part[2][tid], part[3][tid]));
+          x = make_double2(x.x * f, x.y * f);
+          v[tid] = x;
+          acc = cadd(acc, x);
+          on = fabs(x.x) > small || fabs(x.y) > small;
+        }
+      }
+      if (!__syncthreads_or(on ? 1 : 0)) break;
+    }
+    if (s + 1 < steps) {
+      __syncthreads();
+      if (tid < me) v[tid] = acc;
+      __syncthreads();
+    }
+  }
+  if (tid < m) cout[((size_t)t * gridDim.x + w) * m + tid] = tid < me ? acc : cz();
+}
+
+// The same coordinates from the full exponential (k_expm), for one time.
+__global__ void k_first_col(int nslots, const TileInfo* __restrict__ tiles, const int* __restrict__ map, int m,
+                            const double2* __restrict__ Aexp, const double2* __restrict__ cvec,
                             double2* __restrict__ cout) {
   const int w = blockIdx.x * blockDim.x + threadIdx.x;
   if (w >= nslots || map[w] < 0) return;
@@ -148,6 +260,49 @@ __global__ void k_first_col(int nslots, const TileInfo* __restrict__ tiles, cons
   const double2* E = Aexp + (size_t)w * m * m;
   for (int j = 0; j < m; ++j) cout[(size_t)w * m + j] = j < me ? cscale(beta, E[j]) : cz();
 }
+
+// y_t = Q c_t for up to NT times from one read of the basis, for the tile of a
+// pass item; dynamic shared memory [NT][m][32] complex.
+template <int NT>
+__global__ void __launch_bounds__(256)
+    k_apply(const TileInfo* __restrict__ tiles, const int2* __restrict__ items, int m, int nslots,
+            const int* __restrict__ map, const int* __restrict__ scol, const double2* __restrict__ Q,
+            const double2* __restrict__ c, Times tm, int t0) {
+  extern __shared__ double2 asm_[];
+  const int2 it = items[blockIdx.x];
+  const TileInfo& T = tiles[it.x];
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  const int w = it.x * SPC_LANES + tx;
+  const bool act = map[w] >= 0;
+  const int me = T.m;
+  for (int k = ty; k < NT * me; k += SPC_WARPS)
+    asm_[((k / me) * m + k % me) * SPC_LANES + tx] =
+        act ? c[((size_t)(t0 + k / me) * nslots + w) * m + k % me] : cz();
+  __syncthreads();
+  if (!act) return;
+  const int n = T.n;
+  const size_t vs = (size_t)n * SPC_LANES;
+  const double2* q = Q + T.q_off + tx;
+  const size_t dst = T.psi_off + scol[w];
+  const int stride = T.nip * SPC_WARPS;
+  for (int r = it.y * SPC_WARPS + ty; r < n; r += stride) {
+    double2 acc[NT];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) acc[t] = cz();
+    const double2* qr = q + (size_t)r * SPC_LANES;
+    for (int j = 0; j < me; ++j) {
+      const double2 x = qr[(size_t)j * vs];
+#pragma unroll
+      for (int t = 0; t < NT; ++t) acc[t] = cfma(x, asm_[(t * m + j) * SPC_LANES + tx], acc[t]);
+    }
+#pragma unroll
+    for (int t = 0; t < NT; ++t) tm.y[t0 + t][dst + (size_t)r * T.ldp] = acc[t];
+  }
+}
+typedef void (*ApplyFn)(const TileInfo*, const int2*, int, int, const int*, const int*, const double2*, const double2*,
+                        Times, int);
+#define APPLY_MAX 4
+static const ApplyFn kApply[APPLY_MAX] = {k_apply<1>, k_apply<2>, k_apply<3>, k_apply<4>};
 
 // lam = ulam + c (cI psi + cP Pi_S psi) with (cI, cP) per tile, Pi_S = |S><S|
 // on the electron pair, |S> = (|ab> - |ba>)/sqrt(2); grid (tiles, row
@@ -319,26 +474,26 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
     pairs.push_back(ConPair{t, jobs[tile_job[t]].slot0, 0, 1, (int64_t)t * SPC_LANES});
   const int npairs = (int)pairs.size();
   // chunks per pair: about two waves of one-warp CTAs over the group (row
-  // blocks included), at least 32 rows of `o` each
+  // blocks and nodes included), at least 8 rows of `o` each
   auto pair_len = [&](const ConPair& P) {
     const GradSlot& Sl = cs[P.js];
     const int64_t Z = tile_n[P.t] / 4;
     return Sl.owner == -1 ? Z : (Sl.owner == -2 ? 4 * Z / Sl.g : 2 * Z / Sl.g);
   };
   auto nrb_of = [](int G) { return G == 6 ? 2 : 1; };
-  auto chunks_for = [&](int p0, int cnt, int G) {
+  auto chunks_for = [&](int p0, int cnt, int G, int nodes) {
     int64_t L = 1;
     for (int q = p0; q < p0 + cnt; ++q) L = std::max(L, pair_len(pairs[q]));
-    const int64_t by_wave = (int64_t)h->sm_count * 64 / std::max(1, cnt * nrb_of(G));
-    const int64_t by_len = (L + 31) / 32;
+    const int64_t by_wave = (int64_t)h->sm_count * 64 / std::max(1, cnt * nodes * nrb_of(G));
+    const int64_t by_len = (L + 7) / 8;
     return (int)std::max<int64_t>(1, std::min(by_wave, by_len));
   };
-  const int nch_f = chunks_for(pf0, ntiles, 4);
+  const int nch_f = chunks_for(pf0, ntiles, 4, 1);
   std::vector<int> grp_nch(grp_G.size());
   size_t part_need = (size_t)ntiles * nch_f * 16 * SPC_LANES;
   for (size_t gi = 0; gi < grp_G.size(); ++gi) {
-    grp_nch[gi] = chunks_for(grp_p0[gi], grp_cnt[gi], grp_G[gi]);
-    part_need = std::max(part_need, (size_t)grp_cnt[gi] * grp_nch[gi] * grp_G[gi] * grp_G[gi] * SPC_LANES);
+    grp_nch[gi] = chunks_for(grp_p0[gi], grp_cnt[gi], grp_G[gi], nq);
+    part_need = std::max(part_need, (size_t)nq * grp_cnt[gi] * grp_nch[gi] * grp_G[gi] * grp_G[gi] * SPC_LANES);
   }
   const size_t part_cap = part_need;
 
@@ -357,13 +512,13 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
     // to the size asked of it (buffers only grow), so its excess over that
     // size is no help
     auto need = [&](int k, bool keep) {
-      return sb * ((double)m + 4.0 + xs_bytes / 16.0 + (nsteps / k + 1) + k + 1.0 + (keep ? (double)k * nq : (double)nq));
+      return sb * ((double)m + 3.0 + nq + xs_bytes / 16.0 + (nsteps / k + 1) + k + 1.0 + (keep ? (double)k * nq : (double)nq));
     };
     auto extra = [&](int k, bool keep) {
       double x = 0.0;
       auto add = [&](const Handle::Buf& b, double bytes) { x += std::max(0.0, bytes - (double)b.bytes); };
       add(h->Q, sb * m);
-      add(h->gmu, sb);
+      add(h->gmu, sb * nq);
       add(h->glam, 2.0 * sb);
       add(h->P, sb);
       add(h->xsum, xs_bytes / 16.0 * sb);  // the current Krylov vector's digits or Re + Im plane beside P
@@ -407,7 +562,7 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   const size_t plan_bytes = 2 * sizeof(TileInfo) * ntiles + sizeof(int2) * 4 * items_cap +
                             sizeof(int) * 2 * nslots + sizeof(double2) * ntiles + 64;
   if (h->ensure(h->gck, sizeof(double2) * S * n_ck) || h->ensure(h->gseg, sizeof(double2) * S * n_seg) ||
-      h->ensure(h->gnu, sizeof(double2) * S * n_nu) || h->ensure(h->gmu, sizeof(double2) * S) ||
+      h->ensure(h->gnu, sizeof(double2) * S * n_nu) || h->ensure(h->gmu, sizeof(double2) * S * (want_grad ? nq : 1)) ||
       h->ensure(h->glam, sizeof(double2) * S * 2) || h->ensure(h->Q, sizeof(double2) * m * S) ||
       h->ensure(h->P, sizeof(double2) * S) || h->ensure(h->xsum, (size_t)xs_bytes * S) ||
       h->ensure(h->qmax, 2 * sizeof(unsigned) * nslots) || h->ensure(h->xexp, sizeof(int) * nslots) ||
@@ -415,9 +570,9 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
       h->ensure(h->partial, sizeof(double2) * std::max<size_t>((size_t)items_cap * SPC_LANES, part_cap)) ||
       h->ensure(h->counters, sizeof(unsigned) * std::max<size_t>(ntiles, npairs)) ||
       h->ensure(h->coef, sizeof(double2) * nslots) || h->ensure(h->rbeta, sizeof(double) * nslots) ||
-      h->ensure(h->Ahess, sizeof(double2) * mm * nslots) || h->ensure(h->Aexp, sizeof(double2) * mm * nslots) ||
-      h->ensure(h->cvec, sizeof(double2) * m * nslots) || h->ensure(h->cvec2, sizeof(double2) * m * nslots) ||
-      h->ensure(h->flag, sizeof(int) * nslots) || h->ensure(h->err, 16) ||
+      h->ensure(h->Ahess, sizeof(double2) * mm * nslots) ||
+      h->ensure(h->cvec, sizeof(double2) * m * nslots) || h->ensure(h->cvec2, sizeof(double2) * m * nslots * (nq + 1)) ||
+      h->ensure(h->err, 16) ||
       h->ensure(h->gslots, sizeof(GradSlot) * cs.size() + sizeof(ConPair) * npairs) ||
       h->ensure(h->gracc, sizeof(double2) * std::max<int64_t>(rtot, 1) * con) ||
       h->ensure(h->gfacc, sizeof(double2) * nslots * con) || h->ensure(h->plan, plan_bytes) ||
@@ -428,9 +583,8 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   double2 *d_Q = (double2*)h->Q.p, *d_P = (double2*)h->P.p, *d_part = (double2*)h->partial.p;
   unsigned* d_qmax = (unsigned*)h->qmax.p;
   unsigned* d_cnt = (unsigned*)h->counters.p;
-  double2 *d_A = (double2*)h->Ahess.p, *d_E = (double2*)h->Aexp.p, *d_c = (double2*)h->cvec.p;
+  double2 *d_A = (double2*)h->Ahess.p, *d_c = (double2*)h->cvec.p;
   double2* d_c2 = (double2*)h->cvec2.p;
-  int* d_flag = (int*)h->flag.p;
   int* d_err = (int*)h->err.p;
   GradSlot* d_slots = (GradSlot*)h->gslots.p;
   ConPair* d_pairs = (ConPair*)((char*)h->gslots.p + sizeof(GradSlot) * cs.size());
@@ -500,7 +654,6 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   CK(cudaMemsetAsync(d_cnt, 0, sizeof(unsigned) * std::max<size_t>(ntiles, npairs), st));
   CK(cudaMemsetAsync(d_racc, 0, sizeof(double2) * std::max<int64_t>(rtot, 1) * con, st));
   CK(cudaMemsetAsync(d_facc, 0, sizeof(double2) * nslots * con, st));
-  CK(cudaMemsetAsync(d_flag, 0, sizeof(int) * nslots, st));
   CK(cudaMemsetAsync(h->err.p, 0, 16, st));
   // psi_0 = theta (x) z: into the last segment's buffer when it is the only one
   double2* psi0 = !want_grad ? lam : a_last == 0 ? seg : ck;
@@ -518,7 +671,6 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
       h->count_launch();
     }
   }
-  CK(set_expm_smem(m));
   const dim3 blk(SPC_LANES, SPC_WARPS);
   std::vector<double> xq, wq;
   gauss_legendre01(nq, xq, wq);
@@ -565,18 +717,48 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
     builds += Mtot;
     return SPC_OK;
   };
-  // y = exp(-i tau H) x from the current bases (tau < 0 runs backwards)
-  auto apply = [&](double tau, const TileInfo* tiles, double2* y) {
+  // the series' substeps grow with ||tau H||, the squarings of the full
+  // exponential with its logarithm: a step past 64 (a basis of at most 48
+  // vectors resolves less) takes the latter
+  bool series = true;
+  for (const GradJob& J : jobs) series = series && std::ldexp(dt, std::max(HB.rexp[J.sys], HB.rexp[J.sys + 1])) <= 64.0;
+  if (!series) {
+    if (h->ensure(h->Aexp, sizeof(double2) * mm * nslots)) return SPC_ERR_ALLOC;
+    CK(set_expm_smem(m));
+  }
+  double2* d_E = (double2*)h->Aexp.p;
+  // y_t = exp(-i tau_t H) x from the current bases (tau < 0 runs backwards)
+  const size_t col_smem = sizeof(double2) * mm;
+  const int apply_max = (int)std::max<size_t>(1, std::min<size_t>(APPLY_MAX, (96u << 10) / (sizeof(double2) * m * SPC_LANES)));
+  CK(cudaFuncSetAttribute(k_expm_col<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col_smem));
+  CK(cudaFuncSetAttribute(k_expm_col<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col_smem));
+  for (int t = 1; t <= apply_max; ++t)
+    CK(cudaFuncSetAttribute(kApply[t - 1], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)(sizeof(double2) * t * m * SPC_LANES)));
+  auto apply = [&](const Times& tm, const TileInfo* tiles) {
     int pe = h->prof.begin(st);
-    launch_expm(m, nslots, tiles, d_map, d_A, d_E, tau, d_err, st);
-    h->prof.end(st, pe, PK_EXPM, 8.0 * (double)mm * m * 9.0 * Mtot, 32.0 * (double)mm * Mtot);
-    pe = h->prof.begin(st);
-    k_first_col<<<(nslots + 127) / 128, 128, 0, st>>>(nslots, tiles, d_map, m, d_E, d_c, d_c2);
-    h->prof.end(st, pe, PK_SETUP, 2.0 * m * Mtot, 32.0 * m * Mtot);
-    pe = h->prof.begin(st);
-    k_psi_update<<<nip, blk, 0, st>>>(tiles, d_items, m, d_map, d_scol, d_flag, d_Q, d_c2, y);
-    h->prof.end(st, pe, PK_PSI, 8.0 * m * elems, 16.0 * (m + 1) * elems);
-    h->count_launch(3);
+    if (!series) {
+      for (int t = 0; t < tm.n; ++t) {
+        launch_expm(m, nslots, tiles, d_map, d_A, d_E, tm.tau[t], d_err, st);
+        k_first_col<<<(nslots + 127) / 128, 128, 0, st>>>(nslots, tiles, d_map, m, d_E, d_c,
+                                                          d_c2 + (size_t)t * nslots * m);
+        h->count_launch(2);
+      }
+    } else if (lanczos)
+      k_expm_col<true><<<dim3(nslots, tm.n), 128, col_smem, st>>>(tiles, d_map, m, d_A, d_c, tm, 0, d_c2);
+    else
+      k_expm_col<false><<<dim3(nslots, tm.n), 128, col_smem, st>>>(tiles, d_map, m, d_A, d_c, tm, 0, d_c2);
+    h->prof.end(st, pe, PK_EXPM, 8.0 * 22.0 * (lanczos ? 3.0 * m : (double)mm) * Mtot * tm.n,
+                16.0 * (double)mm * Mtot * tm.n);
+    h->count_launch();
+    for (int t = 0; t < tm.n; t += apply_max) {
+      const int k = std::min(apply_max, tm.n - t);
+      pe = h->prof.begin(st);
+      kApply[k - 1]<<<nip, blk, sizeof(double2) * k * m * SPC_LANES, st>>>(tiles, d_items, m, nslots, d_map, d_scol, d_Q,
+                                                                          d_c2, tm, t);
+      h->prof.end(st, pe, PK_PSI, 8.0 * m * elems * k, 16.0 * (m + k) * elems);
+      h->count_launch();
+    }
   };
   // algorithmic FLOPs of a contraction over the gradient slots / the pair slot
   double con_fg = 0.0, con_ff = 0.0;
@@ -591,24 +773,29 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
       con_ff += f;
   }
   // acc += w * reduced matrices of (mu, nu): forward = the electron pair only
-  auto launch_group = [&](int G, int p0, int cnt, int nc, const double2* mu, const double2* nu, double w,
+  auto launch_group = [&](int G, int p0, int cnt, int nc, const double2* mu, const double2* nu, const ConNodes& w,
                           double2* acc) {
-    const int nb = cnt * nc * nrb_of(G);
+    const dim3 nb(cnt * nc * nrb_of(G), w.n);
     switch (G) {
       case 2:
-        k_contract<2, 2><<<nb, 32, 0, st>>>(d_tf, d_map, d_scol, d_slots, d_pairs, p0, nc, mu, nu, d_part);
+        k_contract<2, 2><<<nb, 32, 0, st>>>(d_tf, d_map, d_scol, d_slots, d_pairs, p0, nc, mu, nu, w.stride,
+                                            d_part);
         break;
       case 3:
-        k_contract<3, 3><<<nb, 32, 0, st>>>(d_tf, d_map, d_scol, d_slots, d_pairs, p0, nc, mu, nu, d_part);
+        k_contract<3, 3><<<nb, 32, 0, st>>>(d_tf, d_map, d_scol, d_slots, d_pairs, p0, nc, mu, nu, w.stride,
+                                            d_part);
         break;
       case 4:
-        k_contract<4, 4><<<nb, 32, 0, st>>>(d_tf, d_map, d_scol, d_slots, d_pairs, p0, nc, mu, nu, d_part);
+        k_contract<4, 4><<<nb, 32, 0, st>>>(d_tf, d_map, d_scol, d_slots, d_pairs, p0, nc, mu, nu, w.stride,
+                                            d_part);
         break;
       case 5:
-        k_contract<5, 5><<<nb, 32, 0, st>>>(d_tf, d_map, d_scol, d_slots, d_pairs, p0, nc, mu, nu, d_part);
+        k_contract<5, 5><<<nb, 32, 0, st>>>(d_tf, d_map, d_scol, d_slots, d_pairs, p0, nc, mu, nu, w.stride,
+                                            d_part);
         break;
       default:
-        k_contract<6, 3><<<nb, 32, 0, st>>>(d_tf, d_map, d_scol, d_slots, d_pairs, p0, nc, mu, nu, d_part);
+        k_contract<6, 3><<<nb, 32, 0, st>>>(d_tf, d_map, d_scol, d_slots, d_pairs, p0, nc, mu, nu, w.stride,
+                                            d_part);
         break;
     }
     const int64_t nt = (int64_t)cnt * G * G * SPC_LANES;
@@ -622,7 +809,7 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
     }
     h->count_launch(2);
   };
-  auto contract = [&](const double2* mu, const double2* nu, double w, bool forward, double2* acc) {
+  auto contract = [&](const double2* mu, const double2* nu, const ConNodes& w, bool forward, double2* acc) {
     int pe = h->prof.begin(st);
     if (forward) {
       launch_group(4, pf0, ntiles, nch_f, mu, nu, w, acc);
@@ -630,15 +817,26 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
       for (size_t gi = 0; gi < grp_G.size(); ++gi)
         launch_group(grp_G[gi], grp_p0[gi], grp_cnt[gi], grp_nch[gi], mu, nu, w, acc);
     }
-    h->prof.end(st, pe, PK_CONTRACT, forward ? con_ff : con_fg, 32.0 * elems);
+    h->prof.end(st, pe, PK_CONTRACT, (forward ? con_ff : con_fg) * w.n, 32.0 * elems * w.n);
   };
+  auto add_time = [](Times& tm, double tau, double2* y) {
+    tm.tau[tm.n] = tau;
+    tm.y[tm.n++] = y;
+  };
+  ConNodes one{}, all{};  // a single pair of states; the nodes of a step
+  one.n = 1;
+  all.n = nq;
+  all.stride = S;
+  for (int q = 0; q < nq; ++q) all.w[q] = wq[q] * dt;
   // basis at psi_k under H: node states nu_q and psi_{k+1}
   auto step_forward = [&](const double2* x, double2* nodes, double2* y) {
     int rc = build(x, d_tf);
     if (rc) return rc;
+    Times tm{};
     if (nodes)
-      for (int q = 0; q < nq; ++q) apply(dt * xq[q], d_tf, nodes + S * q);
-    apply(dt, d_tf, y);
+      for (int q = 0; q < nq; ++q) add_time(tm, dt * xq[q], nodes + S * q);
+    add_time(tm, dt, y);
+    apply(tm, d_tf);
     return SPC_OK;
   };
   const dim3 lgrid(ntiles, std::max(1, h->sm_count * 4 / ntiles));
@@ -653,7 +851,8 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   // and F = sum_k c_k (electron-pair reduced matrix of psi_k)
   double2* cur = psi0;
   for (int k = 0; k < nsteps; ++k) {
-    if (cw[k] != 0.0) contract(cur, cur, cw[k], true, d_facc);
+    one.w[0] = cw[k];
+    if (cw[k] != 0.0) contract(cur, cur, one, true, d_facc);
     double2* nxt;
     if (want_grad && k + 1 >= a_last)
       nxt = seg + S * (k + 1 - a_last);
@@ -665,7 +864,8 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
     if (rc) return rc;
     cur = nxt;
   }
-  if (cw[nsteps] != 0.0) contract(cur, cur, cw[nsteps], true, d_facc);
+  one.w[0] = cw[nsteps];
+  if (cw[nsteps] != 0.0) contract(cur, cur, one, true, d_facc);
   // backward sweep
   if (want_grad) {
     CK(cudaMemsetAsync(lam, 0, sizeof(double2) * S, st));
@@ -685,15 +885,17 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
       if (!cache) {
         int rc = build(seg + S * (k - a), d_tf);
         if (rc) return rc;
-        for (int q = 0; q < nq; ++q) apply(dt * xq[q], d_tf, nodes + S * q);
+        Times tm{};
+        for (int q = 0; q < nq; ++q) add_time(tm, dt * xq[q], nodes + S * q);
+        apply(tm, d_tf);
       }
       int rc = build(lam, d_tb);
       if (rc) return rc;
-      for (int q = 0; q < nq; ++q) {
-        apply(-dt * (1.0 - xq[q]), d_tb, gmu);
-        contract(gmu, nodes + S * q, wq[q] * dt, false, d_racc);
-      }
-      apply(-dt, d_tb, ulam);
+      Times tm{};
+      for (int q = 0; q < nq; ++q) add_time(tm, -dt * (1.0 - xq[q]), gmu + S * q);
+      add_time(tm, -dt, ulam);
+      apply(tm, d_tb);
+      contract(gmu, nodes, all, false, d_racc);
       costate(cw[k], seg + S * (k - a), ulam);
     }
   }

@@ -1298,7 +1298,7 @@ int num_time_points(double dt, double t_end) {
 // Work items per tile, proportional to the tile's rows and summing to about
 // one wave of `resident` CTAs; at least min_rows rows per item.
 static void plan_items(const std::vector<int>& tile_n, int resident, std::vector<int>& first,
-                       std::vector<int>& count, std::vector<int2>& items, int min_rows = 32) {
+                       std::vector<int>& count, std::vector<int2>& items, int min_rows = SPC_WARPS) {
   int64_t W = 0;
   for (int n : tile_n) W += n;
   first.resize(tile_n.size());

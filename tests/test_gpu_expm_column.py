@@ -1,0 +1,38 @@
+"""The stepwise yields' exponential columns (a Taylor series of the vector, and
+the full exponential past ||dt H|| = 64) against the dense model, in Krylov
+spaces that hold the whole space (m = n), so that the exponential is the only
+approximation. A step's phase carries rounding of eps ||dt H|| <= 4e-14 here, a
+window of 8 steps 3e-13 of a population of at most 1: 1e-11 leaves a factor of
+thirty; a wrong substep or branch shows at order one."""
+import numpy as np
+import pytest
+
+import dense
+from spin_dynamics_gb300 import workloads as W
+from spin_dynamics_gb300.dynamics import num_time_points
+from spin_dynamics_gb300.spinsys import GAMMA_E, Electron, SysParam
+
+pytestmark = pytest.mark.gpu
+DT = 1.0 * GAMMA_E / 1000
+
+
+# dt ||H||: below 1, some substeps, just under the line, past it
+@pytest.mark.parametrize("Bz", [0.05, 20.0, 150.0, 600.0])
+@pytest.mark.parametrize("g1, g2", [((2,), (2,)), ((3,), (2, 2)), ((2,), (2, 3))])
+@pytest.mark.parametrize("method", ["mgs", "lanczos"])
+def test_yields_of_strong_fields(sampler, Bz, g1, g2, method):
+    rng = np.random.default_rng(6)
+    A1, A2 = (W._tensors(rng, len(g), -1.5, 1.5, True) for g in (g1, g2))
+    s = SysParam(Electron(g_I=list(g1), A=A1), Electron(g_I=list(g2), A=A2), J=0.03, D=W.axial_dipolar(-0.3),
+                 kS=0.2, kT=0.2)
+    B = np.array([0.1 * Bz, 0.0, Bz])
+    zk = W.random_phase_samples(s.Z, 3, seed=2)
+    t_end = 8 * DT
+    sampler.set_krylov(method)
+    try:
+        got = sampler.stepwise_yields(s, B, zk, DT, t_end, 4 * s.Z)
+    finally:
+        sampler.set_krylov("mgs")
+    H = dense.hamiltonian(s.e1.g_I, A1, s.e2.g_I, A2, B, s.J, s.D, s.kS, s.kT)
+    ref = dense.stepwise_yields(H, zk, DT, num_time_points(DT, t_end), s.kS, s.kT)
+    assert np.max(np.abs(np.subtract(got, ref))) <= 1e-11
