@@ -50,16 +50,6 @@ __device__ __forceinline__ double2 csub(double2 a, double2 b) {
 __device__ __forceinline__ double2 cscale(double s, double2 a) {
   return make_double2(s * a.x, s * a.y);
 }
-// Smith's complex division a / d
-__device__ __forceinline__ double2 cdiv(double2 a, double2 d) {
-  if (fabs(d.x) >= fabs(d.y)) {
-    double r = d.y / d.x, den = d.x + d.y * r;
-    return make_double2((a.x + a.y * r) / den, (a.y - a.x * r) / den);
-  }
-  double r = d.x / d.y, den = d.x * r + d.y;
-  return make_double2((a.x * r + a.y) / den, (a.y * r - a.x) / den);
-}
-
 __device__ __forceinline__ double2 shfl_xor2(double2 v, int mask) {
   v.x = __shfl_xor_sync(0xffffffffu, v.x, mask);
   v.y = __shfl_xor_sync(0xffffffffu, v.y, mask);

@@ -8,7 +8,7 @@ __device__ __forceinline__ unsigned twice(unsigned x) {
 }
 
 // The Krylov-space projectors (k_proj's Grams, same `part` layout) for m <= 32.
-// CTA = (sample, type, split of the nuclear rows). Staged per chunk of GRAM_R
+// k_gram: CTA = (sample, type, split of the nuclear rows). Staged per chunk of GRAM_R
 // rows: the type's vectors V (q1, q2 - q3, q2 + q3 or q4, formed exactly in
 // integers) as digit pairs (re, im), 32 bits each, [digit][vector][row]. With
 // k = (row, part) both operands of V^H V are the same words: the A fragment
@@ -22,8 +22,8 @@ __device__ __forceinline__ unsigned twice(unsigned x) {
 // (T - T^T) / 2 (Im). A k-step adds at most 8 * 16 * 2^14 = 2^21 to a level:
 // after 8 steps the FP32 sums are closed into 64-bit integers in shared memory.
 // V is in units of 2^(E - 60), E the exponent of the basis' largest component.
-// Row stride GRAM_LD = 36 words: the 8 vectors x 4 rows of a fragment load
-// fall into 32 different banks.
+// Row stride GRAM_R + 4 words (36, or 20 with 16 rows): the 8 vectors x 4 rows
+// of a fragment load fall into 32 different banks.
 // Measured, all four Grams of 512 samples at dim 55296, m = 30: 19.3 ms
 // against 71.4 ms for k_proj (which holds the FP64 pipe at 92 %); 64 samples
 // at dim 9216, m = 24: 0.40 against 1.17 ms; 384 samples at dim 2304, m = 16:
@@ -31,33 +31,18 @@ __device__ __forceinline__ unsigned twice(unsigned x) {
 // (m = 30) are a third of the time: staging (one 16-byte load per line, the
 // conversion to digits) and the products do not overlap within a CTA.
 #define GRAM_R 32
-#define GRAM_LD 36
-__host__ __device__ __forceinline__ size_t gram_smem_bytes(int mt) {
-  return sizeof(unsigned) * DIGITS * 16 * mt * GRAM_LD + sizeof(longlong2) * 8 * 256;
+__host__ __device__ __forceinline__ size_t gram_smem_bytes(int mt, int rows = GRAM_R) {
+  return sizeof(unsigned) * DIGITS * 16 * mt * (rows + 4) + sizeof(longlong2) * 8 * 256;
 }
-template <int MT>
-__global__ void __launch_bounds__(256, 2)
-    k_gram(const TileInfo* __restrict__ tiles, const int* __restrict__ map, int m, int ncombo,
-           const double2* __restrict__ Q, const unsigned* __restrict__ qmax, int nsplit, int64_t rps,
-           double2* __restrict__ part, int nslots) {
-  constexpr int MP = 16 * MT;
-  extern __shared__ __align__(16) unsigned char gsm[];
-  longlong2* acc64 = reinterpret_cast<longlong2*>(gsm);               // [8][256]
-  unsigned* V = reinterpret_cast<unsigned*>(acc64 + 8 * 256);         // [DIGITS][MP][GRAM_LD]
-  const int type = blockIdx.x & 3;
-  const int w = blockIdx.x >> 2;
-  if (map[w] < 0) return;
-  const TileInfo& Ti = tiles[w / SPC_LANES];
-  const int64_t Z = Ti.n / 4;
-  const int nsp = proj_splits(nsplit, rps, Z);
-  const int split = blockIdx.y;
-  if (split >= nsp) return;
-  const int me = Ti.m;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
-  const int64_t per = (Z + nsp - 1) / nsp;
-  const int64_t n0 = (int64_t)split * per, n1 = min(Z, n0 + per);
-  const unsigned top = qmax[w];
-  const int emax = (int)(top >> 20);
+// Sums of one type over the rows [n0, n1): T of every block, in units of the
+// digit products, to Tm ([2][MP][MP + 1] doubles in V's place). get(j, row, e) is
+// the component of basis vector j < me at nuclear row `row`, electron state e. The
+// CTA's 256 threads; ends with a barrier.
+template <int MT, int R, typename Get>
+__device__ __forceinline__ void gram_sums(int type, int m, int me, int emax, int64_t n0, int64_t n1, longlong2* acc64,
+                                          unsigned* V, Get get) {
+  constexpr int MP = 16 * MT, LD = R + 4;
+  const int tid = threadIdx.y * 32 + threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
   // this warp's block: part (0 Re, 1 Im), rows 16 mi, columns 16 ni, k-steps
   const int im = warp & 1;
   const int mi = MT == 2 ? (warp >> 1) & 1 : 0, ni = MT == 2 ? warp >> 2 : 0;
@@ -89,23 +74,19 @@ __global__ void __launch_bounds__(256, 2)
         acc64[(4 * t + r) * 256 + tid] = a;
       }
   };
-  const size_t vs = (size_t)Ti.n * SPC_LANES;
-  const int64_t e0 = type == 0 ? 0 : (type == 3 ? 3 * Z : Z);
-  const double2* Qt = Q + Ti.q_off + (w % SPC_LANES) + (size_t)e0 * SPC_LANES;
   int steps = 0;
-  for (int64_t c0 = n0; c0 < n1; c0 += GRAM_R) {
-    const int len = (int)min((int64_t)GRAM_R, n1 - c0);
+  for (int64_t c0 = n0; c0 < n1; c0 += R) {
+    const int len = (int)min((int64_t)R, n1 - c0);
 #pragma unroll 4
-    for (int idx = tid; idx < MP * GRAM_R; idx += 256) {
-      const int j = idx / GRAM_R, nn = idx % GRAM_R;
+    for (int idx = tid; idx < MP * R; idx += 256) {
+      const int j = idx / R, nn = idx % R;
       long long vr = 0, vi = 0;
       if (j < me && nn < len) {
-        const double2* p = Qt + (size_t)j * vs + (size_t)(c0 + nn) * SPC_LANES;
-        const double2 a = *p;
+        const double2 a = get(j, c0 + nn, type == 0 ? 0 : (type == 3 ? 3 : 1));
         vr = to_fixed<8>(a.x, emax);
         vi = to_fixed<8>(a.y, emax);
         if (type == 1 || type == 2) {
-          const double2 b = p[(size_t)Z * SPC_LANES];
+          const double2 b = get(j, c0 + nn, 2);
           const long long br = to_fixed<8>(b.x, emax), bi = to_fixed<8>(b.y, emax);
           vr = type == 1 ? vr - br : vr + br;
           vi = type == 1 ? vi - bi : vi + bi;
@@ -113,10 +94,10 @@ __global__ void __launch_bounds__(256, 2)
       }
       const unsigned long long ur = (unsigned long long)vr + DIGIT_BIAS, ui = (unsigned long long)vi + DIGIT_BIAS;
       const unsigned rl = (unsigned)ur, rh = (unsigned)(ur >> 32), il = (unsigned)ui, ih = (unsigned)(ui >> 32);
-      unsigned* dst = V + j * GRAM_LD + nn;
+      unsigned* dst = V + j * LD + nn;
 #pragma unroll
       for (int d = 0; d < DIGITS; ++d)
-        dst[d * MP * GRAM_LD] = d < 4 ? digit_pair(rh, ih, 3 - d) : digit_pair(rl, il, 7 - d);
+        dst[d * MP * LD] = d < 4 ? digit_pair(rh, ih, 3 - d) : digit_pair(rl, il, 7 - d);
     }
     __syncthreads();
     for (int ks = k0; ks * 8 < len; ks += kstep) {
@@ -129,17 +110,17 @@ __global__ void __launch_bounds__(256, 2)
           for (int d = 0; d < DIGITS; ++d)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-              const unsigned x = Vk[(d * MP + 16 * ni + 8 * t + g) * GRAM_LD + 4 * h];
+              const unsigned x = Vk[(d * MP + 16 * ni + 8 * t + g) * LD + 4 * h];
               B[t][d][h] = im ? __byte_perm(x, x, 0x1032) ^ 0x80000000u : x;
             }
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         unsigned A[4];
-        const unsigned* Va = Vk + (i * MP + 16 * mi + g) * GRAM_LD;
+        const unsigned* Va = Vk + (i * MP + 16 * mi + g) * LD;
         A[0] = Va[0];
-        A[1] = Va[8 * GRAM_LD];
+        A[1] = Va[8 * LD];
         A[2] = Va[4];
-        A[3] = Va[8 * GRAM_LD + 4];
+        A[3] = Va[8 * LD + 4];
         mma_digits(acc[0][2 * i], A, B[0][i][0], B[0][i][1]);
         if (two) mma_digits(acc[1][2 * i], A, B[1][i][0], B[1][i][1]);
 #pragma unroll
@@ -159,8 +140,7 @@ __global__ void __launch_bounds__(256, 2)
   }
   close();
   __syncthreads();
-  // T of every block in units of the digit products, then G = (T +- T^T) / 2
-  double* Tm = reinterpret_cast<double*>(V);  // [2][MP][MP + 1]
+  double* Tm = reinterpret_cast<double*>(V);
   constexpr int TL = MP + 1;
   if (MT == 2 || k0 == 0) {
 #pragma unroll
@@ -179,17 +159,51 @@ __global__ void __launch_bounds__(256, 2)
       }
   }
   __syncthreads();
-  // units: v in 2^(E - 60), products closed at 256^7, T twice the Gram
-  const double unit = ldexp(1.0, 2 * (emax - 1023) - 120 + 56 - 1);
+}
+// G_ij, i <= j, from the sums; unit: V in 2^(E - 60), products closed at 256^7,
+// T twice the Gram. `bad` (an infinite or undefined basis) gives NaN.
+__device__ __forceinline__ double gram_unit(unsigned top) {
+  return top >= 0x7ff00000u ? __longlong_as_double(0x7ff8000000000000ll)
+                            : ldexp(1.0, 2 * ((int)(top >> 20) - 1023) - 120 + 56 - 1);
+}
+template <int MT>
+__device__ __forceinline__ double2 gram_entry(const double* Tm, int i, int j, double unit) {
+  constexpr int MP = 16 * MT, TL = MP + 1;
+  return make_double2((Tm[i * TL + j] + Tm[j * TL + i]) * unit,
+                      (Tm[(MP + i) * TL + j] - Tm[(MP + j) * TL + i]) * unit);
+}
+
+template <int MT>
+__global__ void __launch_bounds__(256, 2)
+    k_gram(const TileInfo* __restrict__ tiles, const int* __restrict__ map, int m, int ncombo,
+           const double2* __restrict__ Q, const unsigned* __restrict__ qmax, int nsplit, int64_t rps,
+           double2* __restrict__ part, int nslots) {
+  constexpr int MP = 16 * MT;
+  extern __shared__ __align__(16) unsigned char gsm[];
+  longlong2* acc64 = reinterpret_cast<longlong2*>(gsm);               // [8][256]
+  unsigned* V = reinterpret_cast<unsigned*>(acc64 + 8 * 256);         // [DIGITS][MP][GRAM_R + 4]
+  const int type = blockIdx.x & 3;
+  const int w = blockIdx.x >> 2;
+  if (map[w] < 0) return;
+  const TileInfo& Ti = tiles[w / SPC_LANES];
+  const int64_t Z = Ti.n / 4;
+  const int nsp = proj_splits(nsplit, rps, Z);
+  const int split = blockIdx.y;
+  if (split >= nsp) return;
+  const int64_t per = (Z + nsp - 1) / nsp;
+  const int64_t n0 = (int64_t)split * per, n1 = min(Z, n0 + per);
+  const unsigned top = qmax[w];
+  const size_t vs = (size_t)Ti.n * SPC_LANES;
+  const double2* Qt = Q + Ti.q_off + (w % SPC_LANES);
+  gram_sums<MT, GRAM_R>(type, m, Ti.m, (int)(top >> 20), n0, n1, acc64, V, [&](int j, int64_t row, int e) {
+    return Qt[(size_t)j * vs + (size_t)(e * Z + row) * SPC_LANES];
+  });
+  const double* Tm = reinterpret_cast<const double*>(V);
+  const double unit = gram_unit(top);
   const int nc = ncombo / 4;
   double2* out = part + ((size_t)split * nslots + w) * ncombo + type * nc;
-  const bool bad = top >= 0x7ff00000u;  // an infinite or undefined basis gives undefined Grams
-  for (int idx = tid; idx < MP * MP; idx += 256) {
+  for (int idx = threadIdx.x; idx < MP * MP; idx += 256) {
     const int i = idx / MP, j = idx % MP;
-    if (i > j || j >= m) continue;
-    double2 gv = make_double2((Tm[i * TL + j] + Tm[j * TL + i]) * unit,
-                              (Tm[(MP + i) * TL + j] - Tm[(MP + j) * TL + i]) * unit);
-    if (bad) gv = make_double2(__longlong_as_double(0x7ff8000000000000ll), __longlong_as_double(0x7ff8000000000000ll));
-    out[i * m - i * (i - 1) / 2 + (j - i)] = gv;
+    if (i <= j && j < m) out[i * m - i * (i - 1) / 2 + (j - i)] = gram_entry<MT>(Tm, i, j, unit);
   }
 }

@@ -376,9 +376,9 @@ int prepare_spmm_rows(Handle* h) {
 // ---------------------------------------------------------------------------
 // expm (src/matrix_exponential.f90:14-87) of -i dt A per sample, column-major
 // m x m matrices in shared memory. expm_one is run by nt threads (index tid)
-// that synchronise as a whole CTA (one sample per CTA) or as one warp (k_expm
-// packs four samples per 128-thread CTA for m <= 16); every element is
-// computed by the same serial loop either way, so both give the same bits.
+// that synchronise as a whole CTA (one sample per CTA) or as one warp
+// (k_expm_warp packs four samples per 128-thread CTA for m <= 16); every element
+// is computed by the same serial loop either way, so both give the same bits.
 template <bool WARP>
 __device__ __forceinline__ void expm_sync() {
   if (WARP)
@@ -430,337 +430,217 @@ __device__ void smem_matmul_band(int m, const double2* A, int la, int ua, const 
   }
 }
 
-// Padé(6,6) coefficient c_k by the reference's recurrence (:54-77),
-// c_0 = 1, c_1 = 1/2, c_k = c_{k-1} (q - k + 1) / (k (2q - k + 1)), folded at
-// compile time with the same IEEE double operations.
-constexpr double pade6_coef(int k) {
+// 1/k!, folded at compile time
+constexpr double inv_factorial(int k) {
   double c = 1.0;
-  for (int j = 1; j <= k; ++j) c = j == 1 ? 0.5 : c * (double)(6 - j + 1) / (double)(j * (2 * 6 - j + 1));
+  for (int j = 2; j <= k; ++j) c /= j;
   return c;
 }
-
-// Complex reciprocal 1/d = conj(d) / |d|^2, for the band path's pivots (the
-// diagonal of a diagonally dominant denominator, |d| of order one).
-__device__ __forceinline__ double2 crcp(double2 d) {
-  const double s = 1.0 / fma(d.x, d.x, d.y * d.y);
-  return make_double2(d.x * s, -d.y * s);
+#define F(k) inv_factorial(k)
+__constant__ double kInvFact[30] = {F(0),  F(1),  F(2),  F(3),  F(4),  F(5),  F(6),  F(7),  F(8),  F(9),
+                                    F(10), F(11), F(12), F(13), F(14), F(15), F(16), F(17), F(18), F(19),
+                                    F(20), F(21), F(22), F(23), F(24), F(25), F(26), F(27), F(28), F(29)};
+#undef F
+// smallest number n of terms with theta^n / n! below 2^-56
+__device__ __forceinline__ int taylor_terms(double theta) {
+  double t = 1.0;
+  int n = 0;
+  while (n < 40 && !(t < 1.4e-17)) t *= theta / ++n;
+  return n;
 }
 
-// Padé(6,6) with scaling and squaring, evaluated on the bands of the input:
-// a Lanczos basis gives a tridiagonal matrix, MGS an upper Hessenberg one.
-// The powers and the Padé sums (each element by the dense evaluation's
-// operations in its order: the skipped terms are exact zeros), the LU
-// factors (while partial pivoting keeps the diagonal, which the
-// denominator's diagonal dominance at the scaled norm < 1/2 makes the rule)
-// and the triangular solves then only touch their bands. On that path the
-// multipliers and the upper solve use the pivots' reciprocals: a complex
-// division is three IEEE divides on the serial path of every step. A pivot
-// off the diagonal restarts the factorisation dense with Smith's division.
+// out = exp(-i dt A) for one sample (the reference's expm, src/matrix_exponential.f90:14-87,
+// takes a Pade form): a Taylor polynomial at a norm of at most 2, then squarings. At
+// that norm its 17-25 terms carry a rounding of a few eps, like Pade(6,6) at a
+// norm below 1/2 with its two or three squarings more, and it has no pivot
+// search, factorisation and triangular solves, whose m serial steps each were
+// longer than an m x m product on one SM.
+// tri (Lanczos): A = T - i kappa with T real, symmetric, tridiagonal. The terms
+// (dt T)^k / k! are real and symmetric, so a term is 3 FMAs per element of the
+// upper triangle and adds to the real or imaginary part in turn.
+// General: powers a, a^2, a^3 and Horner's rule in a^3 (Paterson and Stockmeyer,
+// "On the number of nonscalar multiplications necessary to evaluate
+// polynomials", SIAM J. Comput. 2 (1973) 60-66); the products skip the zeros
+// outside the bands of the powers (an MGS basis gives an upper Hessenberg A).
+// Scratch: 5 m^2 complex.
 template <bool WARP>
 __device__ void expm_one(int m, int mld, const double2* __restrict__ Ain, double2* __restrict__ out, double dt,
-                         double2* sm, double* rowsum, int* piv, int* s_sh, int* p_sh, int tid, int nt,
-                         int* __restrict__ err) {
+                         double2* sm, double* rowsum, int* band, bool tri, int tid, int nt) {
   const int mm = m * m;
-  double2* A2 = sm;
-  double2* X = A2 + mm;
-  double2* E = X + mm;
-  double2* D = E + mm;
-  double2* T = D + mm;
-  // (0,-1)*dt*A and its bandwidths (held in piv[0], piv[1] until the LU)
-  if (tid == 0) piv[0] = piv[1] = 0;
+  // band widths of A, rows' absolute sums
+  if (tid < 2) band[tid] = 0;
   expm_sync<WARP>();
-  {
+  double2* M = sm;
+  double2* A2 = M + mm;
+  double2* A3 = A2 + mm;
+  double2* E = A3 + mm;
+  double2* T = E + mm;
+  if (!tri) {
     int bl = 0, bu = 0;
     for (int i = tid; i < mm; i += nt) {
       const double2 a = Ain[(i % m) + (size_t)(i / m) * mld];
-      const double2 v = make_double2(dt * a.y, -dt * a.x);
-      A2[i] = v;
-      if (v.x != 0.0 || v.y != 0.0) {
+      M[i] = make_double2(dt * a.y, -dt * a.x);
+      if (a.x != 0.0 || a.y != 0.0) {
         bl = max(bl, i % m - i / m);
         bu = max(bu, i / m - i % m);
       }
     }
-    if (bl) atomicMax(&piv[0], bl);
-    if (bu) atomicMax(&piv[1], bu);
+    if (bl) atomicMax(&band[0], bl);
+    if (bu) atomicMax(&band[1], bu);
+    expm_sync<WARP>();
   }
-  expm_sync<WARP>();
-  const int l1 = piv[0], u1 = piv[1];
-  const int l2 = min(2 * l1, m - 1), u2 = min(2 * u1, m - 1);
-  const int l4 = min(2 * l2, m - 1), u4 = min(2 * u2, m - 1);
-  const int l6 = min(l4 + l2, m - 1), u6 = min(u4 + u2, m - 1);
-  const int lN = max(l6, min(l1 + l4, m - 1)), uN = max(u6, min(u1 + u4, m - 1));
-  // L-infinity norm (mat_norm_linf :89-104): the row's band in column order
-  // (the entries outside add exact zeros)
+  const int l1 = tri ? 1 : band[0], u1 = tri ? 1 : band[1];
   for (int i = tid; i < m; i += nt) {
     double s = 0.0;
-    for (int j = max(0, i - l1); j <= min(m - 1, i + u1); ++j) s += hypot(A2[i + j * m].x, A2[i + j * m].y);
+    for (int j = max(0, i - l1); j <= min(m - 1, i + u1); ++j) {
+      const double2 a = tri ? Ain[i + (size_t)j * mld] : M[i + j * m];
+      s += tri ? fabs(dt * a.x) : fabs(a.x) + fabs(a.y);
+    }
     rowsum[i] = s;
   }
   expm_sync<WARP>();
   if (tid < 32) {
-    // the largest row sum by a warp maximum (exact: the same value in any order)
     double an = 0.0;
     for (int i = tid; i < m; i += 32) an = fmax(an, rowsum[i]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) an = fmax(an, __shfl_xor_sync(0xffffffffu, an, o));
     if (tid == 0) {
       int s = 0;
-      if (an > 0.0) {
-        const double l2 = log(an) / log(2.0);  // log_2 (:106-117)
-        const int ee = (int)l2 + 1;            // int() truncates toward zero
-        s = max(0, ee + 1);
+      while (an > 2.0 && an < 1e300) {
+        an *= 0.5;
+        ++s;
       }
-      *s_sh = s;
+      band[2] = s;
+      band[3] = taylor_terms(an);
     }
   }
   expm_sync<WARP>();
-  const int s = *s_sh;
-  const double sc = ldexp(1.0, -s);  // A/2**s, exact
-  for (int i = tid; i < mm; i += nt) A2[i] = make_double2(A2[i].x * sc, A2[i].y * sc);
-  expm_sync<WARP>();
-  // Pade(6,6) numerator N = sum c_k a^k and denominator D = sum (-1)^k c_k a^k
-  // with the reference's coefficient recurrence (:54-77), evaluated from the
-  // even and odd parts (Paterson-Stockmeyer): a^2, a^4, a^6 and
-  // a (c1 + c3 a^2 + c5 a^4), four products instead of five
-  constexpr double ck[7] = {pade6_coef(0), pade6_coef(1), pade6_coef(2), pade6_coef(3),
-                            pade6_coef(4), pade6_coef(5), pade6_coef(6)};
-  smem_matmul_band(m, A2, l1, u1, A2, l1, u1, X, tid, nt);  // a^2
-  expm_sync<WARP>();
-  smem_matmul_band(m, X, l2, u2, X, l2, u2, T, tid, nt);    // a^4
-  expm_sync<WARP>();
-  smem_matmul_band(m, T, l4, u4, X, l2, u2, D, tid, nt);    // a^6
-  expm_sync<WARP>();
-  for (int i = tid; i < mm; i += nt) {
-    const double id = (i % (m + 1) == 0) ? 1.0 : 0.0;
-    const double2 x2 = X[i], x4 = T[i], x6 = D[i];
-    E[i] = make_double2(id + ck[2] * x2.x + ck[4] * x4.x + ck[6] * x6.x, ck[2] * x2.y + ck[4] * x4.y + ck[6] * x6.y);
-    D[i] = make_double2(id * ck[1] + ck[3] * x2.x + ck[5] * x4.x, ck[3] * x2.y + ck[5] * x4.y);
-  }
-  expm_sync<WARP>();
-  smem_matmul_band(m, A2, l1, u1, D, l4, u4, X, tid, nt);   // odd part
-  expm_sync<WARP>();
-  for (int i = tid; i < mm; i += nt) {
-    const double2 ev = E[i], od = X[i];
-    T[i] = cadd(ev, od);  // N
-    D[i] = csub(ev, od);  // D
-    X[i] = D[i];          // kept for a dense restart of the LU
-  }
-  expm_sync<WARP>();
-  // LU of D with partial pivoting (|re|+|im| pivot, as izamax), in place, on
-  // the bands (lN, uN) while every pivot is the diagonal: then no row moves,
-  // the unit-lower factor keeps bandwidth lN and the upper one uN. The
-  // multipliers l_ik = D_ik / D_kk (formed with the pivot's reciprocal in the
-  // same pass as the trailing update) go to the spent A2.
-  bool swapped = false;
-  for (int k = 0; k < m; ++k) {
-    const int ie = min(k + lN, m - 1), je = min(k + uN, m - 1);
-    if (tid < 32) {
-      // non-negative doubles order as their bit patterns: integer compares
-      long long best = -1;
-      int bi = k;
-      for (int i = k + tid; i <= ie; i += 32) {
-        const long long v = __double_as_longlong(fabs(D[i + k * m].x) + fabs(D[i + k * m].y));
-        if (v > best) {
-          best = v;
-          bi = i;
-        }
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const long long ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ob > best || (ob == best && oi < bi)) {
-          best = ob;
-          bi = oi;
-        }
-      }
-      if (tid == 0) {
-        *p_sh = bi;
-        piv[k] = bi;
-        if (best == 0) atomicExch(err, 2);
-      }
+  const int s = band[2], terms = band[3];
+  const double sc = ldexp(1.0, -s);
+  if (tri) {
+    // R_k = (f T)^k / k!, upper triangle; E = sum (-i)^k R_k
+    double* R0 = reinterpret_cast<double*>(M);
+    double* R1 = R0 + mm;
+    unsigned short* tab = reinterpret_cast<unsigned short*>(A2);  // (i, j >= i)
+    double* da = reinterpret_cast<double*>(A3);                   // f * diagonal
+    double* db = da + m;                                          // f * subdiagonal
+    const double f = dt * sc;
+    const int np = m * (m + 1) / 2;
+    for (int i = tid; i < m; i += nt) {
+      da[i] = f * Ain[i + (size_t)i * mld].x;
+      db[i] = i + 1 < m ? f * Ain[i + (size_t)(i + 1) * mld].x : 0.0;
+      for (int j = i; j < m; ++j) tab[i * m - i * (i - 1) / 2 + (j - i)] = (unsigned short)(i << 8 | j);
+    }
+    for (int i = tid; i < mm; i += nt) {
+      const bool d = i % (m + 1) == 0;
+      R0[i] = d ? 1.0 : 0.0;
+      E[i] = make_double2(d ? 1.0 : 0.0, 0.0);
     }
     expm_sync<WARP>();
-    if (*p_sh != k) {  // a row swap: the bands no longer hold
-      swapped = true;
-      break;
-    }
-    const int ri = ie - k, rj = je - k + 1;  // rows k+1..ie, columns k..je
-    for (int idx = tid; idx < ri * rj; idx += nt) {
-      const int i = k + 1 + idx % ri, j = k + idx / ri;
-      const double2 l = cmul(D[i + k * m], crcp(D[k + k * m]));
-      if (j == k)
-        A2[i + k * m] = l;
-      else
-        D[i + j * m] = cfms(l, D[k + j * m], D[i + j * m]);
-    }
-    expm_sync<WARP>();
-  }
-  if (swapped) {
-    // dense restart from the saved denominator
-    for (int i = tid; i < mm; i += nt) D[i] = X[i];
-    expm_sync<WARP>();
-  }
-  const int lL = swapped ? m - 1 : lN, uU = swapped ? m - 1 : uN;
-  for (int k = 0; swapped && k < m; ++k) {
-    if (tid < 32) {
-      double best = -1.0;
-      int bi = k;
-      for (int i = k + tid; i < m; i += 32) {
-        const double v = fabs(D[i + k * m].x) + fabs(D[i + k * m].y);
-        if (v > best) {
-          best = v;
-          bi = i;
-        }
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ob > best || (ob == best && oi < bi)) {
-          best = ob;
-          bi = oi;
-        }
-      }
-      if (tid == 0) {
-        *p_sh = bi;
-        piv[k] = bi;
-        if (best == 0.0) atomicExch(err, 2);
-      }
-    }
-    expm_sync<WARP>();
-    const int pr = *p_sh;
-    if (pr != k)
-      for (int j = tid; j < m; j += nt) {
-        const double2 t0 = D[k + j * m];
-        D[k + j * m] = D[pr + j * m];
-        D[pr + j * m] = t0;
-      }
-    expm_sync<WARP>();
-    const double2 dkk = D[k + k * m];
-    for (int i = k + 1 + tid; i < m; i += nt) D[i + k * m] = cdiv(D[i + k * m], dkk);
-    expm_sync<WARP>();
-    const int rem = m - k - 1;
-    for (int idx = tid; idx < rem * rem; idx += nt) {
-      const int i = k + 1 + idx % rem, j = k + 1 + idx / rem;
-      D[i + j * m] = cfms(D[i + k * m], D[k + j * m], D[i + j * m]);
-    }
-    expm_sync<WARP>();
-  }
-  // E = D^-1 N: the rows of N permuted as the LU's row swaps (P N), then the
-  // unit-lower and the upper triangular solves of all m columns as rank-1
-  // updates over every (row, column) at once, one sync per step
-  int* perm = reinterpret_cast<int*>(rowsum);  // the row sums are spent
-  if (tid == 0) {
-    for (int i = 0; i < m; ++i) perm[i] = i;
-    for (int k = 0; k < m; ++k) {
-      const int a = perm[k];
-      perm[k] = perm[piv[k]];
-      perm[piv[k]] = a;
-    }
-  }
-  expm_sync<WARP>();
-  for (int idx = tid; idx < mm; idx += nt) E[idx] = T[perm[idx % m] + (idx / m) * m];
-  expm_sync<WARP>();
-  // (the factors' entries outside their bands are exact zeros; the band
-  // path's multipliers are in A2, whose diagonal then takes the pivots'
-  // reciprocals for the upper solve)
-  const double2* Lf = swapped ? D : A2;
-  for (int k = 0; k + 1 < m; ++k) {
-    const int rem = min(lL, m - k - 1);
-    for (int idx = tid; idx < rem * m; idx += nt) {
-      const int i = k + 1 + idx % rem, j = idx / rem;
-      E[i + j * m] = cfms(Lf[i + k * m], E[k + j * m], E[i + j * m]);
-    }
-    expm_sync<WARP>();
-  }
-  if (!swapped) {
-    for (int k = tid; k < m; k += nt) A2[k + k * m] = crcp(D[k + k * m]);
-    expm_sync<WARP>();
-  }
-  if (swapped) {
-    for (int k = m - 1; k >= 0; --k) {
-      for (int j = tid; j < m; j += nt) E[k + j * m] = cdiv(E[k + j * m], D[k + k * m]);
-      expm_sync<WARP>();
-      for (int idx = tid; idx < k * m; idx += nt) {
-        const int i = idx % k, j = idx / k;
-        E[i + j * m] = cfms(D[i + k * m], E[k + j * m], E[i + j * m]);
+    for (int k = 1; k < terms; ++k) {
+      const double rk = 1.0 / k;
+      for (int p = tid; p < np; p += nt) {
+        const int i = tab[p] >> 8, j = tab[p] & 255;
+        double r = da[i] * R0[i + j * m];
+        if (i > 0) r = fma(db[i - 1], R0[i - 1 + j * m], r);
+        if (i + 1 < m) r = fma(db[i], i < j ? R0[i + 1 + j * m] : R0[i + (i + 1) * m], r);
+        r *= rk;
+        R1[i + j * m] = r;
+        double* e = reinterpret_cast<double*>(E + i + j * m) + (k & 1);
+        *e += (k & 3) == 1 || (k & 3) == 2 ? -r : r;
       }
       expm_sync<WARP>();
+      double* t = R0;
+      R0 = R1;
+      R1 = t;
     }
+    const double damp = exp(sc * dt * Ain[0].y);  // e^{-kappa dt}, Im A_ii = -kappa
+    for (int p = tid; p < np; p += nt) {
+      const int i = tab[p] >> 8, j = tab[p] & 255;
+      const double2 e = cscale(damp, E[i + j * m]);
+      T[i + j * m] = e;
+      T[j + i * m] = e;
+    }
+    expm_sync<WARP>();
+    double2* t = E;
+    E = T;
+    T = t;
   } else {
-    // one sync per step: row k's solution, E_kj times the pivot's
-    // reciprocal, goes to T (N is spent), and every thread that updates a
-    // row above forms the same product itself
-    for (int k = m - 1; k >= 0; --k) {
-      const int i0 = max(0, k - uU), ri = k - i0 + 1;  // rows i0..k
-      for (int idx = tid; idx < ri * m; idx += nt) {
-        const int i = i0 + idx % ri, j = idx / ri;
-        const double2 ek = cmul(E[k + j * m], A2[k + k * m]);
-        if (i == k)
-          T[k + j * m] = ek;
-        else
-          E[i + j * m] = cfms(D[i + k * m], ek, E[i + j * m]);
+    if (s > 0) {
+      for (int i = tid; i < mm; i += nt) M[i] = cscale(sc, M[i]);
+      expm_sync<WARP>();
+    }
+    const int l2 = min(2 * l1, m - 1), u2 = min(2 * u1, m - 1), l3 = min(3 * l1, m - 1), u3 = min(3 * u1, m - 1);
+    smem_matmul_band(m, M, l1, u1, M, l1, u1, A2, tid, nt);
+    expm_sync<WARP>();
+    smem_matmul_band(m, A2, l2, u2, M, l1, u1, A3, tid, nt);
+    expm_sync<WARP>();
+    const int q = min(9, (terms + 2) / 3 - 1 < 0 ? 0 : (terms + 2) / 3 - 1);  // terms 0 .. 3 q + 2
+    int lE = m - 1, uE = m - 1;
+    for (int j = q; j >= 0; --j) {
+      if (j < q) {
+        smem_matmul_band(m, E, lE, uE, A3, l3, u3, T, tid, nt);
+        expm_sync<WARP>();
+      }
+      const double c0 = kInvFact[3 * j], c1 = kInvFact[3 * j + 1], c2 = kInvFact[3 * j + 2];
+      for (int i = tid; i < mm; i += nt) {
+        double2 e = make_double2(fma(c2, A2[i].x, c1 * M[i].x), fma(c2, A2[i].y, c1 * M[i].y));
+        if (i % (m + 1) == 0) e.x += c0;
+        E[i] = j < q ? cadd(T[i], e) : e;
       }
       expm_sync<WARP>();
     }
-    for (int i = tid; i < mm; i += nt) E[i] = T[i];
-    expm_sync<WARP>();
   }
   // s squarings
   for (int k = 0; k < s; ++k) {
-    smem_matmul(m, E, E, X, tid, nt);
+    smem_matmul(m, E, E, T, tid, nt);
     expm_sync<WARP>();
-    for (int i = tid; i < mm; i += nt) E[i] = X[i];
-    expm_sync<WARP>();
+    double2* t = E;
+    E = T;
+    T = t;
   }
   for (int i = tid; i < mm; i += nt) out[(i % m) + (size_t)(i / m) * mld] = E[i];
 }
 
 __global__ void __launch_bounds__(128)
     k_expm(int mld, int nslots, const TileInfo* __restrict__ tiles, const int* __restrict__ map,
-           const double2* __restrict__ Ahess, double2* __restrict__ Aexp, double dt,
-           int* __restrict__ err) {
+           const double2* __restrict__ Ahess, double2* __restrict__ Aexp, double dt, int tri) {
   extern __shared__ double2 sm[];
   __shared__ double rowsum[SPC_MAX_M];
-  __shared__ int piv[SPC_MAX_M];
-  __shared__ int s_sh, p_sh;
+  __shared__ int band[4];
   const int w = blockIdx.x;
   if (w >= nslots || map[w] < 0) return;
   // working dimension m <= mld (the storage leading dimension)
   const int m = tiles[w / SPC_LANES].m;
-  expm_one<false>(m, mld, Ahess + (size_t)w * mld * mld, Aexp + (size_t)w * mld * mld, dt, sm, rowsum, piv,
-                  &s_sh, &p_sh, threadIdx.x, blockDim.x, err);
+  expm_one<false>(m, mld, Ahess + (size_t)w * mld * mld, Aexp + (size_t)w * mld * mld, dt, sm, rowsum, band, tri != 0,
+                  threadIdx.x, blockDim.x);
 }
 
 // Four samples per 128-thread CTA, one warp each (m <= 16); dynamic shared
 // memory 4 x 5 mld^2 complex.
 __global__ void __launch_bounds__(128)
     k_expm_warp(int mld, int nslots, const TileInfo* __restrict__ tiles, const int* __restrict__ map,
-                const double2* __restrict__ Ahess, double2* __restrict__ Aexp, double dt,
-                int* __restrict__ err) {
+                const double2* __restrict__ Ahess, double2* __restrict__ Aexp, double dt, int tri) {
   extern __shared__ double2 sm[];
   __shared__ double rowsum[4][SPC_MAX_M];
-  __shared__ int piv[4][SPC_MAX_M];
-  __shared__ int s_sh[4], p_sh[4];
+  __shared__ int band[4][4];
   const int g = threadIdx.x >> 5;
   const int w = blockIdx.x * 4 + g;
   if (w >= nslots || map[w] < 0) return;
   const int m = tiles[w / SPC_LANES].m;
   expm_one<true>(m, mld, Ahess + (size_t)w * mld * mld, Aexp + (size_t)w * mld * mld, dt,
-                 sm + (size_t)g * 5 * mld * mld, rowsum[g], piv[g], &s_sh[g], &p_sh[g], threadIdx.x & 31, 32,
-                 err);
+                 sm + (size_t)g * 5 * mld * mld, rowsum[g], band[g], tri != 0, threadIdx.x & 31, 32);
 }
 
-// Launch of the expm of every slot: packed warps for m <= 16.
+// Launch of the expm of every slot: packed warps for m <= 16 where the samples
+// fill the SMs (a lone CTA per sample is four times as quick).
 static void launch_expm(int m, int nslots, const TileInfo* tiles, const int* map, const double2* Ahess,
-                        double2* Aexp, double dt, int* err, cudaStream_t st) {
+                        double2* Aexp, double dt, bool tri, int sm_count, cudaStream_t st) {
   const size_t mm = (size_t)m * m;
-  if (m <= 16)
-    k_expm_warp<<<(nslots + 3) / 4, 128, sizeof(double2) * 20 * mm, st>>>(m, nslots, tiles, map, Ahess, Aexp,
-                                                                          dt, err);
+  if (m <= 16 && nslots >= 16 * sm_count)
+    k_expm_warp<<<(nslots + 3) / 4, 128, sizeof(double2) * 20 * mm, st>>>(m, nslots, tiles, map, Ahess, Aexp, dt, tri);
   else
-    k_expm<<<nslots, 128, sizeof(double2) * 5 * mm, st>>>(m, nslots, tiles, map, Ahess, Aexp, dt, err);
+    k_expm<<<nslots, 128, sizeof(double2) * 5 * mm, st>>>(m, nslots, tiles, map, Ahess, Aexp, dt, tri);
 }
 
 // Shared-memory limits of both expm kernels for Krylov dimension m.
@@ -1902,7 +1782,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
       for (size_t c = 0; c < map.size(); ++c)
         if (map[c] >= 0) zsum += tiles[c / SPC_LANES].n / 4;
       pe = h->prof.begin(st);
-      launch_expm(m, nslots, d_tiles, d_map, d_A, d_E, dt, d_err, st);
+      launch_expm(m, nslots, d_tiles, d_map, d_A, d_E, dt, lanczos, h->sm_count, st);
       h->prof.end(st, pe, PK_EXPM, 8.0 * (double)mm * m * 9.0 * list.size(),
                   32.0 * (double)mm * list.size());
       const dim3 pgrid(gram ? 4 * nslots : nslots, ns);
@@ -2066,8 +1946,6 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
       std::chrono::duration<double>(std::chrono::steady_clock::now() - t_start).count();
   if (err_h[0] == 1)
     return set_error(SPC_ERR_NUMERIC, "time index overflow: the dt loop ran past %d output slots", T);
-  if (err_h[0] == 2)
-    return set_error(SPC_ERR_NUMERIC, "singular Pade denominator in expm");
   return SPC_OK;
 }
 
