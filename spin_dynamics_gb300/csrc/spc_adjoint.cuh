@@ -675,8 +675,34 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   gauss_legendre01(nq, xq, wq);
   int64_t builds = 0;
 
+  // Small systems build their bases a sample per CTA (k_small_basis) where the
+  // vectors of every job fit a CTA's shared memory; past 800 row-samples or 8
+  // samples per SM the tiles' launches are full. Whole gradient of 6 steps at
+  // m = 16, per sample against tiled (MGS | Lanczos): dim 288, 96 samples 7.4 :
+  // 10.7 | 4.6 : 6.2 ms, 300 samples 12.3 : 17.3 | 7.1 : 8.4, 600 samples 22.7 :
+  // 24.0 | 12.4 : 11.0; dim 576, 96 samples 11.0 : 13.0 | 6.7 : 7.2, 300 samples
+  // 22.1 : 22.1 | 12.9 : 11.2; dim 24, 1200 samples 15.0 : 17.0 | 6.1 : 7.6.
+  size_t basis_smem = 0;
+  {
+    int nmax = 0;
+    for (int k = 0; k < nj; ++k) nmax = std::max(nmax, nrow[k]);
+    const size_t need = sizeof(double2) * small_basis_elems(m, nmax);
+    if (m <= SMALL_MAX_M && need + SMALL_STATIC <= h->smem_optin && Mtot <= 8 * h->sm_count && elems <= 800.0 * h->sm_count &&
+        h->sample_path != SPC_SAMPLE_OFF) {
+      CK(cudaFuncSetAttribute(k_small_basis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
+      basis_smem = need;
+    }
+  }
   // Krylov basis of the states `x` (psi layout) under the tiles' Hamiltonians
   auto build = [&](const double2* x, const TileInfo* tiles) {
+    if (basis_smem) {
+      const int pe = h->prof.begin(st);
+      k_small_basis<<<nslots, SMALL_THREADS, basis_smem, st>>>(tiles, d_map, d_scol, x, m, lanczos ? 1 : 0, d_Q, d_A, d_c);
+      h->prof.end(st, pe, PK_SAMPLE, 0.0, 0.0);
+      h->count_launch();
+      builds += Mtot;
+      return SPC_OK;
+    }
     CK(cudaMemsetAsync(d_A, 0, sizeof(double2) * mm * nslots, st));
     CK(cudaMemsetAsync(d_qmax, 0, 2 * sizeof(unsigned) * nslots, st));
     BasisRun br{};

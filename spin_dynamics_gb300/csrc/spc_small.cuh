@@ -424,6 +424,45 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
   if (lane == 0) atomicMax(&ort.top, top);
 }
 
+// The Krylov bases of a small system's samples for the yield gradient, one CTA
+// per slot with its vectors in shared memory, written in the tiles' layout. The
+// tiled build of a step is about 4 m launches of kernels that a few hundred rows
+// fill for microseconds: 32 samples at dim 288, m = 16, MGS take 0.72 ms so and
+// 0.38 ms here (FP64 issue: 16 complex entries a row and 136 vector pairs).
+// Dynamic shared memory: A (m^2), c (m), basis (m n), work and state vector (n each).
+__host__ __device__ __forceinline__ size_t small_basis_elems(int m, int n) {
+  return (size_t)m * m + m + (size_t)(m + 2) * n;
+}
+__global__ void __launch_bounds__(SMALL_THREADS)
+    k_small_basis(const TileInfo* __restrict__ tiles, const int* __restrict__ map, const int* __restrict__ scol,
+                  const double2* __restrict__ x, int m, int lanczos, double2* __restrict__ Q,
+                  double2* __restrict__ Ahess, double2* __restrict__ cvec) {
+  extern __shared__ double2 smem[];
+  __shared__ SmallRed red;
+  __shared__ SmallOrtho ort;
+  const int w = blockIdx.x;
+  if (map[w] < 0) return;
+  const TileInfo& T = tiles[w / SPC_LANES];
+  const SmallJob J{T.n, T.n / 4, T.m, T.rowptr, T.split, T.col, T.val, T.kappa, T.rexp, nullptr};
+  const int n = T.n, tid = threadIdx.x;
+  double2* A = smem;
+  double2* cA = A + m * m;
+  double2* V = cA + m;
+  double2* p = V + (size_t)m * n;
+  double2* psi = p + n;
+  const double2* src = x + T.psi_off + scol[w];
+  for (int r = tid; r < n; r += SMALL_THREADS) psi[r] = src[(size_t)r * T.ldp];
+  __syncthreads();
+  int turn = 0;
+  small_krylov(J, lanczos != 0, T.kappa != nullptr, T.kappa != nullptr ? *T.kappa : 0.0, m, A, cA, V, p, psi, red, ort,
+               turn);
+  __syncthreads();
+  for (int k = tid; k < m * m; k += SMALL_THREADS) Ahess[(size_t)w * m * m + k] = A[k];
+  if (tid < m) cvec[(size_t)w * m + tid] = cA[tid];
+  double2* dst = Q + T.q_off + (w % SPC_LANES);
+  for (int k = tid; k < T.m * n; k += SMALL_THREADS) dst[(size_t)k * SPC_LANES] = V[k];
+}
+
 // max |sum_t P_t - I| over the me x me block of the four Grams (NaN wins):
 // the orthonormality of a Lanczos basis (the Grams sum to Q^H Q). Called by
 // all threads; every thread gets the maximum.

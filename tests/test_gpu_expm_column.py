@@ -36,3 +36,32 @@ def test_yields_of_strong_fields(sampler, Bz, g1, g2, method):
     H = dense.hamiltonian(s.e1.g_I, A1, s.e2.g_I, A2, B, s.J, s.D, s.kS, s.kT)
     ref = dense.stepwise_yields(H, zk, DT, num_time_points(DT, t_end), s.kS, s.kT)
     assert np.max(np.abs(np.subtract(got, ref))) <= 1e-11
+
+
+@pytest.mark.parametrize("m", [1, 7, 8, 9, 16, 32])
+@pytest.mark.parametrize("method", ["mgs", "lanczos"])
+def test_gradient_basis_per_sample(sampler, m, method):
+    """The per-sample basis build of small gradients against the tiled one,
+    over blocks of eight vectors and uneven jobs (dims 12, 48 and 288): the
+    same model, so gradients differ by rounding of the steps, below 1e-13 of
+    their norm for 4 steps (a wrong vector shows at its own size)."""
+    rng = np.random.default_rng(9)
+    systems = []
+    for g1, g2 in (((3,), ()), ((2,), (2, 3)), ((2, 2, 3), (3, 2))):
+        A1, A2 = (W._tensors(rng, len(g), -1.5, 1.5, True) for g in (g1, g2))
+        systems.append(SysParam(Electron(g_I=list(g1), A=A1), Electron(g_I=list(g2), A=A2), J=0.03,
+                                D=W.axial_dipolar(-0.3), kS=0.02, kT=0.02))
+    fields = [np.array([0.02, 0.03, 0.04])] * 3
+    zks = [W.random_phase_samples(s.Z, M, seed=M) for s, M in zip(systems, (1, 33, 5))]
+    out = {}
+    sampler.set_krylov(method)
+    try:
+        for mode in ("auto", "off"):
+            sampler.set_sample_path(mode)
+            out[mode] = sampler.yield_gradient_batch(systems, fields, zks, DT, 4 * DT, m)
+    finally:
+        sampler.set_sample_path("auto")
+        sampler.set_krylov("mgs")
+    for a, b in zip(out["auto"], out["off"]):
+        assert abs(a.Phi_S - b.Phi_S) <= 1e-13 and abs(a.Phi_T - b.Phi_T) <= 1e-13
+        assert np.linalg.norm(a.raw - b.raw) <= 1e-13 * np.linalg.norm(b.raw)
