@@ -26,7 +26,6 @@
 #define SMALL_THREADS 256
 #define SMALL_WARPS (SMALL_THREADS / 32)
 #define SMALL_MAX_M 32
-#define SMALL_ROUNDS 5   // dt-loop pair rounds over 128 threads: 32 * 33 / 2 <= 5 * 128
 #define SMALL_NMAX 2048
 #define SMALL_GRAM_R(mt) ((mt) == 1 ? 32 : 16)  // rows per chunk of the Grams: two CTAs' scratch in an SM at m = 20
 #define SMALL_STATIC 12288  // at least the kernels' static shared memory
@@ -41,27 +40,6 @@ struct SmallJob {
   int rexp;                // ||H|| <= 2^rexp
   const double2* zk;       // M x Z sample vectors of the job
 };
-
-// Stop test of the dt loop, |c_{me-1}|^2 <= tol |c|^2, for the coordinates in a
-// warp's lanes (zero past me). In single precision where that decides it (two
-// sides apart by more than its rounding): five FP64 adds with their shuffles
-// take 545 clocks, more than half of a step's products.
-__device__ __forceinline__ bool krylov_holds(double2 c, int me, double tol) {
-  const float x = (float)c.x, y = (float)c.y;
-  const float own = x * x + y * y;
-  float s = own;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  const float last = __shfl_sync(0xffffffffu, own, me - 1), lim = (float)tol * s;
-  if (lim > 1e-30f && lim < 1e30f && fabsf(last - lim) > 1e-4f * lim) return last <= lim;
-  const double n2 = warp_sum(fma(c.x, c.x, c.y * c.y));
-  const double l2 = __shfl_sync(0xffffffffu, c.x * c.x + c.y * c.y, me - 1);
-  return l2 <= tol * n2;
-}
-
-// Barrier of warps 0-3 (the dt loop's warps; the others wait at the next
-// __syncthreads).
-__device__ __forceinline__ void small_bar4() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 // Sum over the CTA of values whose absolute sum is at most 2^e, or with NORM its
 // square root and that root's reciprocal (0 for a zero sum): every thread gets
@@ -514,7 +492,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2)
   __shared__ int band[4];
   __shared__ SmallRed red;
   __shared__ SmallOrtho ort;
-  __shared__ double2 part[SMALL_WARPS][32];
+  __shared__ double2 part[4][32];
   __shared__ double terms[16];
   __shared__ double cstat[2];
   __shared__ double loop_t;
@@ -565,106 +543,14 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2)
     nb++;
     expm_one<false>(me, m, A, E, dt, X, rowsum, band, lz, tid, SMALL_THREADS);
     __syncthreads();
-    // dt loop (:348-364): c <- E c; P_X(t) = Re(c^H P_X c); stop when the
-    // last Krylov coordinate grows past tol or the window ends. It runs on
-    // warps 0-3, one per scheduler: GB300's FP64 pipe sits in each scheduler
-    // and a warp instruction holds it for the same time whatever its active
-    // lanes, so the step is laid out to issue few FP64 warp instructions:
-    //  * c' = E c with lane = row and warp w over the columns j = w mod 4 (c_j
-    //    by shuffle); every warp adds the four partials in warp order, so
-    //    each holds c' in its lanes and no further barrier is needed;
-    //  * the four forms over the pairs i <= j, with the Hermitian weights in
-    //    W = (s Re P_ij, -s Im P_ij) (s = 1 on the diagonal, 2 above it) and
-    //    g_ij = conj(c_i) c_j shared by the types: 12 FP64 operations a pair;
-    //  * each warp's four sums by a reduce-scatter over its lanes (6 adds
-    //    instead of 20), then the warps' sums added in warp order.
-    // Warps 4-7 wait at the barrier after the loop.
-    const int npair = me * (me + 1) / 2;
     double2* W = X;  // 4 x npair weights in the spent expm scratch
-    for (int idx = tid; idx < 4 * npair; idx += SMALL_THREADS) {
-      const int ty = idx / npair;
-      int rem = idx % npair, i = 0;
-      while (rem >= me - i) {
-        rem -= me - i;
-        ++i;
-      }
-      const double2 pv = P[ty * mm + i + (size_t)(i + rem) * m];
-      const double sw = rem == 0 ? 1.0 : 2.0;
-      W[idx] = make_double2(sw * pv.x, -sw * pv.y);
-    }
+    dt_weights(m, me, P, W, tid, SMALL_THREADS);
     __syncthreads();
     if (warp < 4) {
-      int pi[SMALL_ROUNDS], pj[SMALL_ROUNDS];
-#pragma unroll
-      for (int r = 0; r < SMALL_ROUNDS; ++r) {
-        pi[r] = -1;
-        pj[r] = 0;
-        int rem = r * 128 + tid;
-        if (rem < npair) {
-          int i = 0;
-          while (rem >= me - i) {
-            rem -= me - i;
-            ++i;
-          }
-          pi[r] = i;
-          pj[r] = i + rem;
-        }
-      }
       double2 c = lane < me ? cA[lane] : cz();
-      bool go = true;
-      while (go && t < t_end) {
-        if (k >= T) {  // output full (guard; every thread takes it)
-          if (tid == 0) atomicExch(err, 1);
-          done = true;
-          break;
-        }
-        double2 a = cz();
-        for (int j = warp; j < me; j += 4) {
-          const double2 cj = make_double2(__shfl_sync(0xffffffffu, c.x, j), __shfl_sync(0xffffffffu, c.y, j));
-          if (lane < me) a = cfma(E[lane + j * m], cj, a);
-        }
-        part[warp][lane] = a;
-        small_bar4();
-        double2 cn = cz();
-        if (lane < me) cn = cadd(cadd(cadd(part[0][lane], part[1][lane]), part[2][lane]), part[3][lane]);
-        double f0 = 0.0, f1 = 0.0, f2 = 0.0, f3 = 0.0;
-#pragma unroll
-        for (int r = 0; r < SMALL_ROUNDS; ++r) {
-          if (r * 128 + warp * 32 >= npair) break;  // no pair of this warp left
-          const int i = max(pi[r], 0), j = pj[r];
-          const double cix = __shfl_sync(0xffffffffu, cn.x, i), ciy = __shfl_sync(0xffffffffu, cn.y, i);
-          const double cjx = __shfl_sync(0xffffffffu, cn.x, j), cjy = __shfl_sync(0xffffffffu, cn.y, j);
-          if (pi[r] >= 0) {
-            const double gx = fma(cix, cjx, ciy * cjy), gy = fma(cix, cjy, -ciy * cjx);
-            const int pp = r * 128 + tid;
-            const double2 w0 = W[pp], w1 = W[npair + pp], w2 = W[2 * npair + pp], w3 = W[3 * npair + pp];
-            f0 = fma(w0.x, gx, fma(w0.y, gy, f0));
-            f1 = fma(w1.x, gx, fma(w1.y, gy, f1));
-            f2 = fma(w2.x, gx, fma(w2.y, gy, f2));
-            f3 = fma(w3.x, gx, fma(w3.y, gy, f3));
-          }
-        }
-        // reduce-scatter: lanes 8t..8t+7 end with the warp's sum of form t
-        const bool h16 = (lane & 16) != 0, h8 = (lane & 8) != 0;
-        double ka = h16 ? f2 : f0, kb = h16 ? f3 : f1;
-        ka += __shfl_xor_sync(0xffffffffu, h16 ? f0 : f2, 16);
-        kb += __shfl_xor_sync(0xffffffffu, h16 ? f1 : f3, 16);
-        double v = h8 ? kb : ka;
-        v += __shfl_xor_sync(0xffffffffu, h8 ? ka : kb, 8);
-        v += __shfl_xor_sync(0xffffffffu, v, 4);
-        v += __shfl_xor_sync(0xffffffffu, v, 2);
-        v += __shfl_xor_sync(0xffffffffu, v, 1);
-        if ((lane & 7) == 0) terms[4 * warp + (lane >> 3)] = v;
-        small_bar4();
-        if (tid < 4) {
-          const int slot = tid == 0 ? 2 : (tid == 1 ? 0 : (tid == 2 ? 1 : 3));  // proj type -> obs slot
-          o[slot * T + k] = ((terms[tid] + terms[4 + tid]) + terms[8 + tid]) + terms[12 + tid];
-        }
-        go = krylov_holds(cn, me, tol);
-        c = cn;
-        t = t + dt;
-        k = k + 1;
-        steps++;
+      if (dt_steps(m, me, E, W, c, t, k, steps, T, dt, t_end, tol, o, part, terms)) {
+        if (tid == 0) atomicExch(err, 1);
+        done = true;
       }
       if (warp == 0 && lane < me) cA[lane] = c;  // for psi = Q c
       if (tid == 0) {
@@ -674,7 +560,7 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2)
         loop_done = done ? 1 : 0;
       }
     }
-    __syncthreads();
+    __syncthreads();  // warps 4-7 wait here
     t = loop_t;
     k = loop_k;
     steps = loop_steps;
@@ -866,20 +752,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SMALL_THREADS, 1)
           ctrl.ok = okv ? 1 : 0;
           ctrl_main->ok = okv ? 1 : 0;
         }
-        // Hermitian weights W_t = (s Re P_t, -s Im P_t) of the pairs i <= j
-        // (s = 1 on the diagonal, 2 above it) and the pair table
-        for (int idx = tid; idx < 4 * npair; idx += SMALL_THREADS) {
-          const int ty = idx / npair;
-          int rem = idx % npair, i = 0;
-          while (rem >= me - i) {
-            rem -= me - i;
-            ++i;
-          }
-          const double2 pv = P[ty * mm + i + (size_t)(i + rem) * m];
-          const double sw = rem == 0 ? 1.0 : 2.0;
-          W[idx] = make_double2(sw * pv.x, -sw * pv.y);
-          if (ty == 0) pij[idx] = make_int2(i, i + rem);
-        }
+        dt_weights(m, me, P, W, tid, SMALL_THREADS);
+        for (int idx = tid; idx < npair; idx += SMALL_THREADS) pij[idx] = dt_pair(me, idx);
         __syncthreads();
       }
       // dt loop (:348-364) in segments of at most hmax steps. Main CTA, warps

@@ -78,3 +78,24 @@ def test_undefined_samples_stay_undefined(sampler):
         sampler.set_sample_path("auto")
     for k in KEYS:
         assert np.all(np.isnan(getattr(got, k)[1:5]))
+
+
+@pytest.mark.parametrize("m", [7, 8, 9, 16, 17, 32])
+@pytest.mark.parametrize("more", [0, 1])
+def test_dt_loop_forms(sampler, oracle, m, more):
+    """As many samples as the dt loop takes on a CTA each, and one more (packed
+    into warps up to m = 16)."""
+    import torch
+    s = pair((2,), (2, 3))
+    B = np.array([0.01, 0.03, 0.04])
+    M = 7 * torch.cuda.get_device_properties(0).multi_processor_count + more
+    rp, col, val = general_csr(oracle, s, B)
+    zk = W.random_phase_samples(s.Z, M, seed=m)
+    ref = oracle.trace_sampling(rp, col, val, zk, DT, 30 * DT, m, 1e-6)
+    sampler.set_sample_path("off")
+    try:
+        sampler.build_h(s, B, "general")
+        got = sampler.trace_sampling(zk, DT, 30 * DT, m, 1e-6)
+    finally:
+        sampler.set_sample_path("auto")
+    assert max(np.max(np.abs(getattr(got, k) - ref[k])) for k in KEYS) <= 1e-12
