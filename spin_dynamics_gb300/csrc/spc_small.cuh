@@ -134,13 +134,32 @@ __device__ __forceinline__ double2 block_norm(double v, SmallRed& red, int& turn
   return res;
 }
 
-// Row r of H x. Entries are taken four at a time, all loads before the sums: a
-// row has 4 to 20 entries, and their latency, not their arithmetic, is a row's
-// time. shift adds -i*kappa*x_r.
-__device__ __forceinline__ double2 small_row(const SmallJob& J, const double2* __restrict__ x, int r, bool shift,
+// Vectors are taken by components: thread idx has component idx & 1 (real,
+// imaginary) of row idx / 2, the order in memory. A warp instruction of FP64
+// holds its scheduler's pipe for 64 clocks whatever the lanes in use, and the
+// 288 rows of a small pair are nine warps on four schedulers (three on one);
+// as 576 components they are five half-rows at most against six, and where rows
+// are few a row's chain of multiply-adds is half as long: 64 samples at dim 288,
+// m = 20, 5000 steps 24.3 -> 22.1 ms; dim 48, m = 10 1.98 -> 1.88 ms.
+__device__ __forceinline__ double flip(double v, bool neg) {
+  return __hiloint2double(__double2hiint(v) ^ (neg ? (int)0x80000000 : 0), __double2loint(v));
+}
+// component im of a + v q for the complex v, q
+__device__ __forceinline__ double half_fma(double2 v, double2 q, bool im, double a) {
+  a = fma(v.x, im ? q.y : q.x, a);
+  return fma(flip(v.y, !im), im ? q.x : q.y, a);
+}
+
+// Component idx of H x. Entries are taken four at a time, all loads before the
+// sums: a row has 4 to 20 entries, and their latency, not their arithmetic, is
+// a row's time. shift adds -i*kappa*x_r.
+__device__ __forceinline__ double small_half(const SmallJob& J, const double2* __restrict__ x, int idx, bool shift,
                                              double kap) {
+  const int r = idx >> 1;
+  const bool im = (idx & 1) != 0;
   const int k0 = __ldg(J.rowptr + r), ks = __ldg(J.split + r), k1 = __ldg(J.rowptr + r + 1);
-  double2 a0 = cz(), a1 = cz();
+  const double* xd = reinterpret_cast<const double*>(x) + (idx & 1);
+  double a0 = 0.0, a1 = 0.0;
   for (int k = k0; k < ks; k += 4) {
     double2 v[4], q[4];
 #pragma unroll
@@ -153,35 +172,43 @@ __device__ __forceinline__ double2 small_row(const SmallJob& J, const double2* _
     for (int u = 0; u < 4; ++u)
       if (k + u < ks) {
         if (u & 1)
-          a1 = cfma(v[u], q[u], a1);
+          a1 = half_fma(v[u], q[u], im, a1);
         else
-          a0 = cfma(v[u], q[u], a0);
+          a0 = half_fma(v[u], q[u], im, a0);
       }
   }
   for (int k = ks; k < k1; k += 4) {
-    double v[4];
-    double2 q[4];
+    double v[4], q[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const bool in = k + u < k1;
       v[u] = in ? __ldg(&J.val[k + u].x) : 0.0;
-      q[u] = x[in ? __ldg(J.col + k + u) : r];
+      q[u] = xd[2 * (in ? __ldg(J.col + k + u) : r)];
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u)
       if (k + u < k1) {
-        double2& a = (u & 1) ? a1 : a0;
-        a.x = fma(v[u], q[u].x, a.x);
-        a.y = fma(v[u], q[u].y, a.y);
+        if (u & 1)
+          a1 = fma(v[u], q[u], a1);
+        else
+          a0 = fma(v[u], q[u], a0);
       }
   }
-  double2 y = cadd(a0, a1);
+  double y = a0 + a1;
   if (shift) {
     const double2 xr = x[r];
-    y.x = fma(kap, xr.y, y.x);
-    y.y = fma(-kap, xr.x, y.y);
+    y = fma(flip(kap, im), im ? xr.x : xr.y, y);
   }
   return y;
+}
+
+// psi = Q c (:365) by components, over all threads of the CTA
+__device__ __forceinline__ void small_psi(int me, int n, const double2* Q, const double2* c, double2* psi) {
+  for (int idx = threadIdx.x; idx < 2 * n; idx += SMALL_THREADS) {
+    double a = 0.0;
+    for (int j = 0; j < me; ++j) a = half_fma(c[j], Q[(size_t)j * n + (idx >> 1)], (idx & 1) != 0, a);
+    reinterpret_cast<double*>(psi)[idx] = a;
+  }
 }
 
 // The four projector Grams P_t = V_t^H V_t over the Z nuclear rows (k_gram and
@@ -247,49 +274,42 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
   const int n = J.n, me = J.me, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const size_t mm = (size_t)m * m;
   for (int i = tid; i < (int)mm; i += SMALL_THREADS) A[i] = cz();
+  double* pd = reinterpret_cast<double*>(p);
+  double* Qd = reinterpret_cast<double*>(Q);
+  const double* psid = reinterpret_cast<const double*>(psi);
   // c = ||psi|| e_1, Q_0 = psi / ||psi|| (get_krylov :440-447)
   double acc = 0.0;
-  for (int r = tid; r < n; r += SMALL_THREADS) {
-    const double2 x = psi[r];
-    acc = fma(x.x, x.x, acc);
-    acc = fma(x.y, x.y, acc);
-  }
+  for (int idx = tid; idx < 2 * n; idx += SMALL_THREADS) acc = fma(psid[idx], psid[idx], acc);
   const double2 bn0 = block_norm(acc, red, turn);
   unsigned top = 0;
   if (tid == 0) ort.top = 0;
-  for (int r = tid; r < n; r += SMALL_THREADS) {
-    const double2 x = psi[r];
-    const double2 q = make_double2(x.x * bn0.y, x.y * bn0.y);
-    Q[r] = q;
-    top = max(top, abs_high(q));
+  for (int idx = tid; idx < 2 * n; idx += SMALL_THREADS) {
+    const double q = psid[idx] * bn0.y;
+    Qd[idx] = q;
+    top = max(top, (unsigned)__double2hiint(q) & 0x7fffffffu);
   }
   if (tid < m) cA[tid] = tid == 0 ? make_double2(bn0.x, 0.0) : cz();
   __syncthreads();
   double beta = 0.0;
   for (int i = 0; i < me; ++i) {
     const double2* qi = Q + (size_t)i * n;
+    const double* qid = Qd + (size_t)i * 2 * n;
     double alpha = 0.0;
     int na = 0, ja = 0;  // the block whose projection is still to be subtracted
     if (lz) {
       // p = H q_i - beta_{i-1} Q_{i-1}; alpha_i = Re <Q_i, p>
       double a2 = 0.0;
-      for (int r = tid; r < n; r += SMALL_THREADS) {
-        double2 pv = small_row(J, qi, r, false, kap);
-        if (i > 0) {
-          const double2 q = qi[r - n];
-          pv.x = fma(-beta, q.x, pv.x);
-          pv.y = fma(-beta, q.y, pv.y);
-        }
-        p[r] = pv;
-        const double2 x = qi[r];
-        a2 = fma(x.x, pv.x, a2);
-        a2 = fma(x.y, pv.y, a2);
+      for (int idx = tid; idx < 2 * n; idx += SMALL_THREADS) {
+        double pv = small_half(J, qi, idx, false, kap);
+        if (i > 0) pv = fma(-beta, qid[idx - 2 * n], pv);
+        pd[idx] = pv;
+        a2 = fma(qid[idx], pv, a2);
       }
       alpha = block_sum<false>(a2, J.rexp, red, turn).x;
       if (tid == 0) A[i + i * m] = make_double2(alpha, -kap);
       if (i == me - 1) break;
     } else {
-      for (int r = tid; r < n; r += SMALL_THREADS) p[r] = small_row(J, qi, r, herm, kap);
+      for (int idx = tid; idx < 2 * n; idx += SMALL_THREADS) pd[idx] = small_half(J, qi, idx, herm, kap);
       // MGS (get_krylov :453-456) by blocks: d_v = <Q_v, p>, h_v from the d_v and
       // the block's basis products, p -= sum_v h_v Q_v
       for (int jb = 0; jb <= i; jb += ORTHO_NB) {
@@ -357,11 +377,15 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
             ja = jb;
             na = nb;
           } else {
-            for (int r = tid; r < n; r += SMALL_THREADS) {
-              double2 pv = p[r];
+            for (int idx = tid; idx < 2 * n; idx += SMALL_THREADS) {
+              const bool im = (idx & 1) != 0;
+              double pv = pd[idx];
 #pragma unroll
-              for (int v = 0; v < ORTHO_NB; ++v) pv = cfms(ort.h[v], Q[(size_t)(jb + v) * n + r], pv);
-              p[r] = pv;
+              for (int v = 0; v < ORTHO_NB; ++v) {
+                const double2 h = ort.h[v];
+                pv = half_fma(make_double2(-h.x, -h.y), Q[(size_t)(jb + v) * n + (idx >> 1)], im, pv);
+              }
+              pd[idx] = pv;
             }
           }
         }
@@ -370,18 +394,18 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
     }
     // the last projection, ||p|| and Q_{i+1} = p / ||p||
     double nr = 0.0;
-    for (int r = tid; r < n; r += SMALL_THREADS) {
-      double2 pv = p[r];
+    for (int idx = tid; idx < 2 * n; idx += SMALL_THREADS) {
+      double pv = pd[idx];
       if (lz) {
-        const double2 q = qi[r];
-        pv.x = fma(-alpha, q.x, pv.x);
-        pv.y = fma(-alpha, q.y, pv.y);
+        pv = fma(-alpha, qid[idx], pv);
       } else {
-        for (int v = 0; v < na; ++v) pv = cfms(ort.h[v], Q[(size_t)(ja + v) * n + r], pv);
+        for (int v = 0; v < na; ++v) {
+          const double2 h = ort.h[v];
+          pv = half_fma(make_double2(-h.x, -h.y), Q[(size_t)(ja + v) * n + (idx >> 1)], (idx & 1) != 0, pv);
+        }
       }
-      p[r] = pv;
-      nr = fma(pv.x, pv.x, nr);
-      nr = fma(pv.y, pv.y, nr);
+      pd[idx] = pv;
+      nr = fma(pv, pv, nr);
     }
     const double2 bn = block_sum<true>(nr, 2 * J.rexp, red, turn);
     beta = bn.x;
@@ -389,12 +413,11 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
       A[(i + 1) + i * m] = make_double2(beta, 0.0);
       if (lz) A[i + (i + 1) * m] = make_double2(beta, 0.0);
     }
-    double2* qn = Q + (size_t)(i + 1) * n;
-    for (int r = tid; r < n; r += SMALL_THREADS) {
-      const double2 pv = p[r];
-      const double2 q = make_double2(pv.x * bn.y, pv.y * bn.y);
-      qn[r] = q;
-      top = max(top, abs_high(q));
+    double* qn = Qd + (size_t)(i + 1) * 2 * n;
+    for (int idx = tid; idx < 2 * n; idx += SMALL_THREADS) {
+      const double q = pd[idx] * bn.y;
+      qn[idx] = q;
+      top = max(top, (unsigned)__double2hiint(q) & 0x7fffffffu);
     }
     __syncthreads();
   }
@@ -565,16 +588,8 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2)
     k = loop_k;
     steps = loop_steps;
     done = loop_done != 0;
-    const double2* c = cA;
     if (!done) done = !(t < t_end);
-    if (!done) {
-      // psi = Q c (:365)
-      for (int r = tid; r < n; r += SMALL_THREADS) {
-        double2 acc3 = cz();
-        for (int j = 0; j < me; ++j) acc3 = cfma(Q[(size_t)j * n + r], c[j], acc3);
-        psi[r] = acc3;
-      }
-    }
+    if (!done) small_psi(me, n, Q, cA, psi);
     // c lives in cA; the next build rewrites it after a barrier
     __syncthreads();
   }
@@ -836,14 +851,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SMALL_THREADS, 1)
       steps = steps_build;
     }
     nb++;
-    if (rank == 0 && !done) {
-      // psi = Q c (:365)
-      for (int r = tid; r < n; r += SMALL_THREADS) {
-        double2 acc3 = cz();
-        for (int j = 0; j < me; ++j) acc3 = cfma(Q[(size_t)j * n + r], cA[j], acc3);
-        psi[r] = acc3;
-      }
-    }
+    if (rank == 0 && !done) small_psi(me, n, Q, cA, psi);
     __syncthreads();
   }
   // keep the helper's shared memory alive until the main CTA's last remote
