@@ -1,12 +1,21 @@
 // The dt loop (src/qm_dynamics.f90:348-364) of one sample on four warps, for
 // Krylov dimensions up to 32. Included by spc_propagate.cu inside namespace spc.
 
+// (float)v, cut off instead of rounded, from the words of v: the conversion
+// instruction holds the FP64 pipe as a multiply-add does.
+__device__ __forceinline__ float cut_float(double v) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const int e = (int)(hi >> 20 & 0x7ff) - 896;
+  const unsigned mag = e <= 0 ? 0u : e >= 255 ? 0x7f800000u : (unsigned)e << 23 | (hi & 0xfffff) << 3 | lo >> 29;
+  return __uint_as_float((hi & 0x80000000u) | mag);
+}
+
 // Stop test of the dt loop, |c_{me-1}|^2 <= tol |c|^2, for the coordinates in a
 // warp's lanes (zero past me). In single precision where that decides it (two
 // sides apart by more than its rounding): five FP64 adds with their shuffles
 // take 545 clocks, more than half of a step's products.
 __device__ __forceinline__ bool krylov_holds(double2 c, int me, double tol) {
-  const float x = (float)c.x, y = (float)c.y;
+  const float x = cut_float(c.x), y = cut_float(c.y);
   const float own = x * x + y * y;
   float s = own;
 #pragma unroll
@@ -21,6 +30,7 @@ __device__ __forceinline__ bool krylov_holds(double2 c, int me, double tol) {
 // Barrier of warps 0-3 (the dt loop's warps; a CTA's others wait at its next
 // __syncthreads).
 __device__ __forceinline__ void small_bar4() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ void small_bar5() { asm volatile("bar.sync 2, 160;" ::: "memory"); }  // of warps 0-4
 
 // pair number idx of (i, j >= i) in row order
 __device__ __forceinline__ int2 dt_pair(int me, int idx) {

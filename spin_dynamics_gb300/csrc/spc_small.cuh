@@ -616,8 +616,8 @@ __global__ void __launch_bounds__(SMALL_THREADS, 2)
 //    segments of at most hmax steps (two buffers): the helper evaluates a
 //    segment while the main CTA runs the next one, psi = Q c and the next
 //    Krylov build.
-// The main CTA's dt step is then c' = E c on four warps (one barrier) and the
-// stop test, which each of the four warps evaluates on its own copy of c'.
+// The main CTA's dt step is then c' = E c on four warps and the stop test on a
+// fifth, beside the next step.
 // Control flow is uniform across the cluster: a flag that ends a loop is
 // written to both CTAs' shared memory before a cluster barrier and read after
 // it, and every thread of both CTAs reaches every cluster barrier. The
@@ -690,7 +690,7 @@ __host__ __device__ __forceinline__ size_t pair_help_elems(int m, int hmax) {
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SMALL_THREADS, 1)
     k_small_pair(const SmallJob* __restrict__ jobs, const int* __restrict__ sjob, const int* __restrict__ scol,
                  const int64_t* __restrict__ soff, double2* __restrict__ work, Theta th, int m, int T, double dt,
-                 double t_end, double tol, int lanczos, int vec_smem, int hmax, double* __restrict__ obs,
+                 int nstep, double tol, int lanczos, int vec_smem, int hmax, double* __restrict__ obs,
                  long long* __restrict__ nsteps, unsigned long long* __restrict__ counts, int* __restrict__ err) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
@@ -699,9 +699,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SMALL_THREADS, 1)
   __shared__ int band[4];
   __shared__ SmallRed red;
   __shared__ SmallOrtho ort;
-  __shared__ double2 part[2][4][32];
+  __shared__ double part[4][2 * SMALL_MAX_M];
   __shared__ double terms[16];
   __shared__ double cstat[2];
+  __shared__ int holds;
   __shared__ PairCtrl ctrl;
 
   const int rank = (int)cluster.block_rank();
@@ -742,17 +743,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SMALL_THREADS, 1)
     for (int r = tid; r < n; r += SMALL_THREADS) psi[r] = cmul(th.v[r / Z], zk[r % Z]);
   }
   __syncthreads();
-  double t = 0.0;
-  int k = 1;  // outputs 0 hold the initial populations (k_obs_init)
-  long long steps = 0;
+  // The dt loop's layout: thread (part q, component x) of warps 0-3 has columns
+  // [q ncol, (q + 1) ncol) of row x / 2
+  const int nq = min(4, 64 / me), ncol = (me + nq - 1) / nq;
+  const int dq = tid / (2 * me), dx = tid - dq * 2 * me;
+  const bool dimag = (dx & 1) != 0;
+  int k = 1;  // outputs 0 hold the initial populations (k_obs_init); steps done: k - 1
   int turn = 0;
   unsigned long long nb = 0, nf = 0;
-  bool done = !(0.0 < t_end);
+  bool done = nstep == 0;
   while (!done) {
     bool lz = lanczos != 0 && herm;
-    const double t_build = t;
     const int k_build = k;
-    const long long steps_build = steps;
     for (int attempt = 0; attempt < 2; ++attempt) {
       if (rank == 0) small_krylov(J, lz, herm, kap, m, A, cA, Q, p, psi, red, ort, turn);
       cluster.sync();  // basis, A and c complete
@@ -771,50 +773,72 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SMALL_THREADS, 1)
         for (int idx = tid; idx < npair; idx += SMALL_THREADS) pij[idx] = dt_pair(me, idx);
         __syncthreads();
       }
-      // dt loop (:348-364) in segments of at most hmax steps. Main CTA, warps
-      // 0-3: c' = E c with lane = row and warp w over the columns j = w mod 4
-      // (c_j by shuffle), the four partials (double-buffered by step parity)
-      // added in warp order by every warp, and the stop test by every warp;
-      // warp 0 stores c' into the helper's history. The first segment runs while
-      // the helper forms the Grams and the check of the same basis: a basis that
-      // fails it is rebuilt, and the segment's steps count for nothing.
-      double2 c = (rank == 0 && lane < me) ? cA[lane] : cz();
-      bool go = true;  // the last Krylov coordinate is within the tolerance
-      int buf = 0;
+      // dt loop (:348-364) in segments of at most hmax steps. The first segment
+      // runs while the helper forms the Grams and the check of the same basis: a
+      // basis that fails it is rebuilt, and the segment's steps count for nothing.
+      // c lives in cA. A step is bound by the FP64 pipes of four schedulers and by
+      // latency, so it is laid out for few FP64 instructions in a row: c' = E c by
+      // components, 2 ncol multiply-adds a thread on coefficients in registers,
+      // the parts added by one thread a component; steps are counted (nstep, the
+      // host's count of the reference's t < t_end loop) instead of adding t; and
+      // warp 4 stores c' into the helper's history and applies the stop test while
+      // warps 0-3 already form the next step, which counts for nothing after the
+      // last. Before (lane = row, every warp adding the parts, testing and
+      // carrying t) a step at m = 20 took 3060 clocks, now 1860: 64 samples at
+      // dim 288, 5000 steps 22.1 -> 19.0 ms; dim 48, m = 10, 500 steps 1.88 -> 1.64 ms.
       bool ok = true;
+      int buf = 0;
       for (;;) {
         if (rank == 0) {
-          if (warp < 4) {
+          if (warp < 5) {
+            double2 ec[SMALL_MAX_M / 2];
+#pragma unroll
+            for (int u = 0; u < SMALL_MAX_M / 2; ++u) {
+              const int j = dq * ncol + u;
+              ec[u] = dq < nq && u < ncol && j < me ? E[(dx >> 1) + j * m] : cz();
+              ec[u].y = flip(ec[u].y, !dimag);
+            }
             double2* hist = H_help + (size_t)buf * hmax * m;
             const int k0 = k;
             int cnt = 0;
-            bool overflow = false;
-            while (cnt < hmax && go && t < t_end) {
-              if (k >= T) {  // output full (guard; every chain thread takes it)
-                overflow = true;
-                break;
+            bool go = true, overflow = false;
+            for (;;) {
+              const bool last = cnt == hmax || k > nstep;
+              const bool full = !last && k >= T;  // output full (guard; every chain thread takes it)
+              if (warp == 4) {
+                if (cnt > 0) {
+                  const double2 c = lane < me ? cA[lane] : cz();
+                  if (lane < me) hist[(size_t)(cnt - 1) * m + lane] = c;
+                  const bool in = krylov_holds(c, me, tol);
+                  if (lane == 0) holds = in ? 1 : 0;
+                }
+              } else if (!last && !full && dq < nq) {
+                double a = 0.0;
+#pragma unroll
+                for (int u = 0; u < SMALL_MAX_M / 2; ++u) {
+                  if (u >= ncol) break;
+                  const double2 c = cA[min(dq * ncol + u, me - 1)];
+                  a = fma(ec[u].x, dimag ? c.y : c.x, a);
+                  a = fma(ec[u].y, dimag ? c.x : c.y, a);
+                }
+                part[dq][dx] = a;
               }
-              double2 a = cz();
-              for (int j = warp; j < me; j += 4) {
-                const double2 cj = make_double2(__shfl_sync(0xffffffffu, c.x, j), __shfl_sync(0xffffffffu, c.y, j));
-                if (lane < me) a = cfma(E[lane + j * m], cj, a);
+              small_bar5();
+              if (cnt > 0) go = holds != 0;
+              overflow = go && full;
+              if (!go || last || full) break;
+              if (tid < 2 * me) {
+                double a = part[0][tid];
+                if (nq > 1) a += part[1][tid];
+                if (nq > 2) a += nq > 3 ? part[2][tid] + part[3][tid] : part[2][tid];
+                reinterpret_cast<double*>(cA)[tid] = a;
               }
-              part[cnt & 1][warp][lane] = a;
-              small_bar4();
-              double2 cn = cz();
-              if (lane < me)
-                cn = cadd(cadd(cadd(part[cnt & 1][0][lane], part[cnt & 1][1][lane]), part[cnt & 1][2][lane]),
-                          part[cnt & 1][3][lane]);
-              if (warp == 0 && lane < me) hist[(size_t)cnt * m + lane] = cn;
-              go = krylov_holds(cn, me, tol);
-              c = cn;
-              t = t + dt;
+              small_bar5();
               k = k + 1;
-              steps++;
               cnt++;
             }
-            const bool more = !overflow && cnt == hmax && go && t < t_end;
-            const bool dn = overflow || (!more && !(t < t_end));
+            const bool more = !overflow && cnt == hmax && go && k <= nstep;
+            const bool dn = overflow || (!more && k > nstep);
             if (tid == 0) {
               ctrl.over = overflow ? 1 : 0;
               ctrl.more[buf] = more ? 1 : 0;
@@ -824,7 +848,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SMALL_THREADS, 1)
               ctrl_help->more[buf] = more ? 1 : 0;
               ctrl_help->done[buf] = dn ? 1 : 0;
             }
-            if (!more && warp == 0 && lane < me) cA[lane] = c;  // for psi = Q c
           }
           __syncthreads();
         }
@@ -846,9 +869,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SMALL_THREADS, 1)
       cluster.sync();
       nf++;
       lz = false;  // rebuild this basis with full MGS
-      t = t_build;
       k = k_build;
-      steps = steps_build;
     }
     nb++;
     if (rank == 0 && !done) small_psi(me, n, Q, cA, psi);
@@ -858,7 +879,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SMALL_THREADS, 1)
   // access has completed
   cluster.sync();
   if (rank == 0 && tid == 0) {
-    atomicAdd((unsigned long long*)nsteps, (unsigned long long)steps);
+    atomicAdd((unsigned long long*)nsteps, (unsigned long long)(k - 1));
     atomicAdd(&counts[0], nb);
     atomicAdd(&counts[1], nf);
   }
@@ -1000,9 +1021,12 @@ static int propagate_small(Handle* h, const double* theta, const double* init_po
   }
   int pe = h->prof.begin(st);
   if (pair) {
+    // steps of the reference's loop (t += dt while t < t_end), past T the guard's
+    int nstep = 0;
+    for (double t = 0.0; t < t_end && nstep < T; t = t + dt) ++nstep;
     k_small_pair<<<2 * G, SMALL_THREADS, psmem, st>>>((const SmallJob*)plan, (const int*)(plan + o_sjob),
                                                       (const int*)(plan + o_scol), (const int64_t*)(plan + o_soff),
-                                                      (double2*)h->Q.p, th, m, T, dt, t_end, tol, lanczos ? 1 : 0,
+                                                      (double2*)h->Q.p, th, m, T, dt, nstep, tol, lanczos ? 1 : 0,
                                                       pvec ? 1 : 0, hmax, d_obs, d_nsteps, d_counts, d_err);
   } else {
     const size_t vbytes = sizeof(double2) * (size_t)(m + 2) * nmax;

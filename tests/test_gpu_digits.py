@@ -99,3 +99,30 @@ def test_dt_loop_forms(sampler, oracle, m, more):
     finally:
         sampler.set_sample_path("auto")
     assert max(np.max(np.abs(getattr(got, k) - ref[k])) for k in KEYS) <= 1e-12
+
+
+@pytest.mark.parametrize("mode", ["on", "single"])
+@pytest.mark.parametrize("m, steps, scale", [(1, 2, 1.0), (2, 9, 1.0), (7, 40, 1.0), (15, 60, 1.0), (16, 60, 1.0),
+                                             (17, 60, 1.0), (21, 60, 1.0), (22, 60, 1.0), (31, 60, 1.0), (32, 60, 1.0),
+                                             (12, 63, 0.02), (12, 64, 0.02), (12, 65, 0.02), (12, 129, 0.02)])
+def test_dt_loop_per_sample(sampler, oracle, mode, m, steps, scale):
+    """The per-sample kernels' dt loops at the edges of their thread layouts
+    (parts of a row, components past a warp) and of a 64-step history buffer
+    (small steps: one basis carries all of them)."""
+    s = pair((2,), (2, 3))
+    B = np.array([0.01, 0.03, 0.04])
+    rp, col, val = general_csr(oracle, s, B)
+    zk = W.random_phase_samples(s.Z, 5, seed=m)
+    dt = scale * DT
+    t_end = (steps - 0.5) * dt
+    ref = oracle.trace_sampling(rp, col, val, zk, dt, t_end, m, 1e-6)
+    sampler.set_sample_path(mode)
+    try:
+        sampler.build_h(s, B, "general")
+        got = sampler.trace_sampling(zk, dt, t_end, m, 1e-6)
+        stats = sampler.stats()
+    finally:
+        sampler.set_sample_path("auto")
+    assert max(np.max(np.abs(getattr(got, k) - ref[k])) for k in KEYS) <= 1e-12
+    assert stats["krylov_builds"] == int(ref["n_builds"].sum())
+    assert stats["sample_steps"] == 5 * steps
