@@ -1,15 +1,6 @@
 // The dt loop (src/qm_dynamics.f90:348-364) of one sample on four warps, for
 // Krylov dimensions up to 32. Included by spc_propagate.cu inside namespace spc.
 
-// (float)v, cut off instead of rounded, from the words of v: the conversion
-// instruction holds the FP64 pipe as a multiply-add does.
-__device__ __forceinline__ float cut_float(double v) {
-  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
-  const int e = (int)(hi >> 20 & 0x7ff) - 896;
-  const unsigned mag = e <= 0 ? 0u : e >= 255 ? 0x7f800000u : (unsigned)e << 23 | (hi & 0xfffff) << 3 | lo >> 29;
-  return __uint_as_float((hi & 0x80000000u) | mag);
-}
-
 // Stop test of the dt loop, |c_{me-1}|^2 <= tol |c|^2, for the coordinates in a
 // warp's lanes (zero past me). In single precision where that decides it (two
 // sides apart by more than its rounding): five FP64 adds with their shuffles

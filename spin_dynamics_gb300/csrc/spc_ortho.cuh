@@ -66,6 +66,29 @@ __device__ __forceinline__ int acc_dot_exp(const TileInfo& T) { return T.rexp; }
 __device__ __forceinline__ int acc_norm_exp(const TileInfo& T) { return 2 * T.rexp; }
 #define ACC_GRAM_EXP 4
 
+// (float)v, cut off instead of rounded, from the words of v: the conversion
+// instruction holds the FP64 pipe as a multiply-add does.
+__device__ __forceinline__ float cut_float(double v) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const int e = (int)(hi >> 20 & 0x7ff) - 896;
+  const unsigned mag = e <= 0 ? 0u : e >= 255 ? 0x7f800000u : (unsigned)e << 23 | (hi & 0xfffff) << 3 | lo >> 29;
+  return __uint_as_float((hi & 0x80000000u) | mag);
+}
+
+// The leading 20 bits of a double below 2^127 as a float (0 below 2^-126), and a
+// float as a double.
+__device__ __forceinline__ float head_float(double v) {
+  const unsigned h = (unsigned)__double2hiint(v);
+  const unsigned u = max(h & 0x7fffffffu, 896u << 20) - (896u << 20);
+  return __uint_as_float((u << 3) | (h & 0x80000000u));
+}
+__device__ __forceinline__ double wide_float(float f) {
+  const unsigned b = __float_as_uint(f), u = b & 0x7fffffffu;
+  const unsigned h = u < 0x00800000u ? 0u : (u >> 3) + (896u << 20);
+  return __hiloint2double((int)(h | (b & 0x80000000u)), u < 0x00800000u ? 0 : (int)(b << 29));
+}
+#define ORTHO_SMALL 44
+
 struct OrthoArgs {
   PassArgs p;
   AccArgs a;
@@ -91,6 +114,17 @@ struct OrthoArgs {
 // build. Blocks of eight: the newest block's pass holds 15 complex sums and 8
 // vectors in 126 registers. Lanczos at dim 2304, 77 samples: the norm pass 15.3
 // -> 10.1 us, k_spmm_blk with its projection 27.9 -> 19.5 us without the last sum.
+// Small coefficients: where H is Hermitian up to a shift every h_v but the last
+// two is of rounding size. A vector whose coefficients are below 2^(rexp - 44) in
+// all of a tile's samples is subtracted in single precision (q's leading 20
+// bits): an error below 2^-60 of the bound on ||H||, 1/128 of one FP64 rounding
+// of p. 64 FP32 multiply-adds issue in the time of one FP64, and the conversions
+// are done on the words, since the conversion instruction also runs on the FP64
+// pipe. Up to two other vectors are subtracted beside them in FP64; a block with
+// more (unequal rates) takes FP64 throughout. The block's pass and the norm pass
+// at dim 2304, 384 samples, m = 16: 97 -> 68 and 35 -> 31 us; dim 55296, 32
+// samples, m = 30: 200 -> 129 and 69 -> 59 us. A branch for each vector instead
+// made the norm pass slower (40 and 80 us).
 // REAL: Lanczos on the Hermitian part; NA = 1 with ND = 1 takes beta_{i-1}
 // (coef), with ND = 0 alpha_i.
 template <int NA, int ND, bool GRAM, bool REAL>
@@ -100,6 +134,8 @@ __global__ void __launch_bounds__(256, 2) k_ortho(OrthoArgs o) {
   __shared__ double2 h[NA > 0 ? NA : 1][SPC_LANES];
   __shared__ double2 red[NR][SPC_WARPS][SPC_LANES];
   __shared__ unsigned mx[SPC_WARPS][SPC_LANES];
+  __shared__ float2 hs[NA > 0 && !REAL ? NA : 1][SPC_LANES];
+  __shared__ int large[NA > 0 && !REAL ? NA : 1];
   const PassArgs& a = o.p;
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
   const int2 it = a.items[blockIdx.x];
@@ -113,6 +149,7 @@ __global__ void __launch_bounds__(256, 2) k_ortho(OrthoArgs o) {
   const bool tail = ND == 0 && i == T.m - 1;
   if (tail && !first) return;
   if (first) acc_clear(o.a, it.x, tid, 256);
+  unsigned lgm = 0;  // the vectors with large coefficients
   if (NA > 0) {
     const size_t mm = (size_t)a.m * a.m;
     const acc_t* in = acc_tile(o.a, o.a.in, it.x) + tx;
@@ -157,13 +194,13 @@ __global__ void __launch_bounds__(256, 2) k_ortho(OrthoArgs o) {
             } else {
               gv = G[k * SPC_LANES];
             }
-            gk[k] = make_float2((float)gv.x, (float)gv.y);
-            big |= act && !(fabsf(gk[k].x) + fabsf(gk[k].y) < 1e-8f);
+            gk[k] = make_float2(cut_float(gv.x), cut_float(gv.y));
+            big |= act && !(fabsf(gk[k].x) + fabsf(gk[k].y) < 4e-9f);
           }
         }
       }
       // an orthonormal basis (products of rounding size): the corrections are
-      // below 1e-8 of the coefficients, first order and single precision leave
+      // below 4e-9 of the coefficients, first order and single precision leave
       // an error below 1e-15 of them. A basis past a breakdown takes the
       // recurrence in full.
       if (!__syncthreads_or(big ? 1 : 0)) {
@@ -171,11 +208,11 @@ __global__ void __launch_bounds__(256, 2) k_ortho(OrthoArgs o) {
         if (ty < NA) {
 #pragma unroll
           for (int k = 0; k < NA - 1; ++k) {
-            const float hx = (float)h[k][tx].x, hy = (float)h[k][tx].y;
+            const float hx = cut_float(h[k][tx].x), hy = cut_float(h[k][tx].y);
             c.x += gk[k].x * hx - gk[k].y * hy;
             c.y += gk[k].x * hy + gk[k].y * hx;
           }
-          d = make_double2(d.x - (double)c.x, d.y - (double)c.y);
+          d = make_double2(d.x - wide_float(c.x), d.y - wide_float(c.y));
         }
         __syncthreads();
         if (ty < NA) h[ty][tx] = d;
@@ -195,10 +232,19 @@ __global__ void __launch_bounds__(256, 2) k_ortho(OrthoArgs o) {
         }
       }
       if (first && act && ty < NA) a.Ahess[(size_t)w * mm + jv + (size_t)i * a.m] = d;
+      if (ty < NA) {
+        // |h| < 2^(rexp - ORTHO_SMALL) by the exponents; NaN and infinities are large
+        const bool lg = __any_sync(0xffffffffu, act && (int)(abs_high(d) >> 20) - 1023 >= T.rexp - ORTHO_SMALL);
+        hs[ty][tx] = lg ? make_float2(0.f, 0.f) : make_float2(cut_float(d.x), cut_float(d.y));
+        if (tx == 0) large[ty] = lg ? 1 : 0;
+      }
       __syncthreads();
+#pragma unroll
+      for (int v = 0; v < NA; ++v) lgm |= (unsigned)large[v] << v;
     }
   }
   if (tail) return;
+  const int nl = __popc(lgm), v0 = nl > 0 ? __ffs(lgm) - 1 : 0, v1 = nl > 1 ? 31 - __clz(lgm) : 0;
   const int n = act ? T.n : 0;
   const int stride = T.nio * SPC_WARPS;
   const size_t vs = (size_t)T.n * SPC_LANES;
@@ -215,20 +261,30 @@ __global__ void __launch_bounds__(256, 2) k_ortho(OrthoArgs o) {
     double2 qd[ND > 0 ? ND : 1];
 #pragma unroll
     for (int v = 0; v < ND; ++v) qd[v] = Qd[v * vs + off];
-    if (NA > 0) {
+    if (NA > 0 && REAL) {
+      const double2 q = Qa[off];
+      const double c = h[0][tx].x;
+      p.x = fma(-c, q.x, p.x);
+      p.y = fma(-c, q.y, p.y);
+    } else if (NA > 0 && nl > 2) {
+#pragma unroll
+      for (int v = 0; v < NA; ++v) p = cfms(h[v][tx], Qa[v * vs + off], p);
+    } else if (NA > 0) {
+      float sx = 0.f, sy = 0.f;
 #pragma unroll
       for (int v = 0; v < NA; ++v) {
-        const double2 q = Qa[v * vs + off];
-        if (REAL) {
-          const double c = h[v][tx].x;
-          p.x = fma(-c, q.x, p.x);
-          p.y = fma(-c, q.y, p.y);
-        } else {
-          p = cfms(h[v][tx], q, p);
-        }
+        const double2 x = Qa[v * vs + off];
+        const float qx = head_float(x.x), qy = head_float(x.y);
+        const float2 c = hs[v][tx];
+        sx = fmaf(c.x, qx, fmaf(-c.y, qy, sx));
+        sy = fmaf(c.x, qy, fmaf(c.y, qx, sy));
       }
-      P[off] = p;
+      if (nl > 0) p = cfms(h[v0][tx], Qa[v0 * vs + off], p);  // in L1 by now
+      if (nl > 1) p = cfms(h[v1][tx], Qa[v1 * vs + off], p);
+      p.x -= wide_float(sx);
+      p.y -= wide_float(sy);
     }
+    if (NA > 0) P[off] = p;
     if (ND == 0) {
       acc[0].x = fma(p.x, p.x, acc[0].x);
       acc[0].x = fma(p.y, p.y, acc[0].x);

@@ -352,13 +352,13 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
           if (v < nb)
             for (int k = 0; k < v; ++k) {
               const double2 gv = ort.gram[jb + v][k];
-              const float gx = (float)gv.x, gy = (float)gv.y, hx = (float)ort.h[k].x, hy = (float)ort.h[k].y;
-              big |= !(fabsf(gx) + fabsf(gy) < 1e-8f);
+              const float gx = cut_float(gv.x), gy = cut_float(gv.y), hx = cut_float(ort.h[k].x), hy = cut_float(ort.h[k].y);
+              big |= !(fabsf(gx) + fabsf(gy) < 4e-9f);
               c.x += gx * hx - gy * hy;
               c.y += gx * hy + gy * hx;
             }
           if (!__any_sync(0xffffffffu, big)) {
-            d = make_double2(d.x - (double)c.x, d.y - (double)c.y);
+            d = make_double2(d.x - wide_float(c.x), d.y - wide_float(c.y));
           } else {
             for (int k = 0; k + 1 < nb; ++k) {
               const double2 hk = make_double2(__shfl_sync(0xffffffffu, d.x, k), __shfl_sync(0xffffffffu, d.y, k));

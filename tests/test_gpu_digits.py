@@ -126,3 +126,23 @@ def test_dt_loop_per_sample(sampler, oracle, mode, m, steps, scale):
     assert max(np.max(np.abs(getattr(got, k) - ref[k])) for k in KEYS) <= 1e-12
     assert stats["krylov_builds"] == int(ref["n_builds"].sum())
     assert stats["sample_steps"] == 5 * steps
+
+
+@pytest.mark.parametrize("m", [9, 10, 17, 24])
+@pytest.mark.parametrize("kT", [1.0, 1.0 + 1e-12, 1.0 + 1e-9, 1.0 + 1e-6, 1.3])
+def test_small_coefficients(sampler, oracle, m, kT):
+    """Projection coefficients below, around and above the size that is
+    subtracted in single precision: they grow with the difference of the rates."""
+    s = pair((3, 2, 2), (3, 3, 3), kT=kT)
+    B = np.array([0.01, 0.03, 0.04])
+    rp, col, val = general_csr(oracle, s, B)
+    zk = W.random_phase_samples(s.Z, 33, seed=m)
+    ref = oracle.trace_sampling(rp, col, val, zk, DT, 40 * DT, m, 1e-6)
+    sampler.set_krylov("mgs")
+    sampler.set_sample_path("off")
+    try:
+        sampler.build_h(s, B, "general")
+        got = sampler.trace_sampling(zk, DT, 40 * DT, m, 1e-6)
+    finally:
+        sampler.set_sample_path("auto")
+    assert max(np.max(np.abs(getattr(got, k) - ref[k])) for k in KEYS) <= 1e-12
