@@ -683,13 +683,22 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   // 24.0 | 12.4 : 11.0; dim 576, 96 samples 11.0 : 13.0 | 6.7 : 7.2, 300 samples
   // 22.1 : 22.1 | 12.9 : 11.2; dim 24, 1200 samples 15.0 : 17.0 | 6.1 : 7.6.
   size_t basis_smem = 0;
+  int team = 1;
   {
     int nmax = 0;
     for (int k = 0; k < nj; ++k) nmax = std::max(nmax, nrow[k]);
-    const size_t need = sizeof(double2) * small_basis_elems(m, nmax);
+    size_t need = sizeof(double2) * small_basis_elems(m, nmax, 1);
     if (m <= SMALL_MAX_M && need + SMALL_STATIC <= h->smem_optin && Mtot <= 8 * h->sm_count && elems <= 800.0 * h->sm_count &&
         h->sample_path != SPC_SAMPLE_OFF) {
-      CK(cudaFuncSetAttribute(k_small_basis, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
+      // clusters while they find idle SMs and rows to share; whole gradient as
+      // above, one CTA against a cluster (MGS | Lanczos): dim 48, 32 samples 3.72 :
+      // 3.90 | 2.40 : 2.75 ms, dim 144 5.11 : 4.57 | 3.23 : 3.05, dim 288 6.85 :
+      // 4.78 | 4.24 : 3.27, dim 576 9.98 : 6.02 | 5.78 : 4.05; 70 samples (two
+      // CTAs each) dim 144 5.46 : 4.95 | 3.28 : 3.12, dim 576 10.9 : 8.3 | 6.3 : 5.2
+      while (team < SMALL_TEAM && 2 * team * Mtot <= h->sm_count && nmax >= 96) team *= 2;
+      need = sizeof(double2) * small_basis_elems(m, nmax, team);
+      CK(cudaFuncSetAttribute(team > 1 ? k_small_basis<true> : k_small_basis<false>,
+                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
       basis_smem = need;
     }
   }
@@ -697,7 +706,23 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   auto build = [&](const double2* x, const TileInfo* tiles) {
     if (basis_smem) {
       const int pe = h->prof.begin(st);
-      k_small_basis<<<nslots, SMALL_THREADS, basis_smem, st>>>(tiles, d_map, d_scol, x, m, lanczos ? 1 : 0, d_Q, d_A, d_c);
+      if (team > 1) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(team * nslots);
+        cfg.blockDim = dim3(SMALL_THREADS);
+        cfg.dynamicSmemBytes = basis_smem;
+        cfg.stream = st;
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim = {(unsigned)team, 1, 1};
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        CK(cudaLaunchKernelEx(&cfg, k_small_basis<true>, tiles, (const int*)d_map, (const int*)d_scol, x, m,
+                              lanczos ? 1 : 0, team, d_Q, d_A, d_c));
+      } else {
+        k_small_basis<false><<<nslots, SMALL_THREADS, basis_smem, st>>>(tiles, d_map, d_scol, x, m, lanczos ? 1 : 0, 1,
+                                                                        d_Q, d_A, d_c);
+      }
       h->prof.end(st, pe, PK_SAMPLE, 0.0, 0.0);
       h->count_launch();
       builds += Mtot;

@@ -48,12 +48,20 @@ struct SmallJob {
 // as integer multiples of 2^(e - 110) (acc_add's pair of words) a level takes a
 // third of that. red: SMALL_WARPS pairs and the result, two sets that the
 // calls use in turn (`turn`). Called by all threads; one result per two barriers.
+//
+// A sample's rows may be spread over a cluster of up to SMALL_TEAM CTAs (CL):
+// every CTA then sends its partials to all of them and adds the same numbers in
+// the same order.
+#define SMALL_TEAM 4
 struct SmallRed {
-  longlong2 part[2][SMALL_WARPS];
+  longlong2 part[2][SMALL_TEAM * SMALL_WARPS];
   double2 out[2];
 };
-template <bool NORM>
-__device__ __forceinline__ double2 block_sum(double v, int e, SmallRed& red, int& turn) {
+struct SmallTeam {
+  int rank, size;
+};
+template <bool NORM, bool CL = false>
+__device__ __forceinline__ double2 block_sum(double v, int e, SmallRed& red, int& turn, SmallTeam team = {0, 1}) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long b = __double_as_longlong(v);
   const int ex = (int)(b >> 52) & 0x7ff;
@@ -81,15 +89,25 @@ __device__ __forceinline__ double2 block_sum(double v, int e, SmallRed& red, int
     lo += __shfl_xor_sync(0xffffffffu, lo, o);
   }
   if (__any_sync(0xffffffffu, bad)) hi = LLONG_MIN;
-  if (lane == 0) red.part[turn][warp] = make_longlong2(hi, lo);
-  __syncthreads();
+  if (CL) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    if (lane < team.size)
+      cluster.map_shared_rank(&red, lane)->part[turn][team.rank * SMALL_WARPS + warp] = make_longlong2(hi, lo);
+    cluster.sync();
+  } else {
+    if (lane == 0) red.part[turn][warp] = make_longlong2(hi, lo);
+    __syncthreads();
+  }
   if (warp == 0) {
-    const longlong2 x = red.part[turn][lane & (SMALL_WARPS - 1)];
+    const int np = CL ? team.size * SMALL_WARPS : SMALL_WARPS;
+    const longlong2 x = red.part[turn][lane & (np - 1)];
     hi = x.x;
     lo = x.y;
     const bool nan = __any_sync(0xffffffffu, hi == LLONG_MIN);
 #pragma unroll
-    for (int o = SMALL_WARPS / 2; o > 0; o >>= 1) {
+    for (int o = CL ? 16 : SMALL_WARPS / 2; o > 0; o >>= 1) {
+      if (CL && o >= np) continue;
       hi += __shfl_xor_sync(0xffffffffu, hi, o);
       lo += __shfl_xor_sync(0xffffffffu, lo, o);
     }
@@ -268,48 +286,71 @@ struct SmallOrtho {
 // rows by itself, so a block costs one warp's tree of adds and three barriers
 // where a vector at a time cost a CTA sum each. 20 vectors at dim 288: 1.5 M
 // clocks a vector at a time, 1.1 M by blocks; dim 48, 10 vectors: 230 K -> 147 K.
+// CL: the CTA of a cluster that holds rows [r0, r0 + nl) of every vector (Q and p
+// with ns rows); psi (all n rows, in every CTA) becomes the vector that H is
+// applied to. Dots and norms are sums over the cluster, and a new vector's rows
+// go to every CTA: nblocks + 2 cluster barriers a step.
+struct SmallExch {
+  double d[2][SMALL_TEAM][SMALL_WARPS][4];  // a block's dots and products of each CTA, two sets in turn
+};
+template <bool CL = false>
 __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool herm, double kap, int m, double2* A,
-                                             double2* cA, double2* Q, double2* p, const double2* psi,
-                                             SmallRed& red, SmallOrtho& ort, int& turn) {
-  const int n = J.n, me = J.me, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+                                             double2* cA, double2* Q, double2* p,
+                                             std::conditional_t<CL, double2*, const double2*> psi, SmallRed& red,
+                                             SmallOrtho& ort, int& turn, SmallTeam team = {0, 1},
+                                             SmallExch* ex = nullptr) {
+  namespace cg = cooperative_groups;
+  const int me = J.me, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int n = CL ? (J.n + team.size - 1) / team.size : J.n;  // rows of a vector here
+  const int r0 = CL ? team.rank * n : 0, nl = CL ? max(0, min(n, J.n - r0)) : n;
+  int turn_ex = 0;
   const size_t mm = (size_t)m * m;
   for (int i = tid; i < (int)mm; i += SMALL_THREADS) A[i] = cz();
   double* pd = reinterpret_cast<double*>(p);
   double* Qd = reinterpret_cast<double*>(Q);
-  const double* psid = reinterpret_cast<const double*>(psi);
+  auto* psid = reinterpret_cast<std::conditional_t<CL, double, const double>*>(psi);
   // c = ||psi|| e_1, Q_0 = psi / ||psi|| (get_krylov :440-447)
   double acc = 0.0;
-  for (int idx = tid; idx < 2 * n; idx += SMALL_THREADS) acc = fma(psid[idx], psid[idx], acc);
+  for (int idx = tid; idx < 2 * J.n; idx += SMALL_THREADS) acc = fma(psid[idx], psid[idx], acc);
   const double2 bn0 = block_norm(acc, red, turn);
   unsigned top = 0;
   if (tid == 0) ort.top = 0;
-  for (int idx = tid; idx < 2 * n; idx += SMALL_THREADS) {
+  for (int idx = tid; idx < 2 * J.n; idx += SMALL_THREADS) {
     const double q = psid[idx] * bn0.y;
-    Qd[idx] = q;
+    if constexpr (CL) {
+      psid[idx] = q;
+      if (idx >= 2 * r0 && idx < 2 * (r0 + nl)) Qd[idx - 2 * r0] = q;
+    } else {
+      Qd[idx] = q;
+    }
     top = max(top, (unsigned)__double2hiint(q) & 0x7fffffffu);
   }
   if (tid < m) cA[tid] = tid == 0 ? make_double2(bn0.x, 0.0) : cz();
-  __syncthreads();
+  if (CL)
+    cg::this_cluster().sync();  // every CTA has psi before another one's rows arrive there
+  else
+    __syncthreads();
   double beta = 0.0;
   for (int i = 0; i < me; ++i) {
     const double2* qi = Q + (size_t)i * n;
+    const double2* x = CL ? psi : qi;
     const double* qid = Qd + (size_t)i * 2 * n;
     double alpha = 0.0;
     int na = 0, ja = 0;  // the block whose projection is still to be subtracted
     if (lz) {
       // p = H q_i - beta_{i-1} Q_{i-1}; alpha_i = Re <Q_i, p>
       double a2 = 0.0;
-      for (int idx = tid; idx < 2 * n; idx += SMALL_THREADS) {
-        double pv = small_half(J, qi, idx, false, kap);
+      for (int idx = tid; idx < 2 * nl; idx += SMALL_THREADS) {
+        double pv = small_half(J, x, idx + 2 * r0, false, kap);
         if (i > 0) pv = fma(-beta, qid[idx - 2 * n], pv);
         pd[idx] = pv;
         a2 = fma(qid[idx], pv, a2);
       }
-      alpha = block_sum<false>(a2, J.rexp, red, turn).x;
+      alpha = block_sum<false, CL>(a2, J.rexp, red, turn, team).x;
       if (tid == 0) A[i + i * m] = make_double2(alpha, -kap);
       if (i == me - 1) break;
     } else {
-      for (int idx = tid; idx < 2 * n; idx += SMALL_THREADS) pd[idx] = small_half(J, qi, idx, herm, kap);
+      for (int idx = tid; idx < 2 * nl; idx += SMALL_THREADS) pd[idx] = small_half(J, x, idx + 2 * r0, herm, kap);
       // MGS (get_krylov :453-456) by blocks: d_v = <Q_v, p>, h_v from the d_v and
       // the block's basis products, p -= sum_v h_v Q_v
       for (int jb = 0; jb <= i; jb += ORTHO_NB) {
@@ -320,10 +361,10 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
           const double2* qv = Q + (size_t)(jb + warp) * n;
           const bool prod = newest && warp < nb - 1;  // also <Q_v, Q_i>
           double2 d = cz(), gp = cz();
-          for (int r = lane; r < n; r += 32) {
-            const double2 x = qv[r];
-            d = cjfma(x, p[r], d);
-            if (prod) gp = cjfma(x, qi[r], gp);
+          for (int r = lane; r < nl; r += 32) {
+            const double2 q = qv[r];
+            d = cjfma(q, p[r], d);
+            if (prod) gp = cjfma(q, qi[r], gp);
           }
           // the four sums, two halves of the lanes at a time
           const bool h16 = (lane & 16) != 0, h8 = (lane & 8) != 0;
@@ -335,14 +376,35 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
           v += __shfl_xor_sync(0xffffffffu, v, 4);
           v += __shfl_xor_sync(0xffffffffu, v, 2);
           v += __shfl_xor_sync(0xffffffffu, v, 1);
-          if (lane == 0) ort.h[warp].x = v;
-          if (lane == 8) ort.h[warp].y = v;
-          // <Q_i, Q_v> = conj <Q_v, Q_i>
-          if (prod && lane == 16) ort.gram[i][warp].x = v;
-          if (prod && lane == 24) ort.gram[i][warp].y = -v;
+          if (CL) {
+            if ((lane & 7) < team.size)
+              cg::this_cluster().map_shared_rank(ex, lane & 7)->d[turn_ex][team.rank][warp][lane >> 3] = v;
+          } else {
+            if (lane == 0) ort.h[warp].x = v;
+            if (lane == 8) ort.h[warp].y = v;
+            // <Q_i, Q_v> = conj <Q_v, Q_i>
+            if (prod && lane == 16) ort.gram[i][warp].x = v;
+            if (prod && lane == 24) ort.gram[i][warp].y = -v;
+          }
         }
-        __syncthreads();
+        const int set = turn_ex;
+        turn_ex ^= 1;
+        if (CL)
+          cg::this_cluster().sync();
+        else
+          __syncthreads();
         if (warp == 0) {
+          if (CL) {
+            // four lanes a vector: the components in rank order
+            const int v = lane >> 2, u = lane & 3;
+            if (v < nb) {
+              double y = ex->d[set][0][v][u];
+              for (int c = 1; c < team.size; ++c) y += ex->d[set][c][v][u];
+              double* to = reinterpret_cast<double*>(u < 2 ? &ort.h[v] : &ort.gram[i][v]);
+              if (u < 2 || (newest && v < nb - 1)) to[u & 1] = u == 3 ? -y : y;
+            }
+            __syncwarp();
+          }
           // first-order corrections where the basis is orthonormal to rounding,
           // the recurrence otherwise
           const int v = lane;
@@ -377,7 +439,7 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
             ja = jb;
             na = nb;
           } else {
-            for (int idx = tid; idx < 2 * n; idx += SMALL_THREADS) {
+            for (int idx = tid; idx < 2 * nl; idx += SMALL_THREADS) {
               const bool im = (idx & 1) != 0;
               double pv = pd[idx];
 #pragma unroll
@@ -394,7 +456,7 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
     }
     // the last projection, ||p|| and Q_{i+1} = p / ||p||
     double nr = 0.0;
-    for (int idx = tid; idx < 2 * n; idx += SMALL_THREADS) {
+    for (int idx = tid; idx < 2 * nl; idx += SMALL_THREADS) {
       double pv = pd[idx];
       if (lz) {
         pv = fma(-alpha, qid[idx], pv);
@@ -407,19 +469,24 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
       pd[idx] = pv;
       nr = fma(pv, pv, nr);
     }
-    const double2 bn = block_sum<true>(nr, 2 * J.rexp, red, turn);
+    const double2 bn = block_sum<true, CL>(nr, 2 * J.rexp, red, turn, team);
     beta = bn.x;
     if (tid == 0) {
       A[(i + 1) + i * m] = make_double2(beta, 0.0);
       if (lz) A[i + (i + 1) * m] = make_double2(beta, 0.0);
     }
     double* qn = Qd + (size_t)(i + 1) * 2 * n;
-    for (int idx = tid; idx < 2 * n; idx += SMALL_THREADS) {
+    for (int idx = tid; idx < 2 * nl; idx += SMALL_THREADS) {
       const double q = pd[idx] * bn.y;
       qn[idx] = q;
+      if constexpr (CL)
+        for (int c = 0; c < team.size; ++c) cg::this_cluster().map_shared_rank(psid, c)[2 * r0 + idx] = q;
       top = max(top, (unsigned)__double2hiint(q) & 0x7fffffffu);
     }
-    __syncthreads();
+    if (CL)
+      cg::this_cluster().sync();
+    else
+      __syncthreads();
   }
   top = __reduce_max_sync(0xffffffffu, top);
   if (lane == 0) atomicMax(&ort.top, top);
@@ -431,37 +498,48 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
 // fill for microseconds: 32 samples at dim 288, m = 16, MGS take 0.72 ms so and
 // 0.38 ms here (FP64 issue: 16 complex entries a row and 136 vector pairs).
 // Dynamic shared memory: A (m^2), c (m), basis (m n), work and state vector (n each).
-__host__ __device__ __forceinline__ size_t small_basis_elems(int m, int n) {
-  return (size_t)m * m + m + (size_t)(m + 2) * n;
+// With samples for at most half or a quarter of the SMs a cluster of two or four
+// CTAs takes each (`size` CTAs, rows split): 0.38 -> 0.20 ms.
+__host__ __device__ __forceinline__ size_t small_basis_elems(int m, int n, int team) {
+  return (size_t)m * m + m + (size_t)(m + 1) * ((n + team - 1) / team) + n;
 }
+template <bool CL>
 __global__ void __launch_bounds__(SMALL_THREADS)
     k_small_basis(const TileInfo* __restrict__ tiles, const int* __restrict__ map, const int* __restrict__ scol,
-                  const double2* __restrict__ x, int m, int lanczos, double2* __restrict__ Q,
+                  const double2* __restrict__ x, int m, int lanczos, int size, double2* __restrict__ Q,
                   double2* __restrict__ Ahess, double2* __restrict__ cvec) {
   extern __shared__ double2 smem[];
   __shared__ SmallRed red;
   __shared__ SmallOrtho ort;
-  const int w = blockIdx.x;
-  if (map[w] < 0) return;
+  __shared__ SmallExch ex;
+  const int w = CL ? blockIdx.x / size : blockIdx.x;
+  if (map[w] < 0) return;  // every CTA of a cluster
   const TileInfo& T = tiles[w / SPC_LANES];
   const SmallJob J{T.n, T.n / 4, T.m, T.rowptr, T.split, T.col, T.val, T.kappa, T.rexp, nullptr};
-  const int n = T.n, tid = threadIdx.x;
+  const SmallTeam team{CL ? (int)(blockIdx.x % size) : 0, CL ? size : 1};
+  const int n = T.n, tid = threadIdx.x, ns = (n + team.size - 1) / team.size, r0 = team.rank * ns;
   double2* A = smem;
   double2* cA = A + m * m;
   double2* V = cA + m;
-  double2* p = V + (size_t)m * n;
-  double2* psi = p + n;
+  double2* p = V + (size_t)m * ns;
+  double2* psi = p + ns;
   const double2* src = x + T.psi_off + scol[w];
   for (int r = tid; r < n; r += SMALL_THREADS) psi[r] = src[(size_t)r * T.ldp];
   __syncthreads();
   int turn = 0;
-  small_krylov(J, lanczos != 0, T.kappa != nullptr, T.kappa != nullptr ? *T.kappa : 0.0, m, A, cA, V, p, psi, red, ort,
-               turn);
+  const bool herm = T.kappa != nullptr;
+  small_krylov<CL>(J, lanczos != 0, herm, herm ? *T.kappa : 0.0, m, A, cA, V, p, psi, red, ort, turn, team, &ex);
   __syncthreads();
-  for (int k = tid; k < m * m; k += SMALL_THREADS) Ahess[(size_t)w * m * m + k] = A[k];
-  if (tid < m) cvec[(size_t)w * m + tid] = cA[tid];
+  if (team.rank == 0) {
+    for (int k = tid; k < m * m; k += SMALL_THREADS) Ahess[(size_t)w * m * m + k] = A[k];
+    if (tid < m) cvec[(size_t)w * m + tid] = cA[tid];
+  }
   double2* dst = Q + T.q_off + (w % SPC_LANES);
-  for (int k = tid; k < T.m * n; k += SMALL_THREADS) dst[(size_t)k * SPC_LANES] = V[k];
+  for (int k = tid; k < T.m * ns; k += SMALL_THREADS) {
+    const int j = k / ns, r = r0 + k - j * ns;
+    if (r < n) dst[((size_t)j * n + r) * SPC_LANES] = V[k];
+  }
+  if (CL) cooperative_groups::this_cluster().sync();  // no CTA leaves before the others' last access
 }
 
 // max |sum_t P_t - I| over the me x me block of the four Grams (NaN wins):

@@ -65,3 +65,30 @@ def test_gradient_basis_per_sample(sampler, m, method):
     for a, b in zip(out["auto"], out["off"]):
         assert abs(a.Phi_S - b.Phi_S) <= 1e-13 and abs(a.Phi_T - b.Phi_T) <= 1e-13
         assert np.linalg.norm(a.raw - b.raw) <= 1e-13 * np.linalg.norm(b.raw)
+
+
+@pytest.mark.parametrize("method, m", [("mgs", 1), ("mgs", 7), ("mgs", 9), ("mgs", 17), ("mgs", 32), ("lanczos", 16)])
+@pytest.mark.parametrize("g1, g2, M, kT", [((3, 2), (2, 2), 1, 0.02), ((3, 3), (3,), 7, 0.02), ((2, 2, 3), (3, 2), 3, 0.05),
+                                           ((3, 2), (2, 3), 40, 0.02)])
+def test_gradient_basis_on_clusters(sampler, method, m, g1, g2, M, kT):
+    """A sample's rows over clusters of four and two CTAs (dims 96, 108, 288 and
+    144) against the tiled build, to the same 1e-13."""
+    if method == "lanczos":
+        kT = 0.02  # equal rates
+    rng = np.random.default_rng(11)
+    A1, A2 = (W._tensors(rng, len(g), -1.5, 1.5, True) for g in (g1, g2))
+    s = SysParam(Electron(g_I=list(g1), A=A1), Electron(g_I=list(g2), A=A2), J=0.03, D=W.axial_dipolar(-0.3), kS=0.02,
+                 kT=kT)
+    zk = W.random_phase_samples(s.Z, M, seed=M)
+    out = {}
+    sampler.set_krylov(method)
+    try:
+        for mode in ("auto", "off"):
+            sampler.set_sample_path(mode)
+            out[mode] = sampler.yield_gradient_batch([s], [np.array([0.02, 0.03, 0.04])], [zk], DT, 4 * DT, m)[0]
+    finally:
+        sampler.set_sample_path("auto")
+        sampler.set_krylov("mgs")
+    a, b = out["auto"], out["off"]
+    assert abs(a.Phi_S - b.Phi_S) <= 1e-13 and abs(a.Phi_T - b.Phi_T) <= 1e-13
+    assert np.linalg.norm(a.raw - b.raw) <= 1e-13 * np.linalg.norm(b.raw)
