@@ -24,23 +24,27 @@ __device__ __forceinline__ unsigned twice(unsigned x) {
 // V is in units of 2^(E - 60), E the exponent of the basis' largest component.
 // Row stride GRAM_R + 4 words (36, or 20 with 16 rows): the 8 vectors x 4 rows
 // of a fragment load fall into 32 different banks.
-// Measured, all four Grams of 512 samples at dim 55296, m = 30: 19.3 ms
-// against 71.4 ms for k_proj (which holds the FP64 pipe at 92 %); 64 samples
-// at dim 9216, m = 24: 0.40 against 1.17 ms; 384 samples at dim 2304, m = 16:
-// 0.26 against 0.59 ms. The 256 clocks of products per nuclear row and sample
-// (m = 30) are a third of the time: staging (one 16-byte load per line, the
-// conversion to digits) and the products do not overlap within a CTA.
+// The next chunk's components are copied to shared memory while a chunk's
+// products run: without that a warp waited on global loads in 2.8 of 8.4 clocks.
+// Measured, all four Grams of 512 samples at dim 55296, m = 30: 18.7 ms (21.6
+// without the copies) against 71.4 ms for k_proj (which holds the FP64 pipe at
+// 92 %); 64 samples at dim 9216, m = 24: 0.40 (0.45) against 1.17 ms; 384
+// samples at dim 2304, m = 16: 0.23 (0.28) against 0.59 ms. The products take a
+// third of the time, the loads (one 32-byte sector a component, the type's
+// vectors read once more for S and T0) and their conversion to digits the rest.
 #define GRAM_R 32
 __host__ __device__ __forceinline__ size_t gram_smem_bytes(int mt, int rows = GRAM_R) {
   return sizeof(unsigned) * DIGITS * 16 * mt * (rows + 4) + sizeof(longlong2) * 8 * 256;
 }
 // Sums of one type over the rows [n0, n1): T of every block, in units of the
 // digit products, to Tm ([2][MP][MP + 1] doubles in V's place). get(j, row, e) is
-// the component of basis vector j < me at nuclear row `row`, electron state e. The
-// CTA's 256 threads; ends with a barrier.
-template <int MT, int R, typename Get>
+// the address of the component of basis vector j < me at nuclear row `row`,
+// electron state e. AHEAD: the next chunk's components are copied to raw while
+// the products run (a thread copies what it converts). The CTA's 256 threads;
+// ends with a barrier.
+template <int MT, int R, bool AHEAD, typename Get>
 __device__ __forceinline__ void gram_sums(int type, int m, int me, int emax, int64_t n0, int64_t n1, longlong2* acc64,
-                                          unsigned* V, Get get) {
+                                          unsigned* V, double2* raw, Get get) {
   constexpr int MP = 16 * MT, LD = R + 4;
   const int tid = threadIdx.y * 32 + threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
   // this warp's block: part (0 Re, 1 Im), rows 16 mi, columns 16 ni, k-steps
@@ -74,19 +78,35 @@ __device__ __forceinline__ void gram_sums(int type, int m, int me, int emax, int
         acc64[(4 * t + r) * 256 + tid] = a;
       }
   };
+  const int e0 = type == 0 ? 0 : (type == 3 ? 3 : 1);
+  const bool sum2 = type == 1 || type == 2;
+  auto copy = [&](int64_t c0) {
+    const int len = (int)min((int64_t)R, n1 - c0);
+#pragma unroll 4
+    for (int idx = tid; idx < MP * R; idx += 256) {
+      const int j = idx / R, nn = idx % R;
+      if (j < me && nn < len) {
+        copy16<false>(raw + idx, get(j, c0 + nn, e0));
+        if (sum2) copy16<false>(raw + MP * R + idx, get(j, c0 + nn, 2));
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  if (AHEAD && n0 < n1) copy(n0);
   int steps = 0;
   for (int64_t c0 = n0; c0 < n1; c0 += R) {
     const int len = (int)min((int64_t)R, n1 - c0);
+    if (AHEAD) asm volatile("cp.async.wait_all;" ::: "memory");
 #pragma unroll 4
     for (int idx = tid; idx < MP * R; idx += 256) {
       const int j = idx / R, nn = idx % R;
       long long vr = 0, vi = 0;
       if (j < me && nn < len) {
-        const double2 a = get(j, c0 + nn, type == 0 ? 0 : (type == 3 ? 3 : 1));
+        const double2 a = AHEAD ? raw[idx] : *get(j, c0 + nn, e0);
         vr = to_fixed<8>(a.x, emax);
         vi = to_fixed<8>(a.y, emax);
-        if (type == 1 || type == 2) {
-          const double2 b = get(j, c0 + nn, 2);
+        if (sum2) {
+          const double2 b = AHEAD ? raw[MP * R + idx] : *get(j, c0 + nn, 2);
           const long long br = to_fixed<8>(b.x, emax), bi = to_fixed<8>(b.y, emax);
           vr = type == 1 ? vr - br : vr + br;
           vi = type == 1 ? vi - bi : vi + bi;
@@ -99,6 +119,7 @@ __device__ __forceinline__ void gram_sums(int type, int m, int me, int emax, int
       for (int d = 0; d < DIGITS; ++d)
         dst[d * MP * LD] = d < 4 ? digit_pair(rh, ih, 3 - d) : digit_pair(rl, il, 7 - d);
     }
+    if (AHEAD && c0 + R < n1) copy(c0 + R);
     __syncthreads();
     for (int ks = k0; ks * 8 < len; ks += kstep) {
       const unsigned* Vk = V + ks * 8 + q;
@@ -173,6 +194,7 @@ __device__ __forceinline__ double2 gram_entry(const double* Tm, int i, int j, do
                       (Tm[(MP + i) * TL + j] - Tm[(MP + j) * TL + i]) * unit);
 }
 
+__host__ __device__ __forceinline__ size_t gram_raw_bytes(int mt) { return sizeof(double2) * 2 * 16 * mt * GRAM_R; }
 template <int MT>
 __global__ void __launch_bounds__(256, 2)
     k_gram(const TileInfo* __restrict__ tiles, const int* __restrict__ map, int m, int ncombo,
@@ -195,8 +217,9 @@ __global__ void __launch_bounds__(256, 2)
   const unsigned top = qmax[w];
   const size_t vs = (size_t)Ti.n * SPC_LANES;
   const double2* Qt = Q + Ti.q_off + (w % SPC_LANES);
-  gram_sums<MT, GRAM_R>(type, m, Ti.m, (int)(top >> 20), n0, n1, acc64, V, [&](int j, int64_t row, int e) {
-    return Qt[(size_t)j * vs + (size_t)(e * Z + row) * SPC_LANES];
+  double2* raw = reinterpret_cast<double2*>(gsm + gram_smem_bytes(MT));
+  gram_sums<MT, GRAM_R, true>(type, m, Ti.m, (int)(top >> 20), n0, n1, acc64, V, raw, [&](int j, int64_t row, int e) {
+    return &Qt[(size_t)j * vs + (size_t)(e * Z + row) * SPC_LANES];
   });
   const double* Tm = reinterpret_cast<const double*>(V);
   const double unit = gram_unit(top);

@@ -1492,7 +1492,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
   const bool gram = m <= 32;
   const int gram_mt = m <= 16 ? 1 : 2;
   const void* gram_fn = gram_mt == 1 ? (const void*)k_gram<1> : (const void*)k_gram<2>;
-  const size_t gram_smem = gram_smem_bytes(gram_mt);
+  const size_t gram_smem = gram_smem_bytes(gram_mt) + gram_raw_bytes(gram_mt);
   CK(cudaFuncSetAttribute(gram_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gram_smem));
   const int res_proj = gram ? std::max(1, resident(gram_fn, 256, gram_smem) / 4)
                             : resident(proj_fn, proj_threads, proj_smem);

@@ -244,8 +244,8 @@ __device__ __forceinline__ void small_grams(int m, int me, int n, int Z, unsigne
   const double* Tm = reinterpret_cast<const double*>(V);
   const double unit = gram_unit(top);
   for (int t = 0; t < 4; ++t) {
-    gram_sums<MT, SMALL_GRAM_R(MT)>(t, me, me, (int)(top >> 20), 0, Z, acc64, V,
-                  [&](int j, int64_t row, int e) { return Q[(size_t)j * n + (size_t)(e * Z + (int)row)]; });
+    gram_sums<MT, SMALL_GRAM_R(MT), false>(t, me, me, (int)(top >> 20), 0, Z, acc64, V, nullptr,
+                  [&](int j, int64_t row, int e) { return &Q[(size_t)j * n + (size_t)(e * Z + (int)row)]; });
     double2* Pt = P + (size_t)t * m * m;
     for (int idx = threadIdx.x; idx < MP * MP; idx += SMALL_THREADS) {
       const int i = idx / MP, j = idx % MP;
