@@ -174,12 +174,28 @@ __global__ void __launch_bounds__(256) k_norm(PassArgs a) {
 #include "spc_digits.cuh"
 #include "spc_blocks.cuh"
 
+// One exchange of a transposition over lanes: b of the lane without bit `o` for a
+// of the lane with it.
+__device__ __forceinline__ void lane_swap(uint4& a, uint4& b, int o) {
+  const bool up = (threadIdx.x & o) != 0;
+  const uint4 s = up ? a : b;
+  const uint4 r = make_uint4(__shfl_xor_sync(0xffffffffu, s.x, o), __shfl_xor_sync(0xffffffffu, s.y, o),
+                             __shfl_xor_sync(0xffffffffu, s.z, o), __shfl_xor_sync(0xffffffffu, s.w, o));
+  if (up)
+    a = r;
+  else
+    b = r;
+}
+
 // Q_{jd} = P / ||P||  (Q_0 = psi[:, scol] / ||psi||),
 // and beside it the operand of the next SpMM: with DIG the packed digits of
 // Q_{jd} that k_spmm_blk reads, [n][32][4] (a thread takes the four electron
-// rows of a nuclear index and writes 64 bytes), else the plane Re + Im of
+// rows of a nuclear index), else the plane Re + Im of
 // k_spmm's three-product form in P's layout (p_off); grid = pass items.
 // Q_0 takes the norm that k_norm left, Q_{jd > 0} the accumulated one.
+// Bound by memory traffic (48 bytes an element); a thread's own 64 bytes as four
+// stores 64 bytes apart from its neighbours' took 277 us at dim 55296, 512
+// samples, transposed over four lanes 230 us (5.9 TB/s).
 template <bool DIG>
 __global__ void __launch_bounds__(256) k_scale(PassArgs a, AccArgs A, int jd, void* __restrict__ XS) {
   __shared__ double s_rb[SPC_LANES];
@@ -198,26 +214,38 @@ __global__ void __launch_bounds__(256) k_scale(PassArgs a, AccArgs A, int jd, vo
     }
   }
   __syncthreads();
-  if (a.map[w] < 0) return;
+  const bool act = a.map[w] >= 0;
+  const unsigned actm = __ballot_sync(0xffffffffu, act);
+  if (DIG ? actm == 0u : !act) return;
   const double rb = s_rb[tx];
   const int n = T.n;
   const int stride = T.nip * SPC_WARPS;
   double2* dst = const_cast<double2*>(a.Q) + T.q_off + (size_t)jd * n * SPC_LANES + tx;
-  const double2* src = jd == 0 ? a.psi + T.psi_off + a.scol[w] : a.P + T.p_off + tx;
+  const double2* src = jd == 0 ? a.psi + T.psi_off + (act ? a.scol[w] : 0) : a.P + T.p_off + tx;
   const size_t ld = jd == 0 ? T.ldp : SPC_LANES;
   if (DIG) {
     const int ex = s_ex[tx], Z = n / 4;
-    uint4* dx = (uint4*)XS + T.p_off + tx * 4;
+    const int g = tx & ~3, q = tx & 3;
+    uint4* dx = (uint4*)XS + T.p_off + g * 4 + q;
     for (int k = it.y * SPC_WARPS + threadIdx.y; k < Z; k += stride) {
       double2 x[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) x[e] = src[((size_t)e * Z + k) * ld];
+      for (int e = 0; e < 4; ++e) x[e] = act ? src[((size_t)e * Z + k) * ld] : cz();
+      uint4 d[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const double2 q = make_double2(x[e].x * rb, x[e].y * rb);
-        dst[((size_t)e * Z + k) * SPC_LANES] = q;
-        dx[(size_t)k * 128 + e] = pack_digits(q, ex);
+        const double2 y = make_double2(x[e].x * rb, x[e].y * rb);
+        if (act) dst[((size_t)e * Z + k) * SPC_LANES] = y;
+        d[e] = pack_digits(y, ex);
       }
+      // lane 4 s + q's row e to lane 4 s + e: four lanes then write a sample's 64 bytes
+      lane_swap(d[0], d[1], 1);
+      lane_swap(d[2], d[3], 1);
+      lane_swap(d[0], d[2], 2);
+      lane_swap(d[1], d[3], 2);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (actm >> (g + j) & 1) dx[(size_t)k * 128 + 4 * j] = d[j];
     }
   } else {
     double* xs = (double*)XS + T.p_off + tx;
