@@ -27,7 +27,8 @@
 // recomputes each segment from its checkpoint, and the Krylov basis built at
 // psi_k for psi_{k+1} also gives the node states exp(-i H x_q dt) psi_k, kept
 // for the segment. Per step: three Krylov builds (forward, recompute, costate)
-// and 2*nq + 2 basis applications. When a segment's node states do not fit in
+// and 2*nq + 2 basis applications, up to four of a build's from one read of the
+// basis. When a segment's node states do not fit in
 // device memory they are rebuilt per step instead (four builds per step).
 // Without a gradient only the forward sweep runs (one build per step).
 
@@ -501,7 +502,10 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   // Krylov build per step saved). K = 0 picks the largest spacing whose
   // states fit in device memory (fewest recomputed segments), else the
   // spacing of least memory with node states rebuilt per step.
+  // nqm: costate node states formed at a time, all of a step's nodes or, where
+  // memory is short, one after the other
   bool cache = false;
+  int nqm = nq;
   if (want_grad) {
     size_t free_b = 0, total_b = 0;
     CK(cudaMemGetInfo(&free_b, &total_b));
@@ -512,13 +516,13 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
     // to the size asked of it (buffers only grow), so its excess over that
     // size is no help
     auto need = [&](int k, bool keep) {
-      return sb * ((double)m + 3.0 + nq + xs_bytes / 16.0 + (nsteps / k + 1) + k + 1.0 + (keep ? (double)k * nq : (double)nq));
+      return sb * ((double)m + 3.0 + nqm + xs_bytes / 16.0 + (nsteps / k + 1) + k + 1.0 + (keep ? (double)k * nq : (double)nq));
     };
     auto extra = [&](int k, bool keep) {
       double x = 0.0;
       auto add = [&](const Handle::Buf& b, double bytes) { x += std::max(0.0, bytes - (double)b.bytes); };
       add(h->Q, sb * m);
-      add(h->gmu, sb * nq);
+      add(h->gmu, sb * nqm);
       add(h->glam, 2.0 * sb);
       add(h->P, sb);
       add(h->xsum, xs_bytes / 16.0 * sb);  // the current Krylov vector's digits or Re + Im plane beside P
@@ -549,7 +553,10 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
     } else {
       cache = extra(K, true) <= avail;
     }
-    if (!cache && extra(K, false) > avail)
+    if (!cache && extra(K, false) > avail) nqm = 1;
+    // the digits' plane and the small sums may use the 15 % kept free
+    const double slack = (xs_bytes / 16.0 - 0.5) * sb + (double)acc_bytes(ntiles) + (double)gram_bytes(ntiles, m);
+    if (!cache && extra(K, false) > avail + slack)
       return set_error(SPC_ERR_ALLOC,
                        "yield gradient needs %.1f GB of device memory at checkpoint spacing %d (%.1f GB free)",
                        need(K, false) / 1e9, K, free_b / 1e9);
@@ -562,7 +569,7 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   const size_t plan_bytes = 2 * sizeof(TileInfo) * ntiles + sizeof(int2) * 4 * items_cap +
                             sizeof(int) * 2 * nslots + sizeof(double2) * ntiles + 64;
   if (h->ensure(h->gck, sizeof(double2) * S * n_ck) || h->ensure(h->gseg, sizeof(double2) * S * n_seg) ||
-      h->ensure(h->gnu, sizeof(double2) * S * n_nu) || h->ensure(h->gmu, sizeof(double2) * S * (want_grad ? nq : 1)) ||
+      h->ensure(h->gnu, sizeof(double2) * S * n_nu) || h->ensure(h->gmu, sizeof(double2) * S * (want_grad ? nqm : 1)) ||
       h->ensure(h->glam, sizeof(double2) * S * 2) || h->ensure(h->Q, sizeof(double2) * m * S) ||
       h->ensure(h->P, sizeof(double2) * S) || h->ensure(h->xsum, (size_t)xs_bytes * S) ||
       h->ensure(h->qmax, 2 * sizeof(unsigned) * nslots) || h->ensure(h->xexp, sizeof(int) * nslots) ||
@@ -873,11 +880,8 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
     tm.tau[tm.n] = tau;
     tm.y[tm.n++] = y;
   };
-  ConNodes one{}, all{};  // a single pair of states; the nodes of a step
+  ConNodes one{};  // a single pair of states
   one.n = 1;
-  all.n = nq;
-  all.stride = S;
-  for (int q = 0; q < nq; ++q) all.w[q] = wq[q] * dt;
   // basis at psi_k under H: node states nu_q and psi_{k+1}
   auto step_forward = [&](const double2* x, double2* nodes, double2* y) {
     int rc = build(x, d_tf);
@@ -941,11 +945,19 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
       }
       int rc = build(lam, d_tb);
       if (rc) return rc;
-      Times tm{};
-      for (int q = 0; q < nq; ++q) add_time(tm, -dt * (1.0 - xq[q]), gmu + S * q);
-      add_time(tm, -dt, ulam);
-      apply(tm, d_tb);
-      contract(gmu, nodes, all, false, d_racc);
+      for (int q0 = 0; q0 < nq; q0 += nqm) {
+        ConNodes some{};
+        some.n = std::min(nqm, nq - q0);
+        some.stride = S;
+        Times tm{};
+        for (int q = 0; q < some.n; ++q) {
+          some.w[q] = wq[q0 + q] * dt;
+          add_time(tm, -dt * (1.0 - xq[q0 + q]), gmu + S * q);
+        }
+        if (q0 + some.n == nq) add_time(tm, -dt, ulam);
+        apply(tm, d_tb);
+        contract(gmu, nodes + S * q0, some, false, d_racc);
+      }
       costate(cw[k], seg + S * (k - a), ulam);
     }
   }

@@ -353,7 +353,12 @@ __global__ void __launch_bounds__(BLK_THREADS, 4)
 // runs on them), three launches in all.
 static int prepare_blocks(Handle* h, Handle::BlockStore& S, const std::vector<const int*>& rowptr,
                           const std::vector<const int*>& col, const std::vector<const double2*>& val) {
-  if (S.ready) return SPC_OK;
+  if (S.ready) {
+    // a call that failed after building returned without waiting for its stream
+    if (S.stream != h->stream && S.built && cudaStreamWaitEvent(h->stream, S.built, 0) != cudaSuccess)
+      return set_error(SPC_ERR_CUDA, "waiting for the blocks failed: %s", cudaGetErrorString(cudaGetLastError()));
+    return SPC_OK;
+  }
   std::vector<BlkDesc> d;
   std::vector<BlkNuc> nu;
   int64_t selfs = 0, tabs = 0, nbrs = 0;
@@ -411,6 +416,9 @@ static int prepare_blocks(Handle* h, Handle::BlockStore& S, const std::vector<co
     h->count_launch(2);
     e = cudaGetLastError();
   }
+  if (e == cudaSuccess && !S.built) e = cudaEventCreateWithFlags(&S.built, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventRecord(S.built, h->stream);
+  S.stream = h->stream;
   if (e != cudaSuccess) {
     S.ready = false;
     return set_error(SPC_ERR_CUDA, "block fragments of the Hamiltonian failed: %s", cudaGetErrorString(e));

@@ -75,6 +75,8 @@ Handle::~Handle() {
   if (d_rowptr) cudaFree(d_rowptr);
   if (d_col) cudaFree(d_col);
   if (d_val) cudaFree(d_val);
+  for (BlockStore* s : {&blk_one, &blk_batch})
+    if (s->built) cudaEventDestroy(s->built);
   if (own_stream) cudaStreamDestroy(own_stream);
 }
 

@@ -170,6 +170,9 @@ struct Handle {
     Buf self, tab, nbr, desc;
     std::vector<BlockSys> sys;
     bool ready = false;
+    // the stream that built the blocks and the end of it, for calls on another one
+    cudaStream_t stream = nullptr;
+    cudaEvent_t built = nullptr;
     void describe(std::vector<BlockSys> s) {
       sys = std::move(s);
       ready = false;

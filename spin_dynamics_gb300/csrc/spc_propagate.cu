@@ -16,19 +16,18 @@
 //
 // Per round:
 //   norm/scale passes      c = ||psi|| e1, Q0 = psi/||psi||      (get_krylov :445-449)
-//   m x [ SpMM p = H Q_i ; MGS (or Lanczos) passes ; scale ]       (:451-465)
-//   Pade-6 expm of -i dt A per sample, one CTA each               (matrix_exponential.f90)
+//   m x [ SpMM p = H Q_i ; MGS by blocks (or Lanczos) ; scale ]    (:451-465)
+//   Taylor expm of -i dt A per sample, one CTA or warp each       (matrix_exponential.f90)
 //   Krylov projectors as Hermitian Grams per sample               (convert_to_krylov :469-498)
-//   dt loop per sample, one warp each                             (:351-364)
+//   dt loop per sample, a CTA each or packed into warps           (:351-364)
 //   psi = Q c                                                      (:365)
 //
 // Row kernels run over work items (tile, phase): an item takes every
 // (items_of_tile * 8)-th row of its tile starting at phase*8 + warp, so row
 // lengths balance and all items of a tile sweep its rows together. Item
 // counts per tile are proportional to the tile's rows and sum to about one
-// wave of resident CTAs. Reductions are two-level and in a fixed order
-// (per-item partials, then the last item of each tile sums them), so results
-// do not depend on scheduling.
+// wave of resident CTAs. Sums over rows are integers (spc_ortho.cuh) or in a
+// fixed order, so results do not depend on scheduling.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -1252,7 +1251,7 @@ static int use_blocks(Handle* h, bool single, const std::vector<int>& systems, H
   }
   const int rc = prepare_blocks(h, S, rp, cl, vl);
   if (rc == SPC_OK) *out = &S;
-  return rc;
+  return rc == SPC_ERR_ALLOC ? SPC_OK : rc;  // no room for the blocks: the CSR kernel
 }
 static void tile_blocks(TileInfo& t, const Handle::BlockStore& S, int sys) {
   const BlockSys& b = S.sys[sys];
@@ -1316,9 +1315,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
   }
   // basis + work vector (complex) + the current vector's digits or Re + Im
   // plane (XS)
-  const double xs_bytes = blocks ? 16.0 : 8.0;
-  const double need_fl = 16.0 * (double)qcap + (16.0 + xs_bytes) * (double)pcap + slot_fixed * slots_cap +
-                         tile_fixed * tiles_cap;
+  double xs_bytes = blocks ? 16.0 : 8.0;
   const double need_global = 16.0 * (double)psi_total + 8.0 * 4.0 * (double)T * G + 16.0 * G;
   double budget;
   {
@@ -1352,6 +1349,13 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
     budget = (double)free_b + held - need_global - (512.0 * (1 << 20) + 0.02 * (double)total_b);
     if (h->mem_limit) budget = std::min(budget, (double)h->mem_limit - need_global);
   }
+  // where not even a tile fits with the digits, the CSR kernel and its plane
+  if (blocks && (16.0 * m + 32.0) * nmax * SPC_LANES + slot_fixed * SPC_LANES + tile_fixed > budget) {
+    blocks = nullptr;
+    xs_bytes = 8.0;
+  }
+  const double need_fl = 16.0 * (double)qcap + (16.0 + xs_bytes) * (double)pcap + slot_fixed * slots_cap +
+                         tile_fixed * tiles_cap;
   int64_t qfl = qcap, pfl = pcap;
   int slots_fl = slots_cap, tiles_fl = tiles_cap;
   const bool chunked = need_fl > budget;
@@ -1363,7 +1367,9 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
     slots_fl = tiles_fl * SPC_LANES;
     const double fl = 16.0 * (double)qfl + (16.0 + xs_bytes) * (double)pfl + slot_fixed * slots_fl +
                       tile_fixed * tiles_fl;
-    if (fl > budget)
+    // a single tile's small sums do not decide
+    const double sums = tiles_fl == 1 ? (double)acc_bytes(1) + (double)gram_bytes(1, m) + 12.0 * SPC_LANES : 0.0;
+    if (fl > budget + sums)
       return set_error(SPC_ERR_ALLOC,
                        "one 32-sample tile of dimension %d at Krylov dimension %d needs %.3g bytes; "
                        "%.3g are available",

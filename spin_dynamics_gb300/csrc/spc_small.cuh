@@ -14,13 +14,12 @@
 // Calls with few samples give each sample a cluster of two CTAs instead
 // (k_small_pair, below).
 //
-// Per sample the arithmetic is the tiled path's: the SpMM row loop of k_spmm,
+// Per sample the arithmetic is the tiled path's: the entries of k_spmm's rows,
 // real-coefficient Lanczos on the Hermitian part (orthonormality checked from
 // the projector Grams, MGS rebuild when it fails) or MGS, expm_one, the four
-// Hermitian projector Grams, the reference's dt-loop semantics. Reductions
-// are two-level and in a fixed order (a warp tree, then warp 0's tree over the
-// warps' partials), so results repeat bit for bit; they differ from the tiled
-// path's by rounding.
+// Hermitian projector Grams, the reference's dt-loop semantics. Reductions are
+// integer or two-level in a fixed order, so results repeat bit for bit; they
+// differ from the tiled path's by rounding.
 // Control flow is uniform across the CTA: every barrier is reached by all
 // threads, and a sample leaves the loop only when the whole CTA does.
 #define SMALL_THREADS 256

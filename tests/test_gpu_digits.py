@@ -8,6 +8,7 @@ import pytest
 
 from conftest import general_csr, iso_csr
 from spin_dynamics_gb300 import workloads as W
+from spin_dynamics_gb300._native import SpcError
 from spin_dynamics_gb300.spinsys import GAMMA_E, Electron, SysParam
 
 pytestmark = pytest.mark.gpu
@@ -146,3 +147,37 @@ def test_small_coefficients(sampler, oracle, m, kT):
     finally:
         sampler.set_sample_path("auto")
     assert max(np.max(np.abs(getattr(got, k) - ref[k])) for k in KEYS) <= 1e-12
+
+
+def test_least_memory(sampler):
+    """The least memory limit that the call accepts is the same for the general
+    builder's Hamiltonian (whose kernel wants a vector's digits beside it) as for
+    the reference builder's, and at that limit the populations are the same."""
+    s = pair((2, 2, 3), (3, 2), iso=True)
+    zk = W.random_phase_samples(s.Z, 40, seed=2)
+
+    def run(limit):
+        sampler.set_memory_limit(limit)
+        return sampler.trace_sampling(zk, DT, 6 * DT, 2, 1e-6)
+
+    least = []
+    sampler.set_sample_path("off")
+    try:
+        for mode, B in (("reference", 0.05), ("general", np.array([0.0, 0.0, 0.05]))):
+            sampler.build_h(s, B, mode)
+            whole = run(0)
+            lo, hi = 1 << 18, 1 << 24
+            while hi - lo > 1:
+                mid = (lo + hi) // 2
+                try:
+                    got = run(mid)
+                    hi = mid
+                except SpcError:
+                    lo = mid
+            got = run(hi)
+            least.append(hi)
+            assert max(np.max(np.abs(getattr(got, k) - getattr(whole, k))) for k in KEYS) <= 1e-13
+    finally:
+        sampler.set_memory_limit(0)
+        sampler.set_sample_path("auto")
+    assert least[0] == least[1]
