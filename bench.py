@@ -39,11 +39,12 @@ from spin_dynamics_gb300 import workloads as W  # noqa: E402
 # |Delta Phi_S| check against the oracle on the first vectors of the timed set.
 METRIC = "sample-steps/s at dim 55296: batched+adjoint vs plain on GB300 at |\u0394\u03a6S|\u22641e-10"
 
-# DRAM traffic per k_spmm launch (dram__bytes_read.sum + dram__bytes_write.sum)
-# from one ncu capture at 64 sample columns (409 MB = 33 MB of Hamiltonian +
-# 376 MB that scales with the columns), scaled to the launch's column count.
-SPMM_TRAFFIC_H = 33.2e6
-SPMM_TRAFFIC_PER_COLUMN = (409.1e6 - 33.2e6) / 64
+# DRAM traffic per k_spmm_blk launch (dram__bytes_read.sum + dram__bytes_write.sum)
+# from one ncu capture at 64 sample columns (300 MB = 16 MB of Hamiltonian blocks and
+# neighbour lists + 284 MB that scales with the columns), scaled to the launch's
+# column count.
+SPMM_TRAFFIC_H = 16e6
+SPMM_TRAFFIC_PER_COLUMN = (300.1e6 - 16e6) / 64
 
 
 def parse():
@@ -874,7 +875,9 @@ def main():
                           "peak_source": peak_src,
                           "fp64": {"achieved_tflops": ach_tf, "peak_tflops": r["fp64_peak"] / 1e12,
                                    "frac": (ach_tf * 1e12 / r["fp64_peak"]) if ach_tf else None,
-                                   "peak_source": "measured DFMA probe (spc_fp64_peak)"}},
+                                   "peak_source": "measured DFMA probe (spc_fp64_peak)",
+                                   "note": "operations of the FP64 form of the product; spmm and projectors run "
+                                           "them as exact digits on the FP16 tensor cores, so frac may exceed 1"}},
                 kernel_share=share, batched=r["batched"], adjoint=r["adjoint"],
                 batched_adjoint=r["batch_adjoint"], symmetry=r["symmetry"], small=r["small"], cpu_baseline=cpu,
                 accuracy=accuracy)
