@@ -234,7 +234,9 @@ __global__ void __launch_bounds__(256, 2) k_ortho(OrthoArgs o) {
       if (first && act && ty < NA) a.Ahess[(size_t)w * mm + jv + (size_t)i * a.m] = d;
       if (ty < NA) {
         // |h| < 2^(rexp - ORTHO_SMALL) by the exponents; NaN and infinities are large
-        const bool lg = __any_sync(0xffffffffu, act && (int)(abs_high(d) >> 20) - 1023 >= T.rexp - ORTHO_SMALL);
+        // as are all where products would leave the range of single precision
+        const bool lg = T.rexp < -40 || T.rexp > 100 ||
+                        __any_sync(0xffffffffu, act && (int)(abs_high(d) >> 20) - 1023 >= T.rexp - ORTHO_SMALL);
         hs[ty][tx] = lg ? make_float2(0.f, 0.f) : make_float2(cut_float(d.x), cut_float(d.y));
         if (tx == 0) large[ty] = lg ? 1 : 0;
       }

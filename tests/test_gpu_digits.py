@@ -181,3 +181,25 @@ def test_least_memory(sampler):
         sampler.set_memory_limit(0)
         sampler.set_sample_path("auto")
     assert least[0] == least[1]
+
+
+@pytest.mark.parametrize("method", ["mgs", "auto"])
+@pytest.mark.parametrize("scale", [2.0**-90, 2.0**-45, 2.0**40, 2.0**105])
+def test_extreme_units(sampler, oracle, method, scale):
+    """A CSR in units far from those of the builders: scaled by a power of two,
+    with dt scaled back, every number keeps its digits, past the range of single
+    precision too."""
+    s = W.small_pair()
+    rp, col, val = iso_csr(oracle, s, 0.05)
+    zk = W.random_phase_samples(s.Z, 5, seed=3)
+    dt = DT / scale
+    ref = oracle.trace_sampling(rp, col, val, zk, DT, 40 * DT, 17, 1e-6)
+    sampler.set_krylov(method)
+    sampler.set_sample_path("off")
+    try:
+        sampler.set_h(rp, col, val * scale)
+        got = sampler.trace_sampling(zk, dt, 40 * dt, 17, 1e-6)
+    finally:
+        sampler.set_sample_path("auto")
+        sampler.set_krylov("mgs")
+    assert max(np.max(np.abs(getattr(got, k) - ref[k])) for k in KEYS) <= 1e-12
