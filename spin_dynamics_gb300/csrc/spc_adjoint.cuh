@@ -615,7 +615,9 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   // the three-term recurrence only on explicit request: no projector Gram
   // verifies these bases (the trace-sampling path checks its own)
   bool lanczos = h->krylov_method == 1;
-  for (const GradJob& J : jobs) lanczos = lanczos && HB.herm[J.sys] && HB.herm[J.sys + 1];
+  bool all_herm = true;
+  for (const GradJob& J : jobs) all_herm = all_herm && HB.herm[J.sys] && HB.herm[J.sys + 1];
+  lanczos = lanczos && all_herm;
   std::vector<int> fp, cp, fs, csn;
   std::vector<int2> items_p, items_s;
   plan_items(tile_n, resident((const void*)k_scale<true>), fp, cp, items_p);
@@ -739,6 +741,7 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
     CK(cudaMemsetAsync(d_qmax, 0, 2 * sizeof(unsigned) * nslots, st));
     BasisRun br{};
     br.tiles = tiles;
+    br.herm = all_herm;
     br.items_p = d_items;
     br.items_s = d_items_s;
     br.items_b = d_items_b;

@@ -94,6 +94,7 @@ struct OrthoArgs {
   AccArgs a;
   int ja, jd;      // first vector to subtract, first to project on
   double2* gram;   // [tile][basis vector][8][32]: <Q_j, Q_k> of the vectors k < j of j's block
+  float far;       // size past which a product <Q_j, Q_k>, k < j - 1, calls for the recurrence
 };
 #define ORTHO_NB 8
 
@@ -125,11 +126,19 @@ struct OrthoArgs {
 // at dim 2304, 384 samples, m = 16: 97 -> 68 and 35 -> 31 us; dim 55296, 32
 // samples, m = 30: 200 -> 129 and 69 -> 59 us. A branch for each vector instead
 // made the norm pass slower (40 and 80 us).
+// HERM (every tile Hermitian up to a shift): the products of the new vector with
+// the ones before its neighbour in FP32. They multiply coefficients h_k, k < i - 1,
+// which are of the size of the basis' defect of orthogonality d times ||H||; an
+// error of 1e-6 of the products adds 1e-6 d ||H|| and less. With them the products
+// cost one FP64 sum instead of up to seven: dim 2304, 384 samples, m = 16, a newest
+// block's pass 48 -> 42 us alone and 68 -> 54 us after a block; dim 55296, 32 samples,
+// m = 30: 103 -> 96 and 129 -> 114 us.
 // REAL: Lanczos on the Hermitian part; NA = 1 with ND = 1 takes beta_{i-1}
 // (coef), with ND = 0 alpha_i.
-template <int NA, int ND, bool GRAM, bool REAL>
+template <int NA, int ND, bool GRAM, bool REAL, bool HERM = false>
 __global__ void __launch_bounds__(256, 2) k_ortho(OrthoArgs o) {
   constexpr int NG = GRAM && ND > 1 ? ND - 1 : 0, NS = ND + NG;
+  constexpr int NF = HERM && NG > 1 ? NG - 1 : 0;  // products in FP32
   constexpr int NR = ND == 0 ? 1 : (NS < 4 ? NS : 4);  // sums reduced at a time
   __shared__ double2 h[NA > 0 ? NA : 1][SPC_LANES];
   __shared__ double2 red[NR][SPC_WARPS][SPC_LANES];
@@ -195,7 +204,7 @@ __global__ void __launch_bounds__(256, 2) k_ortho(OrthoArgs o) {
               gv = G[k * SPC_LANES];
             }
             gk[k] = make_float2(cut_float(gv.x), cut_float(gv.y));
-            big |= act && !(fabsf(gk[k].x) + fabsf(gk[k].y) < 4e-9f);
+            big |= act && !(fabsf(gk[k].x) + fabsf(gk[k].y) < (k == ty - 1 ? 4e-9f : o.far));
           }
         }
       }
@@ -256,6 +265,9 @@ __global__ void __launch_bounds__(256, 2) k_ortho(OrthoArgs o) {
   double2 acc[NS > 0 ? NS : 1];
 #pragma unroll
   for (int v = 0; v < (NS > 0 ? NS : 1); ++v) acc[v] = cz();
+  float2 accf[NF > 0 ? NF : 1];
+#pragma unroll
+  for (int v = 0; v < (NF > 0 ? NF : 1); ++v) accf[v] = make_float2(0.f, 0.f);
   unsigned top = 0;
   for (int r = it.y * SPC_WARPS + ty; r < n; r += stride) {
     const size_t off = (size_t)r * SPC_LANES;
@@ -302,8 +314,19 @@ __global__ void __launch_bounds__(256, 2) k_ortho(OrthoArgs o) {
       }
     }
 #pragma unroll
-    for (int v = 0; v < NG; ++v) acc[ND + v] = cjfma(qd[v], qd[ND > 0 ? ND - 1 : 0], acc[ND + v]);
+    for (int v = NF; v < NG; ++v) acc[ND + v] = cjfma(qd[v], qd[ND > 0 ? ND - 1 : 0], acc[ND + v]);
+    if (NF > 0) {
+      const float nx = head_float(qd[ND > 0 ? ND - 1 : 0].x), ny = head_float(qd[ND > 0 ? ND - 1 : 0].y);
+#pragma unroll
+      for (int v = 0; v < NF; ++v) {
+        const float qx = head_float(qd[v].x), qy = head_float(qd[v].y);
+        accf[v].x = fmaf(qx, nx, fmaf(qy, ny, accf[v].x));
+        accf[v].y = fmaf(qx, ny, fmaf(-qy, nx, accf[v].y));
+      }
+    }
   }
+#pragma unroll
+  for (int v = 0; v < NF; ++v) acc[ND + v] = make_double2(wide_float(accf[v].x), wide_float(accf[v].y));
   // the CTA's sums over its warps, then to the accumulators: warp y takes sum
   // y / 2's real or imaginary part
   acc_t* out = acc_tile(o.a, o.a.out, it.x) + tx;
@@ -366,14 +389,17 @@ typedef void (*OrthoFn)(OrthoArgs);
 // The pass of a block: `nd` dots after subtracting nothing or a full block (nd
 // = 8 on an older block; the newest block also forms its basis products), or
 // the norm after the last block's `na` vectors.
+template <bool HERM>
 static OrthoFn ortho_fn(int na, int nd, bool newest) {
   static const OrthoFn old[2] = {k_ortho<0, 8, false, false>, k_ortho<8, 8, false, false>};
-  static const OrthoFn lone[8] = {k_ortho<0, 1, true, false>, k_ortho<0, 2, true, false>, k_ortho<0, 3, true, false>,
-                                  k_ortho<0, 4, true, false>, k_ortho<0, 5, true, false>, k_ortho<0, 6, true, false>,
-                                  k_ortho<0, 7, true, false>, k_ortho<0, 8, true, false>};
-  static const OrthoFn next[8] = {k_ortho<8, 1, true, false>, k_ortho<8, 2, true, false>, k_ortho<8, 3, true, false>,
-                                  k_ortho<8, 4, true, false>, k_ortho<8, 5, true, false>, k_ortho<8, 6, true, false>,
-                                  k_ortho<8, 7, true, false>, k_ortho<8, 8, true, false>};
+  static const OrthoFn lone[8] = {
+      k_ortho<0, 1, true, false, HERM>, k_ortho<0, 2, true, false, HERM>, k_ortho<0, 3, true, false, HERM>,
+      k_ortho<0, 4, true, false, HERM>, k_ortho<0, 5, true, false, HERM>, k_ortho<0, 6, true, false, HERM>,
+      k_ortho<0, 7, true, false, HERM>, k_ortho<0, 8, true, false, HERM>};
+  static const OrthoFn next[8] = {
+      k_ortho<8, 1, true, false, HERM>, k_ortho<8, 2, true, false, HERM>, k_ortho<8, 3, true, false, HERM>,
+      k_ortho<8, 4, true, false, HERM>, k_ortho<8, 5, true, false, HERM>, k_ortho<8, 6, true, false, HERM>,
+      k_ortho<8, 7, true, false, HERM>, k_ortho<8, 8, true, false, HERM>};
   static const OrthoFn norm[8] = {k_ortho<1, 0, false, false>, k_ortho<2, 0, false, false>, k_ortho<3, 0, false, false>,
                                   k_ortho<4, 0, false, false>, k_ortho<5, 0, false, false>, k_ortho<6, 0, false, false>,
                                   k_ortho<7, 0, false, false>, k_ortho<8, 0, false, false>};

@@ -1141,6 +1141,7 @@ struct BasisRun {
   int ntiles;
   void* xs;                // Re + Im plane or packed digits of the current vector
   bool lanczos;
+  bool herm;               // every tile is Hermitian up to a shift
   // profile: vector elements, all stored entries, FP64 operations of k_spmm
   double elems, nnz_work, spmm_flops;
 };
@@ -1176,7 +1177,7 @@ static cudaError_t enqueue_basis(Handle* h, BasisRun& B) {
   };
   // na vectors from ja subtracted, nd from jd projected on (0: the norm)
   const auto ortho = [&](OrthoFn fn, int ja, int na, int jd, int nd, int extra, double per) {
-    OrthoArgs o{pa, A, ja, jd, B.gram};
+    OrthoArgs o{pa, A, ja, jd, B.gram, B.herm ? 1e-5f : 4e-9f};
     o.p.items = B.items_o;
     const int pe = h->prof.begin(st);
     fn<<<B.nio, blk, 0, st>>>(o);
@@ -1219,11 +1220,11 @@ static cudaError_t enqueue_basis(Handle* h, BasisRun& B) {
       for (int jd = 0; jd <= i; jd += ORTHO_NB) {
         const int nd = std::min(ORTHO_NB, i + 1 - jd);
         const bool newest = jd + nd == i + 1;
-        ortho(ortho_fn(na, nd, newest), ja, na, jd, nd, newest ? nd - 1 : 0, 8.0);
+        ortho(B.herm ? ortho_fn<true>(na, nd, newest) : ortho_fn<false>(na, nd, newest), ja, na, jd, nd, newest ? nd - 1 : 0, 8.0);
         ja = jd;
         na = nd;
       }
-      ortho(ortho_fn(na, 0, false), ja, na, 0, 0, 0, 8.0);
+      ortho(ortho_fn<false>(na, 0, false), ja, na, 0, 0, 0, 8.0);
     }
     if (i < m - 1) scale(i + 1);
   }
@@ -1541,7 +1542,9 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
   int64_t builds = 0, rounds = 0, fallbacks = 0;
   const dim3 blk(SPC_LANES, SPC_WARPS);
   bool lanczos_ok = h->krylov_method == 1 || h->krylov_method == 2;
-  for (const JobSpec& j : jobs) lanczos_ok = lanczos_ok && j.herm_shift;
+  bool all_herm = true;
+  for (const JobSpec& j : jobs) all_herm = all_herm && j.herm_shift;
+  lanczos_ok = lanczos_ok && all_herm;
   std::vector<char> hplan;
   // round graphs of this call: plan shape -> (executable graph, launches in it)
   struct GraphCache : std::map<std::vector<int64_t>, std::pair<cudaGraphExec_t, int64_t>> {
@@ -1678,6 +1681,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
       CK(cudaMemsetAsync(d_qmax, 0, 2 * sizeof(unsigned) * slots_fl, st));
       BasisRun br{};
       br.tiles = d_tiles;
+      br.herm = all_herm;
       br.items_p = d_items_p;
       br.items_s = d_items_s;
       br.items_b = d_items_b;

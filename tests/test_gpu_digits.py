@@ -203,3 +203,29 @@ def test_extreme_units(sampler, oracle, method, scale):
         sampler.set_sample_path("auto")
         sampler.set_krylov("mgs")
     assert max(np.max(np.abs(getattr(got, k) - ref[k])) for k in KEYS) <= 1e-12
+
+
+@pytest.mark.parametrize("m", [8, 12, 20])
+@pytest.mark.parametrize("size", [1e-14, 1e-10, 1e-7, 1e-4])
+def test_weak_couplings(sampler, m, size):
+    """Hyperfine couplings so weak that a basis passes near an invariant subspace
+    of the electrons' part: vectors past it lose orthogonality, and the products
+    of basis vectors (single precision but for neighbours where H is Hermitian
+    up to a shift) carry the projections. Against the per-sample kernel, whose
+    products are all FP64; what is left of a defect reaches the populations
+    through the coupling alone."""
+    rng = np.random.default_rng(6)
+    A1, A2 = ([a * size for a in W._tensors(rng, len(g), -2.0, 2.0, True)] for g in ((3, 2), (2, 2)))
+    s = SysParam.from_input_units(Electron(g_I=[3, 2], A=A1), Electron(g_I=[2, 2], A=A2), J=0.01,
+                                  D=W.axial_dipolar(-0.4), kS_per_us=1.0, kT_per_us=1.0)
+    zk = W.random_phase_samples(s.Z, 5, seed=m)
+    sampler.set_krylov("mgs")
+    out = {}
+    try:
+        sampler.build_h(s, np.array([0.01, 0.03, 0.04]), "general")
+        for mode in ("off", "single"):
+            sampler.set_sample_path(mode)
+            out[mode] = sampler.trace_sampling(zk, DT, 40 * DT, m, 1e-6)
+    finally:
+        sampler.set_sample_path("auto")
+    assert max(np.max(np.abs(getattr(out["off"], k) - getattr(out["single"], k))) for k in KEYS) <= 1e-12
