@@ -87,6 +87,16 @@ __device__ __forceinline__ double wide_float(float f) {
   const unsigned h = u < 0x00800000u ? 0u : (u >> 3) + (896u << 20);
   return __hiloint2double((int)(h | (b & 0x80000000u)), u < 0x00800000u ? 0 : (int)(b << 29));
 }
+// The same with infinities and NaN kept.
+__device__ __forceinline__ double wide_any(float f) {
+  const double v = wide_float(f);
+  const bool special = (__float_as_uint(f) & 0x7f800000u) == 0x7f800000u;
+  return __hiloint2double(__double2hiint(v) + (special ? 896 << 20 : 0), __double2loint(v));
+}
+// Whether coefficients of a Hamiltonian with ||H|| <= 2^rexp stay in the range of
+// single precision, with room for their products: what they lose below 2^-126 is
+// under 2^-86 of the bound.
+__device__ __forceinline__ bool single_range(int rexp) { return rexp >= -40 && rexp <= 100; }
 #define ORTHO_SMALL 44
 
 struct OrthoArgs {
@@ -183,7 +193,7 @@ __global__ void __launch_bounds__(256, 2) k_ortho(OrthoArgs o) {
       const int jv = o.ja + ty;
       double2 d = cz();
       float2 gk[ORTHO_NB - 1];
-      bool big = false;
+      bool big = !single_range(T.rexp);
       double2* G = o.gram + ((size_t)it.x * a.m + jv) * ORTHO_NB * SPC_LANES + tx;
       if (ty < NA) {
         d = make_double2(acc_get(in + 4 * ty * SPC_LANES, acc_dot_exp(T)),
@@ -209,9 +219,13 @@ __global__ void __launch_bounds__(256, 2) k_ortho(OrthoArgs o) {
         }
       }
       // an orthonormal basis (products of rounding size): the corrections are
-      // below 4e-9 of the coefficients, first order and single precision leave
-      // an error below 1e-15 of them. A basis past a breakdown takes the
-      // recurrence in full.
+      // below 4e-9 of the coefficients (1e-5 of small ones between far vectors
+      // where HERM), and first order and single precision leave at most 7e-15
+      // (7 products, two factors cut to 23 bits) of the largest. The coefficient
+      // recorded is the one subtracted, so H Q = Q A holds to rounding all the
+      // same, and what is missing adds to a defect of orthogonality of the
+      // products' own size. A basis past a breakdown takes the recurrence in
+      // full, as do units past single precision.
       if (!__syncthreads_or(big ? 1 : 0)) {
         float2 c = make_float2(0.f, 0.f);
         if (ty < NA) {
@@ -221,7 +235,7 @@ __global__ void __launch_bounds__(256, 2) k_ortho(OrthoArgs o) {
             c.x += gk[k].x * hx - gk[k].y * hy;
             c.y += gk[k].x * hy + gk[k].y * hx;
           }
-          d = make_double2(d.x - wide_float(c.x), d.y - wide_float(c.y));
+          d = make_double2(d.x - wide_any(c.x), d.y - wide_any(c.y));
         }
         __syncthreads();
         if (ty < NA) h[ty][tx] = d;
@@ -244,7 +258,7 @@ __global__ void __launch_bounds__(256, 2) k_ortho(OrthoArgs o) {
       if (ty < NA) {
         // |h| < 2^(rexp - ORTHO_SMALL) by the exponents; NaN and infinities are large
         // as are all where products would leave the range of single precision
-        const bool lg = T.rexp < -40 || T.rexp > 100 ||
+        const bool lg = !single_range(T.rexp) ||
                         __any_sync(0xffffffffu, act && (int)(abs_high(d) >> 20) - 1023 >= T.rexp - ORTHO_SMALL);
         hs[ty][tx] = lg ? make_float2(0.f, 0.f) : make_float2(cut_float(d.x), cut_float(d.y));
         if (tx == 0) large[ty] = lg ? 1 : 0;

@@ -404,12 +404,12 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
             }
             __syncwarp();
           }
-          // first-order corrections where the basis is orthonormal to rounding,
-          // the recurrence otherwise
+          // first-order corrections where the basis is orthonormal to rounding
+          // and the units suit single precision, the recurrence otherwise
           const int v = lane;
           double2 d = v < nb ? ort.h[v] : cz();
           float2 c = make_float2(0.f, 0.f);
-          bool big = false;
+          bool big = !single_range(J.rexp);
           if (v < nb)
             for (int k = 0; k < v; ++k) {
               const double2 gv = ort.gram[jb + v][k];
@@ -419,7 +419,7 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
               c.y += gx * hy + gy * hx;
             }
           if (!__any_sync(0xffffffffu, big)) {
-            d = make_double2(d.x - wide_float(c.x), d.y - wide_float(c.y));
+            d = make_double2(d.x - wide_any(c.x), d.y - wide_any(c.y));
           } else {
             for (int k = 0; k + 1 < nb; ++k) {
               const double2 hk = make_double2(__shfl_sync(0xffffffffu, d.x, k), __shfl_sync(0xffffffffu, d.y, k));
