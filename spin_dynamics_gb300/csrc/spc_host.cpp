@@ -268,8 +268,10 @@ int make_host_system(const spc_system* sys, int mode, HostSystem& hs) {
   return SPC_OK;
 }
 
+// The limits are those of square norms in a double: 2^1024, and 2^-1020 as the
+// least bound that a normal number can pass.
 int norm_exponent(double bound) {
-  return std::isfinite(bound) && bound > 0.0 ? std::min(400, std::max(-400, std::ilogb(bound) + 2)) : 0;
+  return std::isfinite(bound) && bound > 0.0 ? std::min(512, std::max(-510, std::ilogb(bound) + 2)) : 0;
 }
 
 int norm_exponent(const HostSystem& hs, int mode) {

@@ -41,3 +41,15 @@ def test_past_single_precision(sampler, oracle, mode, m, power):
     zk = W.random_phase_samples(s.Z, 5, seed=3)
     ref = oracle.trace_sampling(rp, col, val, zk, DT, 40 * DT, m, 1e-6)
     assert worst(given(sampler, rp, col, val * 2.0**power, zk, DT * 2.0**-power, 40, m, "mgs", mode), ref) <= 1e-12
+
+
+@pytest.mark.parametrize("mode", ["off", "on", "single"])
+@pytest.mark.parametrize("method", ["mgs", "auto"])
+@pytest.mark.parametrize("power", [-480, -420, 420, 480])
+def test_units_to_the_range_of_squares(sampler, oracle, mode, method, power):
+    """Square norms to the ends of a double's range."""
+    s = W.small_pair()
+    rp, col, val = iso_csr(oracle, s, 0.05)
+    zk = W.random_phase_samples(s.Z, 5, seed=3)
+    ref = oracle.trace_sampling(rp, col, val, zk, DT, 40 * DT, 17, 1e-6)
+    assert worst(given(sampler, rp, col, val * 2.0**power, zk, DT * 2.0**-power, 40, 17, method, mode), ref) <= 1e-12
