@@ -97,7 +97,7 @@ __device__ __forceinline__ double wide_any(float f) {
 // single precision, with room for their products: what they lose below 2^-126 is
 // under 2^-86 of the bound.
 __device__ __forceinline__ bool single_range(int rexp) { return rexp >= -40 && rexp <= 100; }
-#define ORTHO_SMALL 44
+#define ORTHO_SMALL 44  // bits of a coefficient below the last beta
 
 struct OrthoArgs {
   PassArgs p;
@@ -126,13 +126,16 @@ struct OrthoArgs {
 // vectors in 126 registers. Lanczos at dim 2304, 77 samples: the norm pass 15.3
 // -> 10.1 us, k_spmm_blk with its projection 27.9 -> 19.5 us without the last sum.
 // Small coefficients: where H is Hermitian up to a shift every h_v but the last
-// two is of rounding size. A vector whose coefficients are below 2^(rexp - 44) in
-// all of a tile's samples is subtracted in single precision (q's leading 20
-// bits): an error below 2^-60 of the bound on ||H||, 1/128 of one FP64 rounding
-// of p. 64 FP32 multiply-adds issue in the time of one FP64, and the conversions
-// are done on the words, since the conversion instruction also runs on the FP64
-// pipe. Up to two other vectors are subtracted beside them in FP64; a block with
-// more (unequal rates) takes FP64 throughout. The block's pass and the norm pass
+// two is of rounding size. A vector whose coefficients are below 2^-44 of the
+// last beta (the coefficient of Q_{i-1}, so no more than ||p||) in all of a
+// tile's samples is subtracted in single precision: eight of them, cut to 23
+// bits, times q's leading 20 leave an error below 2^-60 of ||p||, 1/128 of one
+// FP64 rounding of it. (A line at 2^-44 of the bound on ||H|| took everything
+// for small where the state is in a part of H far below the bound.) 64 FP32
+// multiply-adds issue in the time of one FP64, and the conversions are done on
+// the words, since the conversion instruction also runs on the FP64 pipe. Up to
+// two other vectors are subtracted beside them in FP64; a block with more
+// (unequal rates) takes FP64 throughout. The block's pass and the norm pass
 // at dim 2304, 384 samples, m = 16: 97 -> 68 and 35 -> 31 us; dim 55296, 32
 // samples, m = 30: 200 -> 129 and 69 -> 59 us. A branch for each vector instead
 // made the norm pass slower (40 and 80 us).
@@ -194,6 +197,8 @@ __global__ void __launch_bounds__(256, 2) k_ortho(OrthoArgs o) {
       double2 d = cz();
       float2 gk[ORTHO_NB - 1];
       bool big = !single_range(T.rexp);
+      unsigned eb = 0;  // the last beta's exponent
+      if (ty < NA && act && i > 0) eb = abs_high(a.Ahess[(size_t)w * mm + i + (size_t)(i - 1) * a.m]) >> 20;
       double2* G = o.gram + ((size_t)it.x * a.m + jv) * ORTHO_NB * SPC_LANES + tx;
       if (ty < NA) {
         d = make_double2(acc_get(in + 4 * ty * SPC_LANES, acc_dot_exp(T)),
@@ -256,10 +261,11 @@ __global__ void __launch_bounds__(256, 2) k_ortho(OrthoArgs o) {
       }
       if (first && act && ty < NA) a.Ahess[(size_t)w * mm + jv + (size_t)i * a.m] = d;
       if (ty < NA) {
-        // |h| < 2^(rexp - ORTHO_SMALL) by the exponents; NaN and infinities are large
+        // |h| < 2^-ORTHO_SMALL beta by the exponents; NaN and infinities are large
         // as are all where products would leave the range of single precision
-        const bool lg = !single_range(T.rexp) ||
-                        __any_sync(0xffffffffu, act && (int)(abs_high(d) >> 20) - 1023 >= T.rexp - ORTHO_SMALL);
+        // (and a column without a beta)
+        const bool lg = __any_sync(0xffffffffu, act && (eb < 1023 - 60 || eb > 1023 + 100 ||
+                                                        (abs_high(d) >> 20) + ORTHO_SMALL >= eb));
         hs[ty][tx] = lg ? make_float2(0.f, 0.f) : make_float2(cut_float(d.x), cut_float(d.y));
         if (tx == 0) large[ty] = lg ? 1 : 0;
       }

@@ -53,3 +53,36 @@ def test_units_to_the_range_of_squares(sampler, oracle, mode, method, power):
     zk = W.random_phase_samples(s.Z, 5, seed=3)
     ref = oracle.trace_sampling(rp, col, val, zk, DT, 40 * DT, 17, 1e-6)
     assert worst(given(sampler, rp, col, val * 2.0**power, zk, DT * 2.0**-power, 40, 17, method, mode), ref) <= 1e-12
+
+
+def beside(rp, col, val, scale):
+    """H on one half of the nuclear indices and scale * H on the other: the CSR
+    of both, interleaved as (electron, half, index)."""
+    n = len(rp) - 1
+    Z = n // 4
+    row = np.repeat(np.arange(n), np.diff(rp))
+
+    def place(r, half):
+        return (r // Z) * 2 * Z + half * Z + r % Z
+
+    r = np.concatenate([place(row, k) for k in (0, 1)])
+    c = np.concatenate([place(np.asarray(col, np.int64), k) for k in (0, 1)])
+    v = np.concatenate([val, val * scale])
+    o = np.lexsort((c, r))
+    rp2 = np.concatenate([[0], np.cumsum(np.bincount(r, minlength=2 * n))])
+    return rp2.astype(np.int32), c[o].astype(np.int32), v[o]
+
+
+@pytest.mark.parametrize("mode", ["off", "on", "single"])
+@pytest.mark.parametrize("method, kT", [("mgs", 0.0), ("auto", 0.0), ("mgs", 1e-3), ("mgs", 0.3)])
+@pytest.mark.parametrize("m", [9, 17])
+@pytest.mark.parametrize("power", [0, 20, 30])
+def test_large_part_beside(sampler, oracle, mode, method, kT, m, power):
+    """States confined to a part of H that a larger one bounds."""
+    s = W.small_pair()
+    s.kS, s.kT = 0.0, kT
+    rp, col, val = iso_csr(oracle, s, 0.05)
+    zk = W.random_phase_samples(s.Z, 5, seed=3)
+    ref = oracle.trace_sampling(rp, col, val, zk, DT, 40 * DT, m, 1e-6)
+    z2 = np.concatenate([zk, np.zeros_like(zk)], axis=1)
+    assert worst(given(sampler, *beside(rp, col, val, 2.0**power), z2, DT, 40, m, method, mode), ref) <= 1e-12
