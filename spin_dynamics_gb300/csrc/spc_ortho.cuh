@@ -11,7 +11,9 @@
 // order, so results repeat bit for bit, and their only rounding is the last
 // one. The kernel that needs a sum reads it in its prologue. Three sets of
 // accumulators rotate: a kernel adds to one, reads the one before and clears
-// the one after.
+// the one after. A square norm has a third word, 50 bits further down: a vector
+// may be small against ||H|| (a state in a part of H far below the bound), and
+// its norm has a double's bits down to 2^-53 of the bound.
 #define ACC_VECS 15             // complex sums per sample (8 dots + 7 basis products)
 #define ACC_MAX (4 * ACC_VECS)  // largest component's high word
 #define ACC_BAD (4 * ACC_VECS + 1)
@@ -25,8 +27,10 @@ struct AccArgs {
 __device__ __forceinline__ acc_t* acc_tile(const AccArgs& A, int set, int tile) {
   return A.acc + ((size_t)set * A.ntiles + tile) * ACC_ROWS * SPC_LANES;
 }
-// x to the accumulator pair at p (stride 32), |sum| <= 2^e; NaN, infinities and
-// values past the bound mark the sample
+// x to the accumulator pair at p (stride 32; NORM: the upper or the lower pair of
+// three words), |sum| <= 2^e; NaN, infinities and values past the bound mark the
+// sample
+template <bool NORM = false>
 __device__ __forceinline__ void acc_add(acc_t* p, acc_t* bad, double x, int e) {
   const long long b = __double_as_longlong(x);
   const int ex = (int)(b >> 52) & 0x7ff;
@@ -36,8 +40,12 @@ __device__ __forceinline__ void acc_add(acc_t* p, acc_t* bad, double x, int e) {
     return;
   }
   const acc_t man = (b & 0xfffffffffffffll) | (1ull << 52);
-  const int sh = ex - 965 - e;  // <= 59
-  acc_t lo, hi;                 // man * 2^sh as hi 2^50 + lo
+  int sh = ex - 965 - e;  // <= 59
+  if (NORM && sh < 0) {
+    sh += 50;
+    p += SPC_LANES;
+  }
+  acc_t lo, hi;  // man * 2^sh as hi 2^50 + lo
   if (sh >= 0) {
     lo = (man << sh) & ((1ull << 50) - 1);
     hi = sh >= 50 ? man << (sh - 50) : man >> (50 - sh);
@@ -55,6 +63,14 @@ __device__ __forceinline__ void acc_add(acc_t* p, acc_t* bad, double x, int e) {
 }
 __device__ __forceinline__ double acc_get(const acc_t* p, int e) {
   return ldexp(fma((double)(long long)p[0], 1125899906842624.0, (double)(long long)p[SPC_LANES]), e - 110);
+}
+// The sum of three words; the third adds less than 2^-54 of it from 2^16 units of
+// the first on.
+__device__ __forceinline__ double acc_get_norm(const acc_t* p, int e) {
+  const long long hi = (long long)p[0];
+  if (hi >= 65536) return acc_get(p, e);
+  const double t = fma((double)(long long)p[SPC_LANES], 1125899906842624.0, (double)(long long)p[2 * SPC_LANES]);
+  return ldexp(fma((double)hi, 1125899906842624.0 * 1125899906842624.0, t), e - 160);
 }
 __device__ __forceinline__ void acc_clear(const AccArgs& A, int tile, int tid, int nth) {
   acc_t* p = acc_tile(A, A.clear, tile);
@@ -364,7 +380,7 @@ __global__ void __launch_bounds__(256, 2) k_ortho(OrthoArgs o) {
 #pragma unroll
       for (int y = 1; y < SPC_WARPS; ++y) s += im ? red[u][y][tx].y : red[u][y][tx].x;
       const int e = ND == 0 ? acc_norm_exp(T) : (v < ND ? acc_dot_exp(T) : ACC_GRAM_EXP);
-      acc_add(out + (4 * v + 2 * im) * SPC_LANES, out + ACC_BAD * SPC_LANES, s, e);
+      acc_add<ND == 0>(out + (4 * v + 2 * im) * SPC_LANES, out + ACC_BAD * SPC_LANES, s, e);
       if (ND == 0) {
 #pragma unroll
         for (int y = 1; y < SPC_WARPS; ++y) top = max(top, mx[y][tx]);
@@ -381,7 +397,7 @@ __device__ __forceinline__ double ortho_norm(const PassArgs& a, const AccArgs& A
                                              bool record, int* ex) {
   const int w = tile * SPC_LANES + lane;
   const acc_t* in = acc_tile(A, A.in, tile) + lane;
-  double b = sqrt(acc_get(in, acc_norm_exp(T)));
+  double b = sqrt(acc_get_norm(in, acc_norm_exp(T)));
   if (in[ACC_BAD * SPC_LANES]) b = __longlong_as_double(0x7ff8000000000000ll);
   // exact breakdown (p == 0): the next basis vector is 0 instead of 0/0
   const double rb = b > 0.0 ? 1.0 / b : (b == 0.0 ? 0.0 : b);

@@ -45,7 +45,8 @@ struct SmallJob {
 // {sum or root, reciprocal}. A double add's latency is 109 clocks with its
 // shuffle, eight of them in a row and 1010 more for a square root and a division;
 // as integer multiples of 2^(e - 110) (acc_add's pair of words) a level takes a
-// third of that. red: SMALL_WARPS pairs and the result, two sets that the
+// third of that. A square that is not zero counts as one unit at least, so that
+// only a zero vector has a zero norm (small_norm). red: SMALL_WARPS pairs and the result, two sets that the
 // calls use in turn (`turn`). Called by all threads; one result per two barriers.
 //
 // A sample's rows may be spread over a cluster of up to SMALL_TEAM CTAs (CL):
@@ -73,7 +74,8 @@ __device__ __forceinline__ double2 block_sum(double v, int e, SmallRed& red, int
       lo = (long long)((man << sh) & ((1ull << 50) - 1));
       hi = (long long)(sh >= 50 ? man << (sh - 50) : man >> (50 - sh));
     } else {
-      const acc_t u = sh < -62 ? 0 : ((man >> (-sh - 1)) + 1) >> 1;
+      acc_t u = sh < -62 ? 0 : ((man >> (-sh - 1)) + 1) >> 1;
+      if (NORM && u == 0) u = 1;
       lo = (long long)(u & ((1ull << 50) - 1));
       hi = (long long)(u >> 50);
     }
@@ -126,6 +128,19 @@ __device__ __forceinline__ double2 block_sum(double v, int e, SmallRed& red, int
   const double2 res = red.out[turn];
   turn ^= 1;
   return res;
+}
+
+// {root, reciprocal} of a sum of squares bounded by 2^e: taken again in finer
+// units where the first ones left fewer bits than a double's (a vector far
+// below the bound on ||H||).
+template <bool CL>
+__device__ __forceinline__ double2 small_norm(double v, int e, SmallRed& red, int& turn, SmallTeam team) {
+  for (;;) {
+    const double2 r = block_sum<true, CL>(v, e, red, turn, team);
+    const int top = 2 * (((__double2hiint(r.x) >> 20) & 0x7ff) - 1023) + 3;  // the sum is below 2^top
+    if (!(r.x > 0.0) || top >= e - 44 || e < -1000) return r;
+    e = top;
+  }
 }
 
 // Real sum over the CTA in doubles, its root and reciprocal: for a value of any
@@ -468,7 +483,7 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
       pd[idx] = pv;
       nr = fma(pv, pv, nr);
     }
-    const double2 bn = block_sum<true, CL>(nr, 2 * J.rexp, red, turn, team);
+    const double2 bn = small_norm<CL>(nr, 2 * J.rexp, red, turn, team);
     beta = bn.x;
     if (tid == 0) {
       A[(i + 1) + i * m] = make_double2(beta, 0.0);

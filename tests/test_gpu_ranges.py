@@ -76,7 +76,7 @@ def beside(rp, col, val, scale):
 @pytest.mark.parametrize("mode", ["off", "on", "single"])
 @pytest.mark.parametrize("method, kT", [("mgs", 0.0), ("auto", 0.0), ("mgs", 1e-3), ("mgs", 0.3)])
 @pytest.mark.parametrize("m", [9, 17])
-@pytest.mark.parametrize("power", [0, 20, 30])
+@pytest.mark.parametrize("power", [0, 20, 30, 40, 50])
 def test_large_part_beside(sampler, oracle, mode, method, kT, m, power):
     """States confined to a part of H that a larger one bounds."""
     s = W.small_pair()
