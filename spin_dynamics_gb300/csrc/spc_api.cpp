@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "spc_internal.h"
+#include "spc_plan.h"
 
 struct spc_handle {
   spc::Handle h;
@@ -171,14 +172,7 @@ int spc_set_h(spc_handle* h, const spc_csr* H) {
   h->h.nnz = nnz;
   h->h.herm_shift = is_hermitian_plus_shift(n, rp, cl, H->val);
   h->h.blk_one.describe({spc::BlockSys{}});
-  // ||H|| <= sqrt(n) max row sum
-  double rows = 0.0;
-  for (int r = 0; r < n; ++r) {
-    double t = 0.0;
-    for (int k = rp[r]; k < rp[r + 1]; ++k) t += std::fabs(H->val[2 * (size_t)k]) + std::fabs(H->val[2 * (size_t)k + 1]);
-    if (!(t <= rows)) rows = t;
-  }
-  h->h.rexp = spc::norm_exponent(rows * std::sqrt((double)n));
+  h->h.rexp = spc::norm_exponent(spc::csr_norm_bound(n, rp.data(), cl.data(), H->val));
   return spc::prepare_spmm_rows(&h->h);
 }
 
