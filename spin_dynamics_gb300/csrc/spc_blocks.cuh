@@ -23,7 +23,8 @@
 // rounding unit of 2^-57 of the result reaches only when nearly every digit of
 // a row has its largest value and one sign.
 
-#define BLK_MAXNBR 19
+static_assert(128 * 255 * (6 * (4 * BLK_MAXNBR + 8) + 8) < 1 << 24, "sums of digit products stay exact");
+static_assert(BLK_MAXNBR + 1 <= 32, "a list has an entry for each lane at most");
 #define BLK_THREADS 128
 #define BLK_AHEAD 2  // k-steps copied ahead (and the least length of a list)
 #define BLK_IDX (BLK_THREADS / 64)  // nuclear indices of a CTA at a time

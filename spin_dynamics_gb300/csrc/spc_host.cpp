@@ -347,7 +347,7 @@ BlockSys make_block_sys(const HostSystem& hs, int mode) {
   for (int e = 0; e < 4; ++e)
     for (int f = 0; f < 4; ++f)
       if (!std::isfinite(l1(hs.gen.H[e][f]))) return b;
-  if (!std::isfinite(rows) || nbr > 19 || hs.N > INT32_MAX) return b;
+  if (!std::isfinite(rows) || nbr > BLK_MAXNBR || hs.N > INT32_MAX) return b;
   b.Z = hs.Z;
   b.bk = std::max(4, (nbr + 2) / 2 * 2);
   const int eo = off > 0.0 ? std::ilogb(off) : -1000, es = self > 0.0 ? std::ilogb(self) : -1000;

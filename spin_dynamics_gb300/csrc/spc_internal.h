@@ -100,6 +100,10 @@ struct HMeta {
   unsigned long long ncplx;  // entries with a nonzero imaginary part
 };
 
+// Neighbours of a nuclear index (its other states by one step of a nucleus) that
+// k_spmm_blk takes; spc_blocks.cuh states what bounds it.
+constexpr int BLK_MAXNBR = 19;
+
 // Block structure of a general-builder Hamiltonian: multiplicities and strides
 // of the nuclei, length of a nuclear index's block list (itself first, even),
 // unit exponent of the entries and exponent of the closed sums.

@@ -1,0 +1,42 @@
+"""The general builder's product on blocks (k_spmm_blk) against the product on
+the CSR of the same Hamiltonian, given as a CSR. Both carry rounding of order
+1e-16 of ||H|| a step: 1e-13 of populations of at most 1 over a few steps; a
+wrong list entry or an inexact sum of digits shows at 1e-7 and above."""
+import numpy as np
+import pytest
+
+from spin_dynamics_gb300 import workloads as W
+from spin_dynamics_gb300.spinsys import GAMMA_E, Electron, SysParam
+
+pytestmark = pytest.mark.gpu
+DT = 1.0 * GAMMA_E / 1000
+KEYS = ("P_S", "P_T0", "P_Tp", "P_Tm")
+
+
+def pair(g1, g2, seed=4, kT=1.0):
+    rng = np.random.default_rng(seed)
+    A1, A2 = (W._tensors(rng, len(g), -2.0, 2.0, True) for g in (g1, g2))
+    return SysParam.from_input_units(Electron(g_I=list(g1), A=A1), Electron(g_I=list(g2), A=A2), J=0.01,
+                                     D=W.axial_dipolar(-0.4), kS_per_us=1.0, kT_per_us=kT)
+
+
+def difference(a, b):
+    return max(np.max(np.abs(getattr(a, k) - getattr(b, k))) for k in KEYS)
+
+
+@pytest.mark.parametrize("g1, g2", [((3,) * 5, (3,) * 4), ((3,) * 5, (3, 3, 3, 3, 2)), ((3,) * 5, (3,) * 5)])
+def test_longest_lists(sampler, g1, g2):
+    """18 and 19 neighbours (the most that the blocks take) and 20 (the CSR)."""
+    s = pair(g1, g2)
+    zk = W.random_phase_samples(s.Z, 2, seed=1)
+    sampler.build_h(s, np.array([0.01, 0.03, 0.04]), "general")
+    out = {k: [] for k in ("built", "given")}
+    for which in out:
+        if which == "given":
+            sampler.set_h(*sampler.get_h())
+        for method in ("mgs", "auto"):
+            sampler.set_krylov(method)
+            out[which].append(sampler.trace_sampling(zk, DT, 4 * DT, 6, 1e-6))
+    sampler.set_krylov("mgs")
+    for a, b in zip(out["built"], out["given"]):
+        assert difference(a, b) <= 1e-13
