@@ -263,6 +263,7 @@ struct BuildSlice {
   int* split;           // N
   long long* total;     // 1
   bool herm;            // H = A - i*kappa*1: the execution copy holds A
+  int residue;          // BlockSys::residue
   HMeta* meta;          // kappa and complex-entry count of the copy (zeroed)
 };
 
@@ -301,7 +302,8 @@ static int build_slices(Handle* h, std::vector<BuildSlice>& sl, const std::vecto
       k_ref_fill<<<blocks, threads, 0, st>>>(N, Z, nn, b.nuc, b.hs->ref, b.rowptr, b.col, b.val);
     else
       k_gen_fill_tab<<<blocks, threads, 0, st>>>(N, Z, nn, b.nuc, b.hs->gen, b.tab, b.rowptr, b.col, b.val);
-    enqueue_split_rows(N, b.rowptr, b.col, b.val, b.xcol, b.xval, b.xvs, b.split, b.herm, b.meta, st);
+    enqueue_split_rows(N, b.rowptr, b.col, b.val, b.xcol, b.xval, b.xvs, b.split, b.herm, b.residue, b.meta,
+                       st);
     h->count_launch(2);
   }
   if (cudaStreamSynchronize(st) != cudaSuccess)
@@ -356,12 +358,13 @@ int build_h_device(Handle* h, const HostSystem& hs, int mode) {
     return SPC_ERR_ALLOC;
   if (cudaMemsetAsync(h->hmeta.p, 0, sizeof(HMeta), h->stream) != cudaSuccess)
     return set_error(SPC_ERR_CUDA, "Hamiltonian build failed");
+  BlockSys bs = make_block_sys(hs, mode);
   std::vector<BuildSlice> sl(1);
   sl[0] = BuildSlice{&hs, (const NucInfo*)h->bnuc.p, (const double2*)h->btab.p, (int*)h->bcnt.p, h->d_rowptr,
                      h->d_col, h->d_val,
                      (int*)h->xcol.p, (double2*)h->xval.p, (double*)h->xvs.p, (int*)h->xsplit.p,
                      (long long*)h->btot.p,
-                     hs.herm_shift, (HMeta*)h->hmeta.p};
+                     hs.herm_shift, bs.residue(), (HMeta*)h->hmeta.p};
   rc = build_slices(h, sl, {nnz}, mode);
   if (rc) return rc;
   HMeta meta{};
@@ -372,7 +375,8 @@ int build_h_device(Handle* h, const HostSystem& hs, int mode) {
   h->nnz_cplx = (int64_t)meta.ncplx;
   h->herm_shift = hs.herm_shift;
   h->rexp = norm_exponent(hs, mode);
-  h->blk_one.describe({make_block_sys(hs, mode)});
+  bs.check_rows(meta);
+  h->blk_one.describe({std::move(bs)});
   return SPC_OK;
 }
 
@@ -416,31 +420,34 @@ int build_h_batch_device(Handle* h, const std::vector<HostSystem>& hs, int mode)
   if (cudaMemsetAsync(B.meta.p, 0, sizeof(HMeta) * ns, h->stream) != cudaSuccess)
     return set_error(SPC_ERR_CUDA, "Hamiltonian build failed");
   std::vector<BuildSlice> sl(ns);
+  std::vector<BlockSys> bs(ns);
   int64_t coff = 0;
   for (size_t k = 0; k < ns; ++k) {
+    bs[k] = make_block_sys(hs[k], mode);
     sl[k] = BuildSlice{&hs[k], (const NucInfo*)h->bnuc.p + noff[k], (const double2*)h->btab.p, (int*)h->bcnt.p + coff,
                        (int*)B.rowptr.p + B.rp_off[k], (int*)h->xcol.p + B.nz_off[k],
                        (double2*)h->xval.p + B.nz_off[k], (int*)B.col.p + B.nz_off[k],
                        (double2*)B.val.p + B.nz_off[k], (double*)B.vsum.p + B.nz_off[k],
                        (int*)B.split.p + B.rp_off[k],
-                       (long long*)h->btot.p + k, hs[k].herm_shift, (HMeta*)B.meta.p + k};
+                       (long long*)h->btot.p + k, hs[k].herm_shift, bs[k].residue(), (HMeta*)B.meta.p + k};
     coff += hs[k].N;
   }
   rc = build_slices(h, sl, B.nnz, mode);
   B.nnz_cplx.assign(ns, 0);
-  std::vector<BlockSys> bs(ns);
   B.rexp.assign(ns, 0);
   for (size_t k = 0; k < ns; ++k) {
-    bs[k] = make_block_sys(hs[k], mode);
     B.rexp[k] = norm_exponent(hs[k], mode);
   }
-  h->blk_batch.describe(std::move(bs));
   if (!rc && ns) {
     std::vector<HMeta> meta(ns);
     if (cudaMemcpy(meta.data(), B.meta.p, sizeof(HMeta) * ns, cudaMemcpyDeviceToHost) != cudaSuccess)
       rc = set_error(SPC_ERR_CUDA, "Hamiltonian build failed");
-    for (size_t k = 0; k < ns; ++k) B.nnz_cplx[k] = (int64_t)meta[k].ncplx;
+    for (size_t k = 0; k < ns; ++k) {
+      B.nnz_cplx[k] = (int64_t)meta[k].ncplx;
+      bs[k].check_rows(meta[k]);
+    }
   }
+  h->blk_batch.describe(std::move(bs));
   // the single-Hamiltonian execution copy (xcol/xval) served as scratch
   h->n = 0;
   h->nnz = 0;

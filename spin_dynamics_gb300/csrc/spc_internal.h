@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -98,6 +99,9 @@ struct Prof {
 struct HMeta {
   double kappa;              // H_eff = A - i*kappa*1 (systems with herm_shift)
   unsigned long long ncplx;  // entries with a nonzero imaginary part
+  // 0x7ff less the least biased exponent of a row's largest component (the copy's
+  // rows past the rounding of their sums)
+  unsigned least_row;
 };
 
 // Neighbours of a nuclear index (its other states by one step of a nucleus) that
@@ -114,6 +118,14 @@ struct BlockSys {
   std::vector<int64_t> stride;
   int bk = 0, eoff = 0, bexp = 0;
   int64_t self_off = 0, tab_off = 0, nbr_off = 0;  // place in the store, once built
+  // The blocks' units follow the largest component of H, so a row whose own
+  // largest is 2^-r of it has r bits fewer than its CSR. Down to 2^-12 that is no
+  // matter (2^-42 of the row); states confined to smaller rows would see it.
+  // (Rows below 2^-50 are what sums of the largest leave as rounding, or nothing.)
+  int residue() const { return ok ? std::max(0, eoff - 50 + 1023) : 0; }
+  void check_rows(const HMeta& meta) {
+    if (meta.least_row && 0x7ff - (int)meta.least_row - 1023 < eoff - 12) ok = false;
+  }
 };
 BlockSys make_block_sys(const HostSystem& hs, int mode);
 // An exponent with ||H|| <= 2^e, from the rows' absolute sums (|H| is symmetric).
@@ -267,7 +279,7 @@ int build_h_batch_device(Handle* h, const std::vector<HostSystem>& hs, int mode)
 // receives the copy's count of entries with a nonzero imaginary part. xvs[k]
 // = Re + Im of the copy's entry k (the third product of k_spmm's 3M form).
 void enqueue_split_rows(int64_t N, const int* rowptr, const int* col, const double2* val, int* xcol,
-                        double2* xval, double* xvs, int* split, bool herm, HMeta* meta, cudaStream_t st);
+                        double2* xval, double* xvs, int* split, bool herm, int residue, HMeta* meta, cudaStream_t st);
 int propagate(Handle* h, const double* theta, const double* init_pop, const double* zk_dev,
               int M, double dt, double t_end, int m, double tol, double* out_dev, int T);
 // `single`: the jobs are on the handle's own Hamiltonian, not the batch store.

@@ -337,13 +337,15 @@ __global__ void __launch_bounds__(256, 5)
 // each class); split[r] is the index of the row's first real entry, and
 // xvs[k] = Re + Im of entry k. herm (H = A - i*kappa*1, A Hermitian): diagonal
 // entries are stored with their imaginary part removed (real class) and row
-// 0's removed sum is kappa. meta->ncplx counts the copy's complex entries.
+// 0's removed sum is kappa. meta->ncplx counts the copy's complex entries,
+// meta->least_row finds its smallest row from the biased exponent `residue` on.
 __global__ void k_split_rows(int64_t N, const int* __restrict__ rowptr, const int* __restrict__ col,
                              const double2* __restrict__ val, int* __restrict__ xcol,
                              double2* __restrict__ xval, double* __restrict__ xvs, int* __restrict__ split,
-                             int herm, HMeta* __restrict__ meta) {
+                             int herm, unsigned residue, HMeta* __restrict__ meta) {
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long nc = 0;
+  unsigned top = 0;  // high word of the row's largest component
   if (r < N) {
     const int k0 = rowptr[r], k1 = rowptr[r + 1];
     auto cplx = [&](int k) { return val[k].y != 0.0 && !(herm && col[k] == r); };
@@ -353,6 +355,7 @@ __global__ void k_split_rows(int64_t N, const int* __restrict__ rowptr, const in
         xcol[o] = col[k];
         xval[o] = val[k];
         xvs[o] = val[k].x + val[k].y;
+        top = max(top, abs_high(val[k]));
         o++;
       }
     split[r] = o;
@@ -363,20 +366,25 @@ __global__ void k_split_rows(int64_t N, const int* __restrict__ rowptr, const in
         xcol[o] = col[k];
         xval[o] = herm ? make_double2(val[k].x, 0.0) : val[k];
         xvs[o] = val[k].x;
+        top = max(top, abs_high(xval[o]));
         if (herm && col[k] == r) shift += val[k].y;
         o++;
       }
     if (herm && r == 0) meta->kappa = -shift;
   }
   for (int d = 16; d > 0; d >>= 1) nc += __shfl_down_sync(0xffffffffu, nc, d);
-  if ((threadIdx.x & 31) == 0 && nc) atomicAdd(&meta->ncplx, nc);
+  const unsigned least = __reduce_max_sync(0xffffffffu, top && top >> 20 >= residue ? 0x7ffu - min(top >> 20, 0x7ffu) : 0u);
+  if ((threadIdx.x & 31) == 0) {
+    if (nc) atomicAdd(&meta->ncplx, nc);
+    if (least) atomicMax(&meta->least_row, least);
+  }
 }
 
 void enqueue_split_rows(int64_t N, const int* rowptr, const int* col, const double2* val, int* xcol,
-                        double2* xval, double* xvs, int* split, bool herm, HMeta* meta, cudaStream_t st) {
+                        double2* xval, double* xvs, int* split, bool herm, int residue, HMeta* meta, cudaStream_t st) {
   if (N > 0)
     k_split_rows<<<(int)((N + 255) / 256), 256, 0, st>>>(N, rowptr, col, val, xcol, xval, xvs, split,
-                                                          herm ? 1 : 0, meta);
+                                                          herm ? 1 : 0, (unsigned)residue, meta);
 }
 
 int prepare_spmm_rows(Handle* h) {
@@ -390,7 +398,7 @@ int prepare_spmm_rows(Handle* h) {
   if (cudaMemsetAsync(h->hmeta.p, 0, sizeof(HMeta), h->stream) != cudaSuccess)
     return set_error(SPC_ERR_CUDA, "row split of the Hamiltonian failed");
   enqueue_split_rows(N, h->d_rowptr, h->d_col, h->d_val, (int*)h->xcol.p, (double2*)h->xval.p,
-                     (double*)h->xvs.p, (int*)h->xsplit.p, h->herm_shift, (HMeta*)h->hmeta.p, h->stream);
+                     (double*)h->xvs.p, (int*)h->xsplit.p, h->herm_shift, 0, (HMeta*)h->hmeta.p, h->stream);
   h->count_launch();
   cudaError_t e = cudaMemcpyAsync(&meta, h->hmeta.p, sizeof(HMeta), cudaMemcpyDeviceToHost, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);

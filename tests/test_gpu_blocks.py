@@ -40,3 +40,29 @@ def test_longest_lists(sampler, g1, g2):
     sampler.set_krylov("mgs")
     for a, b in zip(out["built"], out["given"]):
         assert difference(a, b) <= 1e-13
+
+
+@pytest.mark.parametrize("method, kT", [("mgs", 1.0), ("auto", 1.0), ("mgs", 0.3)])
+@pytest.mark.parametrize("size", [1.0, 1e4, 1e8])
+def test_large_coupling_out_of_reach(sampler, method, kT, size):
+    """A nucleus of spin 1 whose one coupling, along z, is large, and states with
+    its m = 0 alone: no row of theirs holds the coupling, and the rest of H keeps
+    its digits beside it."""
+    s = pair((3, 2, 2), (3, 2), kT=kT)
+    s.e1.A[0] = np.diag([0.0, 0.0, size])
+    s.e1.gamma_I = [0.0] + s.e1.gammas[1:]
+    zk = W.random_phase_samples(s.Z, 3, seed=2).reshape(3, 3, -1)
+    zk[:, [0, 2]] = 0.0
+    zk = zk.reshape(3, -1) / np.linalg.norm(zk.reshape(3, -1), axis=1, keepdims=True)
+    out = []
+    sampler.set_sample_path("off")
+    sampler.set_krylov(method)
+    try:
+        sampler.build_h(s, np.array([0.01, 0.03, 0.04]), "general")
+        out.append(sampler.trace_sampling(zk, DT, 40 * DT, 12, 1e-6))
+        sampler.set_h(*sampler.get_h())
+        out.append(sampler.trace_sampling(zk, DT, 40 * DT, 12, 1e-6))
+    finally:
+        sampler.set_krylov("mgs")
+        sampler.set_sample_path("auto")
+    assert difference(*out) <= 1e-13
