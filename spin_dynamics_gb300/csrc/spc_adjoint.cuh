@@ -393,15 +393,19 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   }();
   const int items_cap = h->sm_count * 32 + ntiles;
 
-  Handle::BlockStore* blocks = nullptr;
+  std::vector<char> use;
+  Handle::BlockStore* blocks;
   {
     std::vector<int> used;
     for (const GradJob& J : jobs) {
       used.push_back(J.sys);
       used.push_back(J.sys + 1);
     }
-    const int rc = use_blocks(h, false, used, &blocks);
-    if (rc) return rc;
+    blocks = block_store(h, false, used, use);
+    if (blocks) {
+      const int rc = use_blocks(h, false, use, &blocks);
+      if (rc) return rc;
+    }
   }
   const double xs_bytes = blocks ? 16.0 : 8.0;
   // tiles, slot maps, costate coefficients

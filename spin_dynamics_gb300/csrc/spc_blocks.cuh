@@ -350,23 +350,57 @@ __global__ void __launch_bounds__(BLK_THREADS, 4)
   }
 }
 
-// Fragments of every system of a store (lazily, by the first propagation that
-// runs on them), three launches in all.
-static int prepare_blocks(Handle* h, Handle::BlockStore& S, const std::vector<const int*>& rowptr,
-                          const std::vector<const int*>& col, const std::vector<const double2*>& val) {
-  if (S.ready) {
-    // a call that failed after building returned without waiting for its stream
-    if (S.stream != h->stream && S.built && cudaStreamWaitEvent(h->stream, S.built, 0) != cudaSuccess)
-      return set_error(SPC_ERR_CUDA, "waiting for the blocks failed: %s", cudaGetErrorString(cudaGetLastError()));
-    return SPC_OK;
+// Bytes of a store's buffers (self, tab, nbr, desc) with the fragments of the systems in
+// `use`: 1 KB a nuclear index and a table entry.
+struct BlockSizes {
+  size_t self = 0, tab = 0, nbr = 0, desc = 0;
+};
+static BlockSizes block_sizes(const Handle::BlockStore& S, const std::vector<char>& use) {
+  BlockSizes z;
+  size_t nuc = 1, systems = 0;
+  for (size_t k = 0; k < S.sys.size(); ++k) {
+    if (!use[k]) continue;
+    const BlockSys& b = S.sys[k];
+    int64_t entries = 1;
+    for (int g : b.g) entries += 2 * g;
+    z.self += 1024 * (size_t)b.Z;
+    z.tab += 1024 * (size_t)entries;
+    z.nbr += sizeof(int2) * (size_t)(b.Z * b.bk);
+    nuc += b.g.size();
+    ++systems;
+  }
+  z.desc = sizeof(BlkDesc) * systems + sizeof(BlkNuc) * nuc;
+  return z;
+}
+// What the store's buffers come to once they hold `use` (buffers only grow).
+static size_t block_bytes_after(const Handle::BlockStore& S, const std::vector<char>& use) {
+  if (S.has(use)) return S.bytes();
+  const BlockSizes z = block_sizes(S, use);
+  return std::max(S.self.bytes, z.self) + std::max(S.tab.bytes, z.tab) + std::max(S.nbr.bytes, z.nbr) +
+         std::max(S.desc.bytes, z.desc);
+}
+
+// Fragments of the systems in `use`, built by the first propagation that runs on
+// them, two launches in all. Holds nothing where it fails.
+static int prepare_blocks(Handle* h, Handle::BlockStore& S, const std::vector<char>& use,
+                          const std::vector<const int*>& rowptr, const std::vector<const int*>& col,
+                          const std::vector<const double2*>& val) {
+  // a call that failed after building returned without waiting for its stream
+  if (S.stream != h->stream && S.built && cudaStreamWaitEvent(h->stream, S.built, 0) != cudaSuccess)
+    return set_error(SPC_ERR_CUDA, "waiting for the blocks failed: %s", cudaGetErrorString(cudaGetLastError()));
+  if (S.has(use)) return SPC_OK;
+  const BlockSizes z = block_sizes(S, use);
+  if (h->ensure(S.self, z.self) || h->ensure(S.tab, z.tab) || h->ensure(S.nbr, z.nbr) || h->ensure(S.desc, z.desc)) {
+    S.release();
+    return SPC_ERR_ALLOC;
   }
   std::vector<BlkDesc> d;
   std::vector<BlkNuc> nu;
   int64_t selfs = 0, tabs = 0, nbrs = 0;
   int zmax = 1;
   for (size_t k = 0; k < S.sys.size(); ++k) {
+    if (!use[k]) continue;
     BlockSys& b = S.sys[k];
-    if (!b.ok) continue;
     b.self_off = selfs;
     b.tab_off = tabs;
     b.nbr_off = nbrs;
@@ -379,6 +413,9 @@ static int prepare_blocks(Handle* h, Handle::BlockStore& S, const std::vector<co
     x.rowptr = rowptr[k];
     x.col = col[k];
     x.val = val[k];
+    x.self = (uint4*)S.self.p + 64 * selfs;
+    x.tab = (uint4*)S.tab.p + 64 * tabs;
+    x.nbr = (int2*)S.nbr.p + nbrs;
     int t = 1;
     for (size_t j = 0; j < b.g.size(); ++j) {
       nu.push_back(BlkNuc{b.g[j], t, b.stride[j]});
@@ -390,21 +427,8 @@ static int prepare_blocks(Handle* h, Handle::BlockStore& S, const std::vector<co
     nbrs += b.Z * b.bk;
     zmax = std::max(zmax, (int)b.Z);
   }
-  S.ready = true;
-  if (d.empty()) return SPC_OK;
+  S.placed.assign(S.sys.size(), 0);
   const size_t nb = sizeof(BlkDesc) * d.size();
-  if (h->ensure(S.self, 1024 * (size_t)selfs) || h->ensure(S.tab, 1024 * (size_t)tabs) ||
-      h->ensure(S.nbr, sizeof(int2) * (size_t)nbrs) || h->ensure(S.desc, nb + sizeof(BlkNuc) * (nu.size() + 1))) {
-    S.ready = false;
-    return SPC_ERR_ALLOC;
-  }
-  size_t q = 0;
-  for (const BlockSys& b : S.sys)
-    if (b.ok) {
-      d[q].self = (uint4*)S.self.p + 64 * b.self_off;
-      d[q].tab = (uint4*)S.tab.p + 64 * b.tab_off;
-      d[q++].nbr = (int2*)S.nbr.p + b.nbr_off;
-    }
   cudaError_t e = cudaMemcpyAsync(S.desc.p, d.data(), nb, cudaMemcpyHostToDevice, h->stream);
   if (e == cudaSuccess && !nu.empty())
     e = cudaMemcpyAsync((char*)S.desc.p + nb, nu.data(), sizeof(BlkNuc) * nu.size(), cudaMemcpyHostToDevice, h->stream);
@@ -420,9 +444,8 @@ static int prepare_blocks(Handle* h, Handle::BlockStore& S, const std::vector<co
   if (e == cudaSuccess && !S.built) e = cudaEventCreateWithFlags(&S.built, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventRecord(S.built, h->stream);
   S.stream = h->stream;
-  if (e != cudaSuccess) {
-    S.ready = false;
+  if (e != cudaSuccess)
     return set_error(SPC_ERR_CUDA, "block fragments of the Hamiltonian failed: %s", cudaGetErrorString(e));
-  }
+  S.placed = use;
   return SPC_OK;
 }

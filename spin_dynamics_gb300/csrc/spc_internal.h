@@ -181,17 +181,30 @@ struct Handle {
   } hb;
   // Digit fragments of a general-builder Hamiltonian's 4 x 4 blocks for the
   // tensor-core SpMM (spc_blocks.cuh): host description at build time, device
-  // fragments on the first propagation that uses them
+  // fragments of the systems that a propagation uses on the first one that does
   struct BlockStore {
     Buf self, tab, nbr, desc;
     std::vector<BlockSys> sys;
-    bool ready = false;
+    std::vector<char> placed;  // systems whose fragments the buffers hold
     // the stream that built the blocks and the end of it, for calls on another one
     cudaStream_t stream = nullptr;
     cudaEvent_t built = nullptr;
     void describe(std::vector<BlockSys> s) {
       sys = std::move(s);
-      ready = false;
+      placed.assign(sys.size(), 0);
+    }
+    bool has(const std::vector<char>& use) const {
+      for (size_t k = 0; k < use.size(); ++k)
+        if (use[k] && !placed[k]) return false;
+      return true;
+    }
+    size_t bytes() const { return self.bytes + tab.bytes + nbr.bytes + desc.bytes; }
+    void release() {
+      for (Buf* b : {&self, &tab, &nbr, &desc}) {
+        if (b->p) cudaFree(b->p);
+        *b = Buf{};
+      }
+      placed.assign(sys.size(), 0);
     }
   } blk_one, blk_batch;
   // Krylov method: 0 full MGS (the reference's get_krylov), 1 Lanczos, 2 auto

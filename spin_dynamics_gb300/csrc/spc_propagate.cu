@@ -1239,18 +1239,25 @@ static cudaError_t enqueue_basis(Handle* h, BasisRun& B) {
   return cudaSuccess;
 }
 
-// The block store of the handle's own Hamiltonian (single) or of the batch,
-// built if every system that the call uses has one; null otherwise: CSRs the
+// The block store of the handle's own Hamiltonian (single) or of the batch if
+// every system that the call uses has blocks; null otherwise: CSRs the
 // caller gave, the reference builder's (about 9 mostly real entries a row, 20
 // FP64 operations: k_spmm takes 77 us for 32 samples at dim 55296, where
 // k_spmm_blk takes 102 us for the general builder's 15 blocks a row) and systems
-// of more than
-// BLK_MAXNBR neighbours.
-static int use_blocks(Handle* h, bool single, const std::vector<int>& systems, Handle::BlockStore** out) {
-  *out = nullptr;
+// of more than BLK_MAXNBR neighbours. `use` marks the systems.
+static Handle::BlockStore* block_store(Handle* h, bool single, const std::vector<int>& systems, std::vector<char>& use) {
   Handle::BlockStore& S = single ? h->blk_one : h->blk_batch;
-  for (int k : systems)
-    if (k >= (int)S.sys.size() || !S.sys[k].ok) return SPC_OK;
+  use.assign(S.sys.size(), 0);
+  for (int k : systems) {
+    if (k >= (int)S.sys.size() || !S.sys[k].ok) return nullptr;
+    use[k] = 1;
+  }
+  return &S;
+}
+// The fragments of `use` in the store; null (and nothing held) where the device
+// has no room for them.
+static int use_blocks(Handle* h, bool single, const std::vector<char>& use, Handle::BlockStore** store) {
+  Handle::BlockStore& S = **store;
   std::vector<const int*> rp(S.sys.size()), cl(S.sys.size());
   std::vector<const double2*> vl(S.sys.size());
   for (size_t k = 0; k < S.sys.size(); ++k) {
@@ -1258,9 +1265,9 @@ static int use_blocks(Handle* h, bool single, const std::vector<int>& systems, H
     cl[k] = single ? (const int*)h->xcol.p : (const int*)h->hb.col.p + h->hb.nz_off[k];
     vl[k] = single ? (const double2*)h->xval.p : (const double2*)h->hb.val.p + h->hb.nz_off[k];
   }
-  const int rc = prepare_blocks(h, S, rp, cl, vl);
-  if (rc == SPC_OK) *out = &S;
-  return rc == SPC_ERR_ALLOC ? SPC_OK : rc;  // no room for the blocks: the CSR kernel
+  const int rc = prepare_blocks(h, S, use, rp, cl, vl);
+  if (rc == SPC_ERR_ALLOC) *store = nullptr;
+  return rc == SPC_ERR_ALLOC ? SPC_OK : rc;
 }
 static void tile_blocks(TileInfo& t, const Handle::BlockStore& S, int sys) {
   const BlockSys& b = S.sys[sys];
@@ -1315,28 +1322,26 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
   // clocks stay resident for every sample either way.
   const double slot_fixed = 16.0 * (6.0 * mm + m + 1 + (double)nsplit_max * ncombo) + 8.0 + 4.0 + 12.0 + 8.0;
   const double tile_fixed = (double)(sizeof(TileInfo) + sizeof(unsigned)) + (double)acc_bytes(1) + (double)gram_bytes(1, m);
-  Handle::BlockStore* blocks = nullptr;
+  std::vector<char> use;
+  Handle::BlockStore* blocks;
   {
     std::vector<int> used(nj);
     for (int k = 0; k < nj; ++k) used[k] = jobs[k].sys;
-    const int rc = use_blocks(h, single, used, &blocks);
-    if (rc) return rc;
+    blocks = block_store(h, single, used, use);
   }
-  // basis + work vector (complex) + the current vector's digits or Re + Im
-  // plane (XS)
-  double xs_bytes = blocks ? 16.0 : 8.0;
   const double need_global = 16.0 * (double)psi_total + 8.0 * 4.0 * (double)T * G + 16.0 * G;
-  double budget;
-  {
-    size_t free_b = 0, total_b = 0;
-    CK(cudaMemGetInfo(&free_b, &total_b));
-    // a held buffer is reused up to the size this call asks of it (buffers
-    // only grow), so only that much of it counts toward the budget
+  // Bytes for the round's vectors and matrices beside the states, with the digits
+  // (and the blocks' fragments) or without. A held buffer is reused up to the
+  // size this call asks of it (buffers only grow), so only that much of it
+  // counts toward the budget.
+  size_t free_b = 0, total_b = 0;
+  CK(cudaMemGetInfo(&free_b, &total_b));
+  const auto budget_for = [&](bool digits) {
     double held = 0.0;
     auto reuse = [&](const Handle::Buf& b, double bytes) { held += std::min((double)b.bytes, bytes); };
     reuse(h->Q, 16.0 * (double)qcap);
     reuse(h->P, 16.0 * (double)pcap);
-    reuse(h->xsum, xs_bytes * (double)pcap);
+    reuse(h->xsum, (digits ? 16.0 : 8.0) * (double)pcap);
     reuse(h->psi, 16.0 * (double)psi_total);
     reuse(h->obs, 8.0 * 4.0 * (double)T * G);
     const double sl = (double)slots_cap;
@@ -1355,14 +1360,28 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
     reuse(h->tt, 8.0 * G);
     reuse(h->kk, 4.0 * G);
     reuse(h->done, 4.0 * G);
-    budget = (double)free_b + held - need_global - (512.0 * (1 << 20) + 0.02 * (double)total_b);
-    if (h->mem_limit) budget = std::min(budget, (double)h->mem_limit - need_global);
+    const double store = digits ? (double)block_bytes_after(*blocks, use) : 0.0;
+    if (digits) held += (double)blocks->bytes();
+    double b = (double)free_b + held - store - need_global - (512.0 * (1 << 20) + 0.02 * (double)total_b);
+    if (h->mem_limit) b = std::min(b, (double)h->mem_limit - store - need_global);
+    return b;
+  };
+  if (blocks) {
+    // where not even a tile fits with the digits, the CSR kernel and its plane
+    if ((16.0 * m + 32.0) * nmax * SPC_LANES + slot_fixed * SPC_LANES + tile_fixed > budget_for(true)) {
+      blocks->release();
+      blocks = nullptr;
+      CK(cudaMemGetInfo(&free_b, &total_b));
+    }
   }
-  // where not even a tile fits with the digits, the CSR kernel and its plane
-  if (blocks && (16.0 * m + 32.0) * nmax * SPC_LANES + slot_fixed * SPC_LANES + tile_fixed > budget) {
-    blocks = nullptr;
-    xs_bytes = 8.0;
+  const double budget = budget_for(blocks != nullptr);
+  if (blocks) {
+    const int rc = use_blocks(h, single, use, &blocks);
+    if (rc) return rc;
   }
+  // basis + work vector (complex) + the current vector's digits or Re + Im
+  // plane (XS)
+  const double xs_bytes = blocks ? 16.0 : 8.0;
   const double need_fl = 16.0 * (double)qcap + (16.0 + xs_bytes) * (double)pcap + slot_fixed * slots_cap +
                          tile_fixed * tiles_cap;
   int64_t qfl = qcap, pfl = pcap;

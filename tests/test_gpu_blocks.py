@@ -66,3 +66,33 @@ def test_large_coupling_out_of_reach(sampler, method, kT, size):
         sampler.set_krylov("mgs")
         sampler.set_sample_path("auto")
     assert difference(*out) <= 1e-13
+
+
+def test_memory_held(oracle):
+    """A call holds no more device memory than its limit allows, the blocks'
+    fragments (1 KB a nuclear index) included: two jobs of a batch of 64
+    systems, and a call whose limit has no room for the fragments after one
+    that built them."""
+    from spin_dynamics_gb300.dynamics import TraceSampler, device_memory
+    s = pair((3, 3, 2, 2, 2, 2), (2, 2, 2, 2))
+    zk = [W.random_phase_samples(s.Z, 32, seed=k) for k in range(2)]
+    fields = [np.array([0.01, 0.03, 0.04]) * (1 + k) for k in range(64)]
+    slack = 24 << 20  # the plan, tables and the allocator's granularity
+    with TraceSampler(0) as sp:
+        sp.set_sample_path("off")
+        sp.build_h_batch([s] * 64, fields, "general")
+        free0 = device_memory()[0]
+
+        def run(limit):
+            sp.set_memory_limit(limit)
+            got = sp.trace_sampling_batch(zk, DT, 3 * DT, 4, 1e-6, job_sys=[5, 40])
+            return got, free0 - device_memory()[0]
+
+        limit = 64 << 20
+        bounded, held = run(limit)
+        assert held <= limit + slack
+        whole, _ = run(0)
+        need = 16 * 2 * s.Z * 4 * 32  # the states
+        tight, _ = run(need + (32 << 20))
+        for a, b, c in zip(bounded, whole, tight):
+            assert difference(a, b) <= 1e-13 and difference(c, b) <= 1e-13
