@@ -393,21 +393,34 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   }();
   const int items_cap = h->sm_count * 32 + ntiles;
 
-  std::vector<char> use;
-  Handle::BlockStore* blocks;
+  // Small systems build their bases a sample per CTA (k_small_basis) where the
+  // vectors of every job fit a CTA's shared memory; past 800 row-samples or 8
+  // samples per SM the tiles' launches are full. Whole gradient of 6 steps at
+  // m = 16, per sample against tiled (MGS | Lanczos): dim 288, 96 samples 7.4 :
+  // 10.7 | 4.6 : 6.2 ms, 300 samples 12.3 : 17.3 | 7.1 : 8.4, 600 samples 22.7 :
+  // 24.0 | 12.4 : 11.0; dim 576, 96 samples 11.0 : 13.0 | 6.7 : 7.2, 300 samples
+  // 22.1 : 22.1 | 12.9 : 11.2; dim 24, 1200 samples 15.0 : 17.0 | 6.1 : 7.6.
+  size_t basis_smem = 0;
+  int team = 1;
   {
-    std::vector<int> used;
-    for (const GradJob& J : jobs) {
-      used.push_back(J.sys);
-      used.push_back(J.sys + 1);
-    }
-    blocks = block_store(h, false, used, use);
-    if (blocks) {
-      const int rc = use_blocks(h, false, use, &blocks);
-      if (rc) return rc;
+    int nmax = 0;
+    for (int k = 0; k < nj; ++k) nmax = std::max(nmax, nrow[k]);
+    size_t need = sizeof(double2) * small_basis_elems(m, nmax, 1);
+    if (m <= SMALL_MAX_M && need + SMALL_STATIC <= h->smem_optin && Mtot <= 8 * h->sm_count && elems <= 800.0 * h->sm_count &&
+        h->sample_path != SPC_SAMPLE_OFF) {
+      // clusters while they find idle SMs and rows to share; whole gradient as
+      // above, one CTA against a cluster (MGS | Lanczos): dim 48, 32 samples 3.72 :
+      // 3.90 | 2.40 : 2.75 ms, dim 144 5.11 : 4.57 | 3.23 : 3.05, dim 288 6.85 :
+      // 4.78 | 4.24 : 3.27, dim 576 9.98 : 6.02 | 5.78 : 4.05; 70 samples (two
+      // CTAs each) dim 144 5.46 : 4.95 | 3.28 : 3.12, dim 576 10.9 : 8.3 | 6.3 : 5.2
+      while (team < SMALL_TEAM && 2 * team * Mtot <= h->sm_count && nmax >= 96) team *= 2;
+      need = sizeof(double2) * small_basis_elems(m, nmax, team);
+      CK(cudaFuncSetAttribute(team > 1 ? k_small_basis<true> : k_small_basis<false>,
+                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
+      basis_smem = need;
     }
   }
-  const double xs_bytes = blocks ? 16.0 : 8.0;
+  const bool tiled = true;  // the tiles' buffers
   // tiles, slot maps, costate coefficients
   std::vector<TileInfo> tf(ntiles), tb(ntiles);
   std::vector<int> map(nslots), scol(nslots), tile_n(ntiles), tile_job(ntiles);
@@ -438,7 +451,6 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
           x.vsum = (const double*)HB.vsum.p + HB.nz_off[sy];
           x.kappa = HB.herm[sy] ? &((const HMeta*)HB.meta.p)[sy].kappa : nullptr;
           x.rexp = HB.rexp[sy];
-          if (blocks) tile_blocks(x, *blocks, sy);
         }
         for (int l = 0; l < SPC_LANES; ++l) {
           const int s = c * SPC_LANES + l;
@@ -486,86 +498,101 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
     return Sl.owner == -1 ? Z : (Sl.owner == -2 ? 4 * Z / Sl.g : 2 * Z / Sl.g);
   };
   auto nrb_of = [](int G) { return G == 6 ? 2 : 1; };
-  auto chunks_for = [&](int p0, int cnt, int G, int nodes) {
+  auto longest = [&](int p0, int cnt) {
     int64_t L = 1;
     for (int q = p0; q < p0 + cnt; ++q) L = std::max(L, pair_len(pairs[q]));
+    return L;
+  };
+  auto chunks_for = [&](int64_t L, int cnt, int G, int nodes) {
     const int64_t by_wave = (int64_t)h->sm_count * 64 / std::max(1, cnt * nodes * nrb_of(G));
     const int64_t by_len = (L + 7) / 8;
     return (int)std::max<int64_t>(1, std::min(by_wave, by_len));
   };
-  const int nch_f = chunks_for(pf0, ntiles, 4, 1);
-  std::vector<int> grp_nch(grp_G.size());
-  size_t part_need = (size_t)ntiles * nch_f * 16 * SPC_LANES;
-  for (size_t gi = 0; gi < grp_G.size(); ++gi) {
-    grp_nch[gi] = chunks_for(grp_p0[gi], grp_cnt[gi], grp_G[gi], nq);
-    part_need = std::max(part_need, (size_t)nq * grp_cnt[gi] * grp_nch[gi] * grp_G[gi] * grp_G[gi] * SPC_LANES);
-  }
-  const size_t part_cap = part_need;
+  const int nch_f = chunks_for(longest(pf0, ntiles), ntiles, 4, 1);
+  std::vector<int64_t> grp_L(grp_G.size());
+  for (size_t gi = 0; gi < grp_G.size(); ++gi) grp_L[gi] = longest(grp_p0[gi], grp_cnt[gi]);
+  // entries of the contraction's partial sums with `nodes` node states at a time
+  auto part_of = [&](int nodes) {
+    size_t e = (size_t)ntiles * nch_f * 16 * SPC_LANES;
+    for (size_t gi = 0; want_grad && gi < grp_G.size(); ++gi) {
+      const int nch = chunks_for(grp_L[gi], grp_cnt[gi], grp_G[gi], nodes);
+      e = std::max(e, (size_t)nodes * grp_cnt[gi] * nch * grp_G[gi] * grp_G[gi] * SPC_LANES);
+    }
+    return e;
+  };
 
-  // checkpoint spacing K and whether a segment's node states are kept (one
-  // Krylov build per step saved). K = 0 picks the largest spacing whose
-  // states fit in device memory (fewest recomputed segments), else the
-  // spacing of least memory with node states rebuilt per step.
-  // nqm: costate node states formed at a time, all of a step's nodes or, where
-  // memory is short, one after the other
-  bool cache = false;
-  int nqm = nq;
+  // The block product if every Hamiltonian has blocks and the tiles build the bases
+  std::vector<char> use;
+  Handle::BlockStore* blocks = nullptr;
+  if (tiled) {
+    std::vector<int> used;
+    for (const GradJob& J : jobs) {
+      used.push_back(J.sys);
+      used.push_back(J.sys + 1);
+    }
+    blocks = block_store(h, false, used, use);
+  }
+  // Checkpoint spacing, kept node states and costate node states at a time, by the
+  // memory the buffers take past what the handle holds: a held buffer is reused
+  // up to the size asked of it (buffers only grow), so its excess over that size
+  // is no help.
+  GradPlan gp;
+  gp.K = std::max(1, K);
   if (want_grad) {
     size_t free_b = 0, total_b = 0;
     CK(cudaMemGetInfo(&free_b, &total_b));
-    const double avail = 0.85 * (double)free_b - (double)(1 << 28);
     const double sb = sizeof(double2) * (double)S;
-    // bytes of every state buffer of the sweep, and the device memory they
-    // take beyond what the handle already holds: a held buffer is reused up
-    // to the size asked of it (buffers only grow), so its excess over that
-    // size is no help
-    auto need = [&](int k, bool keep) {
-      return sb * ((double)m + 3.0 + nqm + xs_bytes / 16.0 + (nsteps / k + 1) + k + 1.0 + (keep ? (double)k * nq : (double)nq));
+    std::vector<double> part(nq + 1, 0.0);
+    for (int q = 1; q <= nq; ++q)
+      part[q] = sizeof(double2) * (double)std::max(part_of(q), tiled ? (size_t)items_cap * SPC_LANES : 0);
+    const auto past = [](const Handle::Buf& b, double bytes) { return std::max(0.0, bytes - (double)b.bytes); };
+    const auto states = [&](int k, bool keep, int nodes) {
+      return past(h->Q, sb * m) + past(h->gmu, sb * nodes) + past(h->glam, 2.0 * sb) +
+             (tiled ? past(h->P, sb) + past(h->xsum, 0.5 * sb) : 0.0) + past(h->gck, sb * (nsteps / k + 1)) +
+             past(h->gseg, sb * (k + 1)) + past(h->gnu, sb * (keep ? (double)k * nq : (double)nq));
     };
-    auto extra = [&](int k, bool keep) {
-      double x = 0.0;
-      auto add = [&](const Handle::Buf& b, double bytes) { x += std::max(0.0, bytes - (double)b.bytes); };
-      add(h->Q, sb * m);
-      add(h->gmu, sb * nqm);
-      add(h->glam, 2.0 * sb);
-      add(h->P, sb);
-      add(h->xsum, xs_bytes / 16.0 * sb);  // the current Krylov vector's digits or Re + Im plane beside P
-      add(h->acc, (double)acc_bytes(ntiles));
-      add(h->gram, (double)gram_bytes(ntiles, m));
-      add(h->gck, sb * (nsteps / k + 1));
-      add(h->gseg, sb * (k + 1));
-      add(h->gnu, sb * (keep ? (double)k * nq : (double)nq));
+    const double store = blocks ? (double)block_bytes_after(*blocks, use) - (double)blocks->bytes() : 0.0;
+    const auto rest = [&](int nodes, bool digits) {
+      const double slot = sizeof(double2) * (double)nslots;
+      double x = past(h->partial, part[nodes]) + past(h->cvec2, slot * m * (nq + 1)) + past(h->cvec, slot * m) +
+                 past(h->Ahess, slot * mm) + past(h->gracc, sizeof(double2) * (double)rtot * con) +
+                 past(h->gfacc, slot * con);
+      if (tiled) x += past(h->acc, (double)acc_bytes(ntiles)) + past(h->gram, (double)gram_bytes(ntiles, m));
+      if (digits) x += past(h->xsum, sb) - past(h->xsum, 0.5 * sb) + store;
       return x;
     };
-    if (K == 0) {
-      // among the spacings whose states fit, the one that recomputes the
-      // fewest steps (all but the last segment are recomputed), the larger
-      // on a tie
-      int64_t best = -1;
-      for (int k = nsteps; k >= 1; --k) {
-        if (extra(k, true) > avail) continue;
-        const int64_t recomputed = (int64_t)((nsteps - 1) / k) * k;
-        if (best < 0 || recomputed < best) {
-          best = recomputed;
-          K = k;
-        }
-      }
-      if (K)
-        cache = true;
-      else
-        K = std::max(1, (int)std::lround(std::sqrt((double)nsteps)));
-    } else {
-      cache = extra(K, true) <= avail;
+    const int k0 = K > 0 ? K : std::max(1, (int)std::lround(std::sqrt((double)nsteps)));
+    if (blocks && states(k0, false, 1) + rest(1, true) > 0.95 * (double)free_b - (double)(1 << 28)) {
+      blocks->release();
+      blocks = nullptr;
+      CK(cudaMemGetInfo(&free_b, &total_b));
     }
-    if (!cache && extra(K, false) > avail) nqm = 1;
-    // the digits' plane and the small sums may use the 15 % kept free
-    const double slack = (xs_bytes / 16.0 - 0.5) * sb + (double)acc_bytes(ntiles) + (double)gram_bytes(ntiles, m);
-    if (!cache && extra(K, false) > avail + slack)
+    const double avail = 0.85 * (double)free_b - (double)(1 << 28);
+    gp = plan_gradient(nsteps, nq, K, avail, rest(1, blocks != nullptr), [&](int k, bool keep, int nodes) {
+      return states(k, keep, nodes) + rest(nodes, blocks != nullptr);
+    });
+    if (!gp.fits)
       return set_error(SPC_ERR_ALLOC,
                        "yield gradient needs %.1f GB of device memory at checkpoint spacing %d (%.1f GB free)",
-                       need(K, false) / 1e9, K, free_b / 1e9);
+                       sb * ((double)m + 3.0 + (tiled ? 1.5 : 0.0) + (nsteps / gp.K + 1) + gp.K + 1.0 + nq) / 1e9, gp.K,
+                       free_b / 1e9);
   }
-  if (K < 1) K = 1;
+  if (blocks) {
+    const int rc = use_blocks(h, false, use, &blocks);
+    if (rc) return rc;
+    if (blocks)
+      for (int t = 0; t < ntiles; ++t) {
+        tile_blocks(tf[t], *blocks, jobs[tile_job[t]].sys);
+        tile_blocks(tb[t], *blocks, jobs[tile_job[t]].sys + 1);
+      }
+  }
+  const size_t xs_bytes = blocks ? 16 : 8;
+  K = gp.K;
+  const bool cache = gp.keep;
+  const int nqm = gp.nodes;
+  std::vector<int> grp_nch(grp_G.size());
+  for (size_t gi = 0; gi < grp_G.size(); ++gi) grp_nch[gi] = chunks_for(grp_L[gi], grp_cnt[gi], grp_G[gi], nqm);
+  const size_t part_cap = part_of(nqm);
   const int nck = nsteps / K + 1;
   const int a_last = ((nsteps - 1) / K) * K;  // first step of the last segment
   const size_t n_ck = want_grad ? nck : 0, n_seg = want_grad ? K + 1 : 0;
@@ -575,11 +602,11 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   if (h->ensure(h->gck, sizeof(double2) * S * n_ck) || h->ensure(h->gseg, sizeof(double2) * S * n_seg) ||
       h->ensure(h->gnu, sizeof(double2) * S * n_nu) || h->ensure(h->gmu, sizeof(double2) * S * (want_grad ? nqm : 1)) ||
       h->ensure(h->glam, sizeof(double2) * S * 2) || h->ensure(h->Q, sizeof(double2) * m * S) ||
-      h->ensure(h->P, sizeof(double2) * S) || h->ensure(h->xsum, (size_t)xs_bytes * S) ||
+      h->ensure(h->P, sizeof(double2) * (tiled ? S : 0)) || h->ensure(h->xsum, xs_bytes * (tiled ? S : 0)) ||
       h->ensure(h->qmax, 2 * sizeof(unsigned) * nslots) || h->ensure(h->xexp, sizeof(int) * nslots) ||
-      h->ensure(h->acc, acc_bytes(ntiles)) || h->ensure(h->gram, gram_bytes(ntiles, m)) ||
-      h->ensure(h->partial, sizeof(double2) * std::max<size_t>((size_t)items_cap * SPC_LANES, part_cap)) ||
-      h->ensure(h->counters, sizeof(unsigned) * std::max<size_t>(ntiles, npairs)) ||
+      h->ensure(h->acc, tiled ? acc_bytes(ntiles) : 0) || h->ensure(h->gram, tiled ? gram_bytes(ntiles, m) : 0) ||
+      h->ensure(h->partial, sizeof(double2) * std::max<size_t>(tiled ? (size_t)items_cap * SPC_LANES : 0, part_cap)) ||
+      h->ensure(h->counters, sizeof(unsigned) * ntiles) ||
       h->ensure(h->coef, sizeof(double2) * nslots) || h->ensure(h->rbeta, sizeof(double) * nslots) ||
       h->ensure(h->Ahess, sizeof(double2) * mm * nslots) ||
       h->ensure(h->cvec, sizeof(double2) * m * nslots) || h->ensure(h->cvec2, sizeof(double2) * m * nslots * (nq + 1)) ||
@@ -663,7 +690,7 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   CK(cudaMemcpyAsync(d_coefs, coefs.data(), sizeof(double2) * ntiles, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(d_slots, cs.data(), sizeof(GradSlot) * cs.size(), cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(d_pairs, pairs.data(), sizeof(ConPair) * npairs, cudaMemcpyHostToDevice, st));
-  CK(cudaMemsetAsync(d_cnt, 0, sizeof(unsigned) * std::max<size_t>(ntiles, npairs), st));
+  CK(cudaMemsetAsync(d_cnt, 0, sizeof(unsigned) * ntiles, st));
   CK(cudaMemsetAsync(d_racc, 0, sizeof(double2) * std::max<int64_t>(rtot, 1) * con, st));
   CK(cudaMemsetAsync(d_facc, 0, sizeof(double2) * nslots * con, st));
   CK(cudaMemsetAsync(h->err.p, 0, 16, st));
@@ -688,33 +715,6 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   gauss_legendre01(nq, xq, wq);
   int64_t builds = 0;
 
-  // Small systems build their bases a sample per CTA (k_small_basis) where the
-  // vectors of every job fit a CTA's shared memory; past 800 row-samples or 8
-  // samples per SM the tiles' launches are full. Whole gradient of 6 steps at
-  // m = 16, per sample against tiled (MGS | Lanczos): dim 288, 96 samples 7.4 :
-  // 10.7 | 4.6 : 6.2 ms, 300 samples 12.3 : 17.3 | 7.1 : 8.4, 600 samples 22.7 :
-  // 24.0 | 12.4 : 11.0; dim 576, 96 samples 11.0 : 13.0 | 6.7 : 7.2, 300 samples
-  // 22.1 : 22.1 | 12.9 : 11.2; dim 24, 1200 samples 15.0 : 17.0 | 6.1 : 7.6.
-  size_t basis_smem = 0;
-  int team = 1;
-  {
-    int nmax = 0;
-    for (int k = 0; k < nj; ++k) nmax = std::max(nmax, nrow[k]);
-    size_t need = sizeof(double2) * small_basis_elems(m, nmax, 1);
-    if (m <= SMALL_MAX_M && need + SMALL_STATIC <= h->smem_optin && Mtot <= 8 * h->sm_count && elems <= 800.0 * h->sm_count &&
-        h->sample_path != SPC_SAMPLE_OFF) {
-      // clusters while they find idle SMs and rows to share; whole gradient as
-      // above, one CTA against a cluster (MGS | Lanczos): dim 48, 32 samples 3.72 :
-      // 3.90 | 2.40 : 2.75 ms, dim 144 5.11 : 4.57 | 3.23 : 3.05, dim 288 6.85 :
-      // 4.78 | 4.24 : 3.27, dim 576 9.98 : 6.02 | 5.78 : 4.05; 70 samples (two
-      // CTAs each) dim 144 5.46 : 4.95 | 3.28 : 3.12, dim 576 10.9 : 8.3 | 6.3 : 5.2
-      while (team < SMALL_TEAM && 2 * team * Mtot <= h->sm_count && nmax >= 96) team *= 2;
-      need = sizeof(double2) * small_basis_elems(m, nmax, team);
-      CK(cudaFuncSetAttribute(team > 1 ? k_small_basis<true> : k_small_basis<false>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
-      basis_smem = need;
-    }
-  }
   // Krylov basis of the states `x` (psi layout) under the tiles' Hamiltonians
   auto build = [&](const double2* x, const TileInfo* tiles) {
     if (basis_smem) {

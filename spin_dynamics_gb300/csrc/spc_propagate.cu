@@ -42,6 +42,7 @@
 
 #include "spc_common.cuh"
 #include "spc_internal.h"
+#include "spc_plan.h"
 
 namespace spc {
 

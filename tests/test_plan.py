@@ -16,6 +16,16 @@ DRIVER = """
 extern "C" double csr_bound(int n, const int* rp, const int* cl, const double* v) {
   return spc::csr_norm_bound(n, rp, cl, v);
 }
+// a sweep of m basis vectors and states of one unit, partial sums of `part` a node
+extern "C" int grad_plan(int nsteps, int nq, int K, double avail, double slack, double m, double part, int* out) {
+  const spc::GradPlan p = spc::plan_gradient(nsteps, nq, K, avail, slack, [&](int k, bool keep, int nodes) {
+    return m + 4.0 + nodes * (1.0 + part) + (nsteps / k + 1) + (k + 1) + (keep ? (double)k * nq : (double)nq);
+  });
+  out[0] = p.K;
+  out[1] = p.keep;
+  out[2] = p.nodes;
+  return p.fits;
+}
 """
 
 
@@ -62,3 +72,41 @@ def test_norm_bound_of_undefined_entries(plan):
     assert np.isnan(bound(plan, np.diag([1.0, np.nan, 2.0, 3.0])))
     assert bound(plan, np.zeros((4, 4))) == 0.0
     assert np.isfinite(bound(plan, np.eye(4) * 1e300))
+
+
+def planned(plan, nsteps, nq, K, avail, slack=0.0, m=16.0, part=0.0):
+    out = (C.c_int * 3)()
+    fits = plan.grad_plan(nsteps, nq, K, C.c_double(avail), C.c_double(slack), C.c_double(m), C.c_double(part), out)
+    return tuple(out) + (bool(fits),)
+
+
+def need(nsteps, nq, K, keep, nodes, m=16.0, part=0.0):
+    return m + 4 + nodes * (1 + part) + (nsteps // K + 1) + (K + 1) + (K * nq if keep else nq)
+
+
+@pytest.mark.parametrize("part", [0.0, 0.5, 30.0])
+@pytest.mark.parametrize("K", [0, 1, 5, 40])
+@pytest.mark.parametrize("nsteps, nq", [(1, 1), (40, 6), (40, 16)])
+def test_gradient_plan(plan, nsteps, nq, K, part):
+    """At every size of memory: the plan fits; kept node states and the spacing
+    are those that one costate state at a time allows, so that more of them never
+    cost a build; partial sums shrink the nodes before they refuse a call."""
+    K = min(K, nsteps)
+    least = need(nsteps, nq, K or max(1, round(nsteps ** 0.5)), False, 1, part=part)
+    for avail in np.unique(np.concatenate([np.arange(least - 3, least + 60), np.linspace(least, 900, 200)])):
+        k, keep, nodes, fits = planned(plan, nsteps, nq, K, avail, part=part)
+        kept = [c for c in ([K] if K else range(1, nsteps + 1)) if need(nsteps, nq, c, True, 1, part=part) <= avail]
+        assert fits == (bool(kept) or avail >= least)
+        assert bool(keep) == bool(kept)
+        if K:
+            assert k == K
+        elif kept:
+            assert (nsteps - 1) // k * k == min((nsteps - 1) // c * c for c in kept)
+        if fits:
+            assert need(nsteps, nq, k, bool(keep), nodes, part=part) <= avail
+            assert nodes == nq or need(nsteps, nq, k, bool(keep), nodes + 1, part=part) > avail
+
+
+def test_gradient_plan_uses_the_reserve_for_small_buffers(plan):
+    assert planned(plan, 40, 6, 8, need(40, 6, 8, False, 1) - 5, slack=5.0)[3]
+    assert not planned(plan, 40, 6, 8, need(40, 6, 8, False, 1) - 6, slack=5.0)[3]
