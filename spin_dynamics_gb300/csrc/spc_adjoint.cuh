@@ -420,7 +420,7 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
       basis_smem = need;
     }
   }
-  const bool tiled = true;  // the tiles' buffers
+  const bool tiled = basis_smem == 0;
   // tiles, slot maps, costate coefficients
   std::vector<TileInfo> tf(ntiles), tb(ntiles);
   std::vector<int> map(nslots), scol(nslots), tile_n(ntiles), tile_job(ntiles);

@@ -96,3 +96,23 @@ def test_memory_held(oracle):
         tight, _ = run(need + (32 << 20))
         for a, b, c in zip(bounded, whole, tight):
             assert difference(a, b) <= 1e-13 and difference(c, b) <= 1e-13
+
+
+def test_small_gradients_hold_no_tiled_buffers():
+    """A gradient whose bases are built a sample per CTA allocates neither block
+    fragments nor the tiles' work vectors: the tiled build of the same call then
+    takes that much more memory."""
+    from spin_dynamics_gb300.dynamics import TraceSampler, device_memory
+    s = pair((2, 3, 3), (2,))
+    n, jobs = 4 * s.Z, 300
+    fields = [np.array([0.01, 0.03, 0.04]) * (1 + 0.01 * k) for k in range(jobs)]
+    zk = [W.random_phase_samples(s.Z, 1, seed=1)] * jobs
+    held = []
+    with TraceSampler(0) as sp:
+        for mode in ("auto", "off"):
+            sp.set_sample_path(mode)
+            sp.yield_gradient_batch([s] * jobs, fields, zk, DT, 2 * DT, 4, n_quad=1, checkpoint_every=1, hyperfine=False)
+            held.append(device_memory()[0])
+    state = 16 * n * 32 * jobs
+    fragments = 2 * jobs * s.Z * 1024
+    assert held[0] - held[1] >= 0.9 * (2 * state + fragments)
