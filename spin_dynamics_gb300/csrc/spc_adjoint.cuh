@@ -303,6 +303,7 @@ __global__ void __launch_bounds__(256)
 typedef void (*ApplyFn)(const TileInfo*, const int2*, int, int, const int*, const int*, const double2*, const double2*,
                         Times, int);
 #define APPLY_MAX 4
+#define APPLY_SMEM (96u << 10)  // of the coordinates
 static const ApplyFn kApply[APPLY_MAX] = {k_apply<1>, k_apply<2>, k_apply<3>, k_apply<4>};
 
 // lam = ulam + c (cI psi + cP Pi_S psi) with (cI, cP) per tile, Pi_S = |S><S|
@@ -415,8 +416,7 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
       // CTAs each) dim 144 5.46 : 4.95 | 3.28 : 3.12, dim 576 10.9 : 8.3 | 6.3 : 5.2
       while (team < SMALL_TEAM && 2 * team * Mtot <= h->sm_count && nmax >= 96) team *= 2;
       need = sizeof(double2) * small_basis_elems(m, nmax, team);
-      CK(cudaFuncSetAttribute(team > 1 ? k_small_basis<true> : k_small_basis<false>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
+      CK(allow_smem(team > 1 ? k_small_basis<true> : k_small_basis<false>, h->smem_optin - SMALL_STATIC));
       basis_smem = need;
     }
   }
@@ -788,17 +788,15 @@ int yield_gradient_run(Handle* h, const double* theta, const std::vector<GradJob
   for (const GradJob& J : jobs) series = series && std::ldexp(dt, std::max(HB.rexp[J.sys], HB.rexp[J.sys + 1])) <= 64.0;
   if (!series) {
     if (h->ensure(h->Aexp, sizeof(double2) * mm * nslots)) return SPC_ERR_ALLOC;
-    CK(set_expm_smem(m));
+    CK(allow_expm_smem());
   }
   double2* d_E = (double2*)h->Aexp.p;
   // y_t = exp(-i tau_t H) x from the current bases (tau < 0 runs backwards)
   const size_t col_smem = sizeof(double2) * mm;
-  const int apply_max = (int)std::max<size_t>(1, std::min<size_t>(APPLY_MAX, (96u << 10) / (sizeof(double2) * m * SPC_LANES)));
-  CK(cudaFuncSetAttribute(k_expm_col<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col_smem));
-  CK(cudaFuncSetAttribute(k_expm_col<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col_smem));
-  for (int t = 1; t <= apply_max; ++t)
-    CK(cudaFuncSetAttribute(kApply[t - 1], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)(sizeof(double2) * t * m * SPC_LANES)));
+  const int apply_max = (int)std::max<size_t>(1, std::min<size_t>(APPLY_MAX, APPLY_SMEM / (sizeof(double2) * m * SPC_LANES)));
+  CK(allow_smem(k_expm_col<true>, sizeof(double2) * MAX_KRYLOV * MAX_KRYLOV));
+  CK(allow_smem(k_expm_col<false>, sizeof(double2) * MAX_KRYLOV * MAX_KRYLOV));
+  for (ApplyFn fn : kApply) CK(allow_smem(fn, APPLY_SMEM));
   auto apply = [&](const Times& tm, const TileInfo* tiles) {
     int pe = h->prof.begin(st);
     if (!series) {

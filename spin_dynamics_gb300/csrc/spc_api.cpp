@@ -207,7 +207,8 @@ static int check_prop_args(spc_handle* h, const double* theta, const double* ini
   if (h->h.n == 0) return spc::set_error(SPC_ERR_STATE, "no Hamiltonian: call spc_build_h or spc_set_h first");
   if (M < 1) return spc::set_error(SPC_ERR_ARG, "need at least one sample");
   if (!(dt > 0.0)) return spc::set_error(SPC_ERR_ARG, "dt must be positive");
-  if (m < 1 || m > 48) return spc::set_error(SPC_ERR_ARG, "Krylov dimension %d outside [1, 48]", m);
+  if (m < 1 || m > spc::MAX_KRYLOV)
+    return spc::set_error(SPC_ERR_ARG, "Krylov dimension %d outside [1, %d]", m, spc::MAX_KRYLOV);
   if (T < 1) return spc::set_error(SPC_ERR_ARG, "need at least one output slot");
   return SPC_OK;
 }
@@ -304,7 +305,8 @@ int spc_trace_sampling_batch_device(spc_handle* h, int n_jobs, const int* job_sy
   if (!h || n_jobs < 1 || !M || !theta || !init_pop || !zkets_dev || !out_dev)
     return spc::set_error(SPC_ERR_ARG, "spc_trace_sampling_batch: null argument");
   if (!(dt > 0.0)) return spc::set_error(SPC_ERR_ARG, "dt must be positive");
-  if (m < 1 || m > 48) return spc::set_error(SPC_ERR_ARG, "Krylov dimension %d outside [1, 48]", m);
+  if (m < 1 || m > spc::MAX_KRYLOV)
+    return spc::set_error(SPC_ERR_ARG, "Krylov dimension %d outside [1, %d]", m, spc::MAX_KRYLOV);
   if (T != spc::num_time_points(dt, t_end))
     return spc::set_error(SPC_ERR_ARG, "T must be spc_num_time_points(dt, t_end) = %d",
                           spc::num_time_points(dt, t_end));
@@ -348,8 +350,9 @@ int spc_autotune_krylov(spc_handle* h, int n_jobs, const int* job_sys, const int
     return spc::set_error(SPC_ERR_ARG, "spc_autotune_krylov: null argument");
   if (!(dt > 0.0) || !(t_window > 0.0)) return spc::set_error(SPC_ERR_ARG, "dt and t_window must be positive");
   for (int c = 0; c < n_candidates; ++c)
-    if (candidates[c] < 1 || candidates[c] > 48)
-      return spc::set_error(SPC_ERR_ARG, "candidate Krylov dimension %d outside [1, 48]", candidates[c]);
+    if (candidates[c] < 1 || candidates[c] > spc::MAX_KRYLOV)
+      return spc::set_error(SPC_ERR_ARG, "candidate Krylov dimension %d outside [1, %d]", candidates[c],
+                            spc::MAX_KRYLOV);
   CKR(cudaSetDevice(h->h.device));
   spc::Handle& H = h->h;
   const auto& B = H.hb;
@@ -692,7 +695,8 @@ int spc_yield_gradient_batch(spc_handle* h, int n_jobs, const spc_system* system
   if (!h || n_jobs < 1 || !systems || !M || !theta || !zkets || !yields)
     return spc::set_error(SPC_ERR_ARG, "spc_yield_gradient_batch: null argument");
   if (!(dt > 0.0)) return spc::set_error(SPC_ERR_ARG, "dt must be positive");
-  if (m < 1 || m > 48) return spc::set_error(SPC_ERR_ARG, "Krylov dimension %d outside [1, 48]", m);
+  if (m < 1 || m > spc::MAX_KRYLOV)
+    return spc::set_error(SPC_ERR_ARG, "Krylov dimension %d outside [1, %d]", m, spc::MAX_KRYLOV);
   if (n_quad < 0 || n_quad > 16) return spc::set_error(SPC_ERR_ARG, "n_quad %d outside [0, 16]", n_quad);
   if (checkpoint_every < 0) return spc::set_error(SPC_ERR_ARG, "checkpoint_every must be >= 0");
   if (which != SPC_GRAD_ALL && which != SPC_GRAD_FIELD)

@@ -104,6 +104,9 @@ struct HMeta {
   unsigned least_row;
 };
 
+// Largest Krylov dimension that a call takes.
+constexpr int MAX_KRYLOV = 48;
+
 // Neighbours of a nuclear index (its other states by one step of a nucleus) that
 // k_spmm_blk takes; spc_blocks.cuh states what bounds it.
 constexpr int BLK_MAXNBR = 19;

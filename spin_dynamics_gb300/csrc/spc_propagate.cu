@@ -679,15 +679,16 @@ static void launch_expm(int m, int nslots, const TileInfo* tiles, const int* map
     k_expm<<<nslots, 128, sizeof(double2) * 5 * mm, st>>>(m, nslots, tiles, map, Ahess, Aexp, dt, tri);
 }
 
-// Shared-memory limits of both expm kernels for Krylov dimension m.
-static cudaError_t set_expm_smem(int m) {
-  const size_t mm = (size_t)m * m;
-  cudaError_t e = cudaFuncSetAttribute(k_expm, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)(sizeof(double2) * 5 * mm));
-  if (e == cudaSuccess && m <= 16)
-    e = cudaFuncSetAttribute(k_expm_warp, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(sizeof(double2) * 20 * mm));
-  return e;
+// A kernel's limit of dynamic shared memory is the process's, and calls of several
+// threads may run kernels at different Krylov dimensions: every call sets the
+// same limit, that of the largest dimension the kernel takes.
+template <class F>
+static cudaError_t allow_smem(F* fn, size_t bytes) {
+  return cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+static cudaError_t allow_expm_smem() {
+  const cudaError_t e = allow_smem(k_expm, sizeof(double2) * 5 * MAX_KRYLOV * MAX_KRYLOV);
+  return e == cudaSuccess ? allow_smem(k_expm_warp, sizeof(double2) * 20 * 16 * 16) : e;
 }
 
 // ---------------------------------------------------------------------------
@@ -1498,9 +1499,8 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
   CK(cudaGetLastError());
 
   const size_t proj_smem = proj_smem_bytes(m);
-  CK(set_expm_smem(m));
-  if (m <= 32)
-    CK(cudaFuncSetAttribute(k_dtloop_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dt_smem_bytes(m)));
+  CK(allow_expm_smem());
+  CK(allow_smem(k_dtloop_cta, dt_smem_bytes(32)));
   // combinations per thread (an instantiated count) and threads per CTA (a
   // multiple of 32, at most 256): the pair with the fewest padded slots, the
   // smaller count on a tie (every slot, used or not, issues its DFMAs)
@@ -1535,7 +1535,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
     case 20: proj_fn = (const void*)k_proj<20>; break;
     default: proj_fn = (const void*)k_proj<24>; break;
   }
-  CK(cudaFuncSetAttribute(proj_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)proj_smem));
+  CK(allow_smem(proj_fn, proj_smem_bytes(MAX_KRYLOV)));
   // resident CTAs per kernel: item lists are sized to whole waves
   auto resident = [&](const void* fn, int threads, size_t smem) {
     int b = 0;
@@ -1556,7 +1556,7 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
   const int gram_mt = m <= 16 ? 1 : 2;
   const void* gram_fn = gram_mt == 1 ? (const void*)k_gram<1> : (const void*)k_gram<2>;
   const size_t gram_smem = gram_smem_bytes(gram_mt) + gram_raw_bytes(gram_mt);
-  CK(cudaFuncSetAttribute(gram_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gram_smem));
+  CK(allow_smem(gram_fn, gram_smem));
   const int res_proj = gram ? std::max(1, resident(gram_fn, 256, gram_smem) / 4)
                             : resident(proj_fn, proj_threads, proj_smem);
 

@@ -1014,8 +1014,7 @@ static bool small_path_fits(Handle* h, const std::vector<JobSpec>& jobs, int m, 
   if (h->mem_limit) budget = std::min(budget, (double)h->mem_limit);
   if (bytes > budget) return false;
   if (h->sample_path == SPC_SAMPLE_ON || h->sample_path == SPC_SAMPLE_SINGLE) return true;
-  if (cudaFuncSetAttribute(k_small_prop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return false;
+  if (allow_smem(k_small_prop, h->smem_optin - SMALL_STATIC) != cudaSuccess) return false;
   int b = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_small_prop, SMALL_THREADS, smem) != cudaSuccess) return false;
   return wmax <= 2.5e6 && G <= 2LL * h->sm_count * std::max(1, b);
@@ -1097,7 +1096,7 @@ static int propagate_small(Handle* h, const double* theta, const double* init_po
     pvec = sizeof(double2) * pair_main_elems(m, nmax, true) <= budget;
     psmem = std::max(help, sizeof(double2) * pair_main_elems(m, nmax, pvec));
     pair = psmem <= budget &&
-           cudaFuncSetAttribute(k_small_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem) == cudaSuccess;
+           allow_smem(k_small_pair, budget) == cudaSuccess;
     if (pair) {
       // every cluster resident at once (SMs pair up within a GPC, so this can
       // be fewer than half the SMs)
@@ -1127,7 +1126,7 @@ static int propagate_small(Handle* h, const double* theta, const double* init_po
     // where these take 4.5 (201 samples at dim 288, MGS, m = 20)
     const bool vec_smem = G <= h->sm_count && smem + vbytes + SMALL_STATIC <= h->smem_optin;
     if (vec_smem) smem += vbytes;
-    CK(cudaFuncSetAttribute(k_small_prop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK(allow_smem(k_small_prop, budget));
     k_small_prop<<<G, SMALL_THREADS, smem, st>>>((const SmallJob*)plan, (const int*)(plan + o_sjob),
                                                  (const int*)(plan + o_scol), (const int64_t*)(plan + o_soff),
                                                  (double2*)h->Q.p, th, m, T, dt, t_end, tol, lanczos ? 1 : 0,
