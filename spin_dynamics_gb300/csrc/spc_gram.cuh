@@ -197,7 +197,7 @@ __device__ __forceinline__ double2 gram_entry(const double* Tm, int i, int j, do
 __host__ __device__ __forceinline__ size_t gram_raw_bytes(int mt) { return sizeof(double2) * 2 * 16 * mt * GRAM_R; }
 template <int MT>
 __global__ void __launch_bounds__(256, 2)
-    k_gram(const TileInfo* __restrict__ tiles, const int* __restrict__ map, int m, int ncombo,
+    k_gram(const TileInfo* __restrict__ tiles, const int* __restrict__ slots, int m, int ncombo,
            const double2* __restrict__ Q, const unsigned* __restrict__ qmax, int nsplit, int64_t rps,
            double2* __restrict__ part, int nslots) {
   constexpr int MP = 16 * MT;
@@ -205,8 +205,7 @@ __global__ void __launch_bounds__(256, 2)
   longlong2* acc64 = reinterpret_cast<longlong2*>(gsm);               // [8][256]
   unsigned* V = reinterpret_cast<unsigned*>(acc64 + 8 * 256);         // [DIGITS][MP][GRAM_R + 4]
   const int type = blockIdx.x & 3;
-  const int w = blockIdx.x >> 2;
-  if (map[w] < 0) return;
+  const int w = slots[blockIdx.x >> 2];
   const TileInfo& Ti = tiles[w / SPC_LANES];
   const int64_t Z = Ti.n / 4;
   const int nsp = proj_splits(nsplit, rps, Z);
