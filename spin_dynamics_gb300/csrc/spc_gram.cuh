@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(256, 2)
   longlong2* acc64 = reinterpret_cast<longlong2*>(gsm);               // [8][256]
   unsigned* V = reinterpret_cast<unsigned*>(acc64 + 8 * 256);         // [DIGITS][MP][GRAM_R + 4]
   const int type = blockIdx.x & 3;
-  const int w = slots[blockIdx.x >> 2];
+  const int w = slots ? slots[blockIdx.x >> 2] : blockIdx.x >> 2;  // null: every slot has a sample
   const TileInfo& Ti = tiles[w / SPC_LANES];
   const int64_t Z = Ti.n / 4;
   const int nsp = proj_splits(nsplit, rps, Z);

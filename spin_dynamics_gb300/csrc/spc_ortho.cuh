@@ -67,10 +67,14 @@ __device__ __forceinline__ double acc_get(const acc_t* p, int e) {
 // The sum of three words; the third adds less than 2^-54 of it from 2^16 units of
 // the first on.
 __device__ __forceinline__ double acc_get_norm(const acc_t* p, int e) {
-  const long long hi = (long long)p[0];
-  if (hi >= 65536) return acc_get(p, e);
-  const double t = fma((double)(long long)p[SPC_LANES], 1125899906842624.0, (double)(long long)p[2 * SPC_LANES]);
-  return ldexp(fma((double)hi, 1125899906842624.0 * 1125899906842624.0, t), e - 160);
+  const double word = 1125899906842624.0;
+  const long long hi = (long long)p[0], mid = (long long)p[SPC_LANES];
+  double s = fma((double)hi, word, (double)mid);
+  if (hi < 65536) {
+    s = fma((double)hi, word * word, fma((double)mid, word, (double)(long long)p[2 * SPC_LANES]));
+    e -= 50;
+  }
+  return ldexp(s, e - 110);
 }
 __device__ __forceinline__ void acc_clear(const AccArgs& A, int tile, int tid, int nth) {
   acc_t* p = acc_tile(A, A.clear, tile);
@@ -214,7 +218,7 @@ __global__ void __launch_bounds__(256, 2) k_ortho(OrthoArgs o) {
       float2 gk[ORTHO_NB - 1];
       bool big = !single_range(T.rexp);
       unsigned eb = 0;  // the last beta's exponent
-      if (ty < NA && act && i > 0) eb = abs_high(a.Ahess[(size_t)w * mm + i + (size_t)(i - 1) * a.m]) >> 20;
+      if (i > 0) eb = abs_high(a.coef[w]) >> 20;
       double2* G = o.gram + ((size_t)it.x * a.m + jv) * ORTHO_NB * SPC_LANES + tx;
       if (ty < NA) {
         d = make_double2(acc_get(in + 4 * ty * SPC_LANES, acc_dot_exp(T)),
@@ -413,8 +417,8 @@ __device__ __forceinline__ double ortho_norm(const PassArgs& a, const AccArgs& A
       // Hermitian tridiagonal: A(i, i+1) = beta_i, the coefficient of Q_i in
       // the next step's three-term recurrence
       a.Ahess[(size_t)w * mm + i + (size_t)(i + 1) * a.m] = make_double2(b, 0.0);
-      a.coef[w] = make_double2(b, 0.0);
     }
+    a.coef[w] = make_double2(b, 0.0);
     a.xexp[w] = *ex;
     a.qmax[w] = max(a.qmax[w], hq);
   }

@@ -84,7 +84,7 @@ struct PassArgs {
   const double2* psi;
   const int* map;     // slot -> global sample (or -1)
   const int* scol;    // slot -> column in its job's psi
-  double2* coef;      // current Lanczos coefficient beta per slot
+  double2* coef;      // last beta per slot (the next Lanczos coefficient)
   double* rbeta;      // 1/||psi|| per slot
   double2* Ahess;     // Hessenberg matrices, m x m column-major per slot
   double2* cvec;      // Krylov coordinates per slot
@@ -1773,7 +1773,8 @@ int propagate_batch(Handle* h, const double* theta, const double* init_pop,
       const dim3 pgrid(gram ? 4 * (int)list.size() : nslots, ns);
       pe = h->prof.begin(st);
       if (gram) {
-        void* args[] = {(void*)&d_tiles, (void*)&d_slots, (void*)&m, (void*)&ncombo, (void*)&d_Q, (void*)&d_qmax,
+        const int* slots = (int)list.size() < nslots ? d_slots : nullptr;
+        void* args[] = {(void*)&d_tiles, (void*)&slots, (void*)&m, (void*)&ncombo, (void*)&d_Q, (void*)&d_qmax,
                         (void*)&ns, (void*)&rps, (void*)&d_ppart, (void*)&nslots};
         CK(cudaLaunchKernel(gram_fn, pgrid, dim3(256), args, gram_smem, st));
       } else {
