@@ -234,8 +234,69 @@ __device__ __forceinline__ double small_half(const SmallJob& J, const double2* _
   return y;
 }
 
+// Row r of H x, both components by one thread: from SMALL_WIDE rows on, where every
+// scheduler has rows enough and a row's entries loaded twice cost more than the
+// halves even out. 120 samples, m = 8, 40 steps of 1 ns, components -> rows: dim
+// 576 even; dim 1152 general 3.67 -> 3.31, isotropic MGS 3.37 -> 2.82 ms; dim 1728
+// isotropic MGS 4.79 -> 3.83 ms (with a block's dots over all warps, below).
+#define SMALL_WIDE 512
+__device__ __forceinline__ double2 small_row(const SmallJob& J, const double2* __restrict__ x, int r, bool shift,
+                                             double kap) {
+  const int k0 = __ldg(J.rowptr + r), ks = __ldg(J.split + r), k1 = __ldg(J.rowptr + r + 1);
+  double2 a0 = cz(), a1 = cz();
+  for (int k = k0; k < ks; k += 4) {
+    double2 v[4], q[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const bool in = k + u < ks;
+      v[u] = in ? __ldg(J.val + k + u) : cz();
+      q[u] = x[in ? __ldg(J.col + k + u) : r];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (k + u < ks) {
+        if (u & 1)
+          a1 = cfma(v[u], q[u], a1);
+        else
+          a0 = cfma(v[u], q[u], a0);
+      }
+  }
+  for (int k = ks; k < k1; k += 4) {
+    double v[4];
+    double2 q[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const bool in = k + u < k1;
+      v[u] = in ? __ldg(&J.val[k + u].x) : 0.0;
+      q[u] = x[in ? __ldg(J.col + k + u) : r];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (k + u < k1) {
+        double2& a = (u & 1) ? a1 : a0;
+        a.x = fma(v[u], q[u].x, a.x);
+        a.y = fma(v[u], q[u].y, a.y);
+      }
+  }
+  double2 y = cadd(a0, a1);
+  if (shift) {
+    const double2 xr = x[r];
+    y.x = fma(kap, xr.y, y.x);
+    y.y = fma(-kap, xr.x, y.y);
+  }
+  return y;
+}
+
 // psi = Q c (:365) by components, over all threads of the CTA
 __device__ __forceinline__ void small_psi(int me, int n, const double2* Q, const double2* c, double2* psi) {
+  if (n >= SMALL_WIDE) {
+    for (int r = threadIdx.x; r < n; r += SMALL_THREADS) {
+      double2 a = cz();
+      for (int j = 0; j < me; ++j) a = cfma(c[j], Q[(size_t)j * n + r], a);
+      psi[r] = a;
+    }
+    return;
+  }
   for (int idx = threadIdx.x; idx < 2 * n; idx += SMALL_THREADS) {
     double a = 0.0;
     for (int j = 0; j < me; ++j) a = half_fma(c[j], Q[(size_t)j * n + (idx >> 1)], (idx & 1) != 0, a);
@@ -286,6 +347,7 @@ __host__ __device__ __forceinline__ size_t small_gram_elems(int m) { return (gra
 struct SmallOrtho {
   double2 h[ORTHO_NB];
   double2 gram[SMALL_MAX_M][ORTHO_NB];  // <Q_j, Q_k>, k < j of j's block
+  double part[ORTHO_NB][4];             // a warp's dot and product, where several warps share a vector
   unsigned top;                         // high word of the basis' largest component
 };
 
@@ -317,6 +379,7 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
   const int me = J.me, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n = CL ? (J.n + team.size - 1) / team.size : J.n;  // rows of a vector here
   const int r0 = CL ? team.rank * n : 0, nl = CL ? max(0, min(n, J.n - r0)) : n;
+  const bool wide = !CL && n >= SMALL_WIDE;  // rows instead of components
   int turn_ex = 0;
   const size_t mm = (size_t)m * m;
   for (int i = tid; i < (int)mm; i += SMALL_THREADS) A[i] = cz();
@@ -354,7 +417,18 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
     if (lz) {
       // p = H q_i - beta_{i-1} Q_{i-1}; alpha_i = Re <Q_i, p>
       double a2 = 0.0;
-      for (int idx = tid; idx < 2 * nl; idx += SMALL_THREADS) {
+      for (int r = tid; wide && r < n; r += SMALL_THREADS) {
+        double2 pv = small_row(J, x, r, false, kap);
+        const double2 q = qi[r];
+        if (i > 0) {
+          const double2 q0 = qi[r - n];
+          pv.x = fma(-beta, q0.x, pv.x);
+          pv.y = fma(-beta, q0.y, pv.y);
+        }
+        p[r] = pv;
+        a2 = fma(q.y, pv.y, fma(q.x, pv.x, a2));
+      }
+      for (int idx = tid; !wide && idx < 2 * nl; idx += SMALL_THREADS) {
         double pv = small_half(J, x, idx + 2 * r0, false, kap);
         if (i > 0) pv = fma(-beta, qid[idx - 2 * n], pv);
         pd[idx] = pv;
@@ -364,18 +438,22 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
       if (tid == 0) A[i + i * m] = make_double2(alpha, -kap);
       if (i == me - 1) break;
     } else {
-      for (int idx = tid; idx < 2 * nl; idx += SMALL_THREADS) pd[idx] = small_half(J, x, idx + 2 * r0, herm, kap);
+      for (int r = tid; wide && r < n; r += SMALL_THREADS) p[r] = small_row(J, x, r, herm, kap);
+      for (int idx = tid; !wide && idx < 2 * nl; idx += SMALL_THREADS) pd[idx] = small_half(J, x, idx + 2 * r0, herm, kap);
       // MGS (get_krylov :453-456) by blocks: d_v = <Q_v, p>, h_v from the d_v and
       // the block's basis products, p -= sum_v h_v Q_v
       for (int jb = 0; jb <= i; jb += ORTHO_NB) {
         const int nb = min(ORTHO_NB, i + 1 - jb);
         const bool newest = jb + nb == i + 1;
         __syncthreads();  // p and the last block's coefficients
-        if (warp < nb) {
-          const double2* qv = Q + (size_t)(jb + warp) * n;
-          const bool prod = newest && warp < nb - 1;  // also <Q_v, Q_i>
+        // a block of few vectors leaves warps: long ones go to 2, 4 or 8 of them
+        const int lw = !wide || nb > 4 ? 0 : (nb > 2 ? 1 : (nb > 1 ? 2 : 3));
+        const int wv = warp >> lw;
+        if (wv < nb) {
+          const double2* qv = Q + (size_t)(jb + wv) * n;
+          const bool prod = newest && wv < nb - 1;  // also <Q_v, Q_i>
           double2 d = cz(), gp = cz();
-          for (int r = lane; r < nl; r += 32) {
+          for (int r = lane + 32 * (warp & ((1 << lw) - 1)); r < nl; r += 32 << lw) {
             const double2 q = qv[r];
             d = cjfma(q, p[r], d);
             if (prod) gp = cjfma(q, qi[r], gp);
@@ -393,6 +471,8 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
           if (CL) {
             if ((lane & 7) < team.size)
               cg::this_cluster().map_shared_rank(ex, lane & 7)->d[turn_ex][team.rank][warp][lane >> 3] = v;
+          } else if (lw > 0) {
+            if ((lane & 7) == 0) ort.part[warp][lane >> 3] = v;
           } else {
             if (lane == 0) ort.h[warp].x = v;
             if (lane == 8) ort.h[warp].y = v;
@@ -408,12 +488,18 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
         else
           __syncthreads();
         if (warp == 0) {
-          if (CL) {
-            // four lanes a vector: the components in rank order
+          if (CL || lw > 0) {
+            // four lanes a vector: the components in the order of ranks or warps
             const int v = lane >> 2, u = lane & 3;
             if (v < nb) {
-              double y = ex->d[set][0][v][u];
-              for (int c = 1; c < team.size; ++c) y += ex->d[set][c][v][u];
+              double y;
+              if (CL) {
+                y = ex->d[set][0][v][u];
+                for (int c = 1; c < team.size; ++c) y += ex->d[set][c][v][u];
+              } else {
+                y = ort.part[v << lw][u];
+                for (int c = 1; c < 1 << lw; ++c) y += ort.part[(v << lw) + c][u];
+              }
               double* to = reinterpret_cast<double*>(u < 2 ? &ort.h[v] : &ort.gram[i][v]);
               if (u < 2 || (newest && v < nb - 1)) to[u & 1] = u == 3 ? -y : y;
             }
@@ -453,7 +539,13 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
             ja = jb;
             na = nb;
           } else {
-            for (int idx = tid; idx < 2 * nl; idx += SMALL_THREADS) {
+            for (int r = tid; wide && r < n; r += SMALL_THREADS) {
+              double2 pv = p[r];
+#pragma unroll
+              for (int v = 0; v < ORTHO_NB; ++v) pv = cfms(ort.h[v], Q[(size_t)(jb + v) * n + r], pv);
+              p[r] = pv;
+            }
+            for (int idx = tid; !wide && idx < 2 * nl; idx += SMALL_THREADS) {
               const bool im = (idx & 1) != 0;
               double pv = pd[idx];
 #pragma unroll
@@ -470,7 +562,19 @@ __device__ __forceinline__ void small_krylov(const SmallJob& J, bool lz, bool he
     }
     // the last projection, ||p|| and Q_{i+1} = p / ||p||
     double nr = 0.0;
-    for (int idx = tid; idx < 2 * nl; idx += SMALL_THREADS) {
+    for (int r = tid; wide && r < n; r += SMALL_THREADS) {
+      double2 pv = p[r];
+      if (lz) {
+        const double2 q = qi[r];
+        pv.x = fma(-alpha, q.x, pv.x);
+        pv.y = fma(-alpha, q.y, pv.y);
+      } else {
+        for (int v = 0; v < na; ++v) pv = cfms(ort.h[v], Q[(size_t)(ja + v) * n + r], pv);
+      }
+      p[r] = pv;
+      nr = fma(pv.y, pv.y, fma(pv.x, pv.x, nr));
+    }
+    for (int idx = tid; !wide && idx < 2 * nl; idx += SMALL_THREADS) {
       double pv = pd[idx];
       if (lz) {
         pv = fma(-alpha, qid[idx], pv);
