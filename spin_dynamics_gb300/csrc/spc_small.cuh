@@ -701,7 +701,11 @@ __device__ __forceinline__ double small_ortho_err(int me, int m, const double2* 
 // Dynamic shared memory: A, E (m^2 each), P (4 m^2), c and c' (m each),
 // max(5 m^2, small_gram_elems) of expm / projector scratch, all complex, then
 // the vectors when vec_smem.
-__global__ void __launch_bounds__(SMALL_THREADS, 2)
+// CTAS: CTAs in an SM that the registers allow. Two (128 registers) need spills that
+// a lone CTA does not: 120 samples, m = 8, 40 steps of 1 ns, dim 144 0.94 -> 0.86,
+// dim 216 1.05 -> 0.91 ms; 304 samples at dim 432, m = 24 (one CTA fits) 2.57 -> 2.42.
+template <int CTAS>
+__global__ void __launch_bounds__(SMALL_THREADS, CTAS)
     k_small_prop(const SmallJob* __restrict__ jobs, const int* __restrict__ sjob, const int* __restrict__ scol,
                  const int64_t* __restrict__ soff, double2* __restrict__ work, Theta th, int m, int T, double dt,
                  double t_end, double tol, int lanczos, int vec_smem, double* __restrict__ obs,
@@ -1118,9 +1122,9 @@ static bool small_path_fits(Handle* h, const std::vector<JobSpec>& jobs, int m, 
   if (h->mem_limit) budget = std::min(budget, (double)h->mem_limit);
   if (bytes > budget) return false;
   if (h->sample_path == SPC_SAMPLE_ON || h->sample_path == SPC_SAMPLE_SINGLE) return true;
-  if (allow_smem(k_small_prop, h->smem_optin - SMALL_STATIC) != cudaSuccess) return false;
+  if (allow_smem(k_small_prop<2>, h->smem_optin - SMALL_STATIC) != cudaSuccess) return false;
   int b = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_small_prop, SMALL_THREADS, smem) != cudaSuccess) return false;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_small_prop<2>, SMALL_THREADS, smem) != cudaSuccess) return false;
   return wmax <= 2.5e6 && G <= 2LL * h->sm_count * std::max(1, b);
 }
 
@@ -1224,14 +1228,22 @@ static int propagate_small(Handle* h, const double* theta, const double* init_po
                                                       (double2*)h->Q.p, th, m, T, dt, nstep, tol, lanczos ? 1 : 0,
                                                       pvec ? 1 : 0, hmax, d_obs, d_nsteps, d_counts, d_err);
   } else {
+    // With more samples than SMs two CTAs share one where their shared memory lets
+    // them, and their vectors stay in global memory (L2): two waves of lone CTAs
+    // take 6.0 ms where these take 4.5 (201 samples at dim 288, MGS, m = 20).
+    // Otherwise (fewer samples, or m past 20) the CTA has the SM's registers, and
+    // shared memory for its vectors if they fit.
     const size_t vbytes = sizeof(double2) * (size_t)(m + 2) * nmax;
-    // with more samples than SMs two CTAs share one, and their vectors stay in
-    // global memory (L2): two waves of lone CTAs take 6.0 ms
-    // where these take 4.5 (201 samples at dim 288, MGS, m = 20)
-    const bool vec_smem = G <= h->sm_count && smem + vbytes + SMALL_STATIC <= h->smem_optin;
+    int ctas = 1;
+    if (G > h->sm_count) {
+      CK(allow_smem(k_small_prop<2>, budget));
+      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, k_small_prop<2>, SMALL_THREADS, smem));
+    }
+    const bool vec_smem = ctas < 2 && smem + vbytes + SMALL_STATIC <= h->smem_optin;
     if (vec_smem) smem += vbytes;
-    CK(allow_smem(k_small_prop, budget));
-    k_small_prop<<<G, SMALL_THREADS, smem, st>>>((const SmallJob*)plan, (const int*)(plan + o_sjob),
+    const auto prop = ctas < 2 ? k_small_prop<1> : k_small_prop<2>;
+    CK(allow_smem(prop, budget));
+    prop<<<G, SMALL_THREADS, smem, st>>>((const SmallJob*)plan, (const int*)(plan + o_sjob),
                                                  (const int*)(plan + o_scol), (const int64_t*)(plan + o_soff),
                                                  (double2*)h->Q.p, th, m, T, dt, t_end, tol, lanczos ? 1 : 0,
                                                  vec_smem ? 1 : 0, d_obs,

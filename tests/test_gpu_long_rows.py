@@ -1,6 +1,6 @@
 """The per-sample kernels at the edges of their layouts: vectors by components and by
-rows (from 512 rows on), and blocks of 1 to 9 vectors whose dots one or several
-warps take, against the CPU oracle. Rounding of order 1e-15
+rows (from 512 rows on), blocks of 1 to 9 vectors whose dots one or several
+warps take, and one or two CTAs in an SM; against the CPU oracle. Rounding of order 1e-15
 a step over at most 20 steps: 1e-12 leaves a factor of fifty."""
 import numpy as np
 import pytest
@@ -46,3 +46,14 @@ def check(sampler, oracle, s, M, m, method, mode, steps=20):
 @pytest.mark.parametrize("mode", ["on", "single"])
 def test_rows(sampler, oracle, g1, g2, m, method, kT, mode):
     check(sampler, oracle, pair(g1, g2, kT), 2, m, method, mode)
+
+
+@pytest.mark.parametrize("m", [8, 9, 16, 17, 20, 24, 32])
+@pytest.mark.parametrize("more", [0, 1])
+@pytest.mark.parametrize("method, kT", [("mgs", 0.3), ("auto", 1.0)])
+def test_ctas_of_an_sm(sampler, oracle, m, more, method, kT):
+    """As many samples as SMs, and one more (two CTAs in an SM where their shared
+    memory allows)."""
+    import torch
+    M = torch.cuda.get_device_properties(0).multi_processor_count + more
+    check(sampler, oracle, pair((2,), (2, 3), kT), M, m, method, "on")
