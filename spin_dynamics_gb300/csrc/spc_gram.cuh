@@ -60,12 +60,14 @@ __device__ __forceinline__ void gram_sums(int type, int m, int me, int emax, int
 #pragma unroll
       for (int r = 0; r < 4; ++r) acc[t][l][r] = 0.f;
 #pragma unroll
-  for (int r = 0; r < 8; ++r) acc64[r * 256 + tid] = make_longlong2(0, 0);
+  for (int r = 0; r < 8; ++r)
+    if (r < 4 || two) acc64[r * 256 + tid] = make_longlong2(0, 0);
   auto close = [&]() {
 #pragma unroll
     for (int t = 0; t < 2; ++t)
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
+        if (t > 0 && !two) break;
         long long s[DIGITS];
 #pragma unroll
         for (int l = 0; l < DIGITS; ++l) {
@@ -168,6 +170,7 @@ __device__ __forceinline__ void gram_sums(int type, int m, int me, int emax, int
     for (int t = 0; t < 2; ++t)
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
+        if (t > 0 && !two) break;
         longlong2 a = acc64[(4 * t + r) * 256 + tid];
         if (MT == 1)
           for (int o = 1; o < 4; ++o) {
