@@ -143,7 +143,7 @@ struct OrthoArgs {
 // vector. Per Krylov step at m = 24, dim 9216, 64 samples (MGS): 12.5 passes of
 // 29 us before, 3 of 31-82 us now; dim 55296, 32 samples, m = 30: 56.5 -> 27 ms a
 // build. Blocks of eight: the newest block's pass holds 15 complex sums and 8
-// vectors in 126 registers. Lanczos at dim 2304, 77 samples: the norm pass 15.3
+// vectors in 128 registers (with unequal rates it spills 68 bytes). Lanczos at dim 2304, 77 samples: the norm pass 15.3
 // -> 10.1 us, k_spmm_blk with its projection 27.9 -> 19.5 us without the last sum.
 // Small coefficients: where H is Hermitian up to a shift every h_v but the last
 // two is of rounding size. A vector whose coefficients are below 2^-44 of the
