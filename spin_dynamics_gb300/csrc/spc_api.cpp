@@ -162,6 +162,7 @@ int spc_set_h(spc_handle* h, const spc_csr* H) {
     if (cl[k] < 0 || cl[k] >= n) return spc::set_error(SPC_ERR_ARG, "column index out of range");
   }
   CKR(cudaSetDevice(h->h.device));
+  h->h.n = 0;  // a call that fails from here on leaves no Hamiltonian
   if (h->h.ensure_rowptr(n + 1) || h->h.ensure_h_entries(nnz)) return SPC_ERR_ALLOC;
   CKR(cudaMemcpy(h->h.d_rowptr, rp.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice));
   if (nnz > 0) {
@@ -173,7 +174,9 @@ int spc_set_h(spc_handle* h, const spc_csr* H) {
   h->h.herm_shift = is_hermitian_plus_shift(n, rp, cl, H->val);
   h->h.blk_one.describe({spc::BlockSys{}});
   h->h.rexp = spc::norm_exponent(spc::csr_norm_bound(n, rp.data(), cl.data(), H->val));
-  return spc::prepare_spmm_rows(&h->h);
+  const int rc = spc::prepare_spmm_rows(&h->h);
+  if (rc != SPC_OK) h->h.n = 0;
+  return rc;
 }
 
 int spc_h_size(const spc_handle* h, int32_t* n, int64_t* nnz) {

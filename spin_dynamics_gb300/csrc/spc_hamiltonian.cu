@@ -350,6 +350,7 @@ int build_h_device(Handle* h, const HostSystem& hs, int mode) {
   std::vector<size_t> noff;
   int rc = upload_nuclei(h, {&hs}, noff);
   if (rc) return rc;
+  h->n = 0;  // a build that fails from here on leaves no Hamiltonian
   if (h->ensure_rowptr(N + 1) || h->ensure_h_entries(nnz) || h->ensure(h->bcnt, sizeof(int) * N) ||
       h->ensure(h->btot, sizeof(long long)) || h->ensure(h->xcol, sizeof(int) * std::max<int64_t>(nnz, 1)) ||
       h->ensure(h->xval, sizeof(double2) * std::max<int64_t>(nnz, 1)) ||
@@ -382,6 +383,14 @@ int build_h_device(Handle* h, const HostSystem& hs, int mode) {
 
 int build_h_batch_device(Handle* h, const std::vector<HostSystem>& hs, int mode) {
   auto& B = h->hb;
+  // a build that fails leaves no batch
+  struct Undo {
+    Handle* h;
+    bool done = false;
+    ~Undo() {
+      if (!done) h->hb.n.clear();
+    }
+  } undo{h};
   const size_t ns = hs.size();
   B.n.assign(ns, 0);
   B.nnz.assign(ns, 0);
@@ -407,7 +416,10 @@ int build_h_batch_device(Handle* h, const std::vector<HostSystem>& hs, int mode)
   std::vector<size_t> noff;
   int rc = upload_nuclei(h, ptrs, noff);
   if (rc) return rc;
-  // fill into the unsplit scratch (xcol/xval), split into the store
+  // fill into the unsplit scratch (xcol/xval, the single Hamiltonian's execution
+  // copy), split into the store
+  h->n = 0;
+  h->nnz = 0;
   if (h->ensure(B.rowptr, sizeof(int) * rp_tot) || h->ensure(B.split, sizeof(int) * rp_tot) ||
       h->ensure(B.col, sizeof(int) * std::max<int64_t>(nz_tot, 1)) ||
       h->ensure(B.val, sizeof(double2) * std::max<int64_t>(nz_tot, 1)) ||
@@ -448,9 +460,7 @@ int build_h_batch_device(Handle* h, const std::vector<HostSystem>& hs, int mode)
     }
   }
   h->blk_batch.describe(std::move(bs));
-  // the single-Hamiltonian execution copy (xcol/xval) served as scratch
-  h->n = 0;
-  h->nnz = 0;
+  undo.done = rc == SPC_OK;
   return rc;
 }
 
