@@ -416,16 +416,6 @@ def run_ours(args, rank, world, local_rank):
                 sysp=sysp, B=B, sim=sim)
 
 
-def fp64_peak(device):
-    """FP64 FMA peak of the device in FLOP/s, from the library's DFMA probe."""
-    import ctypes as C
-
-    from spin_dynamics_gb300 import _native as nat
-    v = C.c_double()
-    nat.check(nat.lib().spc_fp64_peak(device, C.byref(v)))
-    return v.value * 1e12
-
-
 def digit_flops(system, samples):
     """FP16 operations of one k_spmm_blk launch: per nuclear index and 16 samples an m16n8k16 product for each
     of the 43 digit pairs of the step with the diagonal block and the 35 of every other pair of blocks."""
